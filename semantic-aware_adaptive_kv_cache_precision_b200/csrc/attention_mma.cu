@@ -1,0 +1,719 @@
+// Causal attention over the cache in bfloat16 on the tensor cores, for the sizes the designs
+// use: keys of 64 or 128 columns with values of 64, 128 or 256, and one shared latent row of 576
+// columns whose first 512 are the values. The scores and options are those of
+// `csrc/attention_distance.cu` (logarithmic or linear distance penalty, soft cap, window with kept
+// first tokens, chunks, sinks, gates, two maps a head), which takes every other size and type.
+//
+// Precision: queries, keys and values are bfloat16 and their products exact in fp32; scores,
+// softmax weights, running maxima and sums are fp32. A weight p in [0, 1] enters the second
+// product as hi + lo, two bfloat16 numbers that keep 16 to 17 of its bits, so every value tile is
+// multiplied twice; against 64 bits the outputs (bfloat16) are as far off as with fp32 weights
+// (2.3e-3 relative, all of it the output's own rounding).
+//
+// A block takes the rows of one key/value head and map: ROWS = 16 WR rows are tokens x query heads
+// of the group, so a group's heads share each tile of keys. WR warps go along the rows and WC
+// along the keys of a tile for the scores and along the values' columns for the weighted sum:
+//   * prompts, 128 columns: WR 4, WC 1 (weights stay in registers); tiles of 64 keys, two blocks
+//     an SM.
+//   * prompts, latent rows: WR 4, WC 2, tiles of 32 keys: 64 rows x 512 columns of fp32 sums are
+//     128 registers a thread of 256, and the queries and three tiles fill the shared memory.
+//   * decoded tokens: WR 1, WC 8 and `key_splits` blocks a token; what bounds them is the trip to
+//     memory, so a whole tile of 64 keys is asked for at once by 256 threads.
+// Tiles lie at multiples of their size in the sequence and a row that sees nothing of a tile is
+// left exactly as it was, so a token's result does not depend on which tokens came with it.
+//
+// The products run on mma.sync: at 576 and 512 columns the sums of 128 rows would fill the whole
+// of tensor memory, and the weights in two pieces would pass through it twice.
+#include <float.h>
+
+#include "common.cuh"
+#include "mma.cuh"
+
+struct MmaAttention {
+  const __nv_bfloat16* q;      // row t: + t * q_stride, virtual head h: + h * q_head_stride
+  long long q_stride;
+  int q_head_stride;
+  const __nv_bfloat16* q2;     // columns from q_split on (null: none)
+  long long q2_stride;
+  int q2_head_stride, q_split;
+  const __nv_bfloat16* k_cache;
+  const __nv_bfloat16* v_cache;      // null: the values are the first columns of the key rows
+  int k_row, v_row;
+  const int32_t* positions;
+  const int32_t* token_seq;
+  const int32_t* block_table;
+  int max_blocks, tokens, heads, kv_heads, maps;      // heads: query heads (each of `maps` maps)
+  float scale;
+  int window, chunk, keep;
+  const float* slope;          // logarithmic penalty, with `rate`
+  const float* rate;
+  float softcap;
+  const float* linear;
+  int key_splits;
+  // the outputs: directly (one map, one split), or through `sums` and a second kernel
+  __nv_bfloat16* out;          // [tokens, heads * DV]
+  float* sums;                 // [key_splits, tokens, heads * maps, DV], not yet divided
+  float* stats;                // [key_splits, tokens, heads * maps, 2]: maximum (base 2), sum
+  const float* sink;
+  const __nv_bfloat16* gate;   // a gate a head: + t * gate_stride + h (null: none)
+  long long gate_stride;
+  const float* elem_gate;      // fp32, + t * elem_stride + h * DV + c (null: none)
+  long long elem_stride;
+  const __nv_bfloat16* map_gate;   // two maps: + t * map_gate_stride + h * DV + c (null: none)
+  long long map_gate_stride;
+  float out_scale, lambda, eps;
+  // the split of the work
+  int heads_per_tile, tokens_per_tile, head_tiles;
+};
+
+namespace {
+
+constexpr float kLog2e = 1.4426950408889634f;
+
+__device__ __forceinline__ int first_visible(int pos, int window, int chunk) {
+  if (chunk > 0) return pos - pos % chunk;
+  return (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+}
+
+// 16 bytes into shared memory; zeros without reading where `real` is false
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool real) {
+  const int n = real ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n)
+               : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= FLT_MAX; }
+
+// A score in units of log 2: soft cap, penalty, base change.
+__device__ __forceinline__ float base2_score(const MmaAttention& a, float s, float dist, float sl,
+                                             float rt) {
+  if (a.softcap > 0.f) {     // cap * tanh(s / cap) as cap * (1 - 2 / (e^(2z) + 1))
+    const float z = __fdividef(s * a.scale, a.softcap);
+    s = a.softcap * (1.f - __fdividef(2.f, __expf(2.f * z) + 1.f)) * kLog2e;
+  } else {
+    s *= a.scale * kLog2e;
+  }
+  if (a.slope != nullptr) s -= sl * __log2f(fmaf(rt, dist, 1.f));
+  else if (a.linear != nullptr) s = fmaf(-sl * kLog2e, dist, s);
+  return s;
+}
+
+// What a row's sums become in the output: one warp a row, columns dealt to the lanes by fours.
+template <int DV>
+__device__ __forceinline__ void write_row(const MmaAttention& a, const float* acc, float m, float l,
+                                          int t, int h, int lane) {
+  float corr = 1.f;
+  if (a.sink != nullptr) {       // one more logit in the denominator
+    const float s = a.sink[h] * kLog2e;
+    const float top = fmaxf(m, s);
+    corr = mma::exp2_fast(m - top);
+    l = fmaf(l, corr, mma::exp2_fast(s - top));
+  }
+  float f = a.out_scale * corr / l;
+  if (a.gate != nullptr)
+    f *= 1.f / (1.f + expf(-widen(a.gate[(long long)t * a.gate_stride + h])));
+  const float* eg = a.elem_gate == nullptr ? nullptr
+                                           : a.elem_gate + (long long)t * a.elem_stride + (long long)h * DV;
+  __nv_bfloat16* o = a.out + ((long long)t * a.heads + h) * DV;
+  for (int c = lane * 4; c < DV; c += 128) {
+    const float4 v = *reinterpret_cast<const float4*>(acc + c);
+    float r[4] = {v.x * f, v.y * f, v.z * f, v.w * f};
+    if (eg != nullptr) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r[i] /= 1.f + expf(-eg[c + i]);
+    }
+    *reinterpret_cast<uint2*>(o + c) = make_uint2(mma::pack_bf16(r[0], r[1]), mma::pack_bf16(r[2], r[3]));
+  }
+}
+
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+struct Shape {
+  static constexpr int kRows = 16 * WR, kThreads = 32 * WR * WC;
+  static constexpr int kQStride = DK + 8, kVStride = VINK ? DK + 8 : DV + 8;   // (elements; odd
+  static constexpr int kOStride = DV + 8, kPStride = KT + 8;                    //  times 16 bytes)
+  static constexpr int kQBytes = kRows * kQStride * 2;
+  static constexpr int kKBytes = KT * kQStride * 2;
+  static constexpr int kStageBytes = kKBytes + (VINK ? 0 : KT * kVStride * 2);
+  static constexpr int kPBytes = WC > 1 ? 2 * kRows * kPStride * 2 : 0;
+  static constexpr int kSmall = (2 * WC + 2) * kRows * 4;        // maxima, sums, a row's m and l
+  static constexpr int kMain = kQBytes + STAGES * kStageBytes + kPBytes;
+  static constexpr int kOut = kRows * kOStride * 4;
+  static constexpr int kBytes = (kMain > kOut ? kMain : kOut) + kSmall;
+};
+
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+__global__ void __launch_bounds__(32 * WR * WC)
+attention_mma_kernel(const MmaAttention a) {
+  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES>;
+  constexpr int NT = KT / WC / 8;            // tiles of 8 keys a warp scores
+  constexpr int NV = DV / WC / 8;            // tiles of 8 value columns a warp sums
+  constexpr int KS = DK / 16;
+  static_assert(KT % (8 * WC) == 0 && DV % (16 * WC) == 0 && kCacheBlock % KT == 0, "");
+  static_assert(WC > 1 || (KT % 16 == 0), "");
+  static_assert(NT == 1 || NT % 2 == 0, "");
+  extern __shared__ __align__(16) unsigned char smem[];
+  __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(smem);
+  float* small = reinterpret_cast<float*>(smem + S::kBytes - S::kSmall);
+  float* row_max = small;                    // [WC][rows]
+  float* row_sum = small + WC * S::kRows;    // [WC][rows]
+  float* row_m = small + 2 * WC * S::kRows;  // [rows]
+  float* row_l = row_m + S::kRows;           // [rows]
+  float* os = reinterpret_cast<float*>(smem);
+  const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+  const uint32_t stage0 = base + S::kQBytes;
+  const uint32_t p_base = stage0 + STAGES * S::kStageBytes;
+
+  if (a.sums != nullptr) let_next_kernel_start();      // (the fold waits for this kernel's end)
+  wait_for_previous_kernel();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int wr = warp / WC, wc = warp % WC;
+  // the longest rows of a prompt (its last tokens) start first
+  const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * a.tokens_per_tile;
+  const int hg = a.heads / a.kv_heads, hp = a.heads_per_tile;
+  int y = blockIdx.y;
+  const int head_tile = y % a.head_tiles;
+  y /= a.head_tiles;
+  const int map = y % a.maps, g = y / a.maps;
+  const int h_base = g * hg + head_tile * hp;
+  const int h_count = min(hp, hg - head_tile * hp);
+  const int t_end = min(t0 + a.tokens_per_tile, a.tokens);
+  const int used = (t_end - t0) * hp;        // rows beyond it belong to nobody
+
+  // the queries
+  constexpr int kPieces = DK / 8;
+  for (int i = threadIdx.x; i < S::kRows * kPieces; i += S::kThreads) {
+    const int r = i / kPieces, e = (i - r * kPieces) * 8;
+    const int t = t0 + r / hp, h = (h_base + r % hp) * a.maps + map;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (r < used && r % hp < h_count) {
+      const __nv_bfloat16* src =
+          e < a.q_split ? a.q + (long long)t * a.q_stride + (long long)h * a.q_head_stride + e
+                        : a.q2 + (long long)t * a.q2_stride + (long long)h * a.q2_head_stride +
+                              (e - a.q_split);
+      v = *reinterpret_cast<const uint4*>(src);
+    }
+    *reinterpret_cast<uint4*>(qs + r * S::kQStride + e) = v;
+  }
+
+  // this thread's two rows
+  int rt[2], rpos[2], rfirst[2];
+  float rsl[2] = {0.f, 0.f}, rrt[2] = {0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = wr * 16 + (lane >> 2) + 8 * i;
+    rt[i] = r < used && r % hp < h_count ? t0 + r / hp : -1;
+    rpos[i] = rt[i] >= 0 ? a.positions[rt[i]] : -1;
+    rfirst[i] = rt[i] >= 0 ? first_visible(rpos[i], a.window, a.chunk) : 0;
+    if (rt[i] >= 0) {
+      const int h = h_base + r % hp;
+      if (a.slope != nullptr) {
+        rsl[i] = a.slope[h];
+        rrt[i] = a.rate[h];
+      } else if (a.linear != nullptr) {
+        rsl[i] = a.linear[h];
+      }
+    }
+  }
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  float acc[NV][4];
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+
+  const int split = blockIdx.z;
+  // The tile's tokens in runs of one sequence and consecutive positions (one run for nearly every
+  // tile of a prompt); rows outside the run see none of its keys.
+  for (int s0 = t0; s0 < t_end;) {
+    const int seq = a.token_seq[s0], p0 = a.positions[s0];
+    int s1 = s0 + 1;
+    while (s1 < t_end && a.token_seq[s1] == seq && a.positions[s1] == p0 + (s1 - s0)) ++s1;
+    const int last = p0 + (s1 - s0) - 1;
+    const int low = first_visible(p0, a.window, a.chunk);
+    const int low_last = first_visible(last, a.window, a.chunk);
+    const bool whole = s0 == t0 && s1 == t_end;
+    const int32_t* table = a.block_table + (long long)seq * a.max_blocks;
+    // tiles: those of the kept first tokens that lie before the first visible one's, then on
+    const int from = low / KT;
+    const int kept_all = (a.keep + KT - 1) / KT;
+    const int kept = kept_all < from ? kept_all : from;
+    const int count = kept + last / KT - from + 1;
+    const int share = (count + a.key_splits - 1) / a.key_splits;
+    const int lo = split * share, hi = min(count, lo + share);
+
+    auto fetch = [&](int i) {
+      const int tile = i < kept ? i : from + i - kept;
+      const int j0 = tile * KT;
+      const long long row0 = ((long long)table[j0 / kCacheBlock] * a.kv_heads + g) * kCacheBlock +
+                             j0 % kCacheBlock;
+      const uint32_t ks = stage0 + (i % STAGES) * S::kStageBytes;
+      const __nv_bfloat16* kp = a.k_cache + row0 * a.k_row + map * DK;
+      constexpr int kp16 = DK / 8;
+      for (int x = threadIdx.x; x < KT * kp16; x += S::kThreads) {
+        const int r = x / kp16, e = (x - r * kp16) * 8;
+        copy16(ks + (r * S::kQStride + e) * 2, kp + (long long)r * a.k_row + e, j0 + r <= last);
+      }
+      if constexpr (!VINK) {
+        const __nv_bfloat16* vp = a.v_cache + row0 * a.v_row;
+        constexpr int vp16 = DV / 8;
+        for (int x = threadIdx.x; x < KT * vp16; x += S::kThreads) {
+          const int r = x / vp16, e = (x - r * vp16) * 8;
+          copy16(ks + S::kKBytes + (r * S::kVStride + e) * 2, vp + (long long)r * a.v_row + e,
+                 j0 + r <= last);
+        }
+      }
+    };
+
+    __syncthreads();                 // (queries are there; the run before this one is done)
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+      if (lo + i < hi) fetch(lo + i);
+      copies_commit();
+    }
+    for (int i = lo; i < hi; ++i) {
+      copies_wait<STAGES - 2>();
+      __syncthreads();               // tile i is there, and everybody has left tile i - 1
+      if (i + STAGES - 1 < hi) fetch(i + STAGES - 1);
+      copies_commit();
+      const int tile = i < kept ? i : from + i - kept;
+      const int j0 = tile * KT;
+      const uint32_t ks = stage0 + (i % STAGES) * S::kStageBytes;
+      const uint32_t vs = VINK ? ks : ks + S::kKBytes;
+
+      float s[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+      const uint32_t q_at = base + ((wr * 16 + (lane & 15)) * S::kQStride + (lane >> 4) * 8) * 2;
+      if constexpr (NT == 1) {
+        const uint32_t k_at =
+            ks + ((wc * 8 + (lane & 7)) * S::kQStride + (lane >> 3) * 8) * 2;
+#pragma unroll 4
+        for (int kk = 0; kk < KS; kk += 2) {
+          uint32_t b[4], q0[4], q1[4];
+          mma::ldmatrix_x4(k_at + kk * 32, b[0], b[1], b[2], b[3]);
+          mma::ldmatrix_x4(q_at + kk * 32, q0[0], q0[1], q0[2], q0[3]);
+          mma::ldmatrix_x4(q_at + kk * 32 + 32, q1[0], q1[1], q1[2], q1[3]);
+          mma::bf16_16816(s[0], q0, b[0], b[1]);
+          mma::bf16_16816(s[0], q1, b[2], b[3]);
+        }
+      } else {
+        const uint32_t k_at = ks + ((wc * NT * 8 + (lane & 7) + (lane >> 4) * 8) * S::kQStride +
+                                    ((lane >> 3) & 1) * 8) * 2;
+#pragma unroll(KS <= 8 ? KS : 4)
+        for (int kk = 0; kk < KS; ++kk) {
+          uint32_t q[4];
+          mma::ldmatrix_x4(q_at + kk * 32, q[0], q[1], q[2], q[3]);
+#pragma unroll
+          for (int n = 0; n < NT; n += 2) {
+            uint32_t b[4];
+            mma::ldmatrix_x4(k_at + (n * 8 * S::kQStride) * 2 + kk * 32, b[0], b[1], b[2], b[3]);
+            mma::bf16_16816(s[n], q, b[0], b[1]);
+            mma::bf16_16816(s[n + 1], q, b[2], b[3]);
+          }
+        }
+      }
+
+      // scores, masks, the tile's maxima
+      const bool all_seen = whole && j0 + KT - 1 <= p0 && (j0 >= low_last || j0 + KT <= a.keep);
+      float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int n = 0; n < NT; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int r = e >> 1;
+          const int j = j0 + (wc * NT + n) * 8 + (lane & 3) * 2 + (e & 1);
+          float v = base2_score(a, s[n][e], (float)(rpos[r] - j), rsl[r], rrt[r]);
+          if (!all_seen)
+            v = rt[r] >= s0 && rt[r] < s1 && j <= rpos[r] && (j >= rfirst[r] || j < a.keep)
+                    ? v : -INFINITY;
+          s[n][e] = v;
+          top[r] = fmaxf(top[r], v);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 1));
+        top[r] = fmaxf(top[r], __shfl_xor_sync(0xffffffffu, top[r], 2));
+      }
+      const int my_row = wr * 16 + (lane >> 2);
+      if constexpr (WC > 1) {        // over the warps of these rows
+        if ((lane & 3) == 0) {
+          row_max[wc * S::kRows + my_row] = top[0];
+          row_max[wc * S::kRows + my_row + 8] = top[1];
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + wr), "n"(32 * WC) : "memory");
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int w = 0; w < WC; ++w)
+            top[r] = fmaxf(top[r], row_max[w * S::kRows + my_row + 8 * r]);
+      }
+      float corr[2], shift[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float next = fmaxf(m[r], top[r]);
+        shift[r] = next == -INFINITY ? 0.f : next;     // (nothing seen yet: weights of 0)
+        corr[r] = mma::exp2_fast(m[r] - shift[r]);
+        m[r] = next;
+        l[r] *= corr[r];
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float p = mma::exp2_fast(s[n][e] - shift[e >> 1]);
+          s[n][e] = p;
+          l[e >> 1] += p;
+        }
+      if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          mma::mul2(acc[n][0], acc[n][1], corr[0]);
+          mma::mul2(acc[n][2], acc[n][3], corr[1]);
+        }
+      }
+
+      // the weights as hi + lo, times the values
+      auto halves = [](float x, float y, uint32_t& hi2, uint32_t& lo2) {
+        hi2 = mma::pack_bf16(x, y);
+        const float2 back = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&hi2));
+        lo2 = mma::pack_bf16(x - back.x, y - back.y);
+      };
+      if constexpr (WC > 1) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            uint32_t hi2, lo2;
+            halves(s[n][2 * r], s[n][2 * r + 1], hi2, lo2);
+            const int at = (my_row + 8 * r) * S::kPStride + (wc * NT + n) * 8 + (lane & 3) * 2;
+            uint32_t* ph = reinterpret_cast<uint32_t*>(smem + S::kQBytes + STAGES * S::kStageBytes);
+            ph[at / 2] = hi2;
+            ph[(S::kRows * S::kPStride + at) / 2] = lo2;
+          }
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + wr), "n"(32 * WC) : "memory");
+      }
+      const uint32_t v_at = vs + (((lane & 7) + ((lane >> 3) & 1) * 8) * S::kVStride +
+                                  wc * NV * 8 + (lane >> 4) * 8) * 2;
+#pragma unroll
+      for (int kk = 0; kk < KT / 16; ++kk) {
+        uint32_t ph[4], pl[4];
+        if constexpr (WC > 1) {
+          const uint32_t at =
+              p_base + ((wr * 16 + (lane & 15)) * S::kPStride + kk * 16 + (lane >> 4) * 8) * 2;
+          mma::ldmatrix_x4(at, ph[0], ph[1], ph[2], ph[3]);
+          mma::ldmatrix_x4(at + S::kRows * S::kPStride * 2, pl[0], pl[1], pl[2], pl[3]);
+        } else {
+          constexpr int kLast = NT > 1 ? NT - 1 : 0;
+          const int n0 = 2 * kk, n1 = 2 * kk + 1 <= kLast ? 2 * kk + 1 : kLast;
+          halves(s[n0][0], s[n0][1], ph[0], pl[0]);
+          halves(s[n0][2], s[n0][3], ph[1], pl[1]);
+          halves(s[n1][0], s[n1][1], ph[2], pl[2]);
+          halves(s[n1][2], s[n1][3], ph[3], pl[3]);
+        }
+#pragma unroll
+        for (int n = 0; n < NV; n += 2) {
+          uint32_t b[4];
+          mma::ldmatrix_x4_trans(v_at + (kk * 16 * S::kVStride + n * 8) * 2, b[0], b[1], b[2], b[3]);
+          mma::bf16_16816(acc[n], ph, b[0], b[1]);
+          mma::bf16_16816(acc[n + 1], ph, b[2], b[3]);
+          mma::bf16_16816(acc[n], pl, b[0], b[1]);
+          mma::bf16_16816(acc[n + 1], pl, b[2], b[3]);
+        }
+      }
+    }
+    copies_wait<0>();
+    s0 = s1;
+  }
+
+  // the rows' sums and maxima, and their sums of values, into shared memory
+  bool bad = false;
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bad |= rt[e >> 1] >= 0 && !finite(acc[n][e]);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    l[r] += __shfl_xor_sync(0xffffffffu, l[r], 1);
+    l[r] += __shfl_xor_sync(0xffffffffu, l[r], 2);
+  }
+  const int any_bad = __syncthreads_or(bad);           // (and everybody has left the tiles)
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int row = wr * 16 + (lane >> 2) + 8 * r;
+    if ((lane & 3) == 0) {
+      row_sum[wc * S::kRows + row] = l[r];
+      if (wc == 0) row_m[row] = m[r];
+    }
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+      *reinterpret_cast<float2*>(os + row * S::kOStride + (wc * NV + n) * 8 + (lane & 3) * 2) =
+          make_float2(acc[n][2 * r], acc[n][2 * r + 1]);
+  }
+  __syncthreads();
+  for (int row = threadIdx.x; row < S::kRows; row += S::kThreads) {
+    float sum = row_sum[row];
+    for (int w = 1; w < WC; ++w) sum += row_sum[w * S::kRows + row];
+    row_l[row] = sum;
+  }
+  __syncthreads();
+  for (int row = warp; row < used; row += WR * WC) {
+    if (row % hp >= h_count) continue;
+    const int t = t0 + row / hp, h = h_base + row % hp;
+    float* acc_row = os + row * S::kOStride;
+    if (any_bad) {
+      // An infinity or a NaN among the values: a weight of 0 times it spoils rows that do not
+      // see it, and hi + lo times it is not p times it. Such a block walks its keys one by one.
+      const int pos = a.positions[t], first = first_visible(pos, a.window, a.chunk);
+      const int32_t* table = a.block_table + (long long)a.token_seq[t] * a.max_blocks;
+      // the same share of the run's tiles as above
+      int s0 = t, s1 = t + 1;
+      while (s0 > t0 && a.token_seq[s0 - 1] == a.token_seq[t] &&
+             a.positions[s0 - 1] == a.positions[s0] - 1) --s0;
+      while (s1 < t_end && a.token_seq[s1] == a.token_seq[t] &&
+             a.positions[s1] == a.positions[s1 - 1] + 1) ++s1;
+      const int last = a.positions[s1 - 1];
+      const int from = first_visible(a.positions[s0], a.window, a.chunk) / KT;
+      const int kept_all = (a.keep + KT - 1) / KT;
+      const int kept = kept_all < from ? kept_all : from;
+      const int count = kept + last / KT - from + 1;
+      const int share = (count + a.key_splits - 1) / a.key_splits;
+      const int lo = split * share, hi = min(count, lo + share);
+      const int vh = h * a.maps + map;
+      const float sl = a.slope ? a.slope[h] : a.linear ? a.linear[h] : 0.f;
+      const float rate = a.slope ? a.rate[h] : 0.f;
+      float top = -INFINITY, sum = 0.f;
+      for (int c = lane; c < DV; c += 32) acc_row[c] = 0.f;
+      for (int i = lo; i < hi; ++i) {
+        const int tile = i < kept ? i : from + i - kept;
+        for (int j = tile * KT; j < tile * KT + KT; ++j) {
+          if (j > pos || (j < first && j >= a.keep)) continue;
+          const long long at = ((long long)table[j / kCacheBlock] * a.kv_heads + g) * kCacheBlock +
+                               j % kCacheBlock;
+          float part = 0.f;
+          for (int e = lane; e < DK; e += 32) {
+            const __nv_bfloat16 qv =
+                e < a.q_split
+                    ? a.q[(long long)t * a.q_stride + (long long)vh * a.q_head_stride + e]
+                    : a.q2[(long long)t * a.q2_stride + (long long)vh * a.q2_head_stride + e - a.q_split];
+            part = fmaf(widen(qv), widen(a.k_cache[at * a.k_row + map * DK + e]), part);
+          }
+          const float sc = base2_score(a, warp_sum(part), (float)(pos - j), sl, rate);
+          const float next = fmaxf(top, sc);
+          const float f = exp2f(top - next), p = exp2f(sc - next);
+          sum = fmaf(sum, f, p);
+          const __nv_bfloat16* vr = VINK ? a.k_cache + at * a.k_row : a.v_cache + at * a.v_row;
+          for (int c = lane; c < DV; c += 32) acc_row[c] = fmaf(acc_row[c], f, p * widen(vr[c]));
+          top = next;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        row_m[row] = top;
+        row_l[row] = sum;
+      }
+      __syncwarp();
+    }
+    const float mm = row_m[row], ll = row_l[row];
+    if (a.sums == nullptr) {
+      write_row<DV>(a, acc_row, mm, ll, t, h, lane);
+      continue;
+    }
+    const long long part = ((long long)split * a.tokens + t) * a.heads * a.maps + h * a.maps + map;
+    for (int c = lane * 4; c < DV; c += 128)
+      *reinterpret_cast<float4*>(a.sums + part * DV + c) = *reinterpret_cast<const float4*>(acc_row + c);
+    if (lane == 0) *reinterpret_cast<float2*>(a.stats + part * 2) = make_float2(mm, ll);
+  }
+}
+
+// Splits of a token's keys and maps of a head brought together: one block a token and head, a
+// thread for four columns. A few hundred kilobytes of fresh sums in the L2: its time is its trip
+// there (all splits asked for before the first is used) and the launch.
+template <int DV>
+__global__ void __launch_bounds__(DV / 4) attention_fold_kernel(const MmaAttention a) {
+  wait_for_previous_kernel();
+  const int t = blockIdx.x, h = blockIdx.y, c = threadIdx.x * 4;
+  const long long vheads = (long long)a.heads * a.maps;
+  float o[2][4];
+#pragma unroll
+  for (int map = 0; map < 2; ++map) {
+    if (map >= a.maps) continue;
+    const long long at = (long long)t * vheads + h * a.maps + map, step = a.tokens * vheads;
+    float top = -INFINITY;
+    for (int s = 0; s < a.key_splits; ++s) top = fmaxf(top, a.stats[(at + s * step) * 2]);
+    if (a.sink != nullptr) top = fmaxf(top, a.sink[h] * kLog2e);
+    float total = a.sink != nullptr ? mma::exp2_fast(a.sink[h] * kLog2e - top) : 0.f;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int s = 0; s < a.key_splits; ++s) {
+      const float2 ml = *reinterpret_cast<const float2*>(a.stats + (at + s * step) * 2);
+      const float4 v = *reinterpret_cast<const float4*>(a.sums + (at + s * step) * DV + c);
+      if (ml.x == -INFINITY && ml.y == 0.f) continue;      // (a split without keys)
+      const float f = mma::exp2_fast(ml.x - top);
+      total = fmaf(ml.y, f, total);
+      sum[0] = fmaf(v.x, f, sum[0]);
+      sum[1] = fmaf(v.y, f, sum[1]);
+      sum[2] = fmaf(v.z, f, sum[2]);
+      sum[3] = fmaf(v.w, f, sum[3]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[map][i] = sum[i] / total;
+  }
+  float r[4];
+  if (a.maps == 2) {         // a1 - lambda a2, over its root mean square
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[i] = o[0][i] - a.lambda * o[1][i];
+      ss = fmaf(r[i], r[i], ss);
+    }
+    __shared__ float scratch[33];
+    const float f = rsqrtf(block_sum(ss, scratch) / (float)DV + a.eps) * a.out_scale;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[i] *= f;
+      if (a.map_gate != nullptr)
+        r[i] *= 1.f / (1.f + expf(-widen(a.map_gate[(long long)t * a.map_gate_stride +
+                                                   (long long)h * DV + c + i])));
+    }
+  } else {
+    float f = a.out_scale;
+    if (a.gate != nullptr)
+      f *= 1.f / (1.f + expf(-widen(a.gate[(long long)t * a.gate_stride + h])));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      r[i] = o[0][i] * f;
+      if (a.elem_gate != nullptr)
+        r[i] /= 1.f + expf(-a.elem_gate[(long long)t * a.elem_stride + (long long)h * DV + c + i]);
+    }
+  }
+  *reinterpret_cast<uint2*>(a.out + ((long long)t * a.heads + h) * DV + c) =
+      make_uint2(mma::pack_bf16(r[0], r[1]), mma::pack_bf16(r[2], r[3]));
+}
+
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
+  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES>;
+  static_assert(S::kBytes <= 227 * 1024, "shared memory of a block");
+  auto kernel = attention_mma_kernel<DK, DV, VINK, WR, WC, KT, STAGES>;
+  static PerDeviceOnce configured;
+  if (configured.needs()) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+    if (e != cudaSuccess) return (int)e;
+    configured.done();
+  }
+  const int hg = a.heads / a.kv_heads;
+  a.heads_per_tile = hg < S::kRows ? hg : S::kRows;
+  a.head_tiles = (hg + a.heads_per_tile - 1) / a.heads_per_tile;
+  a.tokens_per_tile = decode ? 1 : S::kRows / a.heads_per_tile;
+  const long long tiles = (a.tokens + a.tokens_per_tile - 1) / a.tokens_per_tile;
+  const long long across = (long long)a.kv_heads * a.maps * a.head_tiles;
+  if (across > 65535) return cudaErrorInvalidValue;
+  const int code = launch_overlapped(kernel, dim3((unsigned)tiles, (unsigned)across, (unsigned)a.key_splits),
+                                     dim3(S::kThreads), S::kBytes, stream, 1, a);
+  if (code != 0 || a.sums == nullptr) return code;
+  return launch_overlapped(attention_fold_kernel<DV>, dim3((unsigned)a.tokens, (unsigned)a.heads),
+                           dim3(DV / 4), 0, stream, 1, a);
+}
+
+}  // namespace
+
+// Everything as in `sakv_cached_attention` (`csrc/attention_distance.cu`) with bfloat16 operands,
+// plus slope and rate of the logarithmic penalty; gate: the pre-activations of a gate a head, map_gate:
+// of two maps' gate element by element (first head's first column; rows *_stride apart). decode 0:
+// blocks of 64 rows of a prompt; 1: a block a token, key/value head, map and split. sums, stats: fp32
+// scratch of key_splits * tokens * heads * maps * (vdim, 2) numbers, needed with two maps or several
+// splits, else null. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
+// = (64, 64), (128, 128), (128, 256) and, with v_cache null, (576, 512); rows that do not begin at
+// multiples of 16 bytes.
+SAKV_EXPORT int sakv_attention_mma(
+    const void* q, long long q_stride, int q_head_stride, const void* q2, long long q2_stride,
+    int q2_head_stride, int q_split, void* out, const void* k_cache, int k_row, const void* v_cache,
+    int v_row, const int32_t* positions, const int32_t* token_seq, const int32_t* block_table,
+    int max_blocks, int tokens, int heads, int kv_heads, int maps, int dim, int vdim, float scale,
+    int window, int chunk, int keep, const float* slope, const float* rate, float softcap,
+    const float* linear, const float* sink, const void* gate, long long gate_stride,
+    const float* elem_gate, long long elem_stride, const void* map_gate, long long map_gate_stride,
+    float out_scale, float lambda, float eps, int decode, int key_splits, float* sums, float* stats,
+    cudaStream_t stream) {
+  if (tokens < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || (maps != 1 && maps != 2) ||
+      window < 0 || chunk < 0 || keep < 0 || (window > 0 && chunk > 0) || softcap < 0.f ||
+      max_blocks <= 0 || key_splits < 1 || key_splits > 64 || (!decode && key_splits > 1) ||
+      k_row < maps * dim || (v_cache != nullptr ? v_row < vdim : k_row < vdim) ||
+      (q2 != nullptr && (q_split < 0 || q_split > dim)) || heads > 65535)
+    return cudaErrorInvalidValue;
+  const bool two_step = maps == 2 || key_splits > 1;
+  if (two_step != (sums != nullptr) || two_step != (stats != nullptr)) return cudaErrorInvalidValue;
+  if (maps == 2 && (gate != nullptr || elem_gate != nullptr)) return cudaErrorInvalidValue;
+  if ((((uintptr_t)q | (uintptr_t)q2 | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) ||
+      ((q_stride | q_head_stride | k_row) & 7) || (v_cache != nullptr && (v_row & 7)) ||
+      (q2 != nullptr && ((q2_stride | q2_head_stride | q_split) & 7)))
+    return cudaErrorInvalidValue;
+  if (tokens == 0) return 0;
+  MmaAttention a = {};
+  a.q = (const __nv_bfloat16*)q;
+  a.q_stride = q_stride;
+  a.q_head_stride = q_head_stride;
+  a.q2 = (const __nv_bfloat16*)q2;
+  a.q2_stride = q2_stride;
+  a.q2_head_stride = q2_head_stride;
+  a.q_split = q2 != nullptr ? q_split : dim;
+  a.k_cache = (const __nv_bfloat16*)k_cache;
+  a.v_cache = (const __nv_bfloat16*)v_cache;
+  a.k_row = k_row;
+  a.v_row = v_row;
+  a.positions = positions;
+  a.token_seq = token_seq;
+  a.block_table = block_table;
+  a.max_blocks = max_blocks;
+  a.tokens = tokens;
+  a.heads = heads;
+  a.kv_heads = kv_heads;
+  a.maps = maps;
+  a.scale = scale;
+  a.window = window;
+  a.chunk = chunk;
+  a.keep = window > 0 ? keep : 0;
+  a.slope = slope;
+  a.rate = rate;
+  a.softcap = softcap;
+  a.linear = linear;
+  a.key_splits = key_splits;
+  a.out = (__nv_bfloat16*)out;
+  a.sums = sums;
+  a.stats = stats;
+  a.sink = sink;
+  a.gate = (const __nv_bfloat16*)gate;
+  a.gate_stride = gate_stride;
+  a.elem_gate = elem_gate;
+  a.elem_stride = elem_stride;
+  a.map_gate = (const __nv_bfloat16*)map_gate;
+  a.map_gate_stride = map_gate_stride;
+  a.out_scale = out_scale;
+  a.lambda = lambda;
+  a.eps = eps;
+  const bool in_key = v_cache == nullptr;
+  if (in_key && dim == 576 && vdim == 512 && maps == 1)
+    return decode ? launch_shape<576, 512, true, 1, 8, 64, 2>(a, true, stream)
+                  : launch_shape<576, 512, true, 4, 2, 32, 3>(a, false, stream);
+  if (in_key) return cudaErrorInvalidValue;
+  if (dim == 128 && vdim == 128)
+    return decode ? launch_shape<128, 128, false, 1, 8, 64, 3>(a, true, stream)
+                  : launch_shape<128, 128, false, 4, 1, 64, 2>(a, false, stream);
+  if (dim == 128 && vdim == 256)
+    return decode ? launch_shape<128, 256, false, 1, 8, 64, 3>(a, true, stream)
+                  : launch_shape<128, 256, false, 4, 1, 32, 2>(a, false, stream);
+  if (dim == 64 && vdim == 64)
+    return decode ? launch_shape<64, 64, false, 1, 4, 64, 3>(a, true, stream)
+                  : launch_shape<64, 64, false, 4, 1, 64, 2>(a, false, stream);
+  return cudaErrorInvalidValue;
+}

@@ -50,6 +50,7 @@ LIBRARIES = {
     "streams": "streams.cu",
     "delta_rule": "delta_rule.cu",
     "attention_distance": "attention_distance.cu",
+    "attention_mma": "attention_mma.cu",
     "layer_norm": "layer_norm.cu",
     "latent": "latent.cu",
     "moe": "moe.cu",

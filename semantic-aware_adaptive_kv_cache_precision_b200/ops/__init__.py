@@ -11,9 +11,9 @@ from __future__ import annotations
 import torch
 
 from ._lib import (BF16, CACHE_BLOCK, F32, KernelError, call, dtype_code, plain_function, ptr,
-                   require_cuda)
+                   require_cuda, sm_count)
 from .linear import Deferred, dense_up, gated_up, linear, per_head
-from . import gemm_tc
+from . import attention_mma, gemm_tc
 from .streams import streams_spread, streams_step, token_shift
 from .recurrent import delta_rule, gated_delta
 from .scan import causal_conv, decay_attention, dual_scan, norm_gate, selective_scan, step_size
@@ -258,6 +258,12 @@ def distance_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
         _check(c is None or (c.dtype == torch.float32 and c.shape == (heads,)
                              and c.is_contiguous()), "slope, rate: fp32 [heads]")
     _check(gate_off is None or 0 <= gate_off <= qkv.shape[1] - heads, "gate_off: inside qkv")
+    if 1 <= splits <= 16 and attention_mma.takes(qkv, dim, k_cache, v_cache, dim, vdim):
+        return attention_mma.attention(
+            qkv, dim, k_cache, v_cache, positions, token_seq, block_table, heads, dim, vdim, scale,
+            window=window, slope=slope, rate=rate,
+            head_gate=None if gate_off is None else qkv[:, gate_off:gate_off + heads],
+            decode=splits > 1, key_splits=splits)
     out = torch.empty((tokens, heads * vdim), dtype=qkv.dtype, device=qkv.device)
     call("sakv_distance_attention", ptr(qkv), dtype_code(qkv.dtype), qkv.stride(0),
          -1 if gate_off is None else int(gate_off), ptr(out), ptr(k_cache), ptr(v_cache),
@@ -496,10 +502,20 @@ def cached_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     _check(max(q.stride(1), 0 if q2 is None else q2.stride(1)) < 2 ** 31, "head stride too large")
     _check(block_table.dtype == torch.int32 and block_table.dim() == 2
            and block_table.is_contiguous(), "block_table: int32 [B, max_blocks]")
+    heads_first = bool(heads_first) and splits == 1
+    decode = heads_first or splits > 1
+    across = max(1, int(key_splits)) * (1 if heads_first else int(splits)) if decode else 1
+    if 1 <= splits <= 16 and across <= 64 and not (window and chunk) \
+            and attention_mma.takes(q, q.stride(1), k_cache, v_cache, dim, vdim, maps, q2, q_split):
+        return attention_mma.attention(
+            q, q.stride(1), k_cache, v_cache, positions, token_seq, block_table, heads, dim, vdim,
+            scale, maps=maps, q2=q2, q_split=q_split, window=window, chunk=chunk,
+            keep_first=keep_first, softcap=softcap, linear=linear_slopes, sink=sink,
+            head_gate=head_gate, elem_gate=elem_gate, map_gate_off=gate_elem_off, lam=lam,
+            out_scale=out_scale, eps=eps, decode=decode, key_splits=across)
     out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
     scratch = tickets = None
     floats = 0
-    heads_first = bool(heads_first) and splits == 1
     if key_splits > 1 and (splits > 1 or heads_first):
         groups = tokens * kv_heads * (heads * maps // kv_heads + 3)
         floats = groups * key_splits * (max(dim, vdim + 2) + 4)

@@ -44,6 +44,9 @@ SIGNATURES = {
                               [P, I, L, I, P, L, I, I, I, P, P, I, P, I, P, P, P, I, I, I, I, I, I,
                                I, F, I, I, F, F, F, I, I, I, P, L, P, I, I, I, P, P, L, P, L, F, P,
                                P]),
+    "sakv_attention_mma": ("attention_mma",
+                           [P, L, I, P, L, I, I, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I,
+                            I, P, P, F, P, P, P, L, P, L, P, L, F, F, F, I, I, P, P, P]),
     "sakv_rms_update": ("norm_update", [P, P, P, F, P, P, F, I, P, I, I, I, F, P]),
     "sakv_rms_join": ("norm_update", [P, P, P, P, P, F, F, F, P, I, F, P, I, I, I, P]),
     "sakv_qk_prepare": ("qk_prepare", [P, L, I, I, I, P, P, I, F, P, P, I, P, P, P, I, P, P, P,

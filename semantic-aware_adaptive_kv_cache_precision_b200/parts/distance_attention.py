@@ -89,18 +89,23 @@ class LogDistanceAttention(Part):
         return ops.linear(attended, self.w_o, self.b_o, out_dtype=torch.float32)
 
     def _splits(self, step, qkv) -> int:
-        """How many warps share a token's keys. One in the 32-bit mode and for prompts (the
+        """How many warps, or on the tensor cores blocks, share a token's keys. One in the 32-bit mode and for prompts (the
         sums then have one order however the tokens are cut); for decode steps in bfloat16 one
         warp for every two chunks of 32 keys that a token can see, up to 16. (A decode
         step's graph is keyed by the width of the block lists, which bounds the length.)"""
         if qkv.dtype == torch.float32 or not step.is_decode:
             return 1
+        s = self.spec
         keys = step.max_len_bound or step.max_len
-        if self.spec.window:
-            keys = min(keys, self.spec.window + 31)
+        if s.window:
+            keys = min(keys, s.window + 31)
         splits = 1
         while splits < 16 and splits * 64 < keys:
             splits *= 2
+        if (s.head_dim, s.value_dim, False) in ops.attention_mma.SHAPES:
+            # (blocks: no more than four an SM, each brings its own partial sums)
+            while splits > 2 and step.tokens * s.kv_heads * splits > 4 * ops.sm_count():
+                splits //= 2
         return splits
 
     def forward(self, h, step, view, residual, write_cache=True):
