@@ -39,6 +39,34 @@ __device__ __forceinline__ float exp_less_one(float x) {
   return x > -0.125f ? series : __expf(x) - 1.f;
 }
 
+// Between the two passes over a prompt's runs: one number of the state is carried from run to run.
+// What run j left at p[j * step] is replaced by what came before it, which fades by fade(j) + 1
+// over the run. Bound by memory (every run's state is read and written once): the runs' numbers are
+// asked for eight at a time before the first is used, since the store of one keeps the compiler
+// from asking for the next (the dual form, 16 sequences of up to 8 runs of 1 MB of state: 350 us
+// one by one, 120 now; one sequence of 47 runs of the fading state: 162 and 25).
+template <typename Fade>
+__device__ __forceinline__ float carry_runs(float* __restrict__ p, long long step, int runs, float s,
+                                            Fade fade) {
+  constexpr int kAhead = 8;
+  for (int j0 = 0; j0 < runs; j0 += kAhead) {
+    float left[kAhead], f[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (j0 + k < runs) left[k] = p[(j0 + k) * step];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (j0 + k < runs) f[k] = fade(j0 + k);
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (j0 + k < runs) {
+        p[(j0 + k) * step] = s;
+        s += fmaf(f[k], s, left[k]);
+      }
+  }
+  return s;
+}
+
 // ---------------------------------------------------------------------------------------
 // The short causal convolution. Token i of a sequence's part in this step reads its own
 // input and the taps - 1 before it: from the step while there are any, from the state (the
@@ -293,13 +321,9 @@ __global__ void scan_carry_kernel(const W* __restrict__ a_log, float* __restrict
   const int runs = (cu_seqlens[b + 1] - cu_seqlens[b] + chunk_len - 1) / chunk_len;
   const float a = -expf(widen(a_log[cn]));
   float* home = state + (long long)slots[b] * per + cn;
-  float s = *home;
-  for (int j = 0; j < runs; ++j) {
-    float* p = scratch + ((long long)b * max_chunks + j) * per + cn;
-    const float left = *p;
-    *p = s;
-    s += fmaf(expm1f(a * dt_sums[((long long)b * max_chunks + j) * channels + c]), s, left);
-  }
+  const float* sums = dt_sums + (long long)b * max_chunks * channels + c;
+  const float s = carry_runs(scratch + (long long)b * max_chunks * per + cn, per, runs, *home,
+                             [&](int j) { return expm1f(a * sums[(long long)j * channels]); });
   if (keep_state) *home = s;
 }
 
@@ -463,14 +487,11 @@ __global__ void decay_carry_kernel(const float* __restrict__ decay_less_one,
   const int runs = (n + chunk_len - 1) / chunk_len;
   const float log_fade = log1pf(decay_less_one[e / per_head]);
   float* home = state + (long long)slots[b] * per + e;
-  float s = *home;
-  for (int j = 0; j < runs; ++j) {
-    float* p = scratch + ((long long)b * max_chunks + j) * per + e;
-    const float left = *p;
-    *p = s;
-    const int len = n - j * chunk_len < chunk_len ? n - j * chunk_len : chunk_len;
-    s += fmaf(expm1f(log_fade * static_cast<float>(len)), s, left);
-  }
+  const float s = carry_runs(
+      scratch + (long long)b * max_chunks * per + e, per, runs, *home, [&](int j) {
+        const int len = n - j * chunk_len < chunk_len ? n - j * chunk_len : chunk_len;
+        return expm1f(log_fade * static_cast<float>(len));
+      });
   if (keep_state) *home = s;
 }
 
@@ -674,13 +695,10 @@ __global__ void dual_carry_kernel(const float* __restrict__ a, float* __restrict
   const int h = static_cast<int>(e / per_head);
   const int runs = (cu_seqlens[b + 1] - cu_seqlens[b] + chunk_len - 1) / chunk_len;
   float* home = state + (long long)slots[b] * per + e;
-  float s = *home;
-  for (int j = 0; j < runs; ++j) {
-    float* p = scratch + ((long long)b * max_chunks + j) * per + e;
-    const float left = *p;
-    *p = s;
-    s += fmaf(expm1f(a[h] * dt_sums[((long long)b * max_chunks + j) * heads + h]), s, left);
-  }
+  const float rate = a[h];
+  const float* sums = dt_sums + (long long)b * max_chunks * heads + h;
+  const float s = carry_runs(scratch + (long long)b * max_chunks * per + e, per, runs, *home,
+                             [&](int j) { return expm1f(rate * sums[(long long)j * heads]); });
   if (keep_state) *home = s;
 }
 
