@@ -10,7 +10,7 @@
 //   o = S^T r;   out = o / sqrt(mean(o^2) + eps) * norm_w * sigmoid(g)
 //
 // Three kernels. `delta_prepare` works out what does not depend on the state, for all tokens
-// side by side (a warp a token and head): w, u and a * u, fp32 [tokens, 3, heads * dim].
+// side by side: w, u and a * u, fp32 [tokens, 3, heads * dim].
 // `delta_scan` is the recurrence: a block has some neighbouring columns of one head's state
 // for one sequence (columns never meet, so a head may be spread over several blocks when
 // there are few heads and sequences) and walks the sequence's tokens of this step in chunks
@@ -29,47 +29,85 @@ namespace {
 
 __device__ __forceinline__ float sigmoidf(float z) { return 1.f / (1.f + expf(-z)); }
 
-constexpr int kPrepareTokens = 8;      // tokens (warps) of a block of `delta_prepare`
+constexpr int kPrepareThreads = 256;
 
+// A warp's lanes share out a head's channels and a block takes `per_block` tokens: a channel's row of
+// W2 (in shared memory) is read once for eight of them, whose factors lie side by side. 120 -> 87 us
+// over 2,048 tokens of 32 heads of 64, rank 64 (with a warp a token every product read its weight
+// and its factor from shared memory).
 template <typename W>
-__global__ void __launch_bounds__(kPrepareTokens * 32)
+__global__ void __launch_bounds__(kPrepareThreads)
 delta_prepare_kernel(const float* __restrict__ proj, long long proj_stride, int off_k, int off_a,
                      int off_l, const W* __restrict__ w2, const W* __restrict__ w0,
                      const W* __restrict__ a_bias, float* __restrict__ prepared, int tokens,
-                     int heads, int dim, int rank, float decay_scale, float key_eps) {
-  extern __shared__ float shared[];
+                     int heads, int dim, int rank, int per_block, float decay_scale,
+                     float key_eps) {
+  extern __shared__ __align__(16) float shared[];
+  float* s_l = shared;                              // [rank][tokens of the block]
+  float* s_inv = s_l + rank * per_block;            // [tokens of the block]
   const int ld2 = rank + 1;                         // padded rows of W2: no bank conflicts
-  float* s_w2 = shared;                             // [dim][rank + 1]
-  float* s_l = s_w2 + dim * ld2;                    // [warps][rank]
+  float* s_w2 = s_inv + per_block;                  // [dim][rank + 1]
   let_next_kernel_start();
   const int head = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kWarps = kPrepareThreads / 32;
   const int base = head * dim;
   for (int i = threadIdx.x; i < dim * rank; i += blockDim.x)
     s_w2[(i / rank) * ld2 + i % rank] = widen(w2[(long long)base * rank + i]);
   wait_for_previous_kernel();
-  const long long t = (long long)blockIdx.x * kPrepareTokens + warp;
-  const bool live = t < tokens;
-  const float* row = proj + (live ? t : 0) * proj_stride;
-  float* l = s_l + warp * rank;
-  for (int j = lane; j < rank; j += 32) l[j] = tanhf(row[off_l + j]);
-  __syncthreads();
-  if (!live) return;
-  float kk = 0.f;
-  for (int c = lane; c < dim; c += 32) {
-    const float k = row[off_k + base + c];
-    kk = fmaf(k, k, kk);
+  const long long t0 = (long long)blockIdx.x * per_block;
+  const int count = tokens - t0 < per_block ? static_cast<int>(tokens - t0) : per_block;
+  for (int i = threadIdx.x; i < per_block * rank; i += blockDim.x) {
+    const int tt = i / rank, j = i - tt * rank;
+    s_l[j * per_block + tt] = tt < count ? tanhf(proj[(t0 + tt) * proj_stride + off_l + j]) : 0.f;
   }
-  const float inv = 1.f / sqrtf(warp_sum(kk) + key_eps);
+  for (int tt = warp; tt < count; tt += kWarps) {
+    const float* row = proj + (t0 + tt) * proj_stride;
+    float kk = 0.f;
+    for (int c = lane; c < dim; c += 32) {
+      const float k = row[off_k + base + c];
+      kk = fmaf(k, k, kk);
+    }
+    kk = warp_sum(kk);
+    if (lane == 0) s_inv[tt] = 1.f / sqrtf(kk + key_eps);
+  }
+  __syncthreads();
   const long long hd = (long long)heads * dim;
-  float* dst = prepared + t * 3 * hd + base;
-  for (int c = lane; c < dim; c += 32) {
-    float z = widen(w0[base + c]);
+  constexpr int kTogether = 8;                      // (per_block is a multiple of it)
+  const int runs = (dim + 31) / 32;                 // of 32 channels
+  for (int job = warp; job < runs * (per_block / kTogether); job += kWarps) {
+    const int c = job % runs * 32 + lane, tt0 = job / runs * kTogether;
+    if (tt0 >= count || c >= dim) continue;
+    float z[kTogether];
+#pragma unroll
+    for (int q = 0; q < kTogether; ++q) z[q] = widen(w0[base + c]);
     const float* w2row = s_w2 + c * ld2;
-    for (int j = 0; j < rank; ++j) z = fmaf(w2row[j], l[j], z);
-    const float u = row[off_k + base + c] * inv;
-    dst[c] = expf(-decay_scale * sigmoidf(z));
-    dst[hd + c] = u;
-    dst[2 * hd + c] = sigmoidf(row[off_a + base + c] + widen(a_bias[base + c])) * u;
+#pragma unroll 4
+    for (int j = 0; j < rank; ++j) {
+      const float w = w2row[j];
+      const float4 l0 = *reinterpret_cast<const float4*>(s_l + j * per_block + tt0);
+      const float4 l1 = *reinterpret_cast<const float4*>(s_l + j * per_block + tt0 + 4);
+      z[0] = fmaf(w, l0.x, z[0]); z[1] = fmaf(w, l0.y, z[1]);
+      z[2] = fmaf(w, l0.z, z[2]); z[3] = fmaf(w, l0.w, z[3]);
+      z[4] = fmaf(w, l1.x, z[4]); z[5] = fmaf(w, l1.y, z[5]);
+      z[6] = fmaf(w, l1.z, z[6]); z[7] = fmaf(w, l1.w, z[7]);
+    }
+    const float bias = widen(a_bias[base + c]);
+    float k[kTogether], a[kTogether];
+#pragma unroll
+    for (int q = 0; q < kTogether; ++q) {           // (asked for together)
+      const float* row = proj + (t0 + min(tt0 + q, count - 1)) * proj_stride + base + c;
+      k[q] = row[off_k];
+      a[q] = row[off_a];
+    }
+#pragma unroll
+    for (int q = 0; q < kTogether; ++q) {
+      if (tt0 + q >= count) break;
+      float* dst = prepared + (t0 + tt0 + q) * 3 * hd + base;
+      const float u = k[q] * s_inv[tt0 + q];
+      dst[c] = expf(-decay_scale * sigmoidf(z[q]));
+      dst[hd + c] = u;
+      dst[2 * hd + c] = sigmoidf(a[q] + bias) * u;
+    }
   }
 }
 
@@ -89,11 +127,46 @@ __device__ __forceinline__ void copies_wait_all_but_last() {
   asm volatile("cp.async.wait_group 1;" ::: "memory");
 }
 
+// Two fp32 numbers in one register pair, and the two-wide arithmetic on them.
+typedef unsigned long long Two;
+__device__ __forceinline__ Two two(float a, float b) {
+  Two d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
+  Two d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ Two mul2(Two a, Two b) {
+  Two d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float both(Two v) {
+  float a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+  return a + b;
+}
+
 // One block: `cols` neighbouring columns of one head's state for one sequence. A column's
 // rows are dealt to R neighbouring lanes, dim / R <= RPT rows each. VEC: rows are read four
-// at a time (dim / R a multiple of 4, everything 16-byte aligned). The raw o = S^T r goes to
-// `raw` [tokens, heads * dim] fp32 for `delta_finish`.
-template <int RPT, int R, bool VEC>
+// at a time (dim / R a multiple of 4, everything 16-byte aligned); WHOLE: dim / R is RPT.
+// The raw o = S^T r goes to `raw` [tokens, heads * dim] fp32 for `delta_finish`.
+//
+// What bounds it is the chain from token to token: the sum u^T S over a column's R lanes (a
+// shuffle tree) and the update that waits for it. The WHOLE form keeps out of that chain what does
+// not belong to it: R tokens are one straight run of code, so that the next token's vectors can be
+// read meanwhile; S is held in pairs for two-wide arithmetic; and the outputs' sums wait until R
+// tokens have left theirs, when each lane finishes one token's (R - 1 exchanges instead of
+// R log2 R, the same tree of additions). One sequence of 2,048 tokens, 32 heads of 64, behind its
+// prepare kernel: 842 us before, 373 now (of which the launch in plain order 206, see
+// `launch_scan`). Tried and no faster (380 to 450): two columns a thread, bulk copies of the vectors
+// (60 ns each), a copying warp of its own, vectors read by volatile loads a token ahead, 4 or 16
+// lanes a column. Without its shuffles, copies and reads of shared memory, which lie in one chain
+// each with the next, the bare arithmetic takes 118.
+template <int RPT, int R, bool VEC, bool WHOLE>
 __global__ void __launch_bounds__(512)
 delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off_r, int off_k,
                   int off_v, const float* __restrict__ prepared, float* __restrict__ state,
@@ -103,7 +176,7 @@ delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off
   extern __shared__ __align__(16) float shared[];
   // a token's per-row vectors lie part by part with four floats between the parts, so that the
   // R lanes of a column read from different banks
-  const int rpt = dim / R;
+  const int rpt = WHOLE ? RPT : dim / R;
   const int ldp = rpt + (R > 1 ? 4 : 0), ldt = R * ldp;      // a part's, a token's stride
   const int per_buffer = chunk * (5 * ldt + cols);
   let_next_kernel_start();
@@ -119,6 +192,9 @@ delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off
   float S[RPT];
 #pragma unroll
   for (int i = 0; i < RPT; ++i) S[i] = (mine && i < rpt) ? my_state[(long long)i * dim] : 0.f;
+  Two S2[RPT / 2];                                 // (WHOLE: the same in pairs, instead of S)
+#pragma unroll
+  for (int i = 0; i < RPT / 2; ++i) S2[i] = two(S[2 * i], S[2 * i + 1]);
 
   const bool aligned = VEC && dim % 4 == 0 && cols % 4 == 0 && proj_stride % 4 == 0 &&
                        off_r % 4 == 0 && off_k % 4 == 0 && off_v % 4 == 0 &&
@@ -195,7 +271,61 @@ delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off
     __syncthreads();                                 // the chunk has landed, for everyone
     const float* rows = shared + buffer * per_buffer + part * ldp;
     const float* vals = shared + buffer * per_buffer + chunk * 5 * ldt + (mine ? mycol : 0);
-    for (int tt = 0; tt < count; ++tt) {             // the recurrence
+    if constexpr (WHOLE) {
+      // a token: the lane's share of its o, before the sum over the lanes
+      auto token = [&](int tt) {
+        const float* x = rows + tt * 5 * ldt;
+        Two r[RPT / 2], k[RPT / 2], w[RPT / 2], u[RPT / 2], b[RPT / 2];
+        auto read = [&](Two (&to)[RPT / 2], const float* from) {
+#pragma unroll
+          for (int i = 0; i < RPT / 2; i += 2) {
+            const ulonglong2 got = *reinterpret_cast<const ulonglong2*>(from + 2 * i);
+            to[i] = got.x;
+            to[i + 1] = got.y;
+          }
+        };
+        read(u, x + 3 * ldt);
+        read(b, x + 4 * ldt);
+        read(k, x + ldt);
+        read(w, x + 2 * ldt);
+        read(r, x);
+        const float v = vals[tt * cols];
+        Two sum = mul2(u[0], S2[0]);
+#pragma unroll
+        for (int i = 1; i < RPT / 2; ++i) sum = fma2(u[i], S2[i], sum);
+        const float sa = sum_over_parts<R>(both(sum));
+        const Two taken = two(-sa, -sa), put = two(v, v);
+        Two o = two(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < RPT / 2; ++i) {
+          S2[i] = fma2(w[i], S2[i], fma2(b[i], taken, mul2(k[i], put)));
+          o = fma2(S2[i], r[i], o);
+        }
+        return both(o);
+      };
+      int tt = 0;
+      for (; tt + R <= count; tt += R) {
+        float o[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) o[q] = token(tt + q);
+#pragma unroll
+        for (int step = 1, n = R / 2; step < R; step <<= 1, n >>= 1) {
+          const bool odd = (part & step) != 0;
+#pragma unroll
+          for (int i = 0; i < R / 2; ++i)
+            if (i < n) {
+              const float keep = odd ? o[2 * i + 1] : o[2 * i], give = odd ? o[2 * i] : o[2 * i + 1];
+              o[i] = keep + __shfl_xor_sync(0xffffffffu, give, step);
+            }
+        }
+        if (mine) raw[(long long)(t0 + tt + part) * hd + base + col] = o[0];
+      }
+      for (; tt < count; ++tt) {
+        const float o = sum_over_parts<R>(token(tt));
+        if (mine && part == 0) raw[(long long)(t0 + tt) * hd + base + col] = o;
+      }
+    }
+    for (int tt = 0; !WHOLE && tt < count; ++tt) {   // the recurrence
       const float* x = rows + tt * 5 * ldt;          // r, k, w, u, a*u: ldt apart
       const float v = vals[tt * cols];
       float sa = 0.f, o = 0.f;
@@ -237,6 +367,11 @@ delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off
     }
     __syncthreads();                                 // everyone is done with this buffer
   }
+  if constexpr (WHOLE) {
+#pragma unroll
+    for (int i = 0; i < RPT / 2; ++i)
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(S[2 * i]), "=f"(S[2 * i + 1]) : "l"(S2[i]));
+  }
   if (keep_state && mine) {
 #pragma unroll
     for (int i = 0; i < RPT; ++i)
@@ -269,7 +404,7 @@ __global__ void delta_finish_kernel(const float* __restrict__ raw, const float* 
 
 constexpr size_t kScanBudget = 96 * 1024;
 
-template <int RPT, int R, bool VEC>
+template <int RPT, int R, bool VEC, bool WHOLE>
 int launch_scan(const float* proj, long long proj_stride, const int* off, const float* prepared,
                 float* state, const int32_t* cu_seqlens, const int32_t* slots, float* raw,
                 int sequences, int heads, int dim, int chunk, int keep_state,
@@ -292,25 +427,39 @@ int launch_scan(const float* proj, long long proj_stride, const int* off, const 
   if (bytes(chunk) > kScanBudget) return cudaErrorInvalidValue;
   const int threads = ((cols * R + 31) / 32) * 32;
   static PerDeviceOnce configured;
-  auto kernel = delta_scan_kernel<RPT, R, VEC>;
+  auto kernel = delta_scan_kernel<RPT, R, VEC, WHOLE>;
   if (configured.needs()) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)kScanBudget);
     if (e != cudaSuccess) return (int)e;
     configured.done();
   }
-  return launch_overlapped(kernel, dim3(heads, sequences, (dim + cols - 1) / cols), dim3(threads),
-                           bytes(chunk), stream, 1, proj, proj_stride, off[0], off[1], off[2],
-                           prepared, state, cu_seqlens, slots, raw, heads, dim, cols, chunk,
-                           keep_state);
+  // A prompt's blocks begin when the kernel before them has left the SMs, so that each finds one
+  // of its own: begun while it drains, two or three of them share an SM, and the longest decides
+  // (2,048 tokens, 32 heads of 64: 585 us a scan behind its prepare kernel, 379 in plain order).
+  // For a few tokens the early start is worth more.
+  const dim3 grid(heads, sequences, (dim + cols - 1) / cols);
+  if (chunk >= 8)
+    return launch_ordered(kernel, grid, dim3(threads), bytes(chunk), stream, proj, proj_stride, off[0],
+                          off[1], off[2], prepared, state, cu_seqlens, slots, raw, heads, dim, cols,
+                          chunk, keep_state);
+  return launch_overlapped(kernel, grid, dim3(threads), bytes(chunk), stream, 1, proj, proj_stride,
+                           off[0], off[1], off[2], prepared, state, cu_seqlens, slots, raw, heads, dim,
+                           cols, chunk, keep_state);
 }
 
 int pick_scan(const float* proj, long long proj_stride, const int* off, const float* prepared,
               float* state, const int32_t* cu_seqlens, const int32_t* slots, float* raw,
               int sequences, int heads, int dim, int chunk, int keep_state, cudaStream_t stream) {
-#define SAKV_SCAN(RPT, R, VEC)                                                                  \
-  return launch_scan<RPT, R, VEC>(proj, proj_stride, off, prepared, state, cu_seqlens, slots,   \
-                                  raw, sequences, heads, dim, chunk, keep_state, stream)
+#define SAKV_SCAN_AS(RPT, R, VEC, WHOLE)                                                        \
+  return launch_scan<RPT, R, VEC, WHOLE>(proj, proj_stride, off, prepared, state, cu_seqlens,   \
+                                         slots, raw, sequences, heads, dim, chunk, keep_state,  \
+                                         stream)
+#define SAKV_SCAN(RPT, R, VEC)                                 \
+  do {                                                         \
+    if (VEC && dim == RPT * R) SAKV_SCAN_AS(RPT, R, VEC, VEC); \
+    SAKV_SCAN_AS(RPT, R, VEC, false);                          \
+  } while (0)
   // a column's rows over R lanes, four rows at a time: the most lanes (up to 16) that leave
   // a lane 8 rows, or 4 where dim is small; dims that 16 does not divide: one lane a column
   if (dim % 16 == 0) {
@@ -330,6 +479,7 @@ int pick_scan(const float* proj, long long proj_stride, const int* off, const fl
   if (dim <= 128) SAKV_SCAN(128, 1, false);
   SAKV_SCAN(256, 1, false);
 #undef SAKV_SCAN
+#undef SAKV_SCAN_AS
 }
 
 template <typename W>
@@ -338,8 +488,13 @@ int run(const float* proj, long long proj_stride, const int* off, const void* w2
         const int32_t* cu_seqlens, const int32_t* slots, void* out, int out_dtype, int tokens,
         int sequences, int heads, int dim, int rank, int chunk, float decay_scale, float key_eps,
         float eps, int keep_state, cudaStream_t stream) {
-  constexpr size_t kPrepareBudget = 200 * 1024;
-  const size_t smem = ((size_t)dim * (rank + 1) + (size_t)kPrepareTokens * rank) * sizeof(float);
+  constexpr size_t kPrepareBudget = 227 * 1024;
+  // tokens of a block of `delta_prepare`: 32, fewer where there are few or the weights leave no room
+  auto prepare_bytes = [&](int n) { return (size_t)(dim + n) * (rank + 1) * sizeof(float); };
+  int per_block = 32;
+  while (per_block > 8 && (per_block / 2 >= tokens || prepare_bytes(per_block) > kPrepareBudget))
+    per_block /= 2;
+  const size_t smem = prepare_bytes(per_block);
   if (smem > kPrepareBudget) return cudaErrorInvalidValue;
   static PerDeviceOnce configured;
   if (configured.needs()) {
@@ -350,10 +505,10 @@ int run(const float* proj, long long proj_stride, const int* off, const void* w2
     configured.done();
   }
   int code = launch_overlapped(
-      delta_prepare_kernel<W>, dim3((tokens + kPrepareTokens - 1) / kPrepareTokens, heads),
-      dim3(kPrepareTokens * 32), smem, stream, 1, proj, proj_stride, off[1], off[4], off[5],
+      delta_prepare_kernel<W>, dim3((tokens + per_block - 1) / per_block, heads),
+      dim3(kPrepareThreads), smem, stream, 1, proj, proj_stride, off[1], off[4], off[5],
       (const W*)w2, (const W*)w0, (const W*)a_bias, prepared, tokens, heads, dim, rank,
-      decay_scale, key_eps);
+      per_block, decay_scale, key_eps);
   if (code != 0) return code;
   code = pick_scan(proj, proj_stride, off, prepared, state, cu_seqlens, slots, raw, sequences,
                    heads, dim, chunk, keep_state, stream);

@@ -778,6 +778,10 @@ int launch_scan(DeltaScan p, int sequences, int max_new, bool groups, cudaStream
     if (e != cudaSuccess) return (int)e;
     configured[form].done();
   }
+  // (a prompt's blocks begin when the kernel before them has left the SMs: begun while it drains
+  // they share SMs with one another and the longest decides; two sequences of 2,048 and 1,111
+  // tokens, 16 heads of 128 x 128: 677 us behind its inputs' kernel, 481 in plain order)
+  if (groups) return launch_ordered(kernel, grid, dim3(across * RS), bytes(chunk), stream, p);
   return launch_overlapped(kernel, grid, dim3(across * RS), bytes(chunk), stream, 1, p);
 }
 

@@ -17,8 +17,8 @@ def takes(q: torch.Tensor, head_stride: int, k_cache: torch.Tensor, v_cache, dim
     """Whether the tensor-core kernel takes the call: bfloat16, one of the compiled pairs of
     widths, and every row of queries, keys and values beginning at a multiple of 16 bytes (they are
     copied in pieces of 16). It is the faster one for all of these, from one decoded token on
-    (against the kernel that scores a key a lane, us: a prompt of 3,001 tokens 13,008 -> 583 over
-    latent rows, 3,444 -> 124 at 128 columns; one decoded token 95 -> 22 and 114 -> 15)."""
+    (against the kernel that scores a key a lane, us: a prompt of 3,001 tokens 13,058 -> 883 over
+    latent rows, 3,492 -> 295 at 128 columns; one decoded token 94 -> 27 and 92 -> 14)."""
     if q.dtype != torch.bfloat16 or SHAPES.get((dim, vdim, v_cache is None), 0) < maps:
         return False
     rows = [(q, q.stride(0), head_stride), (k_cache, k_cache.shape[3], 0)]
