@@ -21,16 +21,20 @@
 namespace {
 
 constexpr int kMaxPerLane = 8;  // head_dim <= 256
+constexpr int kTogether = 8;    // keys taken at a time
 
-template <typename T>
-__global__ void attention_plain_kernel(const T* __restrict__ q, long long q_stride,
-                                       T* __restrict__ out, const T* __restrict__ k_cache,
-                                       const T* __restrict__ v_cache,
-                                       const int32_t* __restrict__ positions,
-                                       const int32_t* __restrict__ token_seq,
-                                       const int32_t* __restrict__ block_table, int max_blocks,
-                                       int tokens, int heads, int kv_heads, int head_dim,
-                                       float scale, int window) {
+// A warp a (token, head). Bound by the chain from key to key (a trip to memory, a sum over the lanes,
+// the running maximum): keys are taken eight at a time, from multiples of eight on, so their rows
+// and their values' rows are asked for together, their scores are summed side by side and the
+// maximum moves once for the eight. PER: elements a lane.
+template <typename T, int PER>
+__global__ void __launch_bounds__(128)
+attention_plain_kernel(const T* __restrict__ q, long long q_stride, T* __restrict__ out,
+                       const T* __restrict__ k_cache, const T* __restrict__ v_cache,
+                       const int32_t* __restrict__ positions,
+                       const int32_t* __restrict__ token_seq,
+                       const int32_t* __restrict__ block_table, int max_blocks, int tokens,
+                       int heads, int kv_heads, int head_dim, float scale, int window) {
   const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= (long long)tokens * heads) return;
@@ -39,48 +43,86 @@ __global__ void attention_plain_kernel(const T* __restrict__ q, long long q_stri
   const int g = h / (heads / kv_heads);
   const int pos = positions[t];
   const int32_t* table = block_table + (long long)token_seq[t] * max_blocks;
-  const int per_lane = (head_dim + 31) / 32;
 
-  float qr[kMaxPerLane], acc[kMaxPerLane];
+  float qr[PER], acc[PER];
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
-    qr[i] = (i < per_lane && e < head_dim)
-                ? widen(q[(long long)t * q_stride + (long long)h * head_dim + e]) * scale
-                : 0.f;
+    qr[i] = e < head_dim ? widen(q[(long long)t * q_stride + (long long)h * head_dim + e]) * scale : 0.f;
     acc[i] = 0.f;
   }
   float m = -INFINITY, l = 0.f;
   const int first = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
-  for (int j = first; j <= pos; ++j) {
-    const int block = table[j / kCacheBlock];
+  for (int j0 = first / kTogether * kTogether; j0 <= pos; j0 += kTogether) {
+    const int block = table[j0 / kCacheBlock];
     const long long base =
-        (((long long)block * kv_heads + g) * kCacheBlock + j % kCacheBlock) * head_dim;
-    float part = 0.f;
+        (((long long)block * kv_heads + g) * kCacheBlock + j0 % kCacheBlock) * head_dim + lane;
+    float k[kTogether][PER], v[kTogether][PER], s[kTogether];
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
-      const int e = lane + 32 * i;
-      if (i < per_lane && e < head_dim) part += qr[i] * widen(k_cache[base + e]);
+    for (int n = 0; n < kTogether; ++n) {
+      const bool seen = j0 + n >= first && j0 + n <= pos;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const bool real = seen && lane + 32 * i < head_dim;
+        k[n][i] = real ? widen(k_cache[base + (long long)n * head_dim + 32 * i]) : 0.f;
+        v[n][i] = real ? widen(v_cache[base + (long long)n * head_dim + 32 * i]) : 0.f;
+      }
     }
-    const float s = warp_sum(part);
-    const float m_new = fmaxf(m, s);
-    const float corr = expf(m - m_new);
-    const float p = expf(s - m_new);
-    l = l * corr + p;
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) {
-      const int e = lane + 32 * i;
-      if (i < per_lane && e < head_dim) acc[i] = acc[i] * corr + p * widen(v_cache[base + e]);
+    for (int n = 0; n < kTogether; ++n) {
+      s[n] = 0.f;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) s[n] += qr[i] * k[n][i];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int n = 0; n < kTogether; ++n) s[n] += __shfl_xor_sync(0xffffffffu, s[n], o);
+    float m_new = m;
+#pragma unroll
+    for (int n = 0; n < kTogether; ++n)
+      if (j0 + n >= first && j0 + n <= pos) m_new = fmaxf(m_new, s[n]);
+    const float corr = expf(m - m_new);
+    l *= corr;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) acc[i] *= corr;
+#pragma unroll
+    for (int n = 0; n < kTogether; ++n) {
+      if (j0 + n < first || j0 + n > pos) continue;
+      const float p = expf(s[n] - m_new);
+      l += p;
+#pragma unroll
+      for (int i = 0; i < PER; ++i) acc[i] = acc[i] + p * v[n][i];
     }
     m = m_new;
   }
   const float inv = 1.f / l;
 #pragma unroll
-  for (int i = 0; i < kMaxPerLane; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = lane + 32 * i;
-    if (i < per_lane && e < head_dim)
-      out[((long long)t * heads + h) * head_dim + e] = narrow<T>(acc[i] * inv);
+    if (e < head_dim) out[((long long)t * heads + h) * head_dim + e] = narrow<T>(acc[i] * inv);
   }
+}
+
+template <typename T>
+int launch_plain(const void* q, long long q_stride, void* out, const void* k_cache,
+                 const void* v_cache, const int32_t* positions, const int32_t* token_seq,
+                 const int32_t* block_table, int max_blocks, int tokens, int heads, int kv_heads,
+                 int head_dim, float scale, int window, cudaStream_t stream) {
+  const int threads = 128;
+  const long long warps = (long long)tokens * heads;
+  const long long blocks = (warps * 32 + threads - 1) / threads;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+#define SAKV_PLAIN(PER)                                                                           \
+  attention_plain_kernel<T, PER><<<(unsigned)blocks, threads, 0, stream>>>(                       \
+      (const T*)q, q_stride, (T*)out, (const T*)k_cache, (const T*)v_cache, positions, token_seq, \
+      block_table, max_blocks, tokens, heads, kv_heads, head_dim, scale, window)
+  if (head_dim <= 32) SAKV_PLAIN(1);
+  else if (head_dim <= 64) SAKV_PLAIN(2);
+  else if (head_dim <= 128) SAKV_PLAIN(4);
+  else SAKV_PLAIN(8);
+#undef SAKV_PLAIN
+  return launch_status();
 }
 
 }  // namespace
@@ -95,21 +137,12 @@ SAKV_EXPORT int sakv_attention_plain(const void* q, int dtype, long long q_strid
       head_dim > 32 * kMaxPerLane || max_blocks <= 0)
     return cudaErrorInvalidValue;
   if (tokens == 0) return 0;
-  const int threads = 128;
-  const long long warps = (long long)tokens * heads;
-  const long long blocks = (warps * 32 + threads - 1) / threads;
-  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   if (dtype == SAKV_F32)
-    attention_plain_kernel<float><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const float*)q, q_stride, (float*)out, (const float*)k_cache, (const float*)v_cache,
-        positions, token_seq, block_table, max_blocks, tokens, heads, kv_heads, head_dim, scale,
-        window);
-  else if (dtype == SAKV_BF16)
-    attention_plain_kernel<__nv_bfloat16><<<(unsigned)blocks, threads, 0, stream>>>(
-        (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_cache,
-        (const __nv_bfloat16*)v_cache, positions, token_seq, block_table, max_blocks, tokens,
-        heads, kv_heads, head_dim, scale, window);
-  else
-    return cudaErrorInvalidValue;
-  return launch_status();
+    return launch_plain<float>(q, q_stride, out, k_cache, v_cache, positions, token_seq, block_table,
+                               max_blocks, tokens, heads, kv_heads, head_dim, scale, window, stream);
+  if (dtype == SAKV_BF16)
+    return launch_plain<__nv_bfloat16>(q, q_stride, out, k_cache, v_cache, positions, token_seq,
+                                       block_table, max_blocks, tokens, heads, kv_heads, head_dim,
+                                       scale, window, stream);
+  return cudaErrorInvalidValue;
 }
