@@ -54,6 +54,7 @@ LIBRARIES = {
     "layer_norm": "layer_norm.cu",
     "latent": "latent.cu",
     "moe": "moe.cu",
+    "moe_tc": "moe_tc.cu",
     "norm_update": "norm_update.cu",
     "qk_prepare": "qk_prepare.cu",
     "recurrent_scan": "recurrent_scan.cu",

@@ -47,6 +47,7 @@ SIGNATURES = {
     "sakv_attention_mma": ("attention_mma",
                            [P, L, I, P, L, I, I, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I,
                             I, P, P, F, P, P, P, L, P, L, P, L, F, F, F, I, I, P, P, P]),
+    "sakv_moe_tc": ("moe_tc", [P, L, P, P, P, I, P, I, I, F, F, F, I, P]),
     "sakv_rms_update": ("norm_update", [P, P, P, F, P, P, F, I, P, I, I, I, F, P]),
     "sakv_rms_join": ("norm_update", [P, P, P, P, P, F, F, F, P, I, F, P, I, I, I, P]),
     "sakv_qk_prepare": ("qk_prepare", [P, L, I, I, I, P, P, I, F, P, P, I, P, P, P, I, P, P, P,
@@ -112,6 +113,7 @@ PLAIN_SIGNATURES = {
     "sakv_gemm_pair_resident": ("gemm_pair", []),
     "sakv_gemm_tc_splits": ("gemm_tc", [I, I]),
     "sakv_gemm_tc_max_clusters": ("gemm_tc", [I, I, I]),
+    "sakv_moe_tc_error": ("moe_tc", [P]),
     "sakv_gemm_tc_error": ("gemm_tc", [P]),
 }
 

@@ -28,6 +28,29 @@ _counts: dict = {}
 ROUTE_IN_ONE_BLOCK = 64
 
 
+#: fewer tiles of 128 rows x 256 weight rows than this: tiles of 32 x 64, so that more SMs pull weights
+FEW_TILES = 48
+
+
+def tc_takes(rows: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor | None) -> bool:
+    """Whether the tcgen05 kernel takes the grouped product: bfloat16 rows and weight rows of
+    multiples of 8 columns at multiples of 16 bytes; it is as fast as the general kernel from
+    one token on (us, general / this, the gated and the down product of 32 experts of 2048 -> 1024, 4
+    a token: 1 token 41 and 16 / 21 and 14, 64 tokens 76 and 43 / 66 and 39, 400 tokens 111 and 64
+    / 66 and 41, 3,001 tokens 530 and 324 / 104 and 76)."""
+    return (rows.dtype == torch.bfloat16 and w0.shape[2] % 8 == 0 and w0.shape[1] % 8 == 0
+            and w0.shape[0] <= 1024
+            and all(t is None or t.data_ptr() % 16 == 0 for t in (rows, w0, w1)))
+
+
+def few_tiles(rows: int, experts: int, n: int, dual: bool) -> bool:
+    """Whether the grouped product of `rows` rows takes the small tiles. Large / small, us: 32 large
+    tiles (1 token, 4 experts, 2 x 1024 x 2048) 25 / 21, 16 (64 tokens, 2 experts, 2 x 1024 x 1024) 19
+    / 14; 64 (16 tokens, 16 experts, 1024 x 1024) 19 / 21, 128 (the same, gated) 25 / 29."""
+    row_tiles = min(experts, rows) + rows // 128
+    return row_tiles * -(-n // (128 if dual else 256)) < FEW_TILES
+
+
 def tile_rows() -> int:
     return plain_function("sakv_moe_tile_rows")()
 
@@ -119,6 +142,11 @@ def grouped_product(rows: torch.Tensor, r: Routing, w0: torch.Tensor, w1: torch.
     n, k = w0.shape[1], w0.shape[2]
     out = torch.empty((rows.shape[0], n), dtype=rows.dtype if w1 is not None else torch.float32,
                       device=rows.device)
+    if tc_takes(rows, w0, w1):
+        call("sakv_moe_tc", ptr(rows), rows.shape[0], ptr(w0), ptr(w1), ptr(r.offsets), r.experts,
+             ptr(out), n, k, float(limit), float(alpha), float(plus),
+             int(few_tiles(r.tokens * r.top, r.experts, n, w1 is not None)))
+        return out
     call("sakv_moe_product", ptr(rows), dtype_code(rows.dtype), ptr(w0), ptr(w1), w0.stride(0),
          ptr(r.tile_expert), ptr(r.tile_row), ptr(r.offsets), ptr(r.n_tiles), r.max_tiles,
          ptr(out), n, k, int(w1 is not None), float(limit), float(alpha), float(plus))

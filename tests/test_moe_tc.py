@@ -1,0 +1,57 @@
+"""The grouped products of a mixture on tcgen05 (`csrc/moe_tc.cu`): the rules that choose it and its
+tiles (no GPU needed), and its results at the edges of tiles, with experts that nobody chose."""
+
+import pytest
+import torch
+
+from semantic_aware_adaptive_kv_cache_precision_b200.ops import mixture
+from semantic_aware_adaptive_kv_cache_precision_b200.ops._lib import call, ptr
+
+
+def test_the_rules_of_the_tiles():
+    def asks(dtype=torch.bfloat16, n=64, k=64, offset=0, two=True):
+        rows = torch.zeros(4 * k + 8, dtype=dtype)[offset:][:4 * k].view(4, k)
+        w = torch.zeros((3, n, k), dtype=dtype)
+        return mixture.tc_takes(rows, w, w if two else None)
+
+    assert asks() and asks(two=False) and asks(n=8, k=8) and asks(offset=8)
+    assert not asks(dtype=torch.float32) and not asks(n=12) and not asks(k=12) and not asks(offset=4)
+    assert mixture.few_tiles(4, 32, 1024, True) and not mixture.few_tiles(32, 16, 1024, True)
+    assert not mixture.few_tiles(6000, 2, 1024, False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("few", [True, False])
+@pytest.mark.parametrize("n,k", [(8, 8), (64, 72), (136, 200), (264, 1032)])
+@pytest.mark.parametrize("counts", [(1,), (0, 31, 32, 33, 0), (127, 0, 0, 128, 129, 1), (0, 0, 300)])
+def test_products_at_the_edges_of_tiles(counts, n, k, few):
+    """Against float64. A gated output is rounded to bfloat16 once (2^-8 of it) and its activation
+    taken with the hardware's exponential and division (some 2^-20); sums of k products are fp32."""
+    g = torch.Generator(device="cuda").manual_seed(n + k + len(counts))
+
+    def draw(*shape):
+        return torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)
+
+    total, experts = sum(counts), len(counts)
+    rows, gate, up = draw(total + 3, k), draw(experts, n, k), draw(experts, n, k)   # (3 rows of nobody)
+    offsets = torch.tensor([sum(counts[:i]) for i in range(experts + 1)], dtype=torch.int32, device="cuda")
+    plain = torch.full((total + 3, n), 7.0, dtype=torch.float32, device="cuda")
+    gated = torch.full((total + 3, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    limit, alpha, plus = 20.0, 1.25, 0.5
+    call("sakv_moe_tc", ptr(rows), total + 3, ptr(gate), None, ptr(offsets), experts, ptr(plain), n, k,
+         0.0, 0.0, 0.0, int(few))
+    call("sakv_moe_tc", ptr(rows), total + 3, ptr(gate), ptr(up), ptr(offsets), experts, ptr(gated), n, k,
+         limit, alpha, plus, int(few))
+    assert bool((plain[total:] == 7).all()) and bool((gated[total:] == 7).all())
+    for e in range(experts):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        if lo == hi:
+            continue
+        x = rows[lo:hi].double()
+        a, b = x @ gate[e].double().T, x @ up[e].double().T
+        size = x.abs() @ gate[e].double().abs().T
+        assert bool(((plain[lo:hi].double() - a).abs() <= 4 * k ** 0.5 * 2.0 ** -24 * size.max()).all())
+        c, d = a.clamp(max=limit), b.clamp(-limit, limit)
+        want = c * torch.sigmoid(alpha * c) * (d + plus)
+        off = (gated[lo:hi].double() - want).abs()
+        assert bool((off <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all())
