@@ -98,6 +98,56 @@ __global__ void causal_conv_kernel(const float* __restrict__ in, long long strid
   }
 }
 
+// The same for four taps over many tokens: a thread takes a channel of eight tokens in a row, whose
+// inputs are asked for together and each read once instead of once a tap (a sequence that begins
+// among them fills the window anew). Bound by memory: 3,400 tokens of 4,096 channels 113 -> 44 us.
+constexpr int kConvTokens = 8;
+template <typename W, typename C>
+__global__ void __launch_bounds__(256)
+causal_conv4_kernel(const float* __restrict__ in, long long stride, const W* __restrict__ w,
+                    const W* __restrict__ bias, const float* __restrict__ state,
+                    const int32_t* __restrict__ cu_seqlens, const int32_t* __restrict__ token_seq,
+                    const int32_t* __restrict__ slots, C* __restrict__ out, int tokens, int channels) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= channels) return;
+  float k[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) k[j] = widen(w[(long long)c * 4 + j]);
+  const float b0 = bias ? widen(bias[c]) : 0.f;
+  for (long long t0 = (long long)blockIdx.y * kConvTokens; t0 < tokens;
+       t0 += (long long)gridDim.y * kConvTokens) {
+    float x[kConvTokens];
+#pragma unroll
+    for (int q = 0; q < kConvTokens; ++q) x[q] = t0 + q < tokens ? in[(t0 + q) * stride + c] : 0.f;
+    float window[3] = {0.f, 0.f, 0.f};
+    int sequence = -1;
+#pragma unroll
+    for (int q = 0; q < kConvTokens; ++q) {
+      const long long t = t0 + q;
+      if (t >= tokens) break;
+      const int b = token_seq[t];
+      if (b != sequence) {
+        sequence = b;
+        const int i = static_cast<int>(t - cu_seqlens[b]);     // place in this step's part
+        const float* old = state + (long long)slots[b] * 3 * channels;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int back = 3 - j;
+          window[j] = back <= i ? in[(t - back) * stride + c] : old[(long long)(3 - (back - i)) * channels + c];
+        }
+      }
+      float acc = b0;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc = fmaf(window[j], k[j], acc);
+      acc = fmaf(x[q], k[3], acc);
+      out[t * channels + c] = narrow<C>(silu(acc));
+      window[0] = window[1];
+      window[1] = window[2];
+      window[2] = x[q];
+    }
+  }
+}
+
 // The state after the step: the sequence's last taps - 1 inputs. One thread a (sequence,
 // channel) reads what it needs of the old state before it writes.
 __global__ void conv_state_kernel(const float* __restrict__ in, long long stride,
@@ -702,6 +752,104 @@ __global__ void dual_carry_kernel(const float* __restrict__ a, float* __restrict
   if (keep_state) *home = s;
 }
 
+// Eight neighbouring elements as fp32, in 16-byte accesses (p at a multiple of 16 bytes).
+__device__ __forceinline__ void read8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void read8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void write8(float* p, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void write8(__nv_bfloat16* p, const float (&v)[8]) {
+  __nv_bfloat162 h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+}
+
+// `norm_gate_kernel` below for rows of up to 4,096 numbers, multiples of 8 everywhere: a row's numbers
+// stay in registers, eight or sixteen a thread, read and written 16 bytes at a time, gate and values
+// asked for together. `lanes`: how many neighbouring threads share a part (more than 32: the
+// whole block, for the whole row). Bound by memory: 4,128 rows of 2,048 with a gate 42 -> 17 us.
+template <int PER, typename W, typename C>
+__global__ void __launch_bounds__(256)
+norm_gate_vec_kernel(const float* __restrict__ y, const W* __restrict__ w,
+                     const float* __restrict__ gate, long long gate_stride, C* __restrict__ out,
+                     int width, int lanes, int gate_silu, int gate_first, float eps, float scale) {
+  __shared__ float scratch[33];
+  const long long t = blockIdx.x;
+  const int at = threadIdx.x * 8;                  // (of every run of blockDim.x * 8 numbers)
+  const int step = blockDim.x * 8;
+  float v[PER][8], g[PER][8];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int c = at + p * step;
+    if (c < width) {
+      read8(y + t * width + c, v[p]);
+      if (gate) read8(gate + t * gate_stride + c, g[p]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[p][i] = g[p][i] = 0.f;
+    }
+  }
+  if (gate) {
+#pragma unroll
+    for (int p = 0; p < PER; ++p)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        g[p][i] = (gate_silu ? g[p][i] : 1.f) / (1.f + expf(-g[p][i]));
+        if (gate_first) v[p][i] *= g[p][i];
+      }
+  }
+  float ss[PER], r[PER];
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    ss[p] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ss[p] = fmaf(v[p][i], v[p][i], ss[p]);
+  }
+  if (lanes > 32) {                                // the whole row
+    float all = ss[0];
+#pragma unroll
+    for (int p = 1; p < PER; ++p) all += ss[p];
+    const float one = 1.f / sqrtf(block_sum(all, scratch) / static_cast<float>(width) + eps);
+#pragma unroll
+    for (int p = 0; p < PER; ++p) r[p] = one;
+  } else {                                         // parts of `lanes` neighbouring threads' numbers
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      for (int o = 1; o < lanes; o <<= 1) ss[p] += __shfl_xor_sync(0xffffffffu, ss[p], o);
+      r[p] = 1.f / sqrtf(ss[p] / static_cast<float>(lanes * 8) + eps);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < PER; ++p) {
+    const int c = at + p * step;
+    if (c >= width) continue;
+    float k[8];
+    if (w) read8(w + c, k);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float x = v[p][i] * r[p];
+      if (w) x *= k[i];
+      if (gate && !gate_first) x *= g[p][i];
+      v[p][i] = x * scale;
+    }
+    write8(out + t * width + c, v[p]);
+  }
+}
+
 // out[t] = y[t] / sqrt(mean(y[t]^2) + eps) * w * sigmoid(gate[t]) * scale. A block a token.
 // `group` == width: the mean over the whole row (all heads' outputs together); smaller: over
 // each run of `group` numbers (a head's outputs), a warp a run. `w` null: no weight.
@@ -773,10 +921,18 @@ SAKV_EXPORT int sakv_causal_conv(const float* in, long long stride, const void* 
   if (tokens == 0) return 0;
   const long long count = (long long)tokens * channels;
   const dim3 grid(grid_for(count, 256)), block(256);
+  const long long runs = (tokens + kConvTokens - 1) / kConvTokens;
+  const dim3 grid4((unsigned)((channels + 255) / 256), (unsigned)(runs < 65535 ? runs : 65535));
 #define SAKV_CONV(W, C)                                                                          \
+  do {                                                                                           \
+  if (taps == 4)                                                                                 \
+    return launch_ordered(causal_conv4_kernel<W, C>, grid4, block, 0, stream, in, stride,  \
+                             (const W*)w, (const W*)bias, state, cu_seqlens, token_seq, slots,   \
+                             (C*)out, tokens, channels);                                         \
   return launch_ordered(causal_conv_kernel<W, C>, grid, block, 0, stream, in, stride,            \
                         (const W*)w, (const W*)bias, state, cu_seqlens, token_seq, slots,        \
-                        (C*)out, channels, taps, count)
+                        (C*)out, channels, taps, count);  \
+  } while (0)
   if (w_dtype == SAKV_F32 && out_dtype == SAKV_F32) SAKV_CONV(float, float);
   if (w_dtype == SAKV_BF16 && out_dtype == SAKV_BF16) SAKV_CONV(__nv_bfloat16, __nv_bfloat16);
   if (w_dtype == SAKV_BF16 && out_dtype == SAKV_F32) SAKV_CONV(__nv_bfloat16, float);
@@ -1050,11 +1206,28 @@ SAKV_EXPORT int sakv_norm_gate(const float* y, const void* w, int w_dtype, const
       (gate_first && (gate == nullptr || width > 12000)))
     return cudaErrorInvalidValue;
   if (tokens == 0) return 0;
+  // 16-byte pieces everywhere, whole warps, and parts that a power of two of lanes holds, or one part
+  const int part_lanes = group == width ? 64 : group % 8 == 0 ? group / 8 : 0;
+  const int vec_threads = width <= 2048 ? (width / 8 + 31) / 32 * 32 : 256;
+  const bool vec = width % 8 == 0 && width <= 4096 && part_lanes > 0 &&
+                   (part_lanes & (part_lanes - 1)) == 0 && (part_lanes <= 32 || group == width) &&
+                   (gate == nullptr || gate_stride % 4 == 0) &&
+                   !(((uintptr_t)y | (uintptr_t)w | (uintptr_t)gate | (uintptr_t)out) & 15);
 #define SAKV_NG(W, C)                                                                            \
+  do {                                                                                           \
+    if (vec && width <= 2048)                                                                    \
+      return launch_ordered(norm_gate_vec_kernel<1, W, C>, dim3(tokens), dim3(vec_threads), 0, \
+                               stream, y, (const W*)w, gate, gate_stride, (C*)out, width,     \
+                               part_lanes, gate_silu, gate_first, eps, scale);                   \
+    if (vec)                                                                                     \
+      return launch_ordered(norm_gate_vec_kernel<2, W, C>, dim3(tokens), dim3(vec_threads), 0, \
+                               stream, y, (const W*)w, gate, gate_stride, (C*)out, width,     \
+                               part_lanes, gate_silu, gate_first, eps, scale);                   \
   return launch_ordered(norm_gate_kernel<W, C>, dim3(tokens), dim3(256),                         \
                         gate_first ? (size_t)width * sizeof(float) : 0, stream, y,               \
                         (const W*)w, gate, gate_stride, (C*)out, width, group, gate_silu,        \
-                        gate_first, eps, scale)
+                        gate_first, eps, scale);  \
+  } while (0)
   if (w_dtype == SAKV_F32 && out_dtype == SAKV_F32) SAKV_NG(float, float);
   if (w_dtype == SAKV_BF16 && out_dtype == SAKV_BF16) SAKV_NG(__nv_bfloat16, __nv_bfloat16);
   if (w_dtype == SAKV_BF16 && out_dtype == SAKV_F32) SAKV_NG(__nv_bfloat16, float);
