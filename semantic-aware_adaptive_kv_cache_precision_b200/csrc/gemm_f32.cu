@@ -24,8 +24,8 @@ __device__ __forceinline__ void copy_async4(uint32_t dst, const float* src, bool
 // likewise), K in steps of BK through a ring of STAGES copied with cp.async. The order of a sum makes
 // a chain of K dependent multiply-adds, some 4 cycles each, that no split may shorten: what is left to
 // win is that nothing else stands in it (four of them a pair of 16-byte reads, the copies STAGES - 1
-// steps ahead, the first weights already under way while the kernel before this one finishes) and
-// that there are enough tiles for every SM (`sakv_gemm_f32`). `wide`: rows that begin at multiples of 16 bytes.
+// steps ahead) and that there are enough tiles for every SM (`sakv_gemm_f32`). `wide`: rows that begin at
+// multiples of 16 bytes.
 template <int BM, int BN, int TM, int TN, int BK, int STAGES>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_kernel(const float* __restrict__ A, long long lda, const float* __restrict__ W,
@@ -55,16 +55,16 @@ gemm_f32_kernel(const float* __restrict__ A, long long lda, const float* __restr
     }
   };
   auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
-  let_next_kernel_start();
-  for (int s = 0; s < STAGES - 1 && s < steps; ++s) fill(s, W, K, n0, N, BN, BM);
-  wait_for_previous_kernel();
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-  for (int s = 0; s < STAGES - 1; ++s) {       // (the first group holds all the early weights)
-    if (s < steps) fill(s, A, lda, m0, M, BM, 0);
+  for (int s = 0; s < STAGES - 1; ++s) {
+    if (s < steps) {
+      fill(s, W, K, n0, N, BN, BM);
+      fill(s, A, lda, m0, M, BM, 0);
+    }
     commit();
   }
   for (int step = 0; step < steps; ++step) {
@@ -139,7 +139,7 @@ int launch(const float* A, long long lda, const float* W, const float* bias, flo
   const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return cudaErrorInvalidValue;
   const int wide = K % 4 == 0 && lda % 4 == 0 && !(((uintptr_t)A | (uintptr_t)W) & 15);
-  return launch_overlapped(kernel, grid, dim3((BM / TM) * (BN / TN)), kSmem, stream, 1, A, lda, W, bias, C,
+  return launch_ordered(kernel, grid, dim3((BM / TM) * (BN / TN)), kSmem, stream, A, lda, W, bias, C,
                            ldc, M, N, K, accumulate, wide);
 }
 
