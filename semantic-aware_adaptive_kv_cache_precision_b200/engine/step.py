@@ -60,16 +60,41 @@ class StepStager:
         self.turn = 0
         self.last_bytes = 0
         self.generation = 0
+        self._layouts: dict = {}             # (of this generation) see `_layout`
 
     def _ensure(self, count: int) -> None:
         if count <= self.capacity:
             return
         self.capacity = max(1 << 18, 2 * count)
         self.generation += 1                 # device addresses change: captured graphs are stale
+        self._layouts = {}
         self.hosts = [torch.empty(self.capacity, dtype=torch.int32, pin_memory=True)
                       for _ in range(2)]
         self.dev = torch.empty(self.capacity, dtype=torch.int32, device=self.device)
         self.copied = [None, None]
+
+    def _layout(self, T: int, B: int, W: int, shapes: tuple):
+        """(offset of every field, ints in all, the fields' views of the device buffer) for steps of
+        T tokens, B sequences, W wanted rows and block lists of `shapes`: steps of one shape follow
+        one another by the hundred in a decode loop, and making a dozen views takes as long as
+        launching the step."""
+        hit = self._layouts.get((T, B, W, shapes))
+        if hit is not None:
+            return hit
+        fields = [("token_ids", T), ("positions", T), ("token_seq", T), ("cu_seqlens", B + 1),
+                  ("seq_lens", B), ("slots", B), ("want", W)]
+        fields += [(f"table{g}", s[0] * s[1]) for g, s in enumerate(shapes)]
+        offsets, total = {}, 0
+        for name, n in fields:
+            offsets[name] = total
+            total += -(-max(n, 1) // 4) * 4          # 16-byte aligned fields
+        self._ensure(total)
+        views = {name: self.dev[offsets[name]:offsets[name] + n] for name, n in fields}
+        tables = [views.pop(f"table{g}").view(s) for g, s in enumerate(shapes)]
+        if len(self._layouts) >= 64:
+            self._layouts.clear()
+        hit = self._layouts[(T, B, W, shapes)] = (offsets, total, views, tables)
+        return hit
 
     def build(self, slots: list, new_tokens: list, starts: list, want_rows, tables: list,
               device_tokens: torch.Tensor | None = None) -> StepContext:
@@ -91,14 +116,7 @@ class StepStager:
         # 512 steps and its captured graph can be replayed)
         width = -(-max(1, -(-max(ends, default=1) // BLOCK)) // 8) * 8
         tables = [np.ascontiguousarray(t[:, :min(width, t.shape[1])]) for t in tables]
-        fields = [("token_ids", T), ("positions", T), ("token_seq", T), ("cu_seqlens", B + 1),
-                  ("seq_lens", B), ("slots", B), ("want", W)]
-        fields += [(f"table{g}", t.size) for g, t in enumerate(tables)]
-        offsets, total = {}, 0
-        for name, n in fields:
-            offsets[name] = total
-            total += -(-max(n, 1) // 4) * 4          # 16-byte aligned fields
-        self._ensure(total)
+        offsets, total, views, dev_tables = self._layout(T, B, W, tuple(t.shape for t in tables))
         turn = self.turn = 1 - self.turn
         if self.copied[turn] is not None:
             self.copied[turn].synchronize()         # its last copy has left this host buffer
@@ -108,16 +126,23 @@ class StepStager:
             values = np.asarray(values, dtype=np.int32).reshape(-1)
             host[offsets[name]:offsets[name] + values.size] = values
 
-        cu = np.zeros(B + 1, dtype=np.int64)
-        np.cumsum(counts, out=cu[1:])
-        put("token_ids", np.zeros(T) if device_tokens is not None else
-            np.concatenate([np.asarray(t, dtype=np.int64) for t in new_tokens]) if T
-            else np.zeros(0))
-        put("positions", np.concatenate([np.arange(s, s + c) for s, c in zip(starts, counts)])
-            if T else np.zeros(0))
-        put("token_seq", np.repeat(np.arange(B), counts))
-        put("cu_seqlens", cu)
-        put("seq_lens", [s + c for s, c in zip(starts, counts)])
+        if device_tokens is not None or T == 0:
+            host[offsets["token_ids"]:offsets["token_ids"] + T] = 0
+        else:
+            put("token_ids", np.concatenate([np.asarray(t, dtype=np.int64) for t in new_tokens]))
+        if T == B and B and min(counts) == 1:       # a token a sequence
+            order = np.arange(B + 1, dtype=np.int32)
+            put("positions", starts)
+            put("token_seq", order[:B])
+            put("cu_seqlens", order)
+        else:
+            cu = np.zeros(B + 1, dtype=np.int64)
+            np.cumsum(counts, out=cu[1:])
+            put("positions", np.concatenate([np.arange(s, s + c) for s, c in zip(starts, counts)])
+                if T else np.zeros(0))
+            put("token_seq", np.repeat(np.arange(B), counts))
+            put("cu_seqlens", cu)
+        put("seq_lens", ends)
         put("slots", slots)
         put("want", want_rows)
         for g, t in enumerate(tables):
@@ -127,20 +152,13 @@ class StepStager:
         first = offsets["positions"] if in_place else 0      # (the token field comes first)
         self.last_bytes = 4 * (total - first)
         self.dev[first:total].copy_(self.hosts[turn][first:total], non_blocking=True)
-        self.copied[turn] = torch.cuda.Event()
+        if self.copied[turn] is None:
+            self.copied[turn] = torch.cuda.Event()
         self.copied[turn].record()
         if device_tokens is not None and not in_place:
-            self.dev[offsets["token_ids"]:offsets["token_ids"] + T].copy_(device_tokens)
-
-        def view(name, n):
-            return self.dev[offsets[name]:offsets[name] + n]
-
-        dev_tables = [view(f"table{g}", t.size).view(t.shape) for g, t in enumerate(tables)]
+            views["token_ids"].copy_(device_tokens)
         return StepContext(
-            tokens=T, sequences=B, token_ids=view("token_ids", T), positions=view("positions", T),
-            token_seq=view("token_seq", T), cu_seqlens=view("cu_seqlens", B + 1),
-            seq_lens=view("seq_lens", B), slots=view("slots", B), want=view("want", W),
-            tables=dev_tables, new_counts=counts, starts=list(starts), host_slots=list(slots),
+            tokens=T, sequences=B, **views, tables=list(dev_tables), new_counts=counts, starts=list(starts), host_slots=list(slots),
             max_position=max(ends) - 1 if ends else 0, max_new=max(counts, default=0),
             max_len=max(ends, default=0), is_decode=all(c == 1 for c in counts),
             max_len_bound=min(width, max((t.shape[1] for t in tables), default=width)) * BLOCK)
