@@ -8,7 +8,7 @@
 // softmax weights, running maxima and sums are fp32. A weight p in [0, 1] enters the second
 // product as hi + lo, two bfloat16 numbers that keep 16 to 17 of its bits, so every value tile is
 // multiplied twice; against 64 bits the outputs (bfloat16) are as far off as with fp32 weights
-// (2.3e-3 relative, all of it the output's own rounding).
+// (1.6e-3 relative, all of it the output's own rounding).
 //
 // A block takes the rows of one key/value head and map: ROWS = 16 WR rows are tokens x query heads
 // of the group, so a group's heads share each tile of keys. WR warps go along the rows and WC
