@@ -62,6 +62,7 @@ struct MmaAttention {
   const __nv_bfloat16* map_gate;   // two maps: + t * map_gate_stride + h * DV + c (null: none)
   long long map_gate_stride;
   float out_scale, lambda, eps;
+  int ordered;                 // in plain stream order: see `launch_shape`
   // the split of the work
   int heads_per_tile, tokens_per_tile, head_tiles;
 };
@@ -168,7 +169,7 @@ attention_mma_kernel(const MmaAttention a) {
   const uint32_t stage0 = base + S::kQBytes;
   const uint32_t p_base = stage0 + STAGES * S::kStageBytes;
 
-  if (a.sums != nullptr) let_next_kernel_start();      // (the fold waits for this kernel's end)
+  if (a.sums != nullptr && !a.ordered) let_next_kernel_start();   // (the fold waits for this kernel's end)
   wait_for_previous_kernel();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wr = warp / WC, wc = warp % WC;
@@ -618,11 +619,20 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
   const long long tiles = (a.tokens + a.tokens_per_tile - 1) / a.tokens_per_tile;
   const long long across = (long long)a.kv_heads * a.maps * a.head_tiles;
   if (across > 65535) return cudaErrorInvalidValue;
-  const int code = launch_overlapped(kernel, dim3((unsigned)tiles, (unsigned)across, (unsigned)a.key_splits),
-                                     dim3(S::kThreads), S::kBytes, stream, 1, a);
+  const dim3 grid((unsigned)tiles, (unsigned)across, (unsigned)a.key_splits), block(S::kThreads);
+  const dim3 fold_grid((unsigned)a.tokens, (unsigned)a.heads), fold_block(DV / 4);
+  // `ordered`: this attention stands between a library's products and kernels that read fresh
+  // indices. An overlapped launch of the kernels there has once ended in a memory fault whose cause
+  // is not known, so both kernels begin when the one before them has ended and neither lets its
+  // successor start early.
+  if (a.ordered) {
+    const int code = launch_ordered(kernel, grid, block, S::kBytes, stream, a);
+    if (code != 0 || a.sums == nullptr) return code;
+    return launch_ordered(attention_fold_kernel<DV>, fold_grid, fold_block, 0, stream, a);
+  }
+  const int code = launch_overlapped(kernel, grid, block, S::kBytes, stream, 1, a);
   if (code != 0 || a.sums == nullptr) return code;
-  return launch_overlapped(attention_fold_kernel<DV>, dim3((unsigned)a.tokens, (unsigned)a.heads),
-                           dim3(DV / 4), 0, stream, 1, a);
+  return launch_overlapped(attention_fold_kernel<DV>, fold_grid, fold_block, 0, stream, 1, a);
 }
 
 }  // namespace
@@ -632,7 +642,7 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
 // of two maps' gate element by element (first head's first column; rows *_stride apart). decode 0:
 // blocks of 64 rows of a prompt; 1: a block a token, key/value head, map and split. sums, stats: fp32
 // scratch of key_splits * tokens * heads * maps * (vdim, 2) numbers, needed with two maps or several
-// splits, else null. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
+// splits, else null. ordered 1: both kernels in plain stream order. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
 // = (64, 64), (128, 128), (128, 256) and, with v_cache null, (576, 512); rows that do not begin at
 // multiples of 16 bytes.
 SAKV_EXPORT int sakv_attention_mma(
@@ -644,7 +654,7 @@ SAKV_EXPORT int sakv_attention_mma(
     const float* linear, const float* sink, const void* gate, long long gate_stride,
     const float* elem_gate, long long elem_stride, const void* map_gate, long long map_gate_stride,
     float out_scale, float lambda, float eps, int decode, int key_splits, float* sums, float* stats,
-    cudaStream_t stream) {
+    int ordered, cudaStream_t stream) {
   if (tokens < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || (maps != 1 && maps != 2) ||
       window < 0 || chunk < 0 || keep < 0 || (window > 0 && chunk > 0) || softcap < 0.f ||
       max_blocks <= 0 || key_splits < 1 || key_splits > 64 || (!decode && key_splits > 1) ||
@@ -701,6 +711,7 @@ SAKV_EXPORT int sakv_attention_mma(
   a.out_scale = out_scale;
   a.lambda = lambda;
   a.eps = eps;
+  a.ordered = ordered;
   const bool in_key = v_cache == nullptr;
   if (in_key && dim == 576 && vdim == 512 && maps == 1)
     return decode ? launch_shape<576, 512, true, 1, 8, 64, 2>(a, true, stream)

@@ -263,7 +263,7 @@ def distance_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
             qkv, dim, k_cache, v_cache, positions, token_seq, block_table, heads, dim, vdim, scale,
             window=window, slope=slope, rate=rate,
             head_gate=None if gate_off is None else qkv[:, gate_off:gate_off + heads],
-            decode=splits > 1, key_splits=splits)
+            decode=splits > 1, key_splits=splits, ordered=False)
     out = torch.empty((tokens, heads * vdim), dtype=qkv.dtype, device=qkv.device)
     call("sakv_distance_attention", ptr(qkv), dtype_code(qkv.dtype), qkv.stride(0),
          -1 if gate_off is None else int(gate_off), ptr(out), ptr(k_cache), ptr(v_cache),

@@ -32,9 +32,11 @@ def takes(q: torch.Tensor, head_stride: int, k_cache: torch.Tensor, v_cache, dim
 def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_table, heads, dim, vdim,
               scale, *, maps=1, q2=None, q_split=0, window=None, chunk=None, keep_first=0, slope=None,
               rate=None, softcap=None, linear=None, sink=None, head_gate=None, elem_gate=None,
-              map_gate_off=None, lam=0.0, out_scale=1.0, eps=0.0, decode=False, key_splits=1):
+              map_gate_off=None, lam=0.0, out_scale=1.0, eps=0.0, decode=False, key_splits=1,
+              ordered=True):
     """The arguments as `ops.cached_attention` and `ops.distance_attention` have checked them.
-    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt."""
+    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt. `ordered`: the kernels begin when the one before them has
+    ended (False: overlapped with it, for a caller whose neighbours are this library's own kernels)."""
     tokens = q.shape[0]
     out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
     if not decode:
@@ -55,7 +57,8 @@ def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_tabl
          ptr(linear), ptr(sink), ptr(head_gate), 0 if head_gate is None else head_gate.stride(0),
          ptr(elem_gate), 0 if elem_gate is None else elem_gate.stride(0),
          None if map_gate_off is None else q.data_ptr() + 2 * map_gate_off, q.stride(0),
-         float(out_scale), float(lam), float(eps), int(decode), int(key_splits), ptr(sums), ptr(stats))
+         float(out_scale), float(lam), float(eps), int(decode), int(key_splits), ptr(sums), ptr(stats),
+         int(ordered))
     if sums is not None and tokens:
         _lib.launches += 1          # the call launched the fold kernel too
     return out

@@ -32,6 +32,31 @@ def test_only_bfloat16_rows_at_multiples_of_16_bytes_go_to_the_tensor_cores():
     assert not asks(head=132) and not asks(k_row=132) and not asks(dim=128, vdim=128, latent=True)
 
 
+def test_attention_beside_library_products_is_launched_in_plain_order(monkeypatch):
+    """Only the attention with the logarithmic penalty, whose neighbours are this library's own
+    kernels, may be overlapped with them."""
+    launched = []
+    monkeypatch.setattr(attention_mma, "call", lambda name, *args: launched.append((name, args[-1])))
+    monkeypatch.setattr(ops, "require_cuda", lambda *tensors: None)
+    pos, table = torch.zeros(3, dtype=torch.int32), torch.zeros((1, 1), dtype=torch.int32)
+
+    def cache(width):
+        return torch.zeros((1, 1, 64, width), dtype=BF)
+
+    for form in ({}, {"heads_first": True, "key_splits": 2}):
+        ops.cached_attention(torch.zeros((3, 4, 576), dtype=BF), cache(576), None, pos, pos, table, 4, 576, 512,
+                             1.0, **form)
+        ops.cached_attention(torch.zeros((3, 4, 128), dtype=BF), cache(256), cache(256), pos, pos, table, 2, 128,
+                             256, 1.0, maps=2, **form)
+        ops.cached_attention(torch.zeros((3, 4, 128), dtype=BF), cache(128), cache(128), pos, pos, table, 4, 128,
+                             128, 1.0, **form)
+    assert launched == [("sakv_attention_mma", 1)] * 6
+    slope = torch.zeros(4)
+    ops.distance_attention(torch.zeros((3, 1024), dtype=BF), cache(128), cache(128), pos, pos, table, 4, 1.0, None,
+                           slope, slope)
+    assert launched[6:] == [("sakv_attention_mma", 0)]
+
+
 def case(seed, lens, heads, kv_heads, dim, vdim, maps=1, latent=False):
     """Sequences of `lens` tokens in a cache whose unused positions hold NaN."""
     g = torch.Generator(device="cuda").manual_seed(seed)
