@@ -5,10 +5,9 @@
 // first tokens, chunks, sinks, gates, two maps a head), which takes every other size and type.
 //
 // Precision: queries, keys and values are bfloat16 and their products exact in fp32; scores,
-// softmax weights, running maxima and sums are fp32. A weight p in [0, 1] enters the second
-// product as hi + lo, two bfloat16 numbers that keep 16 to 17 of its bits, so every value tile is
-// multiplied twice; against 64 bits the outputs (bfloat16) are as far off as with fp32 weights
-// (1.6e-3 relative, all of it the output's own rounding).
+// softmax weights, running maxima and sums are fp32, worked out with the functions of the general
+// kernel (expf, log1pf). A weight enters the second product as the sum of three bfloat16 numbers,
+// which hold all 24 of its bits, so every value tile is multiplied three times.
 //
 // A block takes the rows of one key/value head and map: ROWS = 16 WR rows are tokens x query heads
 // of the group, so a group's heads share each tile of keys. WR warps go along the rows and WC
@@ -53,7 +52,7 @@ struct MmaAttention {
   // the outputs: directly (one map, one split), or through `sums` and a second kernel
   __nv_bfloat16* out;          // [tokens, heads * DV]
   float* sums;                 // [key_splits, tokens, heads * maps, DV], not yet divided
-  float* stats;                // [key_splits, tokens, heads * maps, 2]: maximum (base 2), sum
+  float* stats;                // [key_splits, tokens, heads * maps, 2]: maximum, sum
   const float* sink;
   const __nv_bfloat16* gate;   // a gate a head: + t * gate_stride + h (null: none)
   long long gate_stride;
@@ -68,8 +67,6 @@ struct MmaAttention {
 };
 
 namespace {
-
-constexpr float kLog2e = 1.4426950408889634f;
 
 __device__ __forceinline__ int first_visible(int pos, int window, int chunk) {
   if (chunk > 0) return pos - pos % chunk;
@@ -90,17 +87,13 @@ __device__ __forceinline__ void copies_wait() {
 
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= FLT_MAX; }
 
-// A score in units of log 2: soft cap, penalty, base change.
-__device__ __forceinline__ float base2_score(const MmaAttention& a, float s, float dist, float sl,
-                                             float rt) {
-  if (a.softcap > 0.f) {     // cap * tanh(s / cap) as cap * (1 - 2 / (e^(2z) + 1))
-    const float z = __fdividef(s * a.scale, a.softcap);
-    s = a.softcap * (1.f - __fdividef(2.f, __expf(2.f * z) + 1.f)) * kLog2e;
-  } else {
-    s *= a.scale * kLog2e;
-  }
-  if (a.slope != nullptr) s -= sl * __log2f(fmaf(rt, dist, 1.f));
-  else if (a.linear != nullptr) s = fmaf(-sl * kLog2e, dist, s);
+// A score from a product: scale, soft cap (as the general kernel takes it of 16-bit keys), penalty.
+__device__ __forceinline__ float score_of(const MmaAttention& a, float s, float dist, float sl, float rt) {
+  s *= a.scale;
+  if (a.softcap > 0.f)       // cap * tanh(s / cap) as cap * (1 - 2 / (e^(2z) + 1))
+    s = a.softcap * (1.f - __fdividef(2.f, __expf(2.f * __fdividef(s, a.softcap)) + 1.f));
+  if (a.slope != nullptr) s -= sl * log1pf(rt * dist);
+  else if (a.linear != nullptr) s = fmaf(-sl, dist, s);
   return s;
 }
 
@@ -110,10 +103,10 @@ __device__ __forceinline__ void write_row(const MmaAttention& a, const float* ac
                                           int t, int h, int lane) {
   float corr = 1.f;
   if (a.sink != nullptr) {       // one more logit in the denominator
-    const float s = a.sink[h] * kLog2e;
+    const float s = a.sink[h];
     const float top = fmaxf(m, s);
-    corr = mma::exp2_fast(m - top);
-    l = fmaf(l, corr, mma::exp2_fast(s - top));
+    corr = expf(m - top);
+    l = fmaf(l, corr, expf(s - top));
   }
   float f = a.out_scale * corr / l;
   if (a.gate != nullptr)
@@ -140,7 +133,7 @@ struct Shape {
   static constexpr int kQBytes = kRows * kQStride * 2;
   static constexpr int kKBytes = KT * kQStride * 2;
   static constexpr int kStageBytes = kKBytes + (VINK ? 0 : KT * kVStride * 2);
-  static constexpr int kPBytes = WC > 1 ? 2 * kRows * kPStride * 2 : 0;
+  static constexpr int kPBytes = WC > 1 ? 3 * kRows * kPStride * 2 : 0;   // (a weight's three pieces)
   static constexpr int kSmall = (2 * WC + 2) * kRows * 4;        // maxima, sums, a row's m and l
   static constexpr int kMain = kQBytes + STAGES * kStageBytes + kPBytes;
   static constexpr int kOut = kRows * kOStride * 4;
@@ -330,7 +323,7 @@ attention_mma_kernel(const MmaAttention a) {
         for (int e = 0; e < 4; ++e) {
           const int r = e >> 1;
           const int j = j0 + (wc * NT + n) * 8 + (lane & 3) * 2 + (e & 1);
-          float v = base2_score(a, s[n][e], (float)(rpos[r] - j), rsl[r], rrt[r]);
+          float v = score_of(a, s[n][e], (float)(rpos[r] - j), rsl[r], rrt[r]);
           if (!all_seen)
             v = rt[r] >= s0 && rt[r] < s1 && j <= rpos[r] && (j >= rfirst[r] || j < a.keep)
                     ? v : -INFINITY;
@@ -361,7 +354,7 @@ attention_mma_kernel(const MmaAttention a) {
       for (int r = 0; r < 2; ++r) {
         const float next = fmaxf(m[r], top[r]);
         shift[r] = next == -INFINITY ? 0.f : next;     // (nothing seen yet: weights of 0)
-        corr[r] = mma::exp2_fast(m[r] - shift[r]);
+        corr[r] = expf(m[r] - shift[r]);
         m[r] = next;
         l[r] *= corr[r];
       }
@@ -369,7 +362,7 @@ attention_mma_kernel(const MmaAttention a) {
       for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p = mma::exp2_fast(s[n][e] - shift[e >> 1]);
+          const float p = expf(s[n][e] - shift[e >> 1]);
           s[n][e] = p;
           l[e >> 1] += p;
         }
@@ -381,23 +374,30 @@ attention_mma_kernel(const MmaAttention a) {
         }
       }
 
-      // the weights as hi + lo, times the values
-      auto halves = [](float x, float y, uint32_t& hi2, uint32_t& lo2) {
-        hi2 = mma::pack_bf16(x, y);
-        const float2 back = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&hi2));
-        lo2 = mma::pack_bf16(x - back.x, y - back.y);
+      // the weights as sums of three pieces (what a piece leaves of a number is exact), times the
+      // values
+      auto pieces = [](float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
+        auto take = [&] {
+          uint32_t two = mma::pack_bf16(x, y);
+          const float2 back = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&two));
+          x -= back.x;
+          y -= back.y;
+          return two;
+        };
+        first = take();
+        second = take();
+        third = mma::pack_bf16(x, y);
       };
+      constexpr int kPiece = S::kRows * S::kPStride;        // (elements between two pieces)
       if constexpr (WC > 1) {
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            uint32_t hi2, lo2;
-            halves(s[n][2 * r], s[n][2 * r + 1], hi2, lo2);
             const int at = (my_row + 8 * r) * S::kPStride + (wc * NT + n) * 8 + (lane & 3) * 2;
-            uint32_t* ph = reinterpret_cast<uint32_t*>(smem + S::kQBytes + STAGES * S::kStageBytes);
-            ph[at / 2] = hi2;
-            ph[(S::kRows * S::kPStride + at) / 2] = lo2;
+            uint32_t* ps = reinterpret_cast<uint32_t*>(smem + S::kQBytes + STAGES * S::kStageBytes);
+            pieces(s[n][2 * r], s[n][2 * r + 1], ps[at / 2], ps[(kPiece + at) / 2],
+                   ps[(2 * kPiece + at) / 2]);
           }
         }
         asm volatile("bar.sync %0, %1;" ::"r"(1 + wr), "n"(32 * WC) : "memory");
@@ -406,28 +406,30 @@ attention_mma_kernel(const MmaAttention a) {
                                   wc * NV * 8 + (lane >> 4) * 8) * 2;
 #pragma unroll
       for (int kk = 0; kk < KT / 16; ++kk) {
-        uint32_t ph[4], pl[4];
+        uint32_t p[3][4];
         if constexpr (WC > 1) {
           const uint32_t at =
               p_base + ((wr * 16 + (lane & 15)) * S::kPStride + kk * 16 + (lane >> 4) * 8) * 2;
-          mma::ldmatrix_x4(at, ph[0], ph[1], ph[2], ph[3]);
-          mma::ldmatrix_x4(at + S::kRows * S::kPStride * 2, pl[0], pl[1], pl[2], pl[3]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            mma::ldmatrix_x4(at + i * kPiece * 2, p[i][0], p[i][1], p[i][2], p[i][3]);
         } else {
           constexpr int kLast = NT > 1 ? NT - 1 : 0;
           const int n0 = 2 * kk, n1 = 2 * kk + 1 <= kLast ? 2 * kk + 1 : kLast;
-          halves(s[n0][0], s[n0][1], ph[0], pl[0]);
-          halves(s[n0][2], s[n0][3], ph[1], pl[1]);
-          halves(s[n1][0], s[n1][1], ph[2], pl[2]);
-          halves(s[n1][2], s[n1][3], ph[3], pl[3]);
+          pieces(s[n0][0], s[n0][1], p[0][0], p[1][0], p[2][0]);
+          pieces(s[n0][2], s[n0][3], p[0][1], p[1][1], p[2][1]);
+          pieces(s[n1][0], s[n1][1], p[0][2], p[1][2], p[2][2]);
+          pieces(s[n1][2], s[n1][3], p[0][3], p[1][3], p[2][3]);
         }
 #pragma unroll
         for (int n = 0; n < NV; n += 2) {
           uint32_t b[4];
           mma::ldmatrix_x4_trans(v_at + (kk * 16 * S::kVStride + n * 8) * 2, b[0], b[1], b[2], b[3]);
-          mma::bf16_16816(acc[n], ph, b[0], b[1]);
-          mma::bf16_16816(acc[n + 1], ph, b[2], b[3]);
-          mma::bf16_16816(acc[n], pl, b[0], b[1]);
-          mma::bf16_16816(acc[n + 1], pl, b[2], b[3]);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            mma::bf16_16816(acc[n], p[i], b[0], b[1]);
+            mma::bf16_16816(acc[n + 1], p[i], b[2], b[3]);
+          }
         }
       }
     }
@@ -472,7 +474,7 @@ attention_mma_kernel(const MmaAttention a) {
     float* acc_row = os + row * S::kOStride;
     if (any_bad) {
       // An infinity or a NaN among the values: a weight of 0 times it spoils rows that do not
-      // see it, and hi + lo times it is not p times it. Such a block walks its keys one by one.
+      // see it, and a weight's pieces times it are not the weight times it. Such a block walks its keys one by one.
       const int pos = a.positions[t], first = first_visible(pos, a.window, a.chunk);
       const int32_t* table = a.block_table + (long long)a.token_seq[t] * a.max_blocks;
       // the same share of the run's tiles as above
@@ -507,9 +509,9 @@ attention_mma_kernel(const MmaAttention a) {
                     : a.q2[(long long)t * a.q2_stride + (long long)vh * a.q2_head_stride + e - a.q_split];
             part = fmaf(widen(qv), widen(a.k_cache[at * a.k_row + map * DK + e]), part);
           }
-          const float sc = base2_score(a, warp_sum(part), (float)(pos - j), sl, rate);
+          const float sc = score_of(a, warp_sum(part), (float)(pos - j), sl, rate);
           const float next = fmaxf(top, sc);
-          const float f = exp2f(top - next), p = exp2f(sc - next);
+          const float f = expf(top - next), p = expf(sc - next);
           sum = fmaf(sum, f, p);
           const __nv_bfloat16* vr = VINK ? a.k_cache + at * a.k_row : a.v_cache + at * a.v_row;
           for (int c = lane; c < DV; c += 32) acc_row[c] = fmaf(acc_row[c], f, p * widen(vr[c]));
@@ -550,15 +552,15 @@ __global__ void __launch_bounds__(DV / 4) attention_fold_kernel(const MmaAttenti
     const long long at = (long long)t * vheads + h * a.maps + map, step = a.tokens * vheads;
     float top = -INFINITY;
     for (int s = 0; s < a.key_splits; ++s) top = fmaxf(top, a.stats[(at + s * step) * 2]);
-    if (a.sink != nullptr) top = fmaxf(top, a.sink[h] * kLog2e);
-    float total = a.sink != nullptr ? mma::exp2_fast(a.sink[h] * kLog2e - top) : 0.f;
+    if (a.sink != nullptr) top = fmaxf(top, a.sink[h]);
+    float total = a.sink != nullptr ? expf(a.sink[h] - top) : 0.f;
     float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
     for (int s = 0; s < a.key_splits; ++s) {
       const float2 ml = *reinterpret_cast<const float2*>(a.stats + (at + s * step) * 2);
       const float4 v = *reinterpret_cast<const float4*>(a.sums + (at + s * step) * DV + c);
       if (ml.x == -INFINITY && ml.y == 0.f) continue;      // (a split without keys)
-      const float f = mma::exp2_fast(ml.x - top);
+      const float f = expf(ml.x - top);
       total = fmaf(ml.y, f, total);
       sum[0] = fmaf(v.x, f, sum[0]);
       sum[1] = fmaf(v.y, f, sum[1]);

@@ -212,3 +212,40 @@ def test_a_value_that_is_not_finite_reaches_the_rows_that_see_it_and_no_others(d
         same = torch.isfinite(general)
         if bool(same.any()):
             near(got[same], general[same].double(), 2.0 ** -7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("penalty", ["none", "linear", "logarithm"])
+@pytest.mark.parametrize("splits", [0, 1, 2])
+def test_weights_and_penalties_keep_their_32_bits(penalty, splits):
+    """Two keys whose values nearly cancel: (p0 - c p1) / (p0 + p1), c a bfloat16 number near p0 / p1.
+    What is left shows an error of the weights that rounding the output (2^-8 of it) does not hide: with
+    fp32 weights some 2^-23, with weights of 16 bits or a penalty as log2(1 + x) up to 2^-19 and more."""
+    heads, dim = 64, 128
+    g = torch.Generator(device="cuda").manual_seed(splits)
+    q = torch.zeros((1, heads, dim), dtype=BF, device="cuda")
+    keys = torch.zeros((1, 1, 64, dim), dtype=BF, device="cuda")
+    values = torch.zeros_like(keys)
+    gap = 0.01 + 0.05 * torch.rand(heads, generator=g, device="cuda")        # of the two scores
+    linear = slope = rate = None
+    distance = torch.tensor([1.0, 0.0], dtype=torch.float64, device="cuda")
+    if penalty == "none":
+        keys[0, 0, 0, 0] = 1.0
+        q[0, :, 0] = -gap.to(BF)
+        scores = torch.outer(q[0, :, 0].double(), distance)
+    elif penalty == "linear":
+        linear = gap
+        scores = -torch.outer(gap.double(), distance)
+    else:
+        rate = torch.full((heads,), 1.37 * 2.0 ** -13, device="cuda")
+        slope = gap / rate
+        scores = -slope.double()[:, None] * torch.log1p(torch.outer(rate.double(), distance))
+    c = (1 + torch.arange(dim, device="cuda") / dim / 14).to(BF)
+    values[0, 0, 0], values[0, 0, 1] = c, -1.0
+    want = torch.softmax(scores, 1) @ torch.stack([c.double(), -torch.ones_like(c).double()])
+    zero = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = attention_mma.attention(q, dim, keys, values, zero + 1, zero, zero[:, None], heads, dim, dim, 1.0,
+                                  slope=slope, rate=rate, linear=linear, decode=splits > 0,
+                                  key_splits=max(1, splits))
+    off = (got.view(heads, dim).double() - want).abs() - 2.0 ** -8 * want.abs()
+    assert float(off.max()) <= 2.0 ** -21

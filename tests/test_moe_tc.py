@@ -55,3 +55,22 @@ def test_products_at_the_edges_of_tiles(counts, n, k, few):
         want = c * torch.sigmoid(alpha * c) * (d + plus)
         off = (gated[lo:hi].double() - want).abs()
         assert bool((off <= 2.0 ** -8 * want.abs() + 1e-4 * want.abs().max()).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("few", [True, False])
+def test_the_gated_activation_far_out(few):
+    """g sigmoid(alpha g) where 1 + exp(-alpha g) lies above 2^126: a quotient by an approximate
+    reciprocal is 0 there, the number itself is a normal one."""
+    rows = torch.zeros((3, 8), dtype=torch.bfloat16, device="cuda")
+    rows[:, 0] = torch.tensor([-70.0, -69.5, 1.0])
+    gate = torch.zeros((1, 8, 8), dtype=torch.bfloat16, device="cuda")
+    gate[0, :, 0] = 1.0
+    up = torch.zeros_like(gate)
+    offsets = torch.tensor([0, 3], dtype=torch.int32, device="cuda")
+    out = torch.zeros((3, 8), dtype=torch.bfloat16, device="cuda")
+    call("sakv_moe_tc", ptr(rows), 3, ptr(gate), ptr(up), ptr(offsets), 1, ptr(out), 8, 8, 100.0, 1.2525, 1.0,
+         int(few))
+    x = rows[:, :1].double().expand(3, 8)
+    want = x * torch.sigmoid(1.2525 * x)
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs()).all())
