@@ -511,7 +511,8 @@ attention_mma_kernel(const MmaAttention a) {
           }
           const float sc = score_of(a, warp_sum(part), (float)(pos - j), sl, rate);
           const float next = fmaxf(top, sc);
-          const float f = expf(top - next), p = expf(sc - next);
+          const float shift = next == -INFINITY ? 0.f : next;      // (as above)
+          const float f = expf(top - shift), p = expf(sc - shift);
           sum = fmaf(sum, f, p);
           const __nv_bfloat16* vr = VINK ? a.k_cache + at * a.k_row : a.v_cache + at * a.v_row;
           for (int c = lane; c < DV; c += 32) acc_row[c] = fmaf(acc_row[c], f, p * widen(vr[c]));
@@ -559,8 +560,7 @@ __global__ void __launch_bounds__(DV / 4) attention_fold_kernel(const MmaAttenti
     for (int s = 0; s < a.key_splits; ++s) {
       const float2 ml = *reinterpret_cast<const float2*>(a.stats + (at + s * step) * 2);
       const float4 v = *reinterpret_cast<const float4*>(a.sums + (at + s * step) * DV + c);
-      if (ml.x == -INFINITY && ml.y == 0.f) continue;      // (a split without keys)
-      const float f = expf(ml.x - top);
+      const float f = ml.x == -INFINITY ? 0.f : expf(ml.x - top);      // (a split without keys)
       total = fmaf(ml.y, f, total);
       sum[0] = fmaf(v.x, f, sum[0]);
       sum[1] = fmaf(v.y, f, sum[1]);

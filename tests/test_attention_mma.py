@@ -249,3 +249,29 @@ def test_weights_and_penalties_keep_their_32_bits(penalty, splits):
                                   key_splits=max(1, splits))
     off = (got.view(heads, dim).double() - want).abs() - 2.0 ** -8 * want.abs()
     assert float(off.max()) <= 2.0 ** -21
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first,window", [(0, None), (64, None), (91, 40), (100, 31)])
+def test_a_first_key_that_scores_minus_infinity_counts_for_nothing(first, window):
+    """The key at `first` (a sequence's, a split's or some windows' first) scores -inf with every query; an
+    infinite value at position 110 sends the blocks that see it through their keys one by one."""
+    heads, dim, n = 4, 128, 131
+    draw, keys, values, table, rows = case(5, (n,), heads, 1, dim, dim)
+    q = draw(n, heads, dim)
+    q[:, :, 9] = -q[:, :, 9].abs() - 0.1
+    keys[table[0, first // 64].long(), 0, first % 64, 9] = float("inf")
+    values[table[0, 1].long(), 0, 110 - 64, 3] = float("inf")
+    k, v = rows[0][0].clone(), rows[0][1].clone()
+    k[first, 0, 9], v[110, 0, 3] = float("inf"), float("inf")
+    pos = torch.arange(n, dtype=torch.int32, device="cuda")
+    seq = torch.zeros_like(pos)
+    want = in_64_bits(q, range(n), [0] * n, [(k, v)], heads, 1, dim, 1, dim ** -0.5, window=window or 0)
+    for lo, splits in ((0, 0), (128, 1), (128, 3), (130, 2)):
+        got = attention_mma.attention(q[lo:], dim, keys, values, pos[lo:], seq[lo:], table, heads, dim, dim,
+                                      dim ** -0.5, window=window, decode=splits > 0,
+                                      key_splits=max(1, splits))
+        same = torch.isfinite(want[lo:])
+        assert torch.equal(torch.isnan(got), torch.isnan(want[lo:]))
+        assert torch.equal(torch.isinf(got), torch.isinf(want[lo:]))
+        near(got[same], want[lo:][same])
