@@ -40,6 +40,8 @@ struct MmaAttention {
   int k_row, v_row;
   const int32_t* positions;
   const int32_t* token_seq;
+  const int32_t* cu_seqlens;   // prompts: where each of `sequences` begins among the tokens, or null
+  int sequences;
   const int32_t* block_table;
   int max_blocks, tokens, heads, kv_heads, maps;      // heads: query heads (each of `maps` maps)
   float scale;
@@ -64,6 +66,7 @@ struct MmaAttention {
   int ordered;                 // in plain stream order: see `launch_shape`
   // the split of the work
   int heads_per_tile, tokens_per_tile, head_tiles;
+  int windows_shared;          // grid z are the runs of a window of tokens instead of splits
 };
 
 namespace {
@@ -166,8 +169,44 @@ attention_mma_kernel(const MmaAttention a) {
   wait_for_previous_kernel();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wr = warp / WC, wc = warp % WC;
-  // the longest rows of a prompt (its last tokens) start first
-  const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * a.tokens_per_tile;
+  // The block's tokens. The longest rows of a prompt (its last tokens) start first.
+  const int tile_at = (int)(gridDim.x - 1 - blockIdx.x);
+  int t0 = tile_at * a.tokens_per_tile, t_end = min(t0 + a.tokens_per_tile, a.tokens);
+  if (a.cu_seqlens != nullptr) {
+    // tiles end where a sequence does: the sequence whose tiles hold this one
+    t0 = -1;
+    for (int b0 = 0, base = 0; b0 < a.sequences && t0 < 0; b0 += 32) {
+      const int b = b0 + lane;
+      const int begin = b < a.sequences ? a.cu_seqlens[b] : 0;
+      const int end = b < a.sequences ? min(a.cu_seqlens[b + 1], a.tokens) : 0;
+      const int mine = (end - begin + a.tokens_per_tile - 1) / a.tokens_per_tile;
+      int sum = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      const int at = tile_at - (base + sum - mine);
+      const unsigned here = __ballot_sync(0xffffffffu, at >= 0 && at < mine);
+      if (here != 0) {
+        const int from = __ffs(here) - 1;
+        t0 = __shfl_sync(0xffffffffu, begin + at * a.tokens_per_tile, from);
+        t_end = min(t0 + a.tokens_per_tile, __shfl_sync(0xffffffffu, end, from));
+      }
+      base += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (t0 < 0) return;                      // (the grid has room for every cut into sequences)
+  } else if (a.windows_shared) {
+    // sequences not told: the block takes the z-th run of the window's tokens
+    int run = -1, s1 = t0;
+    for (; s1 < t_end && run < (int)blockIdx.z; ++run) {
+      t0 = s1++;
+      while (s1 < t_end && a.token_seq[s1] == a.token_seq[t0] &&
+             a.positions[s1] == a.positions[s1 - 1] + 1) ++s1;
+    }
+    if (run != (int)blockIdx.z) return;
+    t_end = s1;
+  }
   const int hg = a.heads / a.kv_heads, hp = a.heads_per_tile;
   int y = blockIdx.y;
   const int head_tile = y % a.head_tiles;
@@ -175,7 +214,6 @@ attention_mma_kernel(const MmaAttention a) {
   const int map = y % a.maps, g = y / a.maps;
   const int h_base = g * hg + head_tile * hp;
   const int h_count = min(hp, hg - head_tile * hp);
-  const int t_end = min(t0 + a.tokens_per_tile, a.tokens);
   const int used = (t_end - t0) * hp;        // rows beyond it belong to nobody
 
   // the queries
@@ -220,9 +258,9 @@ attention_mma_kernel(const MmaAttention a) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
 
-  const int split = blockIdx.z;
-  // The tile's tokens in runs of one sequence and consecutive positions (one run for nearly every
-  // tile of a prompt); rows outside the run see none of its keys.
+  const int split = a.windows_shared ? 0 : blockIdx.z;
+  // The tile's tokens in runs of one sequence and consecutive positions (one run for what the engine
+  // issues); rows outside the run see none of its keys.
   for (int s0 = t0; s0 < t_end;) {
     const int seq = a.token_seq[s0], p0 = a.positions[s0];
     int s1 = s0 + 1;
@@ -618,10 +656,23 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
   a.heads_per_tile = hg < S::kRows ? hg : S::kRows;
   a.head_tiles = (hg + a.heads_per_tile - 1) / a.heads_per_tile;
   a.tokens_per_tile = decode ? 1 : S::kRows / a.heads_per_tile;
-  const long long tiles = (a.tokens + a.tokens_per_tile - 1) / a.tokens_per_tile;
+  // A tile of rows walks the keys of one sequence: a step's decoded tokens beside a prompt get blocks
+  // of their own, where one tile would walk the keys of all of them in turn (one prompt of 512 tokens
+  // beside 15 sequences of 2,000 keys, us a layer, general kernel / walked in turn / now: 128 columns, 8
+  // heads of 2 key/value heads 1,228 / 2,161 / 144; two maps of 128 with 256 values, 4 of 2 heads 2,075 / 2,380 /
+  // 146; latent rows, 16 heads 2,174 / 1,114 / 271). With `cu_seqlens` the tiles are counted sequence by sequence on the device, so the
+  // grid has one more a sequence than the tokens alone need; without it a window of consecutive
+  // tokens has as many blocks as it can have runs, most of which find none and leave.
+  long long tiles = (a.tokens + a.tokens_per_tile - 1) / a.tokens_per_tile;
+  if (decode || a.sequences == 1) a.cu_seqlens = nullptr;
+  if (a.cu_seqlens != nullptr) tiles = a.tokens / a.tokens_per_tile + (long long)a.sequences;
+  a.windows_shared = !decode && a.sequences != 1 && a.cu_seqlens == nullptr;
+  if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   const long long across = (long long)a.kv_heads * a.maps * a.head_tiles;
   if (across > 65535) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)tiles, (unsigned)across, (unsigned)a.key_splits), block(S::kThreads);
+  const dim3 grid((unsigned)tiles, (unsigned)across,
+                  a.windows_shared ? (unsigned)a.tokens_per_tile : (unsigned)a.key_splits),
+      block(S::kThreads);
   const dim3 fold_grid((unsigned)a.tokens, (unsigned)a.heads), fold_block(DV / 4);
   // `ordered`: this attention stands between a library's products and kernels that read fresh
   // indices. An overlapped launch of the kernels there has once ended in a memory fault whose cause
@@ -641,7 +692,8 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
 
 // Everything as in `sakv_cached_attention` (`csrc/attention_distance.cu`) with bfloat16 operands,
 // plus slope and rate of the logarithmic penalty; gate: the pre-activations of a gate a head, map_gate:
-// of two maps' gate element by element (first head's first column; rows *_stride apart). decode 0:
+// of two maps' gate element by element (first head's first column; rows *_stride apart). cu_seqlens
+// (int32 [sequences + 1], or null: not known): which tokens each of `sequences` brings. decode 0:
 // blocks of 64 rows of a prompt; 1: a block a token, key/value head, map and split. sums, stats: fp32
 // scratch of key_splits * tokens * heads * maps * (vdim, 2) numbers, needed with two maps or several
 // splits, else null. ordered 1: both kernels in plain stream order. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
@@ -650,8 +702,8 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
 SAKV_EXPORT int sakv_attention_mma(
     const void* q, long long q_stride, int q_head_stride, const void* q2, long long q2_stride,
     int q2_head_stride, int q_split, void* out, const void* k_cache, int k_row, const void* v_cache,
-    int v_row, const int32_t* positions, const int32_t* token_seq, const int32_t* block_table,
-    int max_blocks, int tokens, int heads, int kv_heads, int maps, int dim, int vdim, float scale,
+    int v_row, const int32_t* positions, const int32_t* token_seq, const int32_t* cu_seqlens,
+    int sequences, const int32_t* block_table, int max_blocks, int tokens, int heads, int kv_heads, int maps, int dim, int vdim, float scale,
     int window, int chunk, int keep, const float* slope, const float* rate, float softcap,
     const float* linear, const float* sink, const void* gate, long long gate_stride,
     const float* elem_gate, long long elem_stride, const void* map_gate, long long map_gate_stride,
@@ -659,7 +711,7 @@ SAKV_EXPORT int sakv_attention_mma(
     int ordered, cudaStream_t stream) {
   if (tokens < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || (maps != 1 && maps != 2) ||
       window < 0 || chunk < 0 || keep < 0 || (window > 0 && chunk > 0) || softcap < 0.f ||
-      max_blocks <= 0 || key_splits < 1 || key_splits > 64 || (!decode && key_splits > 1) ||
+      max_blocks <= 0 || sequences < 0 || key_splits < 1 || key_splits > 64 || (!decode && key_splits > 1) ||
       k_row < maps * dim || (v_cache != nullptr ? v_row < vdim : k_row < vdim) ||
       (q2 != nullptr && (q_split < 0 || q_split > dim)) || heads > 65535)
     return cudaErrorInvalidValue;
@@ -685,6 +737,8 @@ SAKV_EXPORT int sakv_attention_mma(
   a.v_row = v_row;
   a.positions = positions;
   a.token_seq = token_seq;
+  a.cu_seqlens = cu_seqlens;
+  a.sequences = sequences;
   a.block_table = block_table;
   a.max_blocks = max_blocks;
   a.tokens = tokens;

@@ -229,11 +229,18 @@ def kv_store(qkv: torch.Tensor, k_off: int, v_off: int, positions: torch.Tensor,
          ptr(v_cache), tokens, kv_heads, dim, vdim)
 
 
+def _check_cu_seqlens(cu_seqlens, block_table):
+    _check(cu_seqlens is None or (cu_seqlens.dtype == torch.int32 and cu_seqlens.is_contiguous()
+                                  and cu_seqlens.shape == (block_table.shape[0] + 1,)),
+           "cu_seqlens: int32 [B + 1]")
+
+
 def distance_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
                        positions: torch.Tensor, token_seq: torch.Tensor,
                        block_table: torch.Tensor, heads: int, scale: float, window: int | None,
                        slope: torch.Tensor | None, rate: torch.Tensor | None,
-                       gate_off: int | None = None, splits: int = 1) -> torch.Tensor:
+                       gate_off: int | None = None, splits: int = 1,
+                       cu_seqlens: torch.Tensor | None = None) -> torch.Tensor:
     """Causal grouped-query attention of every token of the step over its sequence's cache
     with the score `q.k * scale - slope[h] * ln(1 + rate[h] * distance)`; queries are the first
     heads * dim columns of `qkv`, and with `gate_off` each head's output is multiplied by
@@ -242,8 +249,11 @@ def distance_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
     `splits`: 1 (the default) scores 32 keys at a time with one warp for a token's heads of a
     key/value head, and gives a token the same result to the bit however the tokens come; more
     (up to 16) lets that many warps share a token's keys, for steps of few tokens over many
-    keys; 0 is the plain form, one key at a time, which also takes widths above 256."""
-    require_cuda(qkv, k_cache, v_cache, positions, token_seq, block_table, slope, rate)
+    keys; 0 is the plain form, one key at a time, which also takes widths above 256. `cu_seqlens`
+    (int32 [B + 1]): where each sequence's tokens begin in the step, for steps of several sequences
+    whose tokens lie together (found out token by token without it)."""
+    require_cuda(qkv, k_cache, v_cache, positions, token_seq, block_table, slope, rate, cu_seqlens)
+    _check_cu_seqlens(cu_seqlens, block_table)
     tokens = qkv.shape[0]
     kv_heads, dim, vdim = k_cache.shape[1], k_cache.shape[3], v_cache.shape[3]
     _check(qkv.dim() == 2 and qkv.stride(1) == 1 and qkv.shape[1] >= heads * dim,
@@ -263,7 +273,7 @@ def distance_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.
             qkv, dim, k_cache, v_cache, positions, token_seq, block_table, heads, dim, vdim, scale,
             window=window, slope=slope, rate=rate,
             head_gate=None if gate_off is None else qkv[:, gate_off:gate_off + heads],
-            decode=splits > 1, key_splits=splits, ordered=False)
+            decode=splits > 1, key_splits=splits, ordered=False, cu_seqlens=cu_seqlens)
     out = torch.empty((tokens, heads * vdim), dtype=qkv.dtype, device=qkv.device)
     call("sakv_distance_attention", ptr(qkv), dtype_code(qkv.dtype), qkv.stride(0),
          -1 if gate_off is None else int(gate_off), ptr(out), ptr(k_cache), ptr(v_cache),
@@ -435,7 +445,8 @@ def cached_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
                      sink: torch.Tensor | None = None,
                      head_gate: torch.Tensor | None = None,
                      elem_gate: torch.Tensor | None = None, softcap: float | None = None,
-                     linear_slopes: torch.Tensor | None = None) -> torch.Tensor:
+                     linear_slopes: torch.Tensor | None = None,
+                     cu_seqlens: torch.Tensor | None = None) -> torch.Tensor:
     """Causal attention of every token of the step over its sequence's cache, in the general
     form of `csrc/attention_distance.cu`: scores, softmax weights and weighted sums in fp32.
 
@@ -462,9 +473,12 @@ def cached_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
     are ONE token's groups of heads and share every chunk of its keys through shared memory, so
     the rows are read once for all the token's heads; `key_splits` blocks a token then take
     contiguous shares of the chunks. `softcap` c: a scaled score s becomes `c tanh(s / c)`;
-    `linear_slopes` (fp32 [heads]): then `slope[h] * (i - j)` is taken off it."""
+    `linear_slopes` (fp32 [heads]): then `slope[h] * (i - j)` is taken off it. `cu_seqlens` (int32
+    [B + 1]): where each sequence's tokens begin in the step, for steps of several sequences whose
+    tokens lie together (found out token by token without it)."""
     require_cuda(q, k_cache, v_cache, positions, token_seq, block_table, q2, sink, head_gate,
-                 elem_gate, linear_slopes)
+                 elem_gate, linear_slopes, cu_seqlens)
+    _check_cu_seqlens(cu_seqlens, block_table)
     _check(softcap is None or softcap > 0, "softcap must be positive")
     _check(linear_slopes is None or (linear_slopes.dtype == torch.float32
                                      and linear_slopes.shape == (heads,)
@@ -512,7 +526,8 @@ def cached_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
             scale, maps=maps, q2=q2, q_split=q_split, window=window, chunk=chunk,
             keep_first=keep_first, softcap=softcap, linear=linear_slopes, sink=sink,
             head_gate=head_gate, elem_gate=elem_gate, map_gate_off=gate_elem_off, lam=lam,
-            out_scale=out_scale, eps=eps, decode=decode, key_splits=across)
+            out_scale=out_scale, eps=eps, decode=decode, key_splits=across,
+            cu_seqlens=cu_seqlens)
     out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
     scratch = tickets = None
     floats = 0

@@ -45,7 +45,7 @@ SIGNATURES = {
                                I, F, I, I, F, F, F, I, I, I, P, L, P, I, I, I, P, P, L, P, L, F, P,
                                P]),
     "sakv_attention_mma": ("attention_mma",
-                           [P, L, I, P, L, I, I, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, F, I, I,
+                           [P, L, I, P, L, I, I, P, P, I, P, I, P, P, P, I, P, I, I, I, I, I, I, I, F, I, I,
                             I, P, P, F, P, P, P, L, P, L, P, L, F, F, F, I, I, P, P, I, P]),
     "sakv_moe_tc": ("moe_tc", [P, L, P, P, P, I, P, I, I, F, F, F, I, P]),
     "sakv_rms_update": ("norm_update", [P, P, P, F, P, P, F, I, P, I, I, I, F, P]),

@@ -17,8 +17,10 @@ def takes(q: torch.Tensor, head_stride: int, k_cache: torch.Tensor, v_cache, dim
     """Whether the tensor-core kernel takes the call: bfloat16, one of the compiled pairs of
     widths, and every row of queries, keys and values beginning at a multiple of 16 bytes (they are
     copied in pieces of 16). It is the faster one for all of these, from one decoded token on
-    (against the kernel that scores a key a lane, us: a prompt of 3,001 tokens 13,058 -> 883 over
-    latent rows, 3,492 -> 295 at 128 columns; one decoded token 94 -> 27 and 92 -> 14)."""
+    and in steps that mix decoded tokens with a prompt (against the kernel that scores a key a lane, us, 16
+    heads over latent rows and 8 heads of 2 at 128 columns: a prompt of 3,001 tokens 14,597 -> 1,131 and
+    2,587 -> 244; 8 decoded tokens of 2,048 keys 132 -> 37 and 74 -> 39; the mixed steps in
+    `csrc/attention_mma.cu`)."""
     if q.dtype != torch.bfloat16 or SHAPES.get((dim, vdim, v_cache is None), 0) < maps:
         return False
     rows = [(q, q.stride(0), head_stride), (k_cache, k_cache.shape[3], 0)]
@@ -33,9 +35,10 @@ def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_tabl
               scale, *, maps=1, q2=None, q_split=0, window=None, chunk=None, keep_first=0, slope=None,
               rate=None, softcap=None, linear=None, sink=None, head_gate=None, elem_gate=None,
               map_gate_off=None, lam=0.0, out_scale=1.0, eps=0.0, decode=False, key_splits=1,
-              ordered=True):
+              ordered=True, cu_seqlens=None):
     """The arguments as `ops.cached_attention` and `ops.distance_attention` have checked them.
-    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt. `ordered`: the kernels begin when the one before them has
+    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt, of one sequence with `cu_seqlens` (int32 [sequences + 1]: where
+    every sequence's tokens begin), of one run of consecutive tokens without. `ordered`: the kernels begin when the one before them has
     ended (False: overlapped with it, for a caller whose neighbours are this library's own kernels)."""
     tokens = q.shape[0]
     out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
@@ -51,7 +54,8 @@ def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_tabl
     call("sakv_attention_mma", ptr(q), q.stride(0), head_stride, ptr(q2),
          0 if q2 is None else q2.stride(0), 0 if q2 is None else q2.stride(1), q_split, ptr(out),
          ptr(k_cache), k_cache.shape[3], ptr(v_cache), 0 if v_cache is None else v_cache.shape[3],
-         ptr(positions), ptr(token_seq), ptr(block_table), block_table.shape[1], tokens, heads,
+         ptr(positions), ptr(token_seq), ptr(cu_seqlens), block_table.shape[0], ptr(block_table),
+         block_table.shape[1], tokens, heads,
          k_cache.shape[1], maps, dim, vdim, float(scale), int(window) if window else 0,
          int(chunk) if chunk else 0, int(keep_first), ptr(slope), ptr(rate), float(softcap or 0.0),
          ptr(linear), ptr(sink), ptr(head_gate), 0 if head_gate is None else head_gate.stride(0),

@@ -83,7 +83,7 @@ class DifferentialAttention(Part):
             s.heads, s.head_dim, s.value_dim, s.scale, maps=MAPS, chunk=s.chunk, lam=self.lam,
             out_scale=1.0 - s.diff, eps=s.eps,
             gate_elem_off=self.q_cols + self.k_cols + self.v_cols if s.gate else None,
-            **self._decode_form(step, fused))
+            cu_seqlens=step.cu_seqlens, **self._decode_form(step, fused))
         return ops.linear(gated, self.w_o, out_dtype=torch.float32)
 
     def _decode_form(self, step, fused) -> dict:

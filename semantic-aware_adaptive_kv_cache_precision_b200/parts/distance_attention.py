@@ -85,7 +85,7 @@ class LogDistanceAttention(Part):
             qkv, view.keys, view.values, step.positions, step.token_seq, view.block_table,
             s.heads, s.scale, s.window, self.slope, self.rate,
             gate_off=self.q_cols + self.k_cols + self.v_cols if s.head_gate else None,
-            splits=self._splits(step, qkv))
+            splits=self._splits(step, qkv), cu_seqlens=step.cu_seqlens)
         return ops.linear(attended, self.w_o, self.b_o, out_dtype=torch.float32)
 
     def _splits(self, step, qkv) -> int:

@@ -128,7 +128,8 @@ class LatentAttention(Part):
             in_latent, view.keys, None, step.positions, step.token_seq, view.block_table,
             s.heads, rank + s.rot_dim, rank, s.scale, q2=q3[:, :, s.head_dim:], q_split=rank,
             window=s.window, sink=self.sink,
-            head_gate=q[:, q_cols:] if s.head_gate else None, **self._decode_form(step, q))
+            head_gate=q[:, q_cols:] if s.head_gate else None, cu_seqlens=step.cu_seqlens,
+            **self._decode_form(step, q))
         # the weighted sums of latents to each head's values
         heads_out = torch.empty((tokens, s.heads, s.value_dim), dtype=q.dtype, device=q.device)
         ops.per_head(mixed.view(tokens, s.heads, rank), self.w_uv, heads_out)

@@ -135,7 +135,7 @@ class WindowSinkAttention(Part):
             step.token_seq, view.block_table, s.heads, s.head_dim, s.value_dim, s.scale,
             window=s.window, keep_first=s.keep_first if s.window else 0, sink=self.sink,
             out_scale=s.out_scale, elem_gate=gate, softcap=s.softcap, linear_slopes=self.slopes,
-            **self._decode_form(step)).view(q.shape[0], -1)
+            cu_seqlens=step.cu_seqlens, **self._decode_form(step)).view(q.shape[0], -1)
 
     def _temperature(self, step):
         if self.temperature is not None and step.max_position >= self.temperature.numel():

@@ -169,11 +169,20 @@ def test_the_edges_of_tiles_in_every_kind_of_step(heads, kv_heads, dim, vdim, ma
             maps=maps, window=more.get("window"), chunk=more.get("chunk"),
             keep_first=more.get("keep", 0), slope=slope, rate=rate, softcap=more.get("softcap"),
             linear=linear, sink=sink, lam=0.4, eps=1e-6)
-        together = attention_mma.attention(
-            q, dim, keys, values, positions, token_seq, table, heads, dim, vdim, scale, maps=maps,
-            window=more.get("window"), chunk=more.get("chunk"), keep_first=more.get("keep", 0),
-            slope=slope, rate=rate, softcap=more.get("softcap"), linear=linear, sink=sink, lam=0.4, eps=1e-6)
-        assert torch.equal(alone[0], together[-1]), name       # whatever came with it: the same bits
+        counts = [seq.count(0), seq.count(1)]
+        cu = torch.tensor([0, counts[0], len(seq)], dtype=torch.int32, device="cuda")
+        together = {}
+        for told in (False, True):              # (tokens that lie sequence by sequence: told, or found out)
+            if told and seq != [0] * counts[0] + [1] * counts[1]:
+                continue
+            together[told] = attention_mma.attention(
+                q, dim, keys, values, positions, token_seq, table, heads, dim, vdim, scale, maps=maps,
+                window=more.get("window"), chunk=more.get("chunk"), keep_first=more.get("keep", 0),
+                slope=slope, rate=rate, softcap=more.get("softcap"), linear=linear, sink=sink, lam=0.4,
+                eps=1e-6, cu_seqlens=cu if told else None)
+            assert torch.equal(alone[0], together[told][-1]), name      # whatever came with it: the same bits
+        if True in together:
+            assert torch.equal(together[True], together[False]), name
 
 
 @pytest.mark.gpu
@@ -275,3 +284,41 @@ def test_a_first_key_that_scores_minus_infinity_counts_for_nothing(first, window
         assert torch.equal(torch.isnan(got), torch.isnan(want[lo:]))
         assert torch.equal(torch.isinf(got), torch.isinf(want[lo:]))
         near(got[same], want[lo:][same])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,maps,latent", [(8, 2, 128, 128, 1, False), (4, 4, 64, 64, 1, False),
+                                                                 (4, 2, 128, 256, 2, False), (16, 1, 576, 512, 1, True)])
+def test_tokens_of_several_sequences_in_one_step_run_side_by_side(heads, kv_heads, dim, vdim, maps, latent):
+    """Fifteen tokens that each continue a sequence of its own beside a piece of a prompt, as a scheduler
+    mixes them: the rows fit a few tiles, and walked one after another in those tiles' blocks they took
+    many times what one of them takes alone."""
+    lens = [3000 + 7 * i for i in range(15)] + [200]
+    draw, keys, values, table, _ = case(8, lens, heads, kv_heads, dim, vdim, maps, latent)
+    pos = [n - 1 for n in lens[:15]] + list(range(100, 200))
+    seq = list(range(15)) + [15] * 100
+    q = draw(len(pos), heads * maps, dim)
+    positions = torch.tensor(pos, dtype=torch.int32, device="cuda")
+    token_seq = torch.tensor(seq, dtype=torch.int32, device="cuda")
+    cu = torch.tensor(list(range(16)) + [115], dtype=torch.int32, device="cuda")
+
+    def run(n, cu_seqlens):
+        return attention_mma.attention(q[:n], dim, keys, values, positions[:n], token_seq[:n], table, heads, dim,
+                                       vdim, dim ** -0.5, maps=maps, lam=0.3, eps=1e-6, cu_seqlens=cu_seqlens)
+
+    def time(n, cu_seqlens):
+        best = float("inf")
+        for _ in range(5):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            run(n, cu_seqlens)
+            begin.record()
+            for _ in range(10):
+                run(n, cu_seqlens)
+            end.record()
+            end.synchronize()
+            best = min(best, begin.elapsed_time(end))
+        return best
+
+    alone = time(1, cu.clamp(max=1))
+    assert time(115, cu) < 3 * alone and time(115, None) < 3 * alone
+    assert torch.equal(run(115, cu), run(115, None)) and torch.equal(run(1, cu.clamp(max=1)), run(115, cu)[:1])
