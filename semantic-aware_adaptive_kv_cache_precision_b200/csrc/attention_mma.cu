@@ -9,11 +9,15 @@
 // kernel (expf, log1pf). A weight enters the second product as the sum of three bfloat16 numbers,
 // which hold all 24 of its bits, so every value tile is multiplied three times.
 //
-// A block takes the rows of one key/value head and map: ROWS = 16 WR rows are tokens x query heads
-// of the group, so a group's heads share each tile of keys. WR warps go along the rows and WC
+// A block takes the rows of one key/value head: ROWS = 16 WR rows are tokens x query heads of the
+// group (x maps in a prompt, decoded tokens: of one map), so a group's heads share each tile of keys. WR warps go along the rows and WC
 // along the keys of a tile for the scores and along the values' columns for the weighted sum:
 //   * prompts, 128 columns: WR 4, WC 1 (weights stay in registers); tiles of 64 keys, two blocks
 //     an SM.
+//   * prompts, two maps a head: the same with tiles of 32 keys; half of the warps take one map, half the
+//     other, and the block combines them (as blocks of one map each through fp32 sums in device memory,
+//     values of 256 columns: 2 KB a token and head, and 109 us instead of 77 for 16 prompts of 17 to
+//     500 tokens with 4 heads, 313 instead of 296 for one of 3,001).
 //   * prompts, latent rows: WR 4, WC 2, tiles of 32 keys: 64 rows x 512 columns of fp32 sums are
 //     128 registers a thread of 256, and the queries and three tiles fill the shared memory.
 //   * decoded tokens: WR 1, WC 8 and `key_splits` blocks a token; what bounds them is the trip to
@@ -51,7 +55,7 @@ struct MmaAttention {
   float softcap;
   const float* linear;
   int key_splits;
-  // the outputs: directly (one map, one split), or through `sums` and a second kernel
+  // the outputs: directly, or (decoded: two maps or several splits) through `sums` and a second kernel
   __nv_bfloat16* out;          // [tokens, heads * DV]
   float* sums;                 // [key_splits, tokens, heads * maps, DV], not yet divided
   float* stats;                // [key_splits, tokens, heads * maps, 2]: maximum, sum
@@ -128,13 +132,56 @@ __device__ __forceinline__ void write_row(const MmaAttention& a, const float* ac
   }
 }
 
-template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+// The same of a head's two maps: a1 - lambda a2 over its root mean square.
+template <int DV>
+__device__ __forceinline__ void write_pair(const MmaAttention& a, const float* acc1, const float* acc2,
+                                           float2 m, float2 l, int t, int h, int lane) {
+  constexpr int N = DV / 128;
+  float2 corr = make_float2(1.f, 1.f);
+  if (a.sink != nullptr) {
+    const float s = a.sink[h];
+    const float2 top = make_float2(fmaxf(m.x, s), fmaxf(m.y, s));
+    corr = make_float2(expf(m.x - top.x), expf(m.y - top.y));
+    l = make_float2(fmaf(l.x, corr.x, expf(s - top.x)), fmaf(l.y, corr.y, expf(s - top.y)));
+  }
+  const float f1 = corr.x / l.x, f2 = a.lambda * corr.y / l.y;
+  float o[N][4], ss = 0.f;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const float4 x = *reinterpret_cast<const float4*>(acc1 + n * 128 + lane * 4);
+    const float4 y = *reinterpret_cast<const float4*>(acc2 + n * 128 + lane * 4);
+    o[n][0] = x.x * f1 - y.x * f2;
+    o[n][1] = x.y * f1 - y.y * f2;
+    o[n][2] = x.z * f1 - y.z * f2;
+    o[n][3] = x.w * f1 - y.w * f2;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ss = fmaf(o[n][i], o[n][i], ss);
+  }
+  const float r = rsqrtf(warp_sum(ss) / (float)DV + a.eps) * a.out_scale;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = n * 128 + lane * 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[n][i] *= r;
+      if (a.map_gate != nullptr)
+        o[n][i] *= 1.f / (1.f + expf(-widen(a.map_gate[(long long)t * a.map_gate_stride +
+                                                      (long long)h * DV + c + i])));
+    }
+    *reinterpret_cast<uint2*>(a.out + ((long long)t * a.heads + h) * DV + c) =
+        make_uint2(mma::pack_bf16(o[n][0], o[n][1]), mma::pack_bf16(o[n][2], o[n][3]));
+  }
+}
+
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES, int MAPS>
 struct Shape {
   static constexpr int kRows = 16 * WR, kThreads = 32 * WR * WC;
-  static constexpr int kQStride = DK + 8, kVStride = VINK ? DK + 8 : DV + 8;   // (elements; odd
-  static constexpr int kOStride = DV + 8, kPStride = KT + 8;                    //  times 16 bytes)
+  static constexpr int kPairs = kRows / MAPS;       // (token, query head)s of a block
+  static constexpr int kQStride = DK + 8, kKStride = MAPS * DK + 8;            // (elements; odd
+  static constexpr int kVStride = VINK ? kKStride : DV + 8;                     //  times 16 bytes)
+  static constexpr int kOStride = DV + 8, kPStride = KT + 8;
   static constexpr int kQBytes = kRows * kQStride * 2;
-  static constexpr int kKBytes = KT * kQStride * 2;
+  static constexpr int kKBytes = KT * kKStride * 2;
   static constexpr int kStageBytes = kKBytes + (VINK ? 0 : KT * kVStride * 2);
   static constexpr int kPBytes = WC > 1 ? 3 * kRows * kPStride * 2 : 0;   // (a weight's three pieces)
   static constexpr int kSmall = (2 * WC + 2) * kRows * 4;        // maxima, sums, a row's m and l
@@ -143,16 +190,17 @@ struct Shape {
   static constexpr int kBytes = (kMain > kOut ? kMain : kOut) + kSmall;
 };
 
-template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES, int MAPS>
 __global__ void __launch_bounds__(32 * WR * WC)
 attention_mma_kernel(const MmaAttention a) {
-  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES>;
+  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES, MAPS>;
   constexpr int NT = KT / WC / 8;            // tiles of 8 keys a warp scores
   constexpr int NV = DV / WC / 8;            // tiles of 8 value columns a warp sums
   constexpr int KS = DK / 16;
   static_assert(KT % (8 * WC) == 0 && DV % (16 * WC) == 0 && kCacheBlock % KT == 0, "");
   static_assert(WC > 1 || (KT % 16 == 0), "");
   static_assert(NT == 1 || NT % 2 == 0, "");
+  static_assert(MAPS == 1 || (!VINK && S::kPairs % 16 == 0 && DV % 128 == 0), "a warp's rows are of one map");
   extern __shared__ __align__(16) unsigned char smem[];
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(smem);
   float* small = reinterpret_cast<float*>(smem + S::kBytes - S::kSmall);
@@ -211,18 +259,20 @@ attention_mma_kernel(const MmaAttention a) {
   int y = blockIdx.y;
   const int head_tile = y % a.head_tiles;
   y /= a.head_tiles;
-  const int map = y % a.maps, g = y / a.maps;
+  // (MAPS 1: all rows are of one map; else rows from `kPairs` on are of the second)
+  const int map0 = MAPS == 1 ? y % a.maps : 0, g = MAPS == 1 ? y / a.maps : y;
   const int h_base = g * hg + head_tile * hp;
   const int h_count = min(hp, hg - head_tile * hp);
-  const int used = (t_end - t0) * hp;        // rows beyond it belong to nobody
+  const int used = (t_end - t0) * hp;        // pairs beyond it belong to nobody
 
   // the queries
   constexpr int kPieces = DK / 8;
   for (int i = threadIdx.x; i < S::kRows * kPieces; i += S::kThreads) {
     const int r = i / kPieces, e = (i - r * kPieces) * 8;
-    const int t = t0 + r / hp, h = (h_base + r % hp) * a.maps + map;
+    const int pair = r % S::kPairs;
+    const int t = t0 + pair / hp, h = (h_base + pair % hp) * a.maps + map0 + r / S::kPairs;
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (r < used && r % hp < h_count) {
+    if (pair < used && pair % hp < h_count) {
       const __nv_bfloat16* src =
           e < a.q_split ? a.q + (long long)t * a.q_stride + (long long)h * a.q_head_stride + e
                         : a.q2 + (long long)t * a.q2_stride + (long long)h * a.q2_head_stride +
@@ -237,7 +287,7 @@ attention_mma_kernel(const MmaAttention a) {
   float rsl[2] = {0.f, 0.f}, rrt[2] = {0.f, 0.f};
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const int r = wr * 16 + (lane >> 2) + 8 * i;
+    const int r = (wr * 16 + (lane >> 2) + 8 * i) % S::kPairs;
     rt[i] = r < used && r % hp < h_count ? t0 + r / hp : -1;
     rpos[i] = rt[i] >= 0 ? a.positions[rt[i]] : -1;
     rfirst[i] = rt[i] >= 0 ? first_visible(rpos[i], a.window, a.chunk) : 0;
@@ -284,11 +334,11 @@ attention_mma_kernel(const MmaAttention a) {
       const long long row0 = ((long long)table[j0 / kCacheBlock] * a.kv_heads + g) * kCacheBlock +
                              j0 % kCacheBlock;
       const uint32_t ks = stage0 + (i % STAGES) * S::kStageBytes;
-      const __nv_bfloat16* kp = a.k_cache + row0 * a.k_row + map * DK;
-      constexpr int kp16 = DK / 8;
+      const __nv_bfloat16* kp = a.k_cache + row0 * a.k_row + map0 * DK;
+      constexpr int kp16 = MAPS * DK / 8;
       for (int x = threadIdx.x; x < KT * kp16; x += S::kThreads) {
         const int r = x / kp16, e = (x - r * kp16) * 8;
-        copy16(ks + (r * S::kQStride + e) * 2, kp + (long long)r * a.k_row + e, j0 + r <= last);
+        copy16(ks + (r * S::kKStride + e) * 2, kp + (long long)r * a.k_row + e, j0 + r <= last);
       }
       if constexpr (!VINK) {
         const __nv_bfloat16* vp = a.v_cache + row0 * a.v_row;
@@ -325,7 +375,7 @@ attention_mma_kernel(const MmaAttention a) {
       const uint32_t q_at = base + ((wr * 16 + (lane & 15)) * S::kQStride + (lane >> 4) * 8) * 2;
       if constexpr (NT == 1) {
         const uint32_t k_at =
-            ks + ((wc * 8 + (lane & 7)) * S::kQStride + (lane >> 3) * 8) * 2;
+            ks + ((wc * 8 + (lane & 7)) * S::kKStride + (lane >> 3) * 8) * 2;
 #pragma unroll 4
         for (int kk = 0; kk < KS; kk += 2) {
           uint32_t b[4], q0[4], q1[4];
@@ -336,8 +386,8 @@ attention_mma_kernel(const MmaAttention a) {
           mma::bf16_16816(s[0], q1, b[2], b[3]);
         }
       } else {
-        const uint32_t k_at = ks + ((wc * NT * 8 + (lane & 7) + (lane >> 4) * 8) * S::kQStride +
-                                    ((lane >> 3) & 1) * 8) * 2;
+        const uint32_t k_at = ks + ((wc * NT * 8 + (lane & 7) + (lane >> 4) * 8) * S::kKStride +
+                                    wr * 16 / S::kPairs * DK + ((lane >> 3) & 1) * 8) * 2;
 #pragma unroll(KS <= 8 ? KS : 4)
         for (int kk = 0; kk < KS; ++kk) {
           uint32_t q[4];
@@ -345,7 +395,7 @@ attention_mma_kernel(const MmaAttention a) {
 #pragma unroll
           for (int n = 0; n < NT; n += 2) {
             uint32_t b[4];
-            mma::ldmatrix_x4(k_at + (n * 8 * S::kQStride) * 2 + kk * 32, b[0], b[1], b[2], b[3]);
+            mma::ldmatrix_x4(k_at + (n * 8 * S::kKStride) * 2 + kk * 32, b[0], b[1], b[2], b[3]);
             mma::bf16_16816(s[n], q, b[0], b[1]);
             mma::bf16_16816(s[n + 1], q, b[2], b[3]);
           }
@@ -506,70 +556,80 @@ attention_mma_kernel(const MmaAttention a) {
     row_l[row] = sum;
   }
   __syncthreads();
-  for (int row = warp; row < used; row += WR * WC) {
-    if (row % hp >= h_count) continue;
-    const int t = t0 + row / hp, h = h_base + row % hp;
+  // An infinity or a NaN among the values: a weight of 0 times it spoils rows that do not see it, and a
+  // weight's pieces times it are not the weight times it. A warp of such a block walks a row's
+  // keys one by one.
+  auto walk = [&](int row, int t, int h) {
     float* acc_row = os + row * S::kOStride;
-    if (any_bad) {
-      // An infinity or a NaN among the values: a weight of 0 times it spoils rows that do not
-      // see it, and a weight's pieces times it are not the weight times it. Such a block walks its keys one by one.
-      const int pos = a.positions[t], first = first_visible(pos, a.window, a.chunk);
-      const int32_t* table = a.block_table + (long long)a.token_seq[t] * a.max_blocks;
-      // the same share of the run's tiles as above
-      int s0 = t, s1 = t + 1;
-      while (s0 > t0 && a.token_seq[s0 - 1] == a.token_seq[t] &&
-             a.positions[s0 - 1] == a.positions[s0] - 1) --s0;
-      while (s1 < t_end && a.token_seq[s1] == a.token_seq[t] &&
-             a.positions[s1] == a.positions[s1 - 1] + 1) ++s1;
-      const int last = a.positions[s1 - 1];
-      const int from = first_visible(a.positions[s0], a.window, a.chunk) / KT;
-      const int kept_all = (a.keep + KT - 1) / KT;
-      const int kept = kept_all < from ? kept_all : from;
-      const int count = kept + last / KT - from + 1;
-      const int share = (count + a.key_splits - 1) / a.key_splits;
-      const int lo = split * share, hi = min(count, lo + share);
-      const int vh = h * a.maps + map;
-      const float sl = a.slope ? a.slope[h] : a.linear ? a.linear[h] : 0.f;
-      const float rate = a.slope ? a.rate[h] : 0.f;
-      float top = -INFINITY, sum = 0.f;
-      for (int c = lane; c < DV; c += 32) acc_row[c] = 0.f;
-      for (int i = lo; i < hi; ++i) {
-        const int tile = i < kept ? i : from + i - kept;
-        for (int j = tile * KT; j < tile * KT + KT; ++j) {
-          if (j > pos || (j < first && j >= a.keep)) continue;
-          const long long at = ((long long)table[j / kCacheBlock] * a.kv_heads + g) * kCacheBlock +
-                               j % kCacheBlock;
-          float part = 0.f;
-          for (int e = lane; e < DK; e += 32) {
-            const __nv_bfloat16 qv =
-                e < a.q_split
-                    ? a.q[(long long)t * a.q_stride + (long long)vh * a.q_head_stride + e]
-                    : a.q2[(long long)t * a.q2_stride + (long long)vh * a.q2_head_stride + e - a.q_split];
-            part = fmaf(widen(qv), widen(a.k_cache[at * a.k_row + map * DK + e]), part);
-          }
-          const float sc = score_of(a, warp_sum(part), (float)(pos - j), sl, rate);
-          const float next = fmaxf(top, sc);
-          const float shift = next == -INFINITY ? 0.f : next;      // (as above)
-          const float f = expf(top - shift), p = expf(sc - shift);
-          sum = fmaf(sum, f, p);
-          const __nv_bfloat16* vr = VINK ? a.k_cache + at * a.k_row : a.v_cache + at * a.v_row;
-          for (int c = lane; c < DV; c += 32) acc_row[c] = fmaf(acc_row[c], f, p * widen(vr[c]));
-          top = next;
+    const int pos = a.positions[t], first = first_visible(pos, a.window, a.chunk);
+    const int32_t* table = a.block_table + (long long)a.token_seq[t] * a.max_blocks;
+    // the same share of the run's tiles as above
+    int s0 = t, s1 = t + 1;
+    while (s0 > t0 && a.token_seq[s0 - 1] == a.token_seq[t] &&
+           a.positions[s0 - 1] == a.positions[s0] - 1) --s0;
+    while (s1 < t_end && a.token_seq[s1] == a.token_seq[t] &&
+           a.positions[s1] == a.positions[s1 - 1] + 1) ++s1;
+    const int last = a.positions[s1 - 1];
+    const int from = first_visible(a.positions[s0], a.window, a.chunk) / KT;
+    const int kept_all = (a.keep + KT - 1) / KT;
+    const int kept = kept_all < from ? kept_all : from;
+    const int count = kept + last / KT - from + 1;
+    const int share = (count + a.key_splits - 1) / a.key_splits;
+    const int lo = split * share, hi = min(count, lo + share);
+    const int map = map0 + row / S::kPairs, vh = h * a.maps + map;
+    const float sl = a.slope ? a.slope[h] : a.linear ? a.linear[h] : 0.f;
+    const float rate = a.slope ? a.rate[h] : 0.f;
+    float top = -INFINITY, sum = 0.f;
+    for (int c = lane; c < DV; c += 32) acc_row[c] = 0.f;
+    for (int i = lo; i < hi; ++i) {
+      const int tile = i < kept ? i : from + i - kept;
+      for (int j = tile * KT; j < tile * KT + KT; ++j) {
+        if (j > pos || (j < first && j >= a.keep)) continue;
+        const long long at = ((long long)table[j / kCacheBlock] * a.kv_heads + g) * kCacheBlock +
+                             j % kCacheBlock;
+        float part = 0.f;
+        for (int e = lane; e < DK; e += 32) {
+          const __nv_bfloat16 qv =
+              e < a.q_split
+                  ? a.q[(long long)t * a.q_stride + (long long)vh * a.q_head_stride + e]
+                  : a.q2[(long long)t * a.q2_stride + (long long)vh * a.q2_head_stride + e - a.q_split];
+          part = fmaf(widen(qv), widen(a.k_cache[at * a.k_row + map * DK + e]), part);
         }
+        const float sc = score_of(a, warp_sum(part), (float)(pos - j), sl, rate);
+        const float next = fmaxf(top, sc);
+        const float shift = next == -INFINITY ? 0.f : next;      // (as above)
+        const float f = expf(top - shift), p = expf(sc - shift);
+        sum = fmaf(sum, f, p);
+        const __nv_bfloat16* vr = VINK ? a.k_cache + at * a.k_row : a.v_cache + at * a.v_row;
+        for (int c = lane; c < DV; c += 32) acc_row[c] = fmaf(acc_row[c], f, p * widen(vr[c]));
+        top = next;
       }
-      __syncwarp();
-      if (lane == 0) {
-        row_m[row] = top;
-        row_l[row] = sum;
-      }
-      __syncwarp();
     }
-    const float mm = row_m[row], ll = row_l[row];
+    __syncwarp();
+    if (lane == 0) {
+      row_m[row] = top;
+      row_l[row] = sum;
+    }
+    __syncwarp();
+  };
+  for (int pair = warp; pair < used; pair += WR * WC) {
+    if (pair % hp >= h_count) continue;
+    const int t = t0 + pair / hp, h = h_base + pair % hp;
+    if (any_bad)
+      for (int m = 0; m < MAPS; ++m) walk(pair + m * S::kPairs, t, h);
+    const float* acc_row = os + pair * S::kOStride;
+    const float mm = row_m[pair], ll = row_l[pair];
+    if constexpr (MAPS == 2) {
+      constexpr int o = S::kPairs;
+      write_pair<DV>(a, acc_row, acc_row + o * S::kOStride, make_float2(mm, row_m[pair + o]),
+                     make_float2(ll, row_l[pair + o]), t, h, lane);
+      continue;
+    }
     if (a.sums == nullptr) {
       write_row<DV>(a, acc_row, mm, ll, t, h, lane);
       continue;
     }
-    const long long part = ((long long)split * a.tokens + t) * a.heads * a.maps + h * a.maps + map;
+    const long long part = ((long long)split * a.tokens + t) * a.heads * a.maps + h * a.maps + map0;
     for (int c = lane * 4; c < DV; c += 128)
       *reinterpret_cast<float4*>(a.sums + part * DV + c) = *reinterpret_cast<const float4*>(acc_row + c);
     if (lane == 0) *reinterpret_cast<float2*>(a.stats + part * 2) = make_float2(mm, ll);
@@ -640,11 +700,11 @@ __global__ void __launch_bounds__(DV / 4) attention_fold_kernel(const MmaAttenti
       make_uint2(mma::pack_bf16(r[0], r[1]), mma::pack_bf16(r[2], r[3]));
 }
 
-template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES>
+template <int DK, int DV, bool VINK, int WR, int WC, int KT, int STAGES, int MAPS>
 int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
-  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES>;
+  using S = Shape<DK, DV, VINK, WR, WC, KT, STAGES, MAPS>;
   static_assert(S::kBytes <= 227 * 1024, "shared memory of a block");
-  auto kernel = attention_mma_kernel<DK, DV, VINK, WR, WC, KT, STAGES>;
+  auto kernel = attention_mma_kernel<DK, DV, VINK, WR, WC, KT, STAGES, MAPS>;
   static PerDeviceOnce configured;
   if (configured.needs()) {
     const cudaError_t e =
@@ -653,9 +713,9 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
     configured.done();
   }
   const int hg = a.heads / a.kv_heads;
-  a.heads_per_tile = hg < S::kRows ? hg : S::kRows;
+  a.heads_per_tile = hg < S::kPairs ? hg : S::kPairs;
   a.head_tiles = (hg + a.heads_per_tile - 1) / a.heads_per_tile;
-  a.tokens_per_tile = decode ? 1 : S::kRows / a.heads_per_tile;
+  a.tokens_per_tile = decode ? 1 : S::kPairs / a.heads_per_tile;
   // A tile of rows walks the keys of one sequence: a step's decoded tokens beside a prompt get blocks
   // of their own, where one tile would walk the keys of all of them in turn (one prompt of 512 tokens
   // beside 15 sequences of 2,000 keys, us a layer, general kernel / walked in turn / now: 128 columns, 8
@@ -668,7 +728,7 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
   if (a.cu_seqlens != nullptr) tiles = a.tokens / a.tokens_per_tile + (long long)a.sequences;
   a.windows_shared = !decode && a.sequences != 1 && a.cu_seqlens == nullptr;
   if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-  const long long across = (long long)a.kv_heads * a.maps * a.head_tiles;
+  const long long across = (long long)a.kv_heads * (MAPS == 1 ? a.maps : 1) * a.head_tiles;
   if (across > 65535) return cudaErrorInvalidValue;
   const dim3 grid((unsigned)tiles, (unsigned)across,
                   a.windows_shared ? (unsigned)a.tokens_per_tile : (unsigned)a.key_splits),
@@ -695,8 +755,8 @@ int launch_shape(MmaAttention& a, bool decode, cudaStream_t stream) {
 // of two maps' gate element by element (first head's first column; rows *_stride apart). cu_seqlens
 // (int32 [sequences + 1], or null: not known): which tokens each of `sequences` brings. decode 0:
 // blocks of 64 rows of a prompt; 1: a block a token, key/value head, map and split. sums, stats: fp32
-// scratch of key_splits * tokens * heads * maps * (vdim, 2) numbers, needed with two maps or several
-// splits, else null. ordered 1: both kernels in plain stream order. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
+// scratch of key_splits * tokens * heads * maps * (vdim, 2) numbers, needed for decoded tokens with
+// two maps or several splits, else null. ordered 1: both kernels in plain stream order. Refused (the caller's rule sends them elsewhere): other widths than (dim, vdim)
 // = (64, 64), (128, 128), (128, 256) and, with v_cache null, (576, 512); rows that do not begin at
 // multiples of 16 bytes.
 SAKV_EXPORT int sakv_attention_mma(
@@ -715,7 +775,7 @@ SAKV_EXPORT int sakv_attention_mma(
       k_row < maps * dim || (v_cache != nullptr ? v_row < vdim : k_row < vdim) ||
       (q2 != nullptr && (q_split < 0 || q_split > dim)) || heads > 65535)
     return cudaErrorInvalidValue;
-  const bool two_step = maps == 2 || key_splits > 1;
+  const bool two_step = (maps == 2 && decode) || key_splits > 1;
   if (two_step != (sums != nullptr) || two_step != (stats != nullptr)) return cudaErrorInvalidValue;
   if (maps == 2 && (gate != nullptr || elem_gate != nullptr)) return cudaErrorInvalidValue;
   if ((((uintptr_t)q | (uintptr_t)q2 | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) ||
@@ -770,17 +830,19 @@ SAKV_EXPORT int sakv_attention_mma(
   a.ordered = ordered;
   const bool in_key = v_cache == nullptr;
   if (in_key && dim == 576 && vdim == 512 && maps == 1)
-    return decode ? launch_shape<576, 512, true, 1, 8, 64, 2>(a, true, stream)
-                  : launch_shape<576, 512, true, 4, 2, 32, 3>(a, false, stream);
+    return decode ? launch_shape<576, 512, true, 1, 8, 64, 2, 1>(a, true, stream)
+                  : launch_shape<576, 512, true, 4, 2, 32, 3, 1>(a, false, stream);
   if (in_key) return cudaErrorInvalidValue;
   if (dim == 128 && vdim == 128)
-    return decode ? launch_shape<128, 128, false, 1, 8, 64, 3>(a, true, stream)
-                  : launch_shape<128, 128, false, 4, 1, 64, 2>(a, false, stream);
+    return decode      ? launch_shape<128, 128, false, 1, 8, 64, 3, 1>(a, true, stream)
+           : maps == 1 ? launch_shape<128, 128, false, 4, 1, 64, 2, 1>(a, false, stream)
+                       : launch_shape<128, 128, false, 4, 1, 32, 2, 2>(a, false, stream);
   if (dim == 128 && vdim == 256)
-    return decode ? launch_shape<128, 256, false, 1, 8, 64, 3>(a, true, stream)
-                  : launch_shape<128, 256, false, 4, 1, 32, 2>(a, false, stream);
-  if (dim == 64 && vdim == 64)
-    return decode ? launch_shape<64, 64, false, 1, 4, 64, 3>(a, true, stream)
-                  : launch_shape<64, 64, false, 4, 1, 64, 2>(a, false, stream);
+    return decode      ? launch_shape<128, 256, false, 1, 8, 64, 3, 1>(a, true, stream)
+           : maps == 1 ? launch_shape<128, 256, false, 4, 1, 32, 2, 1>(a, false, stream)
+                       : launch_shape<128, 256, false, 4, 1, 32, 2, 2>(a, false, stream);
+  if (dim == 64 && vdim == 64 && maps == 1)
+    return decode ? launch_shape<64, 64, false, 1, 4, 64, 3, 1>(a, true, stream)
+                  : launch_shape<64, 64, false, 4, 1, 64, 2, 1>(a, false, stream);
   return cudaErrorInvalidValue;
 }

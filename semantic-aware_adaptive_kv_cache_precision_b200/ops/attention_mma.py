@@ -45,7 +45,7 @@ def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_tabl
     if not decode:
         key_splits = 1
     sums = stats = None
-    if maps == 2 or key_splits > 1:
+    if decode and (maps == 2 or key_splits > 1):
         rows = key_splits * tokens * heads * maps
         sums = torch.empty((rows, vdim), dtype=torch.float32, device=q.device)
         stats = torch.empty((rows, 2), dtype=torch.float32, device=q.device)

@@ -140,7 +140,8 @@ STEPS = {                                # (position, sequence) of every token o
     (6, 2, 64, 64, 1, False, {}), (8, 2, 128, 128, 1, False, {"window": 50, "keep": 3, "sink": True}),
     (5, 1, 128, 128, 1, False, {"softcap": 9.0, "linear": True}), (4, 4, 128, 128, 1, False, {"slope": True}),
     (20, 1, 64, 64, 1, False, {"window": 64}), (4, 2, 128, 256, 2, False, {"chunk": 48}),
-    (3, 1, 128, 128, 2, False, {}), (2, 1, 128, 256, 1, False, {"window": 1}),
+    (3, 1, 128, 128, 2, False, {}), (40, 1, 128, 128, 2, False, {"window": 50, "keep": 3, "sink": True}),
+    (35, 1, 128, 256, 2, False, {"softcap": 9.0, "linear": True}), (2, 1, 128, 256, 1, False, {"window": 1}),
     (16, 1, 576, 512, 1, True, {"window": 70, "sink": True}), (3, 1, 576, 512, 1, True, {"chunk": 65})])
 def test_the_edges_of_tiles_in_every_kind_of_step(heads, kv_heads, dim, vdim, maps, latent, more):
     draw, keys, values, table, rows = case(heads + dim, (131, 40), heads, kv_heads, dim, vdim, maps, latent)
@@ -186,22 +187,22 @@ def test_the_edges_of_tiles_in_every_kind_of_step(heads, kv_heads, dim, vdim, ma
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dim,vdim,latent", [(128, 128, False), (576, 512, True)])
+@pytest.mark.parametrize("dim,vdim,maps,latent", [(128, 128, 1, False), (128, 256, 2, False), (576, 512, 1, True)])
 @pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
-def test_a_value_that_is_not_finite_reaches_the_rows_that_see_it_and_no_others(dim, vdim, latent, value,
+def test_a_value_that_is_not_finite_reaches_the_rows_that_see_it_and_no_others(dim, vdim, maps, latent, value,
                                                                                monkeypatch):
     """Position 70 of 131 holds it in one column: rows before it are as without it, rows from it on
     are what the general kernel gives, and other columns are as without it (over a latent row the
     key is the value, so the rows from it on have no number at all)."""
     heads = 4
-    draw, keys, values, table, _ = case(3, (131,), heads, 1, dim, vdim, 1, latent)
-    q = draw(131, heads, dim)
+    draw, keys, values, table, _ = case(3, (131,), heads, 1, dim, vdim, maps, latent)
+    q = draw(131, heads * maps, dim)
     pos = torch.arange(131, dtype=torch.int32, device="cuda")
     seq = torch.zeros(131, dtype=torch.int32, device="cuda")
 
     def run(lo=0, **form):
         return ops.cached_attention(q[lo:], keys, values, pos[lo:], seq[lo:], table, heads, dim, vdim,
-                                    dim ** -0.5, **form)
+                                    dim ** -0.5, maps=maps, lam=0.4, eps=1e-6, **form)
 
     forms = (dict(), dict(lo=128, heads_first=True, key_splits=1), dict(lo=128, heads_first=True, key_splits=3))
     clean = [run(**f) for f in forms]
@@ -322,3 +323,25 @@ def test_tokens_of_several_sequences_in_one_step_run_side_by_side(heads, kv_head
     alone = time(1, cu.clamp(max=1))
     assert time(115, cu) < 3 * alone and time(115, None) < 3 * alone
     assert torch.equal(run(115, cu), run(115, None)) and torch.equal(run(1, cu.clamp(max=1)), run(115, cu)[:1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("vdim", [128, 256])
+def test_a_prompt_of_two_maps_needs_no_memory_beside_its_output(vdim):
+    heads, dim, n = 8, 128, 2000
+    draw, keys, values, table, _ = case(4, (n,), heads, 2, dim, vdim, 2)
+    q = draw(n, 2 * heads, dim)
+    pos = torch.arange(n, dtype=torch.int32, device="cuda")
+    zeros = torch.zeros_like(pos)
+
+    def run():
+        return ops.cached_attention(q, keys, values, pos, zeros, table, heads, dim, vdim, dim ** -0.5, maps=2,
+                                    lam=0.4, eps=1e-6)
+
+    run()
+    torch.cuda.synchronize()
+    held = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = run()
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - held <= out.numel() * 2 + 4096
