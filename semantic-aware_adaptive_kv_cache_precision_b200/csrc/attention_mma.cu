@@ -23,7 +23,9 @@
 //   * decoded tokens: WR 1, WC 8 and `key_splits` blocks a token; what bounds them is the trip to
 //     memory, so a whole tile of 64 keys is asked for at once by 256 threads.
 // Tiles lie at multiples of their size in the sequence and a row that sees nothing of a tile is
-// left exactly as it was, so a token's result does not depend on which tokens came with it.
+// left exactly as it was, so in a prompt a token's result does not depend on which tokens came with
+// it, as long as all values are finite (a block that meets one that is not walks its rows' keys one
+// by one). A decoded token's keys are split by rules that count the step's tokens.
 //
 // The products run on mma.sync: at 576 and 512 columns the sums of 128 rows would fill the whole
 // of tensor memory, and the weights in two pieces would pass through it twice.

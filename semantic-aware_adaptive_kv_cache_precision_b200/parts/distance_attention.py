@@ -85,14 +85,16 @@ class LogDistanceAttention(Part):
             qkv, view.keys, view.values, step.positions, step.token_seq, view.block_table,
             s.heads, s.scale, s.window, self.slope, self.rate,
             gate_off=self.q_cols + self.k_cols + self.v_cols if s.head_gate else None,
-            splits=self._splits(step, qkv), cu_seqlens=step.cu_seqlens)
+            splits=self._splits(step, qkv, view), cu_seqlens=step.cu_seqlens)
         return ops.linear(attended, self.w_o, self.b_o, out_dtype=torch.float32)
 
-    def _splits(self, step, qkv) -> int:
-        """How many warps, or on the tensor cores blocks, share a token's keys. One in the 32-bit mode and for prompts (the
-        sums then have one order however the tokens are cut); for decode steps in bfloat16 one
-        warp for every two chunks of 32 keys that a token can see, up to 16. (A decode
-        step's graph is keyed by the width of the block lists, which bounds the length.)"""
+    def _splits(self, step, qkv, view) -> int:
+        """How many warps (on the tensor cores: blocks) share a token's keys. One in the 32-bit mode
+        and for prompts (the sums then have one order however the tokens are cut); for decode steps
+        in bfloat16 one for every two chunks of 32 keys that a token can see, up to 16. (A decode
+        step's graph is keyed by the width of the block lists, which bounds the length.) Blocks: no
+        more than four an SM, since each brings partial sums of its own; a token's sums then have
+        another order in a large batch."""
         if qkv.dtype == torch.float32 or not step.is_decode:
             return 1
         s = self.spec
@@ -102,8 +104,7 @@ class LogDistanceAttention(Part):
         splits = 1
         while splits < 16 and splits * 64 < keys:
             splits *= 2
-        if (s.head_dim, s.value_dim, False) in ops.attention_mma.SHAPES:
-            # (blocks: no more than four an SM, each brings its own partial sums)
+        if ops.attention_mma.takes(qkv, s.head_dim, view.keys, view.values, s.head_dim, s.value_dim):
             while splits > 2 and step.tokens * s.kv_heads * splits > 4 * ops.sm_count():
                 splits //= 2
         return splits

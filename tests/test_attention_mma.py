@@ -2,12 +2,15 @@
 (no GPU needed), and its results against float64 and against the general kernel at the edges of its
 tiles, in prompts, pieces, steps of scattered tokens and decoded, with infinities among the values."""
 
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 import torch
 
 from semantic_aware_adaptive_kv_cache_precision_b200 import ops
 from semantic_aware_adaptive_kv_cache_precision_b200.ops import attention_mma
+from semantic_aware_adaptive_kv_cache_precision_b200.parts.distance_attention import LogDistanceAttention
 
 BF = torch.bfloat16
 
@@ -55,6 +58,27 @@ def test_attention_beside_library_products_is_launched_in_plain_order(monkeypatc
     ops.distance_attention(torch.zeros((3, 1024), dtype=BF), cache(128), cache(128), pos, pos, table, 4, 1.0, None,
                            slope, slope)
     assert launched[6:] == [("sakv_attention_mma", 0)]
+
+
+def test_only_calls_that_the_tensor_cores_take_have_their_splits_bounded_by_blocks(monkeypatch):
+    """Gates of an odd number of heads behind the queries, keys and values leave rows that do not begin at
+    multiples of 16 bytes: those go to the general kernel, whose splits are warps."""
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    spec = SimpleNamespace(head_dim=128, value_dim=128, window=None, heads=6, kv_heads=2)
+    step = SimpleNamespace(is_decode=True, max_len_bound=4096, max_len=4096, tokens=64)
+    cache = torch.zeros((1, 2, 64, 128), dtype=BF)
+    view = SimpleNamespace(keys=cache, values=cache)
+
+    def splits(columns, dtype=BF):
+        return LogDistanceAttention._splits(SimpleNamespace(spec=spec), step,
+                                            torch.zeros((64, columns), dtype=dtype), view)
+
+    assert splits(10 * 128) == 4 and splits(10 * 128 + 6) == 16 and splits(10 * 128, torch.float32) == 1
+    step.tokens = 1
+    assert splits(10 * 128) == 16
+    spec.head_dim = 96
+    step.tokens = 64
+    assert splits(1280) == 16
 
 
 def case(seed, lens, heads, kv_heads, dim, vdim, maps=1, latent=False):
