@@ -150,6 +150,20 @@ __device__ __forceinline__ float both(Two v) {
   return a + b;
 }
 
+constexpr size_t kScanBudget = 96 * 1024;      // shared memory of a scan's block
+constexpr int kMostChunk = 16;                 // tokens that it takes at a time
+
+// Bytes of two chunks of `n` tokens: five vectors in R parts of `rpt` rows, and `cols` values.
+constexpr size_t scan_bytes(int n, int rpt, int R, int cols) {
+  return (size_t)2 * n * (5 * R * (rpt + (R > 1 ? 4 : 0)) + cols) * sizeof(float);
+}
+
+// Tokens of a straight run in the WHOLE form: one a lane, four with 16 lanes. A chunk never holds 16 tokens
+// of columns that long, and runs of the eight that it holds at 128 rows spill: 16 heads of 128,
+// us, token by token / runs of 8 / of 4: 2,048 tokens 1,043 / 881 / 899, 8 sequences of 300 tokens 820 / 678 / 676,
+// of 5 53 / 47 / 44; 8 heads of 256, 2,048 tokens 2,095 token by token, 1,477 in fours.
+constexpr int scan_run(int R) { return R < 16 ? R : 4; }
+
 // One block: `cols` neighbouring columns of one head's state for one sequence. A column's
 // rows are dealt to R neighbouring lanes, dim / R <= RPT rows each. VEC: rows are read four
 // at a time (dim / R a multiple of 4, everything 16-byte aligned); WHOLE: dim / R is RPT.
@@ -157,10 +171,10 @@ __device__ __forceinline__ float both(Two v) {
 //
 // What bounds it is the chain from token to token: the sum u^T S over a column's R lanes (a
 // shuffle tree) and the update that waits for it. The WHOLE form keeps out of that chain what does
-// not belong to it: R tokens are one straight run of code, so that the next token's vectors can be
-// read meanwhile; S is held in pairs for two-wide arithmetic; and the outputs' sums wait until R
-// tokens have left theirs, when each lane finishes one token's (R - 1 exchanges instead of
-// R log2 R, the same tree of additions). One sequence of 2,048 tokens, 32 heads of 64, behind its
+// not belong to it: `scan_run` tokens are one straight run of code,
+// so that the next token's vectors can be read meanwhile; S is held in pairs for two-wide arithmetic;
+// and the outputs' sums wait until a run's tokens have left theirs, when each lane finishes one token's
+// (R - 1 exchanges instead of R log2 R in a run of R, the same tree of additions). One sequence of 2,048 tokens, 32 heads of 64, behind its
 // prepare kernel: 842 us before, 373 now (of which the launch in plain order 206, see
 // `launch_scan`). Tried and no faster (380 to 450): two columns a thread, bulk copies of the vectors
 // (60 ns each), a copying warp of its own, vectors read by volatile loads a token ahead, 4 or 16
@@ -303,22 +317,26 @@ delta_scan_kernel(const float* __restrict__ proj, long long proj_stride, int off
         }
         return both(o);
       };
+      constexpr int kRun = scan_run(R);
+      static_assert(kRun > 1 && scan_bytes(kRun, RPT, R, 512 / R) <= kScanBudget, "a chunk holds a run");
       int tt = 0;
-      for (; tt + R <= count; tt += R) {
-        float o[R];
+      for (; tt + kRun <= count; tt += kRun) {
+        float o[kRun];
 #pragma unroll
-        for (int q = 0; q < R; ++q) o[q] = token(tt + q);
+        for (int q = 0; q < kRun; ++q) o[q] = token(tt + q);
 #pragma unroll
-        for (int step = 1, n = R / 2; step < R; step <<= 1, n >>= 1) {
+        for (int step = 1, n = kRun / 2; step < kRun; step <<= 1, n >>= 1) {
           const bool odd = (part & step) != 0;
 #pragma unroll
-          for (int i = 0; i < R / 2; ++i)
+          for (int i = 0; i < kRun / 2; ++i)
             if (i < n) {
               const float keep = odd ? o[2 * i + 1] : o[2 * i], give = odd ? o[2 * i] : o[2 * i + 1];
               o[i] = keep + __shfl_xor_sync(0xffffffffu, give, step);
             }
         }
-        if (mine) raw[(long long)(t0 + tt + part) * hd + base + col] = o[0];
+#pragma unroll
+        for (int step = kRun; step < R; step <<= 1) o[0] += __shfl_xor_sync(0xffffffffu, o[0], step);
+        if (mine && part < kRun) raw[(long long)(t0 + tt + part) * hd + base + col] = o[0];
       }
       for (; tt < count; ++tt) {
         const float o = sum_over_parts<R>(token(tt));
@@ -402,8 +420,6 @@ __global__ void delta_finish_kernel(const float* __restrict__ raw, const float* 
         o[c] * inv * widen(norm_w[base + c]) * sigmoidf(proj[t * proj_stride + off_g + base + c]));
 }
 
-constexpr size_t kScanBudget = 96 * 1024;
-
 template <int RPT, int R, bool VEC, bool WHOLE>
 int launch_scan(const float* proj, long long proj_stride, const int* off, const float* prepared,
                 float* state, const int32_t* cu_seqlens, const int32_t* slots, float* raw,
@@ -419,10 +435,10 @@ int launch_scan(const float* proj, long long proj_stride, const int* off, const 
     while (cols * R > 512 && cols % 8 == 0) cols /= 2;
   }
   if (cols * R > 512) return cudaErrorInvalidValue;
-  const int rpt = dim / R, ldt = R * (rpt + (R > 1 ? 4 : 0));
-  auto bytes = [&](int n) { return (size_t)2 * n * (5 * ldt + cols) * sizeof(float); };
+  auto bytes = [&](int n) { return scan_bytes(n, dim / R, R, cols); };
+  const bool prompt = chunk >= 8;            // (what a sequence brings, not what fits)
   if (chunk < 1) chunk = 1;
-  if (chunk > 16) chunk = 16;
+  if (chunk > kMostChunk) chunk = kMostChunk;
   while (chunk > 1 && bytes(chunk) > kScanBudget) chunk /= 2;
   if (bytes(chunk) > kScanBudget) return cudaErrorInvalidValue;
   const int threads = ((cols * R + 31) / 32) * 32;
@@ -439,7 +455,7 @@ int launch_scan(const float* proj, long long proj_stride, const int* off, const 
   // (2,048 tokens, 32 heads of 64: 585 us a scan behind its prepare kernel, 379 in plain order).
   // For a few tokens the early start is worth more.
   const dim3 grid(heads, sequences, (dim + cols - 1) / cols);
-  if (chunk >= 8)
+  if (prompt)
     return launch_ordered(kernel, grid, dim3(threads), bytes(chunk), stream, proj, proj_stride, off[0],
                           off[1], off[2], prepared, state, cu_seqlens, slots, raw, heads, dim, cols,
                           chunk, keep_state);
@@ -455,10 +471,11 @@ int pick_scan(const float* proj, long long proj_stride, const int* off, const fl
   return launch_scan<RPT, R, VEC, WHOLE>(proj, proj_stride, off, prepared, state, cu_seqlens,   \
                                          slots, raw, sequences, heads, dim, chunk, keep_state,  \
                                          stream)
-#define SAKV_SCAN(RPT, R, VEC)                                 \
+#define SAKV_SCAN(RPT, R, VEC) SAKV_SCAN_AS(RPT, R, VEC, false)
+#define SAKV_SCAN_WHOLE(RPT, R)                                \
   do {                                                         \
-    if (VEC && dim == RPT * R) SAKV_SCAN_AS(RPT, R, VEC, VEC); \
-    SAKV_SCAN_AS(RPT, R, VEC, false);                          \
+    if (dim == RPT * R) SAKV_SCAN_AS(RPT, R, true, true);      \
+    SAKV_SCAN_AS(RPT, R, true, false);                         \
   } while (0)
   // a column's rows over R lanes, four rows at a time: the most lanes (up to 16) that leave
   // a lane 8 rows, or 4 where dim is small; dims that 16 does not divide: one lane a column
@@ -466,19 +483,20 @@ int pick_scan(const float* proj, long long proj_stride, const int* off, const fl
     int lanes = 4;
     while (lanes < 16 && dim % (8 * lanes) == 0 && dim / (2 * lanes) >= 8) lanes *= 2;
     const int rpt = dim / lanes;
-    if (lanes == 4 && rpt <= 4) SAKV_SCAN(4, 4, true);
-    if (lanes == 4 && rpt <= 8) SAKV_SCAN(8, 4, true);
+    if (lanes == 4 && rpt <= 4) SAKV_SCAN_WHOLE(4, 4);
+    if (lanes == 4 && rpt <= 8) SAKV_SCAN_WHOLE(8, 4);
     if (lanes == 4 && rpt <= 16) SAKV_SCAN(16, 4, true);
-    if (lanes == 8 && rpt <= 8) SAKV_SCAN(8, 8, true);
+    if (lanes == 8 && rpt <= 8) SAKV_SCAN_WHOLE(8, 8);
     if (lanes == 8 && rpt <= 16) SAKV_SCAN(16, 8, true);
-    if (lanes == 16 && rpt <= 8) SAKV_SCAN(8, 16, true);
-    if (lanes == 16 && rpt <= 16) SAKV_SCAN(16, 16, true);
+    if (lanes == 16 && rpt <= 8) SAKV_SCAN_WHOLE(8, 16);
+    if (lanes == 16 && rpt <= 16) SAKV_SCAN_WHOLE(16, 16);
   }
   if (dim <= 32) SAKV_SCAN(32, 1, false);
   if (dim <= 64) SAKV_SCAN(64, 1, false);
   if (dim <= 128) SAKV_SCAN(128, 1, false);
   SAKV_SCAN(256, 1, false);
 #undef SAKV_SCAN
+#undef SAKV_SCAN_WHOLE
 #undef SAKV_SCAN_AS
 }
 
