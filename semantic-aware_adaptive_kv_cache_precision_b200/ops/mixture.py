@@ -28,27 +28,43 @@ _counts: dict = {}
 ROUTE_IN_ONE_BLOCK = 64
 
 
-#: fewer tiles of 128 rows x 256 weight rows than this: tiles of 32 x 64, so that more SMs pull weights
-FEW_TILES = 48
+#: What a grouped product takes in each form, us: (start, a column of K, tiles that run side by side,
+#: rows and weight rows of a tile), where a product of K columns and `tiles` tiles takes
+#: start + K * column * max(1, tiles / side by side). Fitted to 750 products of 2 to 64 experts, 2 to 12,000 rows
+#: and K of 48 to 2,048, weights from memory; the form chosen with them takes 1.01 times the fastest one's time on
+#: average and at most 1.5 (the tcgen05 forms alone 1.23 and 2.7, the tiles of 32 x 64 alone 1.44).
+FORMS = {False: {"tile": (2.2, 0.0064, 240, 32, 64), "few": (4.6, 0.0036, 121, 32, 64),
+                 "large": (5.3, 0.0062, 78, 128, 256)},
+         True: {"tile": (2.8, 0.0141, 307, 32, 64), "few": (5.4, 0.0040, 134, 32, 32),
+                "large": (6.8, 0.0065, 104, 128, 128)}}
+
+
+def _cost(form: str, rows: int, experts: int, n: int, k: int, dual: bool) -> float:
+    start, column, together, high, wide = FORMS[dual][form]
+    tiles = (min(experts, rows) + rows // high) * -(-n // wide)
+    return start + k * column * max(1.0, tiles / together)
 
 
 def tc_takes(rows: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor | None) -> bool:
     """Whether the tcgen05 kernel takes the grouped product: bfloat16 rows and weight rows of
-    multiples of 8 columns at multiples of 16 bytes; it is as fast as the general kernel from
-    one token on (us, general / this, the gated and the down product of 32 experts of 2048 -> 1024, 4
-    a token: 1 token 41 and 16 / 21 and 14, 64 tokens 76 and 43 / 66 and 39, 400 tokens 111 and 64
-    / 66 and 41, 3,001 tokens 530 and 324 / 104 and 76)."""
+    multiples of 8 columns at multiples of 16 bytes."""
     return (rows.dtype == torch.bfloat16 and w0.shape[2] % 8 == 0 and w0.shape[1] % 8 == 0
             and w0.shape[0] <= 1024
             and all(t is None or t.data_ptr() % 16 == 0 for t in (rows, w0, w1)))
 
 
-def few_tiles(rows: int, experts: int, n: int, dual: bool) -> bool:
-    """Whether the grouped product of `rows` rows takes the small tiles. Large / small, us: 32 large
-    tiles (1 token, 4 experts, 2 x 1024 x 2048) 25 / 21, 16 (64 tokens, 2 experts, 2 x 1024 x 1024) 19
-    / 14; 64 (16 tokens, 16 experts, 1024 x 1024) 19 / 21, 128 (the same, gated) 25 / 29."""
-    row_tiles = min(experts, rows) + rows // 128
-    return row_tiles * -(-n // (128 if dual else 256)) < FEW_TILES
+def tc_faster(rows: int, experts: int, n: int, k: int, dual: bool) -> bool:
+    """Whether one of the tcgen05 kernel's forms is faster than tiles of 32 x 64 on mma.sync, which start
+    sooner: those serve short rows of weights and few rows of narrow models (us, tile / tcgen05: 2
+    rows of 16 experts of 64 x 48 2.1 / 4.5, 32 rows of 16 experts of 1024 x 512 7.0 / 8.4; 128 rows of 2 experts of
+    1024 x 1024 10.2 / 8.7, 8,000 rows of 32 experts of 2048 x 1024 222 / 61)."""
+    cost = {form: _cost(form, rows, experts, n, k, dual) for form in FORMS[dual]}
+    return min(cost["few"], cost["large"]) < cost["tile"]
+
+
+def few_tiles(rows: int, experts: int, n: int, dual: bool, k: int = 1024) -> bool:
+    """Whether the grouped product of `rows` rows takes the tcgen05 kernel's small tiles."""
+    return _cost("few", rows, experts, n, k, dual) < _cost("large", rows, experts, n, k, dual)
 
 
 def tile_rows() -> int:
@@ -142,14 +158,17 @@ def grouped_product(rows: torch.Tensor, r: Routing, w0: torch.Tensor, w1: torch.
     n, k = w0.shape[1], w0.shape[2]
     out = torch.empty((rows.shape[0], n), dtype=rows.dtype if w1 is not None else torch.float32,
                       device=rows.device)
-    if tc_takes(rows, w0, w1):
+    total, dual = r.tokens * r.top, w1 is not None
+    if total == 0:
+        return out
+    if tc_takes(rows, w0, w1) and tc_faster(total, r.experts, n, k, dual):
         call("sakv_moe_tc", ptr(rows), rows.shape[0], ptr(w0), ptr(w1), ptr(r.offsets), r.experts,
              ptr(out), n, k, float(limit), float(alpha), float(plus),
-             int(few_tiles(r.tokens * r.top, r.experts, n, w1 is not None)))
+             int(few_tiles(total, r.experts, n, dual, k)))
         return out
     call("sakv_moe_product", ptr(rows), dtype_code(rows.dtype), ptr(w0), ptr(w1), w0.stride(0),
          ptr(r.tile_expert), ptr(r.tile_row), ptr(r.offsets), ptr(r.n_tiles), r.max_tiles,
-         ptr(out), n, k, int(w1 is not None), float(limit), float(alpha), float(plus))
+         ptr(out), n, k, int(dual), float(limit), float(alpha), float(plus))
     return out
 
 

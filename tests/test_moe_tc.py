@@ -20,6 +20,43 @@ def test_the_rules_of_the_tiles():
     assert not mixture.few_tiles(6000, 2, 1024, False)
 
 
+@pytest.mark.parametrize("rows,experts,n,k,dual,faster", [
+    (2, 16, 64, 48, False, "tile"), (4000, 4, 48, 64, True, "tile"), (32, 16, 1024, 512, False, "tile"),
+    (8000, 32, 64, 48, False, "tile"), (8, 8, 256, 256, True, "tile"), (128, 2, 1024, 1024, False, "few"),
+    (2, 16, 1024, 1024, True, "few"), (8, 4, 1024, 2048, True, "few"), (400, 4, 1024, 1024, True, "large"),
+    (1200, 4, 1024, 1024, False, "large"), (8000, 32, 2048, 1024, False, "large")])
+def test_a_product_takes_the_form_that_was_measured_to_be_the_fastest(rows, experts, n, k, dual, faster):
+    assert mixture.tc_faster(rows, experts, n, k, dual) == (faster != "tile")
+    if faster != "tile":
+        assert mixture.few_tiles(rows, experts, n, dual, k) == (faster == "few")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,experts,top,width,ff", [(1, 4, 2, 64, 48), (33, 16, 2, 256, 256), (70, 4, 2, 1024, 512)])
+def test_a_grouped_product_is_the_same_in_every_form(tokens, experts, top, width, ff, monkeypatch):
+    """bfloat16 products are exact in fp32; the sums may be taken in another order (2^-24 a term)."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+
+    def draw(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    r = mixture.route(draw(tokens, experts), experts, top)
+    rows = mixture.gather_rows(draw(tokens, width).to(torch.bfloat16), r, False)
+    gate, up = draw(experts, ff, width).to(torch.bfloat16), draw(experts, ff, width).to(torch.bfloat16)
+    got = {}
+    for form in ("tile", "few", "large"):
+        with monkeypatch.context() as m:
+            m.setattr(mixture, "tc_faster", lambda *a: form != "tile")
+            m.setattr(mixture, "few_tiles", lambda *a: form == "few")
+            got[form] = (mixture.grouped_product(rows, r, gate, None),
+                         mixture.grouped_product(rows, r, gate, up, 30.0, 1.5).float())
+    bound = 4 * width ** 0.5 * 2.0 ** -24 * float((rows.float().abs() @ gate.float().abs().amax(0).T).max())
+    for form in ("few", "large"):
+        assert float((got[form][0] - got["tile"][0]).abs().max()) <= bound
+        off = (got[form][1] - got["tile"][1]).abs() - 2.0 ** -7 * got["tile"][1].abs()
+        assert float(off.max()) <= 100 * bound                  # (times the other factor, at most 31)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("few", [True, False])
 @pytest.mark.parametrize("n,k", [(8, 8), (64, 72), (136, 200), (264, 1032)])
