@@ -53,6 +53,13 @@ __global__ void logits_kernel(const T* __restrict__ h, const float* __restrict__
   if (lane == 0) out[item] = sum;
 }
 
+// Whether sixteen sums a warp are the faster split: with 80 sums an SM there are warps enough, and a
+// tile of two outputs is half empty (us, a warp a sum / sixteen: 64 tokens of 36 outputs of 2,048 4.9 / 11.6, 400
+// of 16 of 1,024 5.0 / 6.9, 800 of 16 7.2 / 7.0, 400 of 36 of 2,048 13.1 / 11.6, 3,200 of 2 5.1 / 6.8, 3,200 of 4 7.0 / 6.8).
+bool logits_in_tiles(int tokens, int outputs) {
+  return outputs > 2 && (long long)tokens * outputs >= 80LL * sm_count();
+}
+
 // The same for many tokens: a warp takes four tokens and four outputs, so that a piece of a row and of
 // a weight row is read once for four sums; every sum has the same terms in the same order. (A warp a
 // sum read the 300 KB of weights once a token: 3,001 tokens, 36 outputs of 2,048: 75 -> 35 us.)
@@ -581,6 +588,7 @@ combine4_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot
 }  // namespace
 
 SAKV_EXPORT int sakv_moe_tile_rows() { return TM; }
+SAKV_EXPORT int sakv_moe_logits_in_tiles(int tokens, int outputs) { return logits_in_tiles(tokens, outputs); }
 
 static bool form_fits(int experts, int top, int groups, int keep, int group_top) {
   return (group_top == 1 || group_top == 2) && groups >= 1 && groups <= 64 && experts % groups == 0 && keep >= 1 && keep <= groups &&
@@ -637,13 +645,13 @@ SAKV_EXPORT int sakv_moe_logits(const void* h, int dtype, const float* w, float*
   const long long blocks = (count * 32 + 255) / 256;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   const dim3 grid((unsigned)blocks), block(256);
-  // (from 64 tokens on there are warps enough with sixteen sums each)
+  const bool in_tiles = logits_in_tiles(tokens, outputs);
   const long long tiles = (tokens + 3LL) / 4 * ((outputs + 3) / 4);
   const dim3 grid4((unsigned)((tiles * 32 + 255) / 256));
-  if (tokens >= 64 && dtype == SAKV_F32)
+  if (in_tiles && dtype == SAKV_F32)
     return launch_ordered(logits_tile_kernel<float>, grid4, block, 0, stream, (const float*)h, w,
                              out, outputs, width, tokens);
-  if (tokens >= 64 && dtype == SAKV_BF16)
+  if (in_tiles && dtype == SAKV_BF16)
     return launch_ordered(logits_tile_kernel<__nv_bfloat16>, grid4, block, 0, stream,
                              (const __nv_bfloat16*)h, w, out, outputs, width, tokens);
   if (dtype == SAKV_F32)

@@ -1,0 +1,13 @@
+"""Which form a kernel with several takes at which sizes (no GPU needed; on 148 SMs): what was measured to be
+the faster one. That the forms agree is tested in `test_tile_forms_gpu.py`."""
+
+import pytest
+
+from semantic_aware_adaptive_kv_cache_precision_b200.ops._lib import plain_function
+
+
+@pytest.mark.parametrize("tokens,outputs,tiles", [(64, 36, 0), (64, 128, 0), (400, 16, 0), (3200, 2, 0), (100000, 2, 0),
+                                                  (800, 16, 1), (400, 36, 1), (100, 128, 1), (3200, 4, 1),
+                                                  (2 ** 20, 4096, 1)])
+def test_router_logits_in_tiles_only_where_there_are_many(tokens, outputs, tiles):
+    assert plain_function("sakv_moe_logits_in_tiles")(tokens, outputs) == tiles

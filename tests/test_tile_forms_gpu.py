@@ -29,7 +29,8 @@ def test_a_row_of_the_32_bit_product_is_the_same_in_every_tile(M, N, K):
         assert torch.equal(ops.linear(x[:rows], w, bias), got[:rows])
 
 
-@pytest.mark.parametrize("tokens,outputs,width", [(64, 5, 96), (67, 36, 200), (130, 1, 33), (65, 4, 2048)])
+@pytest.mark.parametrize("tokens,outputs,width", [(64, 5, 96), (67, 36, 200), (130, 1, 33), (65, 4, 2048),
+                                                  (2501, 5, 96), (701, 36, 200), (8000, 3, 33), (402, 33, 2048)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_router_logits_of_many_tokens_are_those_of_one(tokens, outputs, width, dtype):
     h, w = draw(tokens, width).to(dtype), draw(outputs, width, seed=1)
