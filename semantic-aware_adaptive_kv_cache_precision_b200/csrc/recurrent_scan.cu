@@ -800,7 +800,10 @@ norm_gate_vec_kernel(const float* __restrict__ y, const W* __restrict__ w,
       if (gate) read8(gate + t * gate_stride + c, g[p]);
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[p][i] = g[p][i] = 0.f;
+      for (int i = 0; i < 8; ++i) {
+        v[p][i] = 0.f;
+        g[p][i] = 1.f;         // (0 / x would take the division's slow path, for the whole warp)
+      }
     }
   }
   if (gate) {
