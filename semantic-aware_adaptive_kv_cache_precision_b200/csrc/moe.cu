@@ -540,6 +540,14 @@ __global__ void combine_kernel(const float* __restrict__ rows, const int32_t* __
   }
 }
 
+// Whether the next form is the faster one: a block takes one token, so its threads want columns enough
+// and the launch tokens enough (us, a column a thread / four: 8 tokens of 4 choices, 1,024 columns 2.4 / 2.7, 256 3.3 /
+// 2.9; 1,024 tokens, 256 columns 3.3 / 2.9, 128 columns 2.6 / 2.8; 4,096 tokens, 128 columns 5.0 / 6.5, 256 columns
+// 7.5 / 6.7, 1,024 columns 26 / 11).
+bool combine_by_tokens(int tokens, int width) {
+  return width >= 256 && (long long)tokens * width >= 1750LL * sm_count();
+}
+
 // The same with four columns a thread in 16-byte accesses, a block's threads along one token's columns
 // (3,001 tokens of 4 choices, 2,048 columns: 58 -> 32 us).
 template <typename T>
@@ -588,6 +596,7 @@ combine4_kernel(const float* __restrict__ rows, const int32_t* __restrict__ slot
 }  // namespace
 
 SAKV_EXPORT int sakv_moe_tile_rows() { return TM; }
+SAKV_EXPORT int sakv_moe_combine_by_tokens(int tokens, int width) { return combine_by_tokens(tokens, width); }
 SAKV_EXPORT int sakv_moe_logits_in_tiles(int tokens, int outputs) { return logits_in_tiles(tokens, outputs); }
 
 static bool form_fits(int experts, int top, int groups, int keep, int group_top) {
@@ -759,7 +768,8 @@ SAKV_EXPORT int sakv_moe_combine(const float* rows, const int32_t* slot_of, cons
   if (tokens == 0) return 0;
   const long long count = (long long)tokens * width;
   const dim3 grid(grid_for(count, 256)), block(256);
-  if (width % 4 == 0 && !(((uintptr_t)rows | (uintptr_t)shared | (uintptr_t)out) & 15)) {
+  if (combine_by_tokens(tokens, width) && width % 4 == 0 &&
+      !(((uintptr_t)rows | (uintptr_t)shared | (uintptr_t)out) & 15)) {
     const dim3 grid4(tokens, width > 1024 ? (width + 1023) / 1024 : 1);
     if (grid4.y <= 65535 && h_dtype == SAKV_F32)
       return launch_ordered(combine4_kernel<float>, grid4, block, 0, stream, rows, slot_of, weights,

@@ -11,3 +11,9 @@ from semantic_aware_adaptive_kv_cache_precision_b200.ops._lib import plain_funct
                                                   (2 ** 20, 4096, 1)])
 def test_router_logits_in_tiles_only_where_there_are_many(tokens, outputs, tiles):
     assert plain_function("sakv_moe_logits_in_tiles")(tokens, outputs) == tiles
+
+
+@pytest.mark.parametrize("tokens,width,by_tokens", [(8, 1024, 0), (64, 1024, 0), (4096, 64, 0), (4096, 128, 0),
+                                                    (1024, 256, 1), (256, 1024, 1), (4096, 2048, 1)])
+def test_a_token_a_block_sums_the_experts_rows_only_in_long_steps(tokens, width, by_tokens):
+    assert plain_function("sakv_moe_combine_by_tokens")(tokens, width) == by_tokens

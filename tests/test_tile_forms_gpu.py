@@ -61,10 +61,11 @@ def test_the_gated_norm_at_every_width(width, group, gate_silu, gate_first, gate
     assert float((got.double() - want).abs().max()) <= 2e-5 * float(want.abs().max())
 
 
-@pytest.mark.parametrize("width", [36, 1024, 2052, 30])
+@pytest.mark.parametrize("tokens,width", [(70, 36), (70, 1024), (70, 2052), (70, 30), (300, 1024), (1100, 260), (150, 2052),
+                                          (1100, 262)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-def test_rows_gathered_and_summed_at_every_width(width, dtype):
-    tokens, experts, top, identity = 70, 5, 3, 2
+def test_rows_gathered_and_summed_at_every_width(tokens, width, dtype):
+    experts, top, identity = 5, 3, 2
     h = draw(tokens, width).to(dtype)
     logits = draw(tokens, experts + identity, seed=3)
     r = mixture.route(logits, experts, top, identity)
@@ -81,3 +82,8 @@ def test_rows_gathered_and_summed_at_every_width(width, dtype):
         want = want + torch.where(real, 2.0 * x.to(dtype).double(), x)
     tolerance = 1e-5 if dtype == torch.float32 else 2e-2        # (a weighted row is rounded to its type)
     assert float((into.double() - want).abs().max()) <= tolerance * float(want.abs().max())
+    few = mixture.route(logits[:9], experts, top, identity)          # (the same tokens in a short step)
+    products = mixture.gather_rows(h[:9], few, True).float() * 2.0
+    again = before[:9].float()
+    mixture.combine(products, few, False, shared[:9], gate[:9], h[:9], again)
+    assert torch.equal(again, into[:9])
