@@ -102,6 +102,14 @@ __global__ void causal_conv_kernel(const float* __restrict__ in, long long strid
 // inputs are asked for together and each read once instead of once a tap (a sequence that begins
 // among them fills the window anew). Bound by memory: 3,400 tokens of 4,096 channels 113 -> 44 us.
 constexpr int kConvTokens = 8;
+
+// Whether that form is the faster one: a thread's eight tokens are a chain, so there have to be threads
+// enough (us, a token a thread / eight in a row: 9 tokens of 4,096 channels 4.3 / 5.4, 128 of 1,024 4.8 / 5.2, 64 of 2,304
+// 4.8 / 5.3, 64 of 4,096 5.7 / 5.4, 256 of 1,024 5.7 / 5.2, 512 of 1,024 7.8 / 5.5).
+bool conv_by_runs(int tokens, int channels, int taps) {
+  return taps == 4 && (long long)tokens * channels >= 1400LL * sm_count();
+}
+
 template <typename W, typename C>
 __global__ void __launch_bounds__(256)
 causal_conv4_kernel(const float* __restrict__ in, long long stride, const W* __restrict__ w,
@@ -915,6 +923,10 @@ int lanes_for(int n, int per_lane) {          // a power of two of lanes that ho
 // [channels, taps], bias [channels] (null: none) of `w_dtype`; state: fp32 [slots, taps - 1,
 // channels], read here and replaced by `sakv_conv_state` afterwards. out: [tokens, channels]
 // of `out_dtype` = silu(convolution).
+SAKV_EXPORT int sakv_conv_by_runs(int tokens, int channels, int taps) {
+  return conv_by_runs(tokens, channels, taps);
+}
+
 SAKV_EXPORT int sakv_causal_conv(const float* in, long long stride, const void* w,
                                  const void* bias, int w_dtype, const float* state,
                                  const int32_t* cu_seqlens, const int32_t* token_seq,
@@ -924,11 +936,12 @@ SAKV_EXPORT int sakv_causal_conv(const float* in, long long stride, const void* 
   if (tokens == 0) return 0;
   const long long count = (long long)tokens * channels;
   const dim3 grid(grid_for(count, 256)), block(256);
+  const bool by_runs = conv_by_runs(tokens, channels, taps);
   const long long runs = (tokens + kConvTokens - 1) / kConvTokens;
   const dim3 grid4((unsigned)((channels + 255) / 256), (unsigned)(runs < 65535 ? runs : 65535));
 #define SAKV_CONV(W, C)                                                                          \
   do {                                                                                           \
-  if (taps == 4)                                                                                 \
+  if (by_runs)                                                                                   \
     return launch_ordered(causal_conv4_kernel<W, C>, grid4, block, 0, stream, in, stride,  \
                              (const W*)w, (const W*)bias, state, cu_seqlens, token_seq, slots,   \
                              (C*)out, tokens, channels);                                         \

@@ -115,6 +115,7 @@ PLAIN_SIGNATURES = {
     "sakv_gemm_tc_max_clusters": ("gemm_tc", [I, I, I]),
     "sakv_moe_tc_error": ("moe_tc", [P]),
     "sakv_moe_logits_in_tiles": ("moe", [I, I]),
+    "sakv_conv_by_runs": ("recurrent_scan", [I, I, I]),
     "sakv_moe_combine_by_tokens": ("moe", [I, I]),
     "sakv_gemm_tc_error": ("gemm_tc", [P]),
 }

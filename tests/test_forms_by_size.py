@@ -17,3 +17,10 @@ def test_router_logits_in_tiles_only_where_there_are_many(tokens, outputs, tiles
                                                     (1024, 256, 1), (256, 1024, 1), (4096, 2048, 1)])
 def test_a_token_a_block_sums_the_experts_rows_only_in_long_steps(tokens, width, by_tokens):
     assert plain_function("sakv_moe_combine_by_tokens")(tokens, width) == by_tokens
+
+
+@pytest.mark.parametrize("tokens,channels,taps,runs", [(9, 4096, 4, 0), (128, 1024, 4, 0), (64, 2304, 4, 0),
+                                                       (64, 4096, 4, 1), (256, 1024, 4, 1), (3400, 4096, 4, 1),
+                                                       (3400, 4096, 3, 0)])
+def test_eight_tokens_a_thread_in_the_convolution_only_in_long_steps(tokens, channels, taps, runs):
+    assert plain_function("sakv_conv_by_runs")(tokens, channels, taps) == runs

@@ -1,6 +1,8 @@
 """Kernels that choose a form by the sizes of a call: every form against float64, and against one
 another where the result must not depend on the form."""
 
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -87,3 +89,33 @@ def test_rows_gathered_and_summed_at_every_width(tokens, width, dtype):
     again = before[:9].float()
     mixture.combine(products, few, False, shared[:9], gate[:9], h[:9], again)
     assert torch.equal(again, into[:9])
+
+
+@pytest.mark.parametrize("channels,counts", [(520, [300, 1, 2, 3, 5, 90, 4]), (4096, [61, 3, 1, 1]), (1300, [170])])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_the_convolution_of_a_long_step_is_that_of_short_ones(channels, counts, dtype):
+    """Sequences begin anywhere among a thread's eight tokens; some have inputs from before the step."""
+    tokens, taps = sum(counts), 4
+    x, w, b = draw(tokens, channels), draw(channels, taps, seed=1).to(dtype), draw(channels, seed=2).to(dtype)
+    before = draw(len(counts), taps - 1, channels, seed=3)
+
+    def conv(rows, counts, state):
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+        starts = [sum(counts[:i]) for i in range(len(counts) + 1)]
+        step = SimpleNamespace(sequences=len(counts), cu_seqlens=ints(starts), slots=ints(list(range(len(counts)))),
+                               token_seq=ints([i for i, c in enumerate(counts) for _ in range(c)]))
+        return ops.causal_conv(rows, channels, w, b, state, step, dtype)
+
+    state = before.clone()
+    got = conv(x, counts, state)
+    at = 0
+    for i, n in enumerate(counts):
+        alone = before[i:i + 1].clone()
+        parts = [conv(x[p:min(p + 33, at + n)], [min(33, at + n - p)], alone) for p in range(at, at + n, 33)]
+        assert torch.equal(torch.cat(parts), got[at:at + n]) and torch.equal(alone[0], state[i])
+        inputs = torch.cat([before[i], x[at:at + n]]).double()
+        sums = sum(inputs[j:j + n] * w[:, j].double() for j in range(taps)) + b.double()
+        want = sums * torch.sigmoid(sums)
+        off = (got[at:at + n].double() - want).abs() - (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs()
+        assert float(off.max()) <= 1e-5 * float(want.abs().max())
+        at += n
