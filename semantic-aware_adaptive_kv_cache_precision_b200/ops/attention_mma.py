@@ -37,9 +37,11 @@ def attention(q, head_stride, k_cache, v_cache, positions, token_seq, block_tabl
               map_gate_off=None, lam=0.0, out_scale=1.0, eps=0.0, decode=False, key_splits=1,
               ordered=True, cu_seqlens=None):
     """The arguments as `ops.cached_attention` and `ops.distance_attention` have checked them.
-    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt, of one sequence with `cu_seqlens` (int32 [sequences + 1]: where
-    every sequence's tokens begin), of one run of consecutive tokens without. `ordered`: the kernels begin when the one before them has
-    ended (False: overlapped with it, for a caller whose neighbours are this library's own kernels)."""
+    `decode`: a block (and `key_splits` of them) takes one token; else 64 rows of a prompt, of one
+    sequence with `cu_seqlens` (int32 [sequences + 1]: where every sequence's tokens begin), of one
+    run of consecutive tokens without. `ordered`: the kernels begin when the one before them has
+    ended (False: overlapped with it, for a caller whose neighbours are this library's own
+    kernels)."""
     tokens = q.shape[0]
     out = torch.empty((tokens, heads * vdim), dtype=q.dtype, device=q.device)
     if not decode:
