@@ -158,7 +158,8 @@ class StepStager:
         if device_tokens is not None and not in_place:
             views["token_ids"].copy_(device_tokens)
         return StepContext(
-            tokens=T, sequences=B, **views, tables=list(dev_tables), new_counts=counts, starts=list(starts), host_slots=list(slots),
+            tokens=T, sequences=B, **views, tables=list(dev_tables), new_counts=counts,
+            starts=list(starts), host_slots=list(slots),
             max_position=max(ends) - 1 if ends else 0, max_new=max(counts, default=0),
             max_len=max(ends, default=0), is_decode=all(c == 1 for c in counts),
             max_len_bound=min(width, max((t.shape[1] for t in tables), default=width)) * BLOCK)

@@ -25,6 +25,8 @@ _FUSED = ("r", "k", "v", "g", "a", "w1")
 
 
 class DeltaRuleMixer(Part):
+    kernel_libraries = ("delta_rule", "gemm_f32", "gemm_tc")
+
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)
         if spec.head_dim > 256:

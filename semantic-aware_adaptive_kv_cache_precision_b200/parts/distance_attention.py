@@ -21,6 +21,8 @@ from .base import Part, register_part
 
 
 class LogDistanceAttention(Part):
+    kernel_libraries = ("attention_distance", "attention_mma", "gemm_f32", "gemm_tc")
+
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)
         s = spec

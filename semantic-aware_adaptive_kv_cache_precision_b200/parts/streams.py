@@ -55,6 +55,8 @@ class StreamBlock(Part):
         self.parts = tuple(x for x in (self.mixer_norm, self.mixer, self.ffn_norm, self.ffn)
                            if x is not None)
         self.graph_safe = all(getattr(part, "graph_safe", True) for part in self.parts)
+        self.kernel_libraries = ("streams",) + tuple(
+            n for part in self.parts for n in getattr(part, "kernel_libraries", ()))
         self.hc = {}
         self.shift = None
 

@@ -101,3 +101,12 @@ def test_the_plain_model_carries_its_state_as_the_equations_say():
     h = rng.standard_normal((n, 7))
     shifted = plain.token_shift(h, np.full(7, 0.25))
     assert np.allclose(shifted[0], 0.75 * h[0]) and np.allclose(shifted[3], 0.75 * h[3] + 0.25 * h[2])
+
+
+def test_a_model_names_the_kernel_libraries_of_its_mixers():
+    """They are compiled side by side when the model is loaded; one that is not named is compiled inside
+    the first step."""
+    spec = sakv.config_from_dict(MIXED).model_spec()
+    names = DecoderModel(spec, "bfloat16", "cpu").kernel_libraries()
+    assert {"streams", "delta_rule", "attention_distance", "attention_mma", "gemm_f32", "gemm_tc"} <= set(names)
+    assert len(names) == len(set(names))
