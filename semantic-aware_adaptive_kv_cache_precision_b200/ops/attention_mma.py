@@ -16,11 +16,12 @@ def takes(q: torch.Tensor, head_stride: int, k_cache: torch.Tensor, v_cache, dim
           maps: int = 1, q2=None, q_split: int = 0) -> bool:
     """Whether the tensor-core kernel takes the call: bfloat16, one of the compiled pairs of
     widths, and every row of queries, keys and values beginning at a multiple of 16 bytes (they are
-    copied in pieces of 16). It is the faster one for all of these, from one decoded token on
-    and in steps that mix decoded tokens with a prompt (against the kernel that scores a key a lane, us, 16
-    heads over latent rows and 8 heads of 2 at 128 columns: a prompt of 3,001 tokens 14,597 -> 1,131 and
-    2,587 -> 244; 8 decoded tokens of 2,048 keys 132 -> 37 and 74 -> 39; the mixed steps in
-    `csrc/attention_mma.cu`)."""
+    copied in pieces of 16). Against the kernel that scores a key a lane, us, 16 heads over latent rows
+    and 8 heads of 2 at 128 columns: a prompt of 3,001 tokens 14,597 -> 1,131 and 2,587 -> 244; 8 decoded
+    tokens of 2,048 keys 132 -> 37 and 74 -> 39; the steps that mix both in `csrc/attention_mma.cu`. Of 150
+    calls from one token on it is slower only where a block's rows are nearly all empty: prompts of 16
+    tokens with a head a key/value head 8 -> 11 (they stay here: a prompt's result must not depend
+    on how it is cut)."""
     if q.dtype != torch.bfloat16 or SHAPES.get((dim, vdim, v_cache is None), 0) < maps:
         return False
     rows = [(q, q.stride(0), head_stride), (k_cache, k_cache.shape[3], 0)]

@@ -30,9 +30,10 @@ ROUTE_IN_ONE_BLOCK = 64
 
 #: What a grouped product takes in each form, us: (start, a column of K, tiles that run side by side,
 #: rows and weight rows of a tile), where a product of K columns and `tiles` tiles takes
-#: start + K * column * max(1, tiles / side by side). Fitted to 750 products of 2 to 64 experts, 2 to 12,000 rows
-#: and K of 48 to 2,048, weights from memory; the form chosen with them takes 1.01 times the fastest one's time on
-#: average and at most 1.5 (the tcgen05 forms alone 1.23 and 2.7, the tiles of 32 x 64 alone 1.44).
+#: start + K * column * max(1, tiles / side by side). Fitted to 750 products of 2 to 64 experts, 2 to
+#: 12,000 rows and K of 48 to 2,048, weights from memory; the form chosen with them takes 1.01 times the
+#: fastest one's time on average and at most 1.5 (the tcgen05 forms alone 1.23 and 2.7, the tiles of
+#: 32 x 64 alone 1.44).
 FORMS = {False: {"tile": (2.2, 0.0064, 240, 32, 64), "few": (4.6, 0.0036, 121, 32, 64),
                  "large": (5.3, 0.0062, 78, 128, 256)},
          True: {"tile": (2.8, 0.0141, 307, 32, 64), "few": (5.4, 0.0040, 134, 32, 32),
@@ -55,9 +56,9 @@ def tc_takes(rows: torch.Tensor, w0: torch.Tensor, w1: torch.Tensor | None) -> b
 
 def tc_faster(rows: int, experts: int, n: int, k: int, dual: bool) -> bool:
     """Whether one of the tcgen05 kernel's forms is faster than tiles of 32 x 64 on mma.sync, which start
-    sooner: those serve short rows of weights and few rows of narrow models (us, tile / tcgen05: 2
-    rows of 16 experts of 64 x 48 2.1 / 4.5, 32 rows of 16 experts of 1024 x 512 7.0 / 8.4; 128 rows of 2 experts of
-    1024 x 1024 10.2 / 8.7, 8,000 rows of 32 experts of 2048 x 1024 222 / 61)."""
+    sooner: those serve short rows of weights and few rows of narrow models (us, tile / tcgen05: 2 rows
+    of 16 experts of 64 x 48 2.1 / 4.5, 32 rows of 16 experts of 1024 x 512 7.0 / 8.4; 128 rows of 2
+    experts of 1024 x 1024 10.2 / 8.7, 8,000 rows of 32 experts of 2048 x 1024 222 / 61)."""
     cost = {form: _cost(form, rows, experts, n, k, dual) for form in FORMS[dual]}
     return min(cost["few"], cost["large"]) < cost["tile"]
 
