@@ -30,7 +30,7 @@
 // The products run on mma.sync. Over latent rows the sums of 128 rows x 512 columns would fill the whole
 // of tensor memory and the weights' pieces would pass through it three times. At 128 / 128 columns a
 // form on tcgen05 (as `csrc/attention_prefill_tc.cu`) is possible and not built: 3,001 tokens of 8 heads
-// of 2 take 245 us, 0.15 PFLOP/s of useful work, three products of P V to one of Q K^T.
+// of 2 take 245 us, 0.075 PFLOP/s of useful work, 0.15 with three products of P V to one of Q K^T.
 #include <float.h>
 
 #include "common.cuh"
