@@ -13,13 +13,13 @@
 // the experts' row offsets on the device.
 //
 //   XR 128, HB 128   prompts: one tcgen05.mma is 128 x 256 x 16 (the tensor cores' full rate), four
-//                    stages of 48 KB. 3,001 tokens of 4 choices among 32 experts, 2 x 1024 x 2048: 104
-//                    us (0.97 PFLOP/s), 530 before on mma.sync in tiles of 32 x 64; 3,160 tokens with 2
-//                    experts, 2 x 1024 x 1024, 31 us, 156 before
+//                    stages of 48 KB. 3,001 tokens of 4 choices among 32 experts, 2 x 1024 x 2048: 101
+//                    us (1.0 PFLOP/s), 530 before on mma.sync in tiles of 32 x 64; 3,160 tokens with 2
+//                    experts, 2 x 1024 x 1024, 27 us, 156 before
 //   XR 32, HB 32     few rows an expert: what counts is that the weights stream, through as many SMs
 //                    as there are tiles; a box of 32 rows, the MMA's other 96 lanes hold whatever lies
 //                    behind them and nobody reads their sums. One token of 4 experts, 2 x
-//                    1024 x 2048: 21 us, 41 before
+//                    1024 x 2048: 14 us, 32 before
 //
 //   warp 0     TMA: boxes of 64 columns of the rows and of the weights into the ring
 //   warp 1     tensor memory; lane 0 issues the products and commits stages and accumulators
