@@ -44,6 +44,7 @@ LIBRARIES = {
     "attention_prefill": "attention_prefill.cu",
     "attention_prefill_tc": "attention_prefill_tc.cu",
     "gemm_tc": "gemm_tc.cu",
+    "gemm_few": "gemm_few.cu",
     "gemm_wide": "gemm_wide.cu",
     "gemm_pair": "gemm_pair.cu",
     "gemm_lib": "gemm_lib.cu",

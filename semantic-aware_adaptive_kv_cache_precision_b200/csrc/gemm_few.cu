@@ -1,0 +1,204 @@
+// The bf16 matrix product of a step of up to 16 tokens: C[m, n] = sum_k X[m, k] W[n, k], weights straight
+// from memory into registers.
+//
+// With this few tokens a product is the streaming of its weights plus what a kernel costs before the first
+// and after the last of them, and in a decode step, a chain of such products of a few megabytes, it is
+// mostly the latter. csrc/gemm_tc.cu (tensor maps, mbarriers, tensor memory, clusters that add their K
+// ranges through each other's shared memory) pays 4 us from one kernel's end to the next for products
+// whose bytes take 1. Here a block of eight warps has 16 rows of W and all of K; a warp asks for its first
+// weights while the kernel before is still running, with nothing to set up and no shared memory that the
+// kernel before could be holding; after the wait come one trip to L2 for x, the products (mma.sync
+// m16n8k16), one meeting of the block and the store.
+//
+// The tensor cores' K index may be any permutation of the columns as long as both operands use the same
+// one: a lane takes eight neighbouring columns of a row with one 16-byte load, and they serve as its
+// numbers of two products. So both operands go from memory to the tensor cores without passing through
+// shared memory, and a warp's load is 64 contiguous bytes of each of eight rows. The warps take groups of
+// 32 columns in turn. Sums are fp32, a warp's own first, then the eight warps' in their order.
+//
+// Epilogues as in csrc/gemm_tc.cu. `parts` > 1: K is cut into that many ranges for blocks of their own
+// (few rows, long K), whose sums are left apart for the reader to add.
+#include "common.cuh"
+#include "mma.cuh"
+
+namespace {
+
+constexpr int kWarps = 8, kThreads = 32 * kWarps;
+constexpr int kRows = 16;
+
+enum : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_ACCUM = 2, EPI_GATED = 3, EPI_CLAMPED = 4, EPI_RELU2 = 5 };
+constexpr bool gated_epi(int epi) { return epi == EPI_GATED || epi == EPI_CLAMPED; }
+
+struct Few {
+  const __nv_bfloat16* x;
+  long long ldx;
+  const __nv_bfloat16* w;            // [rows, K]
+  int M, N, K;
+  int groups;                        // groups of 32 columns of one part
+  int dual_offset;
+  float limit, alpha, plus;
+  const void* bias;
+  int bias_dtype;
+  void* out;
+  long long ldo, part_stride;
+};
+
+__device__ __forceinline__ uint4 stream16(const __nv_bfloat16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ float bias_of(const Few& p, int n) {
+  if (!p.bias) return 0.f;
+  return p.bias_dtype == SAKV_F32 ? static_cast<const float*>(p.bias)[n]
+                                  : widen(static_cast<const __nv_bfloat16*>(p.bias)[n]);
+}
+
+// NT: groups of eight tokens.
+template <int NT, int kEpi>
+__global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
+  constexpr int kSets = gated_epi(kEpi) ? 2 : 1;       // gate and up rows
+  constexpr int kAhead = kSets == 2 ? 3 : 6;           // groups of columns asked for at a time
+  __shared__ float sums[kSets][kWarps][NT * 8][kRows + 1];
+  let_next_kernel_start();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n0 = blockIdx.x * kRows, part = blockIdx.y;
+  const int row = lane >> 2, col = (lane & 3) * 8;
+  // (rows beyond the last are the last one again, and not stored)
+  const __nv_bfloat16* from[kSets][2];
+#pragma unroll
+  for (int s = 0; s < kSets; ++s)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      from[s][h] = p.w + ((long long)s * p.dual_offset + min(n0 + row + 8 * h, p.N - 1)) * p.K + col;
+  const int first = part * p.groups, last = min(first + p.groups, (p.K + 31) / 32);
+  uint4 w[kAhead][kSets][2], x[kAhead][NT];
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  auto ask = [&](int i, int g) {
+    const bool in = g < last && g * 32 + col < p.K;
+#pragma unroll
+    for (int s = 0; s < kSets; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) w[i][s][h] = in ? stream16(from[s][h] + g * 32) : none;
+  };
+  auto ask_x = [&](int i, int g) {
+    const bool in = g < last && g * 32 + col < p.K;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int m = t * 8 + row;
+      x[i][t] = in && m < p.M
+                    ? __ldcg(reinterpret_cast<const uint4*>(p.x + m * p.ldx + g * 32 + col))
+                    : none;
+    }
+  };
+  float acc[kSets][NT][4];
+#pragma unroll
+  for (int s = 0; s < kSets; ++s)
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[s][t][k] = 0.f;
+
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) ask(i, first + warp + i * kWarps);
+  float bias = 0.f;
+  if (threadIdx.x < NT * 8 * kRows && n0 + (int)(threadIdx.x & 15) < p.N && part == 0)
+    bias = bias_of(p, n0 + (threadIdx.x & 15));
+  wait_for_previous_kernel();
+#pragma unroll
+  for (int i = 0; i < kAhead; ++i) ask_x(i, first + warp + i * kWarps);
+  for (int g0 = first + warp; g0 < last; g0 += kAhead * kWarps) {
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+#pragma unroll
+      for (int s = 0; s < kSets; ++s) {
+        const uint32_t a0[4] = {w[i][s][0].x, w[i][s][1].x, w[i][s][0].y, w[i][s][1].y};
+        const uint32_t a1[4] = {w[i][s][0].z, w[i][s][1].z, w[i][s][0].w, w[i][s][1].w};
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          mma::bf16_16816(acc[s][t], a0, x[i][t].x, x[i][t].y);
+          mma::bf16_16816(acc[s][t], a1, x[i][t].z, x[i][t].w);
+        }
+      }
+      const int next = g0 + (i + kAhead) * kWarps;
+      if (next < last) {
+        ask(i, next);
+        ask_x(i, next);
+      } else {                                        // (nothing is left of the last round)
+#pragma unroll
+        for (int s = 0; s < kSets; ++s) w[i][s][0] = w[i][s][1] = none;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) x[i][t] = none;
+      }
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < kSets; ++s)
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        sums[s][warp][t * 8 + (lane & 3) * 2 + (k & 1)][row + 8 * (k >> 1)] = acc[s][t][k];
+  __syncthreads();
+  const int r = threadIdx.x & 15, m = threadIdx.x >> 4, n = n0 + r;
+  if (m >= NT * 8 || m >= p.M || n >= p.N) return;
+  float c[kSets];
+#pragma unroll
+  for (int s = 0; s < kSets; ++s) {
+    c[s] = sums[s][0][m][r];
+#pragma unroll
+    for (int i = 1; i < kWarps; ++i) c[s] += sums[s][i][m][r];
+  }
+  const long long at = m * p.ldo + n + part * p.part_stride;
+  float* out32 = static_cast<float*>(p.out);
+  __nv_bfloat16* out16 = static_cast<__nv_bfloat16*>(p.out);
+  if (kEpi == EPI_F32) {
+    out32[at] = c[0] + bias;
+  } else if (kEpi == EPI_ACCUM) {
+    atomicAdd(out32 + at, c[0] + bias);      // (the only addition to this element)
+  } else if (kEpi == EPI_BF16) {
+    out16[at] = narrow<__nv_bfloat16>(c[0] + bias);
+  } else if (kEpi == EPI_RELU2) {
+    const float z = fmaxf(c[0] + bias, 0.f);
+    out16[at] = narrow<__nv_bfloat16>(z * z);
+  } else if (kEpi == EPI_CLAMPED) {
+    const float g = fminf(c[0], p.limit), u = fminf(fmaxf(c[kSets - 1], -p.limit), p.limit);
+    out16[at] = narrow<__nv_bfloat16>(g / (1.0f + expf(-p.alpha * g)) * (u + p.plus));
+  } else {
+    out16[at] = narrow<__nv_bfloat16>(c[0] / (1.0f + expf(-c[0])) * c[kSets - 1]);
+  }
+}
+
+}  // namespace
+
+// x: [M, K] bf16 rows `ldx` apart; w: [N, K] bf16 (gated: gate rows, and up rows from `dual_offset` on);
+// M up to 16, K and ldx multiples of 8, x and w at multiples of 16 bytes. epi, bias, out, ldo, clamp: as
+// `sakv_gemm_tc`. parts > 1 (EPI_F32): part i's sums at out + i * part_stride, the bias in part 0.
+SAKV_EXPORT int sakv_gemm_few(const void* x, long long ldx, const void* w, int M, int N, int K, int parts,
+                              int epi, int dual_offset, const void* bias, int bias_dtype, void* out,
+                              long long ldo, long long part_stride, float limit, float alpha, float plus,
+                              cudaStream_t stream) {
+  if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K % 8 || ldx % 8 || parts < 1 || parts > 64 || ldo < N ||
+      epi < 0 || epi > EPI_RELU2 || (parts > 1 && epi != EPI_F32) ||
+      (((uintptr_t)x | (uintptr_t)w) & 15))
+    return cudaErrorInvalidValue;
+  const int groups = (K + 31) / 32;
+  Few p = {(const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, (groups + parts - 1) / parts,
+           dual_offset, limit, alpha, plus, bias, bias_dtype, out, ldo, part_stride};
+  const dim3 grid((unsigned)((N + kRows - 1) / kRows), (unsigned)parts);
+#define SAKV_FEW(EPI)                                                                            \
+  if (epi == EPI)                                                                                \
+    return M <= 8 ? launch_overlapped(gemm_few_kernel<1, EPI>, grid, dim3(kThreads), 0, stream, 1, p) \
+                  : launch_overlapped(gemm_few_kernel<2, EPI>, grid, dim3(kThreads), 0, stream, 1, p)
+  SAKV_FEW(EPI_BF16);
+  SAKV_FEW(EPI_F32);
+  SAKV_FEW(EPI_ACCUM);
+  SAKV_FEW(EPI_GATED);
+  SAKV_FEW(EPI_CLAMPED);
+  SAKV_FEW(EPI_RELU2);
+#undef SAKV_FEW
+  return cudaErrorInvalidValue;
+}

@@ -89,6 +89,7 @@ SIGNATURES = {
     "sakv_prefill_attention_tc": ("attention_prefill_tc",
                                   [P, P, P, P, P, I, P, I, P, P, P, P, I, I, I, I, F, I, P]),
     "sakv_gemm_tc": ("gemm_tc", [P, P, I, I, I, I, I, I, I, I, P, I, P, L, L, F, F, F, P]),
+    "sakv_gemm_few": ("gemm_few", [P, L, P, I, I, I, I, I, I, P, I, P, L, L, F, F, F, P]),
     "sakv_gemm_wide": ("gemm_wide", [P, P, I, I, I, I, P, L, P]),
     "sakv_gemm_pair": ("gemm_pair", [P, P, I, I, I, I, P, L, I, F, F, F, P]),
     "sakv_lib_accumulate": ("gemm_lib", [P, L, P, P, L, I, I, I, P, L, P]),

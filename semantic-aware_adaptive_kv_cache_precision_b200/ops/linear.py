@@ -15,7 +15,7 @@ from __future__ import annotations
 
 import torch
 
-from . import gemm_tc, gemm_wide
+from . import gemm_few, gemm_tc, gemm_wide
 from ._lib import KernelError, call, ptr, require_cuda
 
 #: up to this many tokens the library's own tcgen05 kernel runs (weights on the MMA's rows:
@@ -76,6 +76,12 @@ def gated_up(x: torch.Tensor, w_gate_up: torch.Tensor, clamp: tuple | None = Non
     from . import gated_silu
     from .mixture import clamped_act
     inter = w_gate_up.shape[0] // 2
+    if gemm_few.takes(x, w_gate_up):
+        out = torch.empty((x.shape[0], inter), dtype=torch.bfloat16, device=x.device)
+        if clamp is not None:
+            return gemm_few.gemm(x, w_gate_up, None, gemm_tc.EPI_CLAMPED, out, inter,
+                                 dual_offset=inter, clamp=clamp)
+        return gemm_few.gemm(x, w_gate_up, None, gemm_tc.EPI_GATED, out, inter, dual_offset=inter)
     if x.shape[0] <= TC_MAX_TOKENS and inter % 128 == 0 and gemm_tc.takes(x, w_gate_up):
         out = torch.empty((x.shape[0], inter), dtype=torch.bfloat16, device=x.device)
         if clamp is not None:
@@ -97,7 +103,8 @@ def dense_up(x: torch.Tensor, w_up: torch.Tensor) -> torch.Tensor:
     from . import relu_squared
     if x.shape[0] <= TC_MAX_TOKENS and gemm_tc.takes(x, w_up):
         out = torch.empty((x.shape[0], w_up.shape[0]), dtype=torch.bfloat16, device=x.device)
-        return gemm_tc.gemm(x, w_up, None, gemm_tc.EPI_RELU2, out, w_up.shape[0])
+        gemm = gemm_few.gemm if gemm_few.takes(x, w_up) else gemm_tc.gemm
+        return gemm(x, w_up, None, gemm_tc.EPI_RELU2, out, w_up.shape[0])
     up = linear(x, w_up, out_dtype=x.dtype)
     return relu_squared(up, out=up)
 
@@ -171,6 +178,18 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     xb = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
     if tokens <= TC_MAX_TOKENS and gemm_tc.takes(xb, weight) and \
             (bias is None or bias.dtype in (torch.bfloat16, torch.float32)):
+        if gemm_few.takes(xb, weight):
+            if accumulate_into is not None:
+                parts = gemm_few.choose_parts(n, k) if may_defer and acc.is_contiguous() else 1
+                if parts > 1:
+                    sums = torch.empty((parts, tokens, n), dtype=torch.float32, device=x.device)
+                    return Deferred(gemm_few.gemm(xb, weight, bias, gemm_tc.EPI_F32, sums, n,
+                                                  parts=parts))
+                return gemm_few.gemm(xb, weight, bias, gemm_tc.EPI_ACCUM, acc, n)
+            if out_dtype in (torch.float32, torch.bfloat16):
+                out = torch.empty((tokens, n), dtype=out_dtype, device=x.device)
+                epi = gemm_tc.EPI_F32 if out_dtype == torch.float32 else gemm_tc.EPI_BF16
+                return gemm_few.gemm(xb, weight, bias, epi, out, n)
         if accumulate_into is not None:
             parts, splits = gemm_tc.choose_parts(tokens, n, k) \
                 if may_defer and acc.is_contiguous() else (1, 0)

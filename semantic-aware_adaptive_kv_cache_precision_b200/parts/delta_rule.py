@@ -25,7 +25,7 @@ _FUSED = ("r", "k", "v", "g", "a", "w1")
 
 
 class DeltaRuleMixer(Part):
-    kernel_libraries = ("delta_rule", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("delta_rule", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)

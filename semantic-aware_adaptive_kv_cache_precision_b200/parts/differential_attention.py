@@ -28,7 +28,7 @@ MAPS = 2
 
 
 class DifferentialAttention(Part):
-    kernel_libraries = ("attention_distance", "attention_mma", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("attention_distance", "attention_mma", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)

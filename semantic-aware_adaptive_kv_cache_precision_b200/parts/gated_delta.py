@@ -28,7 +28,7 @@ from .base import Part, register_part
 
 
 class GatedDeltaMixer(Part):
-    kernel_libraries = ("gated_delta", "recurrent_scan", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("gated_delta", "recurrent_scan", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)

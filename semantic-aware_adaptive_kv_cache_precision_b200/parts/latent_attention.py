@@ -29,7 +29,7 @@ from .base import Part, build_part, register_part
 
 
 class LatentAttention(Part):
-    kernel_libraries = ("latent", "attention_distance", "attention_mma", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("latent", "attention_distance", "attention_mma", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)

@@ -21,7 +21,7 @@ class GatedMLP(Part):
         self.clamp = (spec.limit, spec.alpha, spec.plus) if spec.activation == "clamped" else None
         self.kernel_libraries = ("moe" if self.clamp else "elementwise",)
         if mode == "bfloat16":
-            self.kernel_libraries += ("gemm_tc", "gemm_pair")
+            self.kernel_libraries += ("gemm_tc", "gemm_few", "gemm_pair")
         if spec.bias:
             raise ValueError("a gated feed-forward with biases is not built")
 

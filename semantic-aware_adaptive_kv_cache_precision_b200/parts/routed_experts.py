@@ -29,7 +29,7 @@ from .base import Part, register_part
 
 
 class RoutedExperts(Part):
-    kernel_libraries = ("moe", "moe_tc", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("moe", "moe_tc", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)

@@ -35,7 +35,7 @@ from .base import Part, build_part, register_part
 
 
 class WindowSinkAttention(Part):
-    kernel_libraries = ("qk_prepare", "attention_distance", "attention_mma", "gemm_f32", "gemm_tc")
+    kernel_libraries = ("qk_prepare", "attention_distance", "attention_mma", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)
