@@ -63,7 +63,6 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
   constexpr int kSets = gated_epi(kEpi) ? 2 : 1;       // gate and up rows
   constexpr int kAhead = kSets == 2 ? 3 : 6;           // groups of columns asked for at a time
   __shared__ float sums[kSets][kWarps][NT * 8][kRows + 1];
-  let_next_kernel_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kRows, part = blockIdx.y;
   const int row = lane >> 2, col = (lane & 3) * 8;
@@ -103,14 +102,15 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
       for (int k = 0; k < 4; ++k) acc[s][t][k] = 0.f;
 
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) ask(i, first + warp + i * kWarps);
+  for (int i = 0; i < kAhead; ++i) ask(i, first + warp * kAhead + i);
   float bias = 0.f;
   if (threadIdx.x < NT * 8 * kRows && n0 + (int)(threadIdx.x & 15) < p.N && part == 0)
     bias = bias_of(p, n0 + (threadIdx.x & 15));
   wait_for_previous_kernel();
+  let_next_kernel_start();
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) ask_x(i, first + warp + i * kWarps);
-  for (int g0 = first + warp; g0 < last; g0 += kAhead * kWarps) {
+  for (int i = 0; i < kAhead; ++i) ask_x(i, first + warp * kAhead + i);
+  for (int g0 = first + warp * kAhead; g0 < last; g0 += kAhead * kWarps) {
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
 #pragma unroll
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
           mma::bf16_16816(acc[s][t], a1, x[i][t].z, x[i][t].w);
         }
       }
-      const int next = g0 + (i + kAhead) * kWarps;
+      const int next = g0 + kAhead * kWarps + i;
       if (next < last) {
         ask(i, next);
         ask_x(i, next);
