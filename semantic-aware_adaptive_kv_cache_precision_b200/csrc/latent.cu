@@ -58,6 +58,73 @@ latent_prepare_kernel(const float* __restrict__ down, long long stride, int q_ra
   }
 }
 
+// The same for latents of up to 4,096 numbers, multiples of four: the query latent (blockIdx.y 1) and the
+// cache row (0) are blocks of their own, which ask for all they read at once and keep it in registers, N
+// groups of four neighbouring numbers a thread. (One block a token in turn over both, each read twice,
+// waited for memory six times one after another.)
+template <int N, typename W, typename T>
+__global__ void __launch_bounds__(kThreads)
+latent_prepare_vec_kernel(const float* __restrict__ down, long long stride, int q_rank, int rank,
+                          int rot, const W* __restrict__ q_weight, const W* __restrict__ kv_weight,
+                          float eps, const int32_t* __restrict__ positions,
+                          const int32_t* __restrict__ token_seq,
+                          const int32_t* __restrict__ block_table, int max_blocks,
+                          const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                          T* __restrict__ q_latent, T* __restrict__ cache, int interleaved, int first) {
+  __shared__ float scratch[kThreads / 32];
+  const long long t = blockIdx.x;
+  const bool query = blockIdx.y + first != 0;
+  const int count = query ? q_rank : rank;
+  const float* src = down + t * stride + (query ? 0 : q_rank);
+  const W* weight = query ? q_weight : kv_weight;
+  float v[N][4], w[N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[n][k] = 0.f;
+    if (c < count) {
+      read4(src + c, v[n]);
+      read4(weight + c, w[n]);
+    }
+  }
+  T* to = q_latent + t * q_rank;
+  const int half = rot / 2, i = threadIdx.x;
+  float u = 0.f, x = 0.f, c = 1.f, s = 0.f;
+  int a = 0, b = 0;
+  if (!query) {
+    const int pos = positions[t];
+    const int block = block_table[(long long)token_seq[t] * max_blocks + pos / kCacheBlock];
+    to = cache + ((long long)block * kCacheBlock + pos % kCacheBlock) * (rank + rot);
+    if (i < half) {
+      c = cos_t[(long long)pos * half + i];
+      s = sin_t[(long long)pos * half + i];
+      a = interleaved ? 2 * i : i;
+      b = interleaved ? 2 * i + 1 : i + half;
+      u = src[rank + a];
+      x = src[rank + b];
+    }
+  }
+  float sum = 0.f;
+#pragma unroll
+  for (int n = 0; n < N; ++n)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sum = fmaf(v[n][k], v[n][k], sum);
+  const float r = rsqrtf(block_sum_once(sum, scratch) / static_cast<float>(count) + eps);
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int at = (n * kThreads + threadIdx.x) * 4;
+    if (at >= count) continue;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[n][k] = v[n][k] * r * w[n][k];
+    write4(to + at, v[n]);
+  }
+  if (!query && i < half) {
+    to[rank + a] = narrow<T>(u * c - x * s);
+    to[rank + b] = narrow<T>(x * c + u * s);
+  }
+}
+
 template <typename T>
 __global__ void rotate_heads_kernel(T* __restrict__ x, long long stride, int head_stride,
                                     int offset, int heads, int rot,
@@ -88,6 +155,26 @@ int prepare(const float* down, long long stride, int q_rank, int rank, int rot,
             const int32_t* token_seq, const int32_t* block_table, int max_blocks,
             const float* cos_t, const float* sin_t, void* q_latent, void* cache, int write_cache,
             int interleaved, int tokens, cudaStream_t stream) {
+  // (by the sizes alone: how a row is summed must not depend on the step)
+  auto aligned = [](const void* p, size_t bytes) { return (uintptr_t)p % bytes == 0; };
+  const int most = q_rank > rank ? q_rank : rank;
+  if (stride % 4 == 0 && q_rank % 4 == 0 && rank % 4 == 0 && rot % 4 == 0 && rot <= 2 * kThreads &&
+      most <= 4096 && aligned(down, 16) && aligned(q_weight, 4 * sizeof(W)) &&
+      aligned(kv_weight, 4 * sizeof(W)) && aligned(q_latent, 4 * sizeof(T)) &&
+      aligned(cache, 4 * sizeof(T))) {
+    const int first = write_cache ? 0 : 1, blocks = (write_cache ? 1 : 0) + (q_rank > 0 ? 1 : 0);
+    if (blocks == 0) return 0;
+    auto go = [&](auto kernel) {
+      return launch_ordered(kernel, dim3(tokens, blocks), dim3(kThreads), 0, stream, down, stride, q_rank,
+                            rank, rot, (const W*)q_weight, (const W*)kv_weight, eps, positions,
+                            token_seq, block_table, max_blocks, cos_t, sin_t, (T*)q_latent, (T*)cache,
+                            interleaved, first);
+    };
+    if (most <= 512) return go(latent_prepare_vec_kernel<1, W, T>);
+    if (most <= 1024) return go(latent_prepare_vec_kernel<2, W, T>);
+    if (most <= 2048) return go(latent_prepare_vec_kernel<4, W, T>);
+    return go(latent_prepare_vec_kernel<8, W, T>);
+  }
   return launch_ordered(latent_prepare_kernel<W, T>, dim3(tokens), dim3(kThreads), 0, stream, down,
                         stride, q_rank, rank, rot, (const W*)q_weight, (const W*)kv_weight, eps,
                         positions, token_seq, block_table, max_blocks, cos_t, sin_t,

@@ -60,9 +60,87 @@ layer_norm_kernel(float* __restrict__ x, const float* __restrict__ y,
     o[i] = narrow<Out>((row[i] - st.x) * st.y * widen(w_before[i]));
 }
 
+// The same for rows of up to 4,096 numbers, multiples of four: a thread keeps N groups of four
+// neighbouring numbers in registers, asks for the row, its addend and the weights at once, and a mean or
+// a variance is one meeting of the block.
+template <int N, typename W, typename Out>
+__global__ void __launch_bounds__(kThreads)
+layer_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y,
+                      const W* __restrict__ w_after, const int32_t* __restrict__ rows,
+                      const W* __restrict__ w_before, Out* __restrict__ out, int hidden, float eps) {
+  __shared__ float scratch[4][kThreads / 32];
+  const long long src = rows ? rows[blockIdx.x] : blockIdx.x;
+  float* in = x + src * hidden;
+  float v[N][4], add[N][4], after[N][4], before[N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (c < hidden) {
+      read4(in + c, v[n]);
+      if (y) {
+        read4(y + src * hidden + c, add[n]);
+        read4(w_after + c, after[n]);
+      }
+      if (out) read4(w_before + c, before[n]);
+    }
+  }
+  // (mean, 1 / sqrt(variance + eps)) of the block's row
+  auto stats = [&](const float (&r)[N][4], float (*sums)[kThreads / 32]) {
+    float s = 0.f;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if ((n * kThreads + threadIdx.x) * 4 < hidden) s += (r[n][0] + r[n][1]) + (r[n][2] + r[n][3]);
+    const float mean = block_sum_once(s, sums[0]) / static_cast<float>(hidden);
+    float q = 0.f;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if ((n * kThreads + threadIdx.x) * 4 < hidden)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float d = r[n][i] - mean;
+          q = fmaf(d, d, q);
+        }
+    const float var = block_sum_once(q, sums[1]) / static_cast<float>(hidden);
+    return make_float2(mean, rsqrtf(var + eps));
+  };
+  if (y) {
+    const float2 st = stats(add, scratch);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int c = (n * kThreads + threadIdx.x) * 4;
+      if (c >= hidden) continue;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[n][i] += (add[n][i] - st.x) * st.y * after[n][i];
+      write4(in + c, v[n]);
+    }
+  }
+  if (!out) return;
+  const float2 st = stats(v, scratch + 2);
+  Out* o = out + (long long)blockIdx.x * hidden;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (c >= hidden) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[n][i] = (v[n][i] - st.x) * st.y * before[n][i];
+    write4(o + c, v[n]);
+  }
+}
+
 template <typename W, typename Out>
 int launch(float* x, const float* y, const void* w_after, const int32_t* rows,
            const void* w_before, void* out, int n, int hidden, float eps, cudaStream_t stream) {
+  const uintptr_t weights = (uintptr_t)w_after | (uintptr_t)w_before;
+  if (hidden % 4 == 0 && hidden <= 4096 && !(((uintptr_t)x | (uintptr_t)y) & 15) &&
+      !(weights & (4 * sizeof(W) - 1)) && !((uintptr_t)out & (4 * sizeof(Out) - 1))) {
+    auto go = [&](auto kernel) {
+      return launch_ordered(kernel, dim3(n), dim3(kThreads), 0, stream, x, y, (const W*)w_after, rows,
+                            (const W*)w_before, (Out*)out, hidden, eps);
+    };
+    if (hidden <= 1024) return go(layer_norm_vec_kernel<1, W, Out>);
+    if (hidden <= 2048) return go(layer_norm_vec_kernel<2, W, Out>);
+    return go(layer_norm_vec_kernel<4, W, Out>);
+  }
   return launch_ordered(layer_norm_kernel<W, Out>, dim3(n), dim3(kThreads),
                            (size_t)hidden * sizeof(float), stream, x, y, (const W*)w_after,
                            rows, (const W*)w_before, (Out*)out, hidden, eps);

@@ -37,7 +37,7 @@ constexpr int TK = 32;          // K step
 
 // Router logits in fp32: a warp a (token, output) walks the row; the order of the sums
 // depends on the width alone.
-template <typename T>
+template <bool FOURS, typename T>
 __global__ void logits_kernel(const T* __restrict__ h, const float* __restrict__ w,
                               float* __restrict__ out, int outputs, int width, long long count) {
   const long long item = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -48,9 +48,27 @@ __global__ void logits_kernel(const T* __restrict__ h, const float* __restrict__
   const T* x = h + t * width;
   const float* row = w + (long long)o * width;
   float sum = 0.f;
-  for (int i = lane; i < width; i += 32) sum = fmaf(widen(x[i]), row[i], sum);
+  if (FOURS) {
+    // a lane's groups of four in turn, several asked for at once
+#pragma unroll 8
+    for (int i = lane * 4; i < width; i += 128) {
+      float a[4], b[4];
+      read4(x + i, a);
+      read4(row + i, b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sum = fmaf(a[k], b[k], sum);
+    }
+  } else {
+    for (int i = lane; i < width; i += 32) sum = fmaf(widen(x[i]), row[i], sum);
+  }
   sum = warp_sum(sum);
   if (lane == 0) out[item] = sum;
+}
+
+// Whether rows go by in groups of four neighbouring numbers (both kernels alike: a sum's order depends
+// on the width alone).
+bool logits_by_fours(const void* h, int dtype, const float* w, int width) {
+  return width % 4 == 0 && (uintptr_t)h % (dtype == SAKV_F32 ? 16 : 8) == 0 && (uintptr_t)w % 16 == 0;
 }
 
 // Whether sixteen sums a warp are the faster split: with 80 sums an SM there are warps enough, and a
@@ -63,7 +81,7 @@ bool logits_in_tiles(int tokens, int outputs) {
 // The same for many tokens: a warp takes four tokens and four outputs, so that a piece of a row and of
 // a weight row is read once for four sums; every sum has the same terms in the same order. (A warp a
 // sum read the 300 KB of weights once a token: 3,001 tokens, 36 outputs of 2,048: 75 -> 35 us.)
-template <typename T>
+template <bool FOURS, typename T>
 __global__ void __launch_bounds__(256)
 logits_tile_kernel(const T* __restrict__ h, const float* __restrict__ w, float* __restrict__ out,
                    int outputs, int width, int tokens) {
@@ -82,18 +100,36 @@ logits_tile_kernel(const T* __restrict__ h, const float* __restrict__ w, float* 
     row[i] = w + (long long)min(o0 + i, outputs - 1) * width;
   }
   float sum[N][N] = {};
+  if (FOURS) {
 #pragma unroll 2
-  for (int i = lane; i < width; i += 32) {
-    float a[N], b[N];
+    for (int i = lane * 4; i < width; i += 128) {
+      float a[N][4], b[N][4];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      a[k] = widen(x[k][i]);
-      b[k] = row[k][i];
+      for (int k = 0; k < N; ++k) {
+        read4(x[k] + i, a[k]);
+        read4(row[k] + i, b[k]);
+      }
+#pragma unroll
+      for (int t = 0; t < N; ++t)
+#pragma unroll
+        for (int o = 0; o < N; ++o)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum[t][o] = fmaf(a[t][q], b[o][q], sum[t][o]);
     }
+  } else {
+#pragma unroll 2
+    for (int i = lane; i < width; i += 32) {
+      float a[N], b[N];
 #pragma unroll
-    for (int t = 0; t < N; ++t)
+      for (int k = 0; k < N; ++k) {
+        a[k] = widen(x[k][i]);
+        b[k] = row[k][i];
+      }
 #pragma unroll
-      for (int o = 0; o < N; ++o) sum[t][o] = fmaf(a[t], b[o], sum[t][o]);
+      for (int t = 0; t < N; ++t)
+#pragma unroll
+        for (int o = 0; o < N; ++o) sum[t][o] = fmaf(a[t], b[o], sum[t][o]);
+    }
   }
 #pragma unroll
   for (int t = 0; t < N; ++t)
@@ -120,11 +156,17 @@ struct RouteForm {
   float scale;
 };
 
+// Up to this many outputs a warp keeps a token's scores in shared memory, worked out once; beyond, it
+// reads its logits again for every choice.
+constexpr int kStaged = 128;
+
+// `staged`: [2][kStaged] floats of shared memory of this warp's own, or null.
 __device__ __forceinline__ void route_token(const float* __restrict__ z, int experts, int top,
                                             int32_t* __restrict__ chosen,
                                             float* __restrict__ weights,
                                             int32_t* counts, int32_t* __restrict__ rank,
-                                            int real, const RouteForm& form, int lane) {
+                                            int real, const RouteForm& form, int lane,
+                                            float* staged) {
   const int softmax = form.softmax;
   const float* __restrict__ bias = form.bias;
   float top_z = -INFINITY, total = 1.f;
@@ -139,7 +181,19 @@ __device__ __forceinline__ void route_token(const float* __restrict__ z, int exp
     return softmax ? expf(logit - top_z) / total : 1.f / (1.f + expf(-logit));
   };
   const bool by_logit = bias == nullptr;
-  auto rank_of = [&](int e) { return by_logit ? z[e] : score(z[e]) + bias[e]; };
+  if (staged) {
+    __syncwarp();                                  // (the warp's token before has been read)
+    for (int e = lane; e < experts; e += 32) {
+      const float logit = z[e], s = score(logit);
+      staged[e] = s;
+      staged[kStaged + e] = by_logit ? logit : s + bias[e];
+    }
+    __syncwarp();
+  }
+  auto score_of = [&](int e) { return staged ? staged[e] : score(z[e]); };
+  auto rank_of = [&](int e) {
+    return staged ? staged[kStaged + e] : by_logit ? z[e] : score(z[e]) + bias[e];
+  };
   const int per_group = experts / form.groups;
   uint64_t open = ~0ull;                           // bit g: group g may be chosen from
   if (form.groups > 1) {
@@ -153,7 +207,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ z, int exp
         if (form.group_top == 2) {                   // (sums are of scores, never of logits)
           float second = -INFINITY;
           for (int e = g * per_group; e < (g + 1) * per_group; ++e) {
-            const float r = by_logit ? score(z[e]) : rank_of(e);
+            const float r = by_logit ? score_of(e) : rank_of(e);
             second = fmaxf(second, fminf(v, r));
             v = fmaxf(v, r);
           }
@@ -205,8 +259,9 @@ __device__ __forceinline__ void route_token(const float* __restrict__ z, int exp
     if ((at & 31) == lane) taken |= 1u << (at >> 5);
     if (lane == 0) {
       chosen[k] = at;
-      weights[k] = score(z[at]);
-      sum_chosen += weights[k];
+      const float s = score_of(at);
+      weights[k] = s;
+      sum_chosen += s;
       rank[k] = at < real ? atomicAdd(counts + at, 1) : -1;
     }
   }
@@ -220,10 +275,12 @@ __global__ void route_kernel(const float* __restrict__ logits, long long ld, int
                              int32_t* __restrict__ chosen, float* __restrict__ weights,
                              int32_t* __restrict__ counts, int32_t* __restrict__ rank,
                              int tokens, int real, const RouteForm form) {
+  __shared__ float staged[4][2 * kStaged];
   const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
   if (t >= tokens) return;
   route_token(logits + t * ld, experts, top, chosen + t * top, weights + t * top, counts,
-              rank + t * top, real, form, threadIdx.x & 31);
+              rank + t * top, real, form, threadIdx.x & 31,
+              experts <= kStaged ? staged[threadIdx.x >> 5] : nullptr);
 }
 
 // Where each expert's rows begin and the tiles of the grouped products, from the experts'
@@ -233,17 +290,33 @@ __device__ __forceinline__ void plan_tiles(const int32_t* counts, int32_t* __res
                                            int32_t* __restrict__ tile_row,
                                            int32_t* __restrict__ n_tiles, int experts,
                                            int max_tiles, int32_t* base) {
-  if (threadIdx.x == 0) {
-    int rows = 0, tiles = 0;
-    for (int e = 0; e < experts; ++e) {
-      offsets[e] = rows;
-      base[e] = tiles;
-      rows += counts[e];
-      tiles += (counts[e] + TM - 1) / TM;
+  if (threadIdx.x < 32) {                          // one warp, 32 experts at a time
+    const int lane = threadIdx.x;
+    int rows = 0, tiles = 0;                       // of the experts before
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      const int e = e0 + lane, mine = e < experts ? counts[e] : 0;
+      const int own = (mine + TM - 1) / TM;
+      int r = mine, t = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int ur = __shfl_up_sync(0xffffffffu, r, o), ut = __shfl_up_sync(0xffffffffu, t, o);
+        if (lane >= o) {
+          r += ur;
+          t += ut;
+        }
+      }
+      if (e < experts) {
+        offsets[e] = rows + r - mine;
+        base[e] = tiles + t - own;
+      }
+      rows += __shfl_sync(0xffffffffu, r, 31);
+      tiles += __shfl_sync(0xffffffffu, t, 31);
     }
-    offsets[experts] = rows;
-    base[experts] = tiles;
-    *n_tiles = tiles < max_tiles ? tiles : max_tiles;
+    if (lane == 0) {
+      offsets[experts] = rows;
+      base[experts] = tiles;
+      *n_tiles = tiles < max_tiles ? tiles : max_tiles;
+    }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < experts; e += blockDim.x) {
@@ -266,13 +339,14 @@ route_plan_kernel(const float* __restrict__ logits, long long ld, int experts, i
                   int32_t* __restrict__ tile_expert, int32_t* __restrict__ tile_row,
                   int32_t* __restrict__ n_tiles, int max_tiles) {
   extern __shared__ int32_t shared_ints[];         // counts [real], then base [real + 1]
+  __shared__ float staged[8][2 * kStaged];
   int32_t* counts = shared_ints;
   for (int e = threadIdx.x; e < real; e += blockDim.x) counts[e] = 0;
   __syncthreads();
   for (int t = threadIdx.x >> 5; t < tokens; t += blockDim.x >> 5)
     route_token(logits + t * ld, experts, top, chosen + (long long)t * top,
                 weights + (long long)t * top, counts, rank + (long long)t * top, real, form,
-                threadIdx.x & 31);
+                threadIdx.x & 31, experts <= kStaged ? staged[threadIdx.x >> 5] : nullptr);
   __syncthreads();
   plan_tiles(counts, offsets, tile_expert, tile_row, n_tiles, real, max_tiles, counts + real);
 }
@@ -657,18 +731,24 @@ SAKV_EXPORT int sakv_moe_logits(const void* h, int dtype, const float* w, float*
   const bool in_tiles = logits_in_tiles(tokens, outputs);
   const long long tiles = (tokens + 3LL) / 4 * ((outputs + 3) / 4);
   const dim3 grid4((unsigned)((tiles * 32 + 255) / 256));
-  if (in_tiles && dtype == SAKV_F32)
-    return launch_ordered(logits_tile_kernel<float>, grid4, block, 0, stream, (const float*)h, w,
-                             out, outputs, width, tokens);
-  if (in_tiles && dtype == SAKV_BF16)
-    return launch_ordered(logits_tile_kernel<__nv_bfloat16>, grid4, block, 0, stream,
-                             (const __nv_bfloat16*)h, w, out, outputs, width, tokens);
-  if (dtype == SAKV_F32)
-    return launch_ordered(logits_kernel<float>, grid, block, 0, stream, (const float*)h, w, out,
-                          outputs, width, count);
-  if (dtype == SAKV_BF16)
-    return launch_ordered(logits_kernel<__nv_bfloat16>, grid, block, 0, stream,
-                          (const __nv_bfloat16*)h, w, out, outputs, width, count);
+  const bool fours = logits_by_fours(h, dtype, w, width);
+#define SAKV_LOGITS(FOURS, T)                                                                    \
+  do {                                                                                           \
+    if (in_tiles)                                                                                \
+      return launch_ordered(logits_tile_kernel<FOURS, T>, grid4, block, 0, stream, (const T*)h,  \
+                            w, out, outputs, width, tokens);                                     \
+    return launch_ordered(logits_kernel<FOURS, T>, grid, block, 0, stream, (const T*)h, w, out,  \
+                          outputs, width, count);                                                \
+  } while (0)
+  if (dtype == SAKV_F32) {
+    if (fours) SAKV_LOGITS(true, float);
+    SAKV_LOGITS(false, float);
+  }
+  if (dtype == SAKV_BF16) {
+    if (fours) SAKV_LOGITS(true, __nv_bfloat16);
+    SAKV_LOGITS(false, __nv_bfloat16);
+  }
+#undef SAKV_LOGITS
   return cudaErrorInvalidValue;
 }
 

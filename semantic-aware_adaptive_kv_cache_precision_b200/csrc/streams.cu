@@ -102,6 +102,106 @@ streams_step_kernel(float* __restrict__ xs, long long stream_stride, int streams
   }
 }
 
+// The same for one, two or four streams of rows of up to 4,096 numbers, multiples of four: a thread
+// takes N groups of four neighbouring columns, asks for all it reads before it uses any (the constants
+// before the kernel before it is done), and keeps the row in registers. A row's time is one trip to
+// memory and one meeting of the block, where the loop above makes a trip every 256 columns, since a
+// store to the streams keeps the next columns' loads behind it.
+template <int S, int N, typename W, typename Out>
+__global__ void __launch_bounds__(kThreads)
+streams_step_vec_kernel(float* __restrict__ xs, long long stream_stride, int width,
+                        const float* __restrict__ y, const W* __restrict__ mix,
+                        const W* __restrict__ out_w, int reduce, const W* __restrict__ in_w,
+                        const W* __restrict__ norm_w, float eps, Out* __restrict__ out,
+                        float* __restrict__ shift_state, const W* __restrict__ shift_w,
+                        const int32_t* __restrict__ token_seq, const int32_t* __restrict__ slots,
+                        int keep_state) {
+  __shared__ float scratch[kThreads / 32];
+  let_next_kernel_start();
+  float c_mix[S][S], c_out[S], c_in[S], weight[N][4], blend[N][4];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+#pragma unroll
+    for (int t = 0; t < S; ++t) c_mix[s][t] = mix ? widen(mix[s * S + t]) : (s == t ? 1.f : 0.f);
+    c_out[s] = out_w ? widen(out_w[s]) : 1.f;
+    c_in[s] = in_w ? widen(in_w[s]) : 1.f;
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (norm_w && c < width) read4(norm_w + c, weight[n]);
+    if (shift_state && c < width) read4(shift_w + c, blend[n]);
+  }
+  wait_for_previous_kernel();
+  const long long row = blockIdx.x;
+  float* x = xs + row * width;
+  float v[N][S][4], add[N][4], prev[N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (c >= width) continue;
+#pragma unroll
+    for (int s = 0; s < S; ++s) read4(x + s * stream_stride + c, v[n][s]);
+    if (y) read4(y + row * width + c, add[n]);
+  }
+  float* kept = shift_state ? shift_state + (long long)slots[token_seq[row]] * width : nullptr;
+  if (kept) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int c = (n * kThreads + threadIdx.x) * 4;
+      if (c < width) read4(kept + c, prev[n]);
+    }
+  }
+  float sq = 0.f, u[N][4];
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (c >= width) continue;
+    if (y) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float now[S];
+#pragma unroll
+        for (int t = 0; t < S; ++t) {
+          float acc = 0.f;
+#pragma unroll
+          for (int s = 0; s < S; ++s) acc = fmaf(c_mix[s][t], v[n][s][i], acc);
+          now[t] = fmaf(c_out[t], add[n][i], acc);
+        }
+#pragma unroll
+        for (int s = 0; s < S; ++s) v[n][s][i] = now[s];
+      }
+#pragma unroll
+      for (int s = 0; s < S; ++s) write4(x + s * stream_stride + c, v[n][s]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float sum = 0.f;
+#pragma unroll
+      for (int s = 0; s < S; ++s) sum = fmaf(c_in[s], v[n][s][i], sum);
+      u[n][i] = sum;
+      sq = fmaf(sum, sum, sq);
+    }
+  }
+  if (!reduce) return;
+  const float r = norm_w ? 1.f / sqrtf(block_sum_once(sq, scratch) / (float)width + eps) : 1.f;
+  Out* o = out + row * width;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int c = (n * kThreads + threadIdx.x) * 4;
+    if (c >= width) continue;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (norm_w) u[n][i] = u[n][i] * r * weight[n][i];
+    if (kept) {
+      if (keep_state) write4(kept + c, u[n]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u[n][i] = fmaf(prev[n][i] - u[n][i], blend[n][i], u[n][i]);
+    }
+    write4(o + c, u[n]);
+  }
+}
+
 template <typename W, typename Out>
 __global__ void token_shift_kernel(const float* __restrict__ h, float* __restrict__ state,
                                    const W* __restrict__ shift,
@@ -148,6 +248,33 @@ int launch_step(float* xs, long long stride, int streams, int tokens, int width,
                 const void* norm_w, float eps, void* out, int out_dtype, float* shift_state,
                 const void* shift_w, const int32_t* token_seq, const int32_t* slots,
                 int keep_state, cudaStream_t stream) {
+  if constexpr (S <= 4) {
+    // whole groups of four, aligned everywhere (bf16 constants and outputs: to 8 bytes)
+    const uintptr_t wide = (uintptr_t)xs | (uintptr_t)y | (uintptr_t)shift_state |
+                           (out_dtype == SAKV_F32 ? (uintptr_t)out : 0) |
+                           (sizeof(W) == 4 ? (uintptr_t)norm_w | (uintptr_t)shift_w : 0);
+    const uintptr_t narrow = (uintptr_t)out | (uintptr_t)norm_w | (uintptr_t)shift_w;
+    if (streams == S && width % 4 == 0 && width <= 4096 && stride % 4 == 0 && !(wide & 15) &&
+        !(narrow & 7)) {
+      auto go = [&](auto kernel, auto* o) {
+        return launch_overlapped(kernel, dim3(tokens), dim3(kThreads), 0, stream, 1, xs, stride, width,
+                                 y, (const W*)mix, (const W*)out_w, reduce, (const W*)in_w,
+                                 (const W*)norm_w, eps, o, shift_state, (const W*)shift_w, token_seq,
+                                 slots, keep_state);
+      };
+#define SAKV_VEC(N)                                                                              \
+  do {                                                                                           \
+    if (out_dtype == SAKV_F32) return go(streams_step_vec_kernel<S, N, W, float>, (float*)out);  \
+    if (out_dtype == SAKV_BF16)                                                                  \
+      return go(streams_step_vec_kernel<S, N, W, __nv_bfloat16>, (__nv_bfloat16*)out);           \
+    return cudaErrorInvalidValue;                                                                \
+  } while (0)
+      if (width <= 1024) SAKV_VEC(1);
+      if (width <= 2048) SAKV_VEC(2);
+      SAKV_VEC(4);
+#undef SAKV_VEC
+    }
+  }
   const size_t smem = reduce ? (size_t)width * sizeof(float) : 0;
   if (smem > 200 * 1024) return cudaErrorInvalidValue;
   auto go = [&](auto kernel, auto* o) {
