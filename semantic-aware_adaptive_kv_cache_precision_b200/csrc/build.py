@@ -59,6 +59,7 @@ LIBRARIES = {
     "norm_update": "norm_update.cu",
     "qk_prepare": "qk_prepare.cu",
     "recurrent_scan": "recurrent_scan.cu",
+    "chunk_scan": "chunk_scan.cu",
     "gated_delta": "gated_delta.cu",
 }
 

@@ -19,12 +19,14 @@
 // unrounded). A sequence's tokens are taken in order by the threads that own a piece of its
 // state, so the result of a token does not depend on how its sequence was cut into steps or
 // on what else is in the step.
-#include "common.cuh"
+#include "scan.cuh"
 
 namespace {
 
-__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+using scan::FadeInput;
+using scan::fade_act;
+using scan::silu;
+using scan::softplus;
 
 // e^x - 1 for x <= 0, to about 1e-7 of ITSELF where x is small (what a decay close to 1 needs:
 // its distance from 1) and to about 2e-7 absolutely elsewhere. EXACT: the library's expm1f
@@ -395,21 +397,6 @@ __global__ void scan_carry_kernel(const W* __restrict__ a_log, float* __restrict
 // ---------------------------------------------------------------------------------------
 constexpr int kRun = 16;          // tokens brought into shared memory at a time
 
-// What shapes q, k and v on their way into shared memory: `act` 1 is silu of each element
-// (0: as projected); `rot` > 0 turns the first `rot` numbers of every head of q and k by the
-// token's position (pairs (i, i + rot / 2), tables [positions, rot / 2] that carry the
-// rotation's magnitude), after the activation; `k_scale` multiplies k after that.
-struct FadeInput {
-  int act;
-  int rot;
-  const int32_t* positions;
-  const float* cos_t;
-  const float* sin_t;
-  float k_scale;
-};
-
-__device__ __forceinline__ float fade_act(float x, int act) { return act ? silu(x) : x; }
-
 // One token's head of q or k from `head` (global) to `to` (shared), `padded` floats of which
 // the first `dim` are real, times `scale`; element `i` is this thread's. A rotated pair is
 // made by the thread of its lower half, which reads both numbers and the angle once.
@@ -433,11 +420,8 @@ __device__ __forceinline__ void fade_stage(const float* __restrict__ head, float
   to[i + half] = (y * c + x * sn) * scale;
 }
 
-// PHASE as in the selective scan: 0 walks a sequence's whole part of the step from the state in
-// its slot; 1 walks one run of `chunk_len` tokens from zero and leaves the end state in scratch
-// memory ([sequences, max_chunks, heads, vdim, dim]), without outputs; 2 walks a run from the
-// state that the carry kernel put there and writes the outputs.
-template <int RP, int PHASE>
+// A long prompt goes through csrc/chunk_scan.cu instead, in the 16-bit mode.
+template <int RP>
 __global__ void decay_attention_kernel(const float* __restrict__ proj, long long stride,
                                        int q_off, int k_off, int v_off,
                                        const float* __restrict__ decay_less_one,
@@ -445,22 +429,15 @@ __global__ void decay_attention_kernel(const float* __restrict__ proj, long long
                                        const int32_t* __restrict__ cu_seqlens,
                                        const int32_t* __restrict__ slots, float* __restrict__ out,
                                        int heads, int dim, int vdim, int rs, int cols,
-                                       int keep_state, int chunk_len, int max_chunks,
-                                       float* __restrict__ scratch, const FadeInput in) {
+                                       int keep_state, const FadeInput in) {
   extern __shared__ __align__(16) float shared[];
   const int padded = rs * RP;                       // dim rounded up to whole lanes
   const int padded_shift = 31 - __clz(padded);
   float* qs = shared;                               // [kRun, padded]
   float* ks = qs + kRun * padded;                   // [kRun, padded]
   float* vs = ks + kRun * padded;                   // [kRun, cols]
-  const int b = PHASE == 0 ? blockIdx.z : blockIdx.z / max_chunks;
-  const int piece = PHASE == 0 ? 0 : blockIdx.z % max_chunks;
-  int first = cu_seqlens[b], last = cu_seqlens[b + 1];
-  if (PHASE != 0) {
-    first += piece * chunk_len;
-    if (first >= last) return;                      // (the whole block)
-    if (last - first > chunk_len) last = first + chunk_len;
-  }
+  const int b = blockIdx.z;
+  const int first = cu_seqlens[b], last = cu_seqlens[b + 1];
   const int h = blockIdx.y, col0 = blockIdx.x * cols;
   const int r = threadIdx.x % rs, j = threadIdx.x / rs;
   const int col = col0 + j;
@@ -468,11 +445,9 @@ __global__ void decay_attention_kernel(const float* __restrict__ proj, long long
   const float fade = decay_less_one[h];        // decay - 1, rounded once from the exact number
   float s[RP];
   const long long place = ((long long)h * vdim + (live ? col : 0)) * dim + r * RP;
-  float* mine = PHASE == 0
-                    ? state + (long long)slots[b] * heads * vdim * dim + place
-                    : scratch + ((long long)b * max_chunks + piece) * heads * vdim * dim + place;
+  float* mine = state + (long long)slots[b] * heads * vdim * dim + place;
 #pragma unroll
-  for (int k = 0; k < RP; ++k) s[k] = (PHASE != 1 && live && r * RP + k < dim) ? mine[k] : 0.f;
+  for (int k = 0; k < RP; ++k) s[k] = (live && r * RP + k < dim) ? mine[k] : 0.f;
   for (int t0 = first; t0 < last; t0 += kRun) {
     const int run = last - t0 < kRun ? last - t0 : kRun;
     __syncthreads();
@@ -480,7 +455,7 @@ __global__ void decay_attention_kernel(const float* __restrict__ proj, long long
       const int tt = e >> padded_shift, i = e & (padded - 1);     // (padded is a power of two)
       const float* row = proj + (long long)(t0 + tt) * stride + (long long)h * dim;
       const int pos = in.rot ? in.positions[t0 + tt] : 0;
-      if (PHASE != 1) fade_stage(row + q_off, qs + tt * padded, i, dim, pos, 1.f, in);
+      fade_stage(row + q_off, qs + tt * padded, i, dim, pos, 1.f, in);
       fade_stage(row + k_off, ks + tt * padded, i, dim, pos, in.k_scale, in);
     }
     for (int e = threadIdx.x; e < run * cols; e += blockDim.x) {
@@ -507,50 +482,21 @@ __global__ void decay_attention_kernel(const float* __restrict__ proj, long long
         s[k + 1] = fmaf(kk.y, v, fmaf(fade, s[k + 1], s[k + 1]));
         s[k + 2] = fmaf(kk.z, v, fmaf(fade, s[k + 2], s[k + 2]));
         s[k + 3] = fmaf(kk.w, v, fmaf(fade, s[k + 3], s[k + 3]));
-        if (PHASE != 1) {
-          const float4 qq = q4[k >> 2];
-          o = fmaf(s[k], qq.x, o);
-          o = fmaf(s[k + 1], qq.y, o);
-          o = fmaf(s[k + 2], qq.z, o);
-          o = fmaf(s[k + 3], qq.w, o);
-        }
+        const float4 qq = q4[k >> 2];
+        o = fmaf(s[k], qq.x, o);
+        o = fmaf(s[k + 1], qq.y, o);
+        o = fmaf(s[k + 2], qq.z, o);
+        o = fmaf(s[k + 3], qq.w, o);
       }
-      if (PHASE != 1) {
-        for (int d = rs >> 1; d > 0; d >>= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
-        if (r == 0 && live) out[((long long)(t0 + tt) * heads + h) * vdim + col] = o;
-      }
+      for (int d = rs >> 1; d > 0; d >>= 1) o += __shfl_xor_sync(0xffffffffu, o, d);
+      if (r == 0 && live) out[((long long)(t0 + tt) * heads + h) * vdim + col] = o;
     }
   }
-  if (live && (PHASE == 1 || (PHASE == 0 && keep_state))) {
+  if (live && keep_state) {
 #pragma unroll
     for (int k = 0; k < RP; ++k)
       if (r * RP + k < dim) mine[k] = s[k];
   }
-}
-
-// Between the two passes over a prompt's runs: one thread a (sequence, head, column, row) walks
-// the runs in order; a run of n tokens fades what came before by decay^n.
-__global__ void decay_carry_kernel(const float* __restrict__ decay_less_one,
-                                   float* __restrict__ state, float* __restrict__ scratch,
-                                   const int32_t* __restrict__ cu_seqlens,
-                                   const int32_t* __restrict__ slots, int sequences, int heads,
-                                   long long per_head, int chunk_len, int max_chunks,
-                                   int keep_state) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long per = heads * per_head;
-  if (idx >= sequences * per) return;
-  const int b = static_cast<int>(idx / per);
-  const long long e = idx - b * per;
-  const int n = cu_seqlens[b + 1] - cu_seqlens[b];
-  const int runs = (n + chunk_len - 1) / chunk_len;
-  const float log_fade = log1pf(decay_less_one[e / per_head]);
-  float* home = state + (long long)slots[b] * per + e;
-  const float s = carry_runs(
-      scratch + (long long)b * max_chunks * per + e, per, runs, *home, [&](int j) {
-        const int len = n - j * chunk_len < chunk_len ? n - j * chunk_len : chunk_len;
-        return expm1f(log_fade * static_cast<float>(len));
-      });
-  if (keep_state) *home = s;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -560,7 +506,7 @@ __global__ void decay_carry_kernel(const float* __restrict__ decay_less_one,
 // group and of the convolution's output type; x for v), the step size dt a (token, head), made
 // here from the projection's column, which multiplies x and chooses the token's decay, and D x
 // added to the output. State in memory: [slots, heads, vdim, dim] (a column's rows together).
-// PHASE as above; a run's decay to the carry kernel is the sum of its step sizes.
+// (A long prompt goes through csrc/chunk_scan.cu instead, in the 16-bit mode.)
 //
 // CV neighbouring columns belong to one thread (4 where the step's walks fill the GPU, else 1):
 // what a token brings for a lane's rows is read once for all of them, and with four the sums
@@ -581,12 +527,10 @@ struct DualScan {
   const int32_t* cu_seqlens;
   const int32_t* slots;
   float* out;                      // [tokens, heads * vdim]
-  int heads, groups, dim, vdim, rs, cols, keep_state, chunk_len, max_chunks;
-  float* scratch;                  // [sequences, max_chunks, heads, vdim, dim]
-  float* dt_sums;                  // [sequences, max_chunks, heads]
+  int heads, groups, dim, vdim, rs, cols, keep_state;
 };
 
-template <int RP, int CV, int PHASE, typename C>
+template <int RP, int CV, typename C>
 __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
   extern __shared__ __align__(16) float shared[];
   const int padded = p.rs * RP;                     // dim rounded up to whole lanes
@@ -596,14 +540,8 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
   float* vs = ks + kRun * padded;                   // [kRun, cols]    x
   float* steps = vs + kRun * p.cols;                // [kRun]          dt
   float* fades = steps + kRun;                      // [kRun]          exp(dt A) - 1
-  const int b = PHASE == 0 ? blockIdx.z : blockIdx.z / p.max_chunks;
-  const int piece = PHASE == 0 ? 0 : blockIdx.z % p.max_chunks;
-  int first = p.cu_seqlens[b], last = p.cu_seqlens[b + 1];
-  if (PHASE != 0) {
-    first += piece * p.chunk_len;
-    if (first >= last) return;                      // (the whole block)
-    if (last - first > p.chunk_len) last = first + p.chunk_len;
-  }
+  const int b = blockIdx.z;
+  const int first = p.cu_seqlens[b], last = p.cu_seqlens[b + 1];
   const int h = blockIdx.y, col0 = blockIdx.x * p.cols;
   const int group_off = h / (p.heads / p.groups) * p.dim;
   const int r = threadIdx.x % p.rs, j = threadIdx.x / p.rs * CV;
@@ -612,8 +550,7 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
   float s[CV][RP];
   const long long per_seq = (long long)p.heads * p.vdim * dim;
   const long long place = ((long long)h * p.vdim + col) * dim + r * RP;    // (used while col < vdim)
-  float* mine = PHASE == 0 ? p.state + p.slots[b] * per_seq + place
-                           : p.scratch + ((long long)b * p.max_chunks + piece) * per_seq + place;
+  float* mine = p.state + p.slots[b] * per_seq + place;
   const bool wide = dim % 4 == 0;                   // (then every lane's rows are 16-byte aligned)
 #pragma unroll
   for (int c = 0; c < CV; ++c) {
@@ -621,13 +558,13 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
 #pragma unroll
     for (int k = 0; k < RP; k += 4) {
       const int at = r * RP + k;
-      if (PHASE != 1 && live && wide && at < dim) {
+      if (live && wide && at < dim) {
         const float4 v = *reinterpret_cast<const float4*>(mine + (long long)c * dim + k);
         s[c][k] = v.x; s[c][k + 1] = v.y; s[c][k + 2] = v.z; s[c][k + 3] = v.w;
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          s[c][k + i] = (PHASE != 1 && live && at + i < dim) ? mine[(long long)c * dim + k + i] : 0.f;
+          s[c][k + i] = (live && at + i < dim) ? mine[(long long)c * dim + k + i] : 0.f;
       }
     }
   }
@@ -636,7 +573,6 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
   int own = r == 0 ? 0 : -1;
   if (CV == 4) own = (r & (p.rs / 4 - 1)) == 0 ? r / (p.rs / 4) : -1;
   if (own >= 0 && col + own >= p.vdim) own = -1;
-  float dt_sum = 0.f;
   for (int t0 = first; t0 < last; t0 += kRun) {
     const int run = last - t0 < kRun ? last - t0 : kRun;
     __syncthreads();
@@ -648,7 +584,7 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
     for (int e = threadIdx.x; e < run * padded; e += blockDim.x) {
       const int tt = e >> padded_shift, i = e & (padded - 1);     // (padded is a power of two)
       const C* row = p.xbc + (long long)(t0 + tt) * p.stride + group_off;
-      if (PHASE != 1) qs[e] = i < dim ? widen(row[p.c_off + i]) : 0.f;
+      qs[e] = i < dim ? widen(row[p.c_off + i]) : 0.f;
       ks[e] = i < dim ? widen(row[p.b_off + i]) : 0.f;
     }
     for (int e = threadIdx.x; e < run * p.cols; e += blockDim.x) {
@@ -670,13 +606,12 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
       }
 #pragma unroll
       for (int c = 0; c < CV; ++c) o[c] = 0.f;
-      dt_sum += dt;
       const float4* k4 = reinterpret_cast<const float4*>(ks + tt * padded + r * RP);
       const float4* q4 = reinterpret_cast<const float4*>(qs + tt * padded + r * RP);
 #pragma unroll
       for (int k = 0; k < RP; k += 4) {
         const float4 kk = k4[k >> 2];
-        const float4 qq = PHASE != 1 ? q4[k >> 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 qq = q4[k >> 2];
 #pragma unroll
         for (int c = 0; c < CV; ++c) {
           // S + (e^(dt A) - 1) S + dt B x: a decay close to 1 keeps its distance from 1
@@ -685,37 +620,33 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
           sc[1] = fmaf(kk.y, v[c], fmaf(fade, sc[1], sc[1]));
           sc[2] = fmaf(kk.z, v[c], fmaf(fade, sc[2], sc[2]));
           sc[3] = fmaf(kk.w, v[c], fmaf(fade, sc[3], sc[3]));
-          if (PHASE != 1) {
-            o[c] = fmaf(sc[0], qq.x, o[c]);
-            o[c] = fmaf(sc[1], qq.y, o[c]);
-            o[c] = fmaf(sc[2], qq.z, o[c]);
-            o[c] = fmaf(sc[3], qq.w, o[c]);
-          }
+          o[c] = fmaf(sc[0], qq.x, o[c]);
+          o[c] = fmaf(sc[1], qq.y, o[c]);
+          o[c] = fmaf(sc[2], qq.z, o[c]);
+          o[c] = fmaf(sc[3], qq.w, o[c]);
         }
       }
-      if (PHASE != 1) {
-        float sum;
-        int d = p.rs >> 1;
-        if constexpr (CV == 4) {                       // (rs >= 4)
-          const bool up = r & d;                       // columns 2, 3 stay with the upper half
-          float a0 = up ? o[2] : o[0], a1 = up ? o[3] : o[1];
-          a0 += __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], d);
-          a1 += __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], d);
-          d >>= 1;
-          const bool odd = r & d;
-          sum = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, d);
-          d >>= 1;
-        } else {
-          sum = o[0];
-        }
-        for (; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        if (own >= 0)
-          p.out[((long long)(t0 + tt) * p.heads + h) * p.vdim + col + own] =
-              fmaf(skip, xs[own], sum);
+      float sum;
+      int d = p.rs >> 1;
+      if constexpr (CV == 4) {                       // (rs >= 4)
+        const bool up = r & d;                       // columns 2, 3 stay with the upper half
+        float a0 = up ? o[2] : o[0], a1 = up ? o[3] : o[1];
+        a0 += __shfl_xor_sync(0xffffffffu, up ? o[0] : o[2], d);
+        a1 += __shfl_xor_sync(0xffffffffu, up ? o[1] : o[3], d);
+        d >>= 1;
+        const bool odd = r & d;
+        sum = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, d);
+        d >>= 1;
+      } else {
+        sum = o[0];
       }
+      for (; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      if (own >= 0)
+        p.out[((long long)(t0 + tt) * p.heads + h) * p.vdim + col + own] =
+            fmaf(skip, xs[own], sum);
     }
   }
-  if (PHASE == 1 || (PHASE == 0 && p.keep_state)) {
+  if (p.keep_state) {
 #pragma unroll
     for (int c = 0; c < CV; ++c) {
       if (col + c >= p.vdim) continue;
@@ -734,30 +665,6 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
       }
     }
   }
-  if (PHASE == 1 && blockIdx.x == 0 && threadIdx.x == 0)
-    p.dt_sums[((long long)b * p.max_chunks + piece) * p.heads + h] = dt_sum;
-}
-
-// Between the two passes over a prompt's runs: one thread a (sequence, head, column, row).
-__global__ void dual_carry_kernel(const float* __restrict__ a, float* __restrict__ state,
-                                  float* __restrict__ scratch, const float* __restrict__ dt_sums,
-                                  const int32_t* __restrict__ cu_seqlens,
-                                  const int32_t* __restrict__ slots, int sequences, int heads,
-                                  long long per_head, int chunk_len, int max_chunks,
-                                  int keep_state) {
-  const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long per = heads * per_head;
-  if (idx >= sequences * per) return;
-  const int b = static_cast<int>(idx / per);
-  const long long e = idx - b * per;
-  const int h = static_cast<int>(e / per_head);
-  const int runs = (cu_seqlens[b + 1] - cu_seqlens[b] + chunk_len - 1) / chunk_len;
-  float* home = state + (long long)slots[b] * per + e;
-  const float rate = a[h];
-  const float* sums = dt_sums + (long long)b * max_chunks * heads + h;
-  const float s = carry_runs(scratch + (long long)b * max_chunks * per + e, per, runs, *home,
-                             [&](int j) { return expm1f(rate * sums[(long long)j * heads]); });
-  if (keep_state) *home = s;
 }
 
 // Eight neighbouring elements as fp32, in 16-byte accesses (p at a multiple of 16 bytes).
@@ -1091,8 +998,7 @@ SAKV_EXPORT int sakv_decay_attention(const float* proj, long long stride, int q_
                                      int v_off, const float* decay, float* state,
                                      const int32_t* cu_seqlens, const int32_t* slots, float* out,
                                      int tokens, int sequences, int heads, int dim, int vdim,
-                                     int keep_state, int chunk_len, int max_chunks, float* scratch,
-                                     int act, int rot, const int32_t* positions,
+                                     int keep_state, int act, int rot, const int32_t* positions,
                                      const float* cos_t, const float* sin_t, float k_scale,
                                      cudaStream_t stream) {
   if (tokens < 0 || sequences < 0 || heads <= 0 || dim <= 0 || dim > 256 || vdim <= 0 ||
@@ -1100,11 +1006,7 @@ SAKV_EXPORT int sakv_decay_attention(const float* proj, long long stride, int q_
     return cudaErrorInvalidValue;
   if (tokens == 0 || sequences == 0) return 0;
   const FadeInput in = {act, rot, positions, cos_t, sin_t, k_scale};
-  const bool runs = chunk_len > 0;
-  if (runs && (max_chunks <= 0 || scratch == nullptr ||
-               (long long)sequences * max_chunks > 65535))
-    return cudaErrorInvalidValue;
-  const long long walks = runs ? (long long)sequences * max_chunks : sequences;
+  const long long walks = sequences;
   const int rp = dim < 128 ? 4 : 8;        // (rows a lane; 16 lanes a column from 128 rows on)
   const int rs = lanes_for(dim, rp);
   int cols = 256 / rs;                       // value columns a block
@@ -1115,50 +1017,30 @@ SAKV_EXPORT int sakv_decay_attention(const float* proj, long long stride, int q_
   if (cols * rs < 32) cols = 32 / rs;        // whole warps
   const dim3 grid((unsigned)((vdim + cols - 1) / cols), (unsigned)heads, (unsigned)walks);
   const size_t smem = (size_t)kRun * (2 * rs * rp + cols) * sizeof(float);
-#define SAKV_FADE(RP, PHASE)                                                                     \
-  launch_ordered(decay_attention_kernel<RP, PHASE>, grid, dim3(cols * rs), smem, stream, proj,   \
-                 stride, q_off, k_off, v_off, decay, state, cu_seqlens, slots, out, heads, dim,  \
-                 vdim, rs, cols, keep_state, chunk_len, max_chunks, scratch, in)
-#define SAKV_FADE_ALL(RP)                                                                        \
-  do {                                                                                           \
-    if (!runs) return SAKV_FADE(RP, 0);                                                          \
-    int code = SAKV_FADE(RP, 1);                                                                 \
-    if (code) return code;                                                                       \
-    const long long per_head = (long long)vdim * dim;                                            \
-    const long long count = (long long)sequences * heads * per_head;                             \
-    code = launch_ordered(decay_carry_kernel, dim3((unsigned)((count + 127) / 128)), dim3(128),  \
-                          0, stream, decay, state, scratch, cu_seqlens, slots, sequences, heads, \
-                          per_head, chunk_len, max_chunks, keep_state);                          \
-    if (code) return code;                                                                       \
-    return SAKV_FADE(RP, 2);                                                                     \
-  } while (0)
-  if (rp == 4) SAKV_FADE_ALL(4);
-  SAKV_FADE_ALL(8);
-#undef SAKV_FADE_ALL
+#define SAKV_FADE(RP)                                                                            \
+  return launch_ordered(decay_attention_kernel<RP>, grid, dim3(cols * rs), smem, stream, proj,   \
+                        stride, q_off, k_off, v_off, decay, state, cu_seqlens, slots, out, heads, \
+                        dim, vdim, rs, cols, keep_state, in)
+  if (rp == 4) SAKV_FADE(4);
+  SAKV_FADE(8);
 #undef SAKV_FADE
 }
 
 // xbc: [tokens, stride] of `c_dtype` with x at column x_off (heads * vdim), B at b_off and C at
 // c_off (groups * dim each); dt: fp32 rows `dt_stride` apart (a column a head); dt_bias, a (the
 // negative decay rates), d_skip: fp32 [heads]; state: fp32 [slots, heads, vdim, dim]. out: fp32
-// [tokens, heads * vdim]. Runs (chunk_len > 0) as in `sakv_selective_scan`, with dt_sums
-// [sequences, max_chunks, heads].
+// [tokens, heads * vdim].
 SAKV_EXPORT int sakv_dual_scan(const void* xbc, int c_dtype, long long stride, int x_off, int b_off,
                                int c_off, const float* dt, long long dt_stride,
                                const float* dt_bias, const float* a, const float* d_skip,
                                float* state, const int32_t* cu_seqlens, const int32_t* slots,
                                float* out, int tokens, int sequences, int heads, int groups,
-                               int dim, int vdim, int keep_state, int chunk_len, int max_chunks,
-                               float* scratch, float* dt_sums, cudaStream_t stream) {
+                               int dim, int vdim, int keep_state, cudaStream_t stream) {
   if (tokens < 0 || sequences < 0 || heads <= 0 || groups <= 0 || heads % groups || dim <= 0 ||
       dim > 256 || vdim <= 0)
     return cudaErrorInvalidValue;
   if (tokens == 0 || sequences == 0) return 0;
-  const bool runs = chunk_len > 0;
-  if (runs && (max_chunks <= 0 || scratch == nullptr || dt_sums == nullptr ||
-               (long long)sequences * max_chunks > 65535))
-    return cudaErrorInvalidValue;
-  const long long walks = runs ? (long long)sequences * max_chunks : sequences;
+  const long long walks = sequences;
   const int rp = dim < 128 ? 4 : 8;        // (rows a lane; 16 lanes a column from 128 rows on)
   const int rs = lanes_for(dim, rp);
   // four columns a thread where the step's blocks then still fill the GPU (a prompt's runs)
@@ -1175,35 +1057,21 @@ SAKV_EXPORT int sakv_dual_scan(const void* xbc, int c_dtype, long long stride, i
   const int cols = lanes_across * cv;        // value columns a block
   const dim3 grid((unsigned)((vdim + cols - 1) / cols), (unsigned)heads, (unsigned)walks);
   const size_t smem = (size_t)kRun * (2 * rs * rp + cols + 2) * sizeof(float);
-#define SAKV_DUAL_CV(RP, CV, PHASE, C)                                                           \
-  launch_ordered(dual_scan_kernel<RP, CV, PHASE, C>, grid, dim3(lanes_across * rs), smem, stream, \
+#define SAKV_DUAL_CV(RP, CV, C)                                                                  \
+  launch_ordered(dual_scan_kernel<RP, CV, C>, grid, dim3(lanes_across * rs), smem, stream,       \
                  DualScan<C>{(const C*)xbc, stride, x_off, b_off, c_off, dt, dt_stride, dt_bias, \
                              a, d_skip, state, cu_seqlens, slots, out, heads, groups, dim, vdim, \
-                             rs, cols, keep_state, chunk_len, max_chunks, scratch, dt_sums})
-#define SAKV_DUAL(RP, PHASE, C)                                                                  \
-  (four ? SAKV_DUAL_CV(RP, 4, PHASE, C) : SAKV_DUAL_CV(RP, 1, PHASE, C))
-#define SAKV_DUAL_ALL(RP, C)                                                                     \
-  do {                                                                                           \
-    if (!runs) return SAKV_DUAL(RP, 0, C);                                                       \
-    int code = SAKV_DUAL(RP, 1, C);                                                              \
-    if (code) return code;                                                                       \
-    const long long per_head = (long long)vdim * dim;                                            \
-    const long long count = (long long)sequences * heads * per_head;                             \
-    code = launch_ordered(dual_carry_kernel, dim3((unsigned)((count + 127) / 128)), dim3(128),   \
-                          0, stream, a, state, scratch, (const float*)dt_sums, cu_seqlens,       \
-                          slots, sequences, heads, per_head, chunk_len, max_chunks, keep_state); \
-    if (code) return code;                                                                       \
-    return SAKV_DUAL(RP, 2, C);                                                                  \
-  } while (0)
+                             rs, cols, keep_state})
+#define SAKV_DUAL(RP, C)                                                                         \
+  return four ? SAKV_DUAL_CV(RP, 4, C) : SAKV_DUAL_CV(RP, 1, C)
   if (c_dtype == SAKV_F32) {
-    if (rp == 4) SAKV_DUAL_ALL(4, float);
-    SAKV_DUAL_ALL(8, float);
+    if (rp == 4) SAKV_DUAL(4, float);
+    SAKV_DUAL(8, float);
   }
   if (c_dtype == SAKV_BF16) {
-    if (rp == 4) SAKV_DUAL_ALL(4, __nv_bfloat16);
-    SAKV_DUAL_ALL(8, __nv_bfloat16);
+    if (rp == 4) SAKV_DUAL(4, __nv_bfloat16);
+    SAKV_DUAL(8, __nv_bfloat16);
   }
-#undef SAKV_DUAL_ALL
 #undef SAKV_DUAL
 #undef SAKV_DUAL_CV
   return cudaErrorInvalidValue;

@@ -59,9 +59,13 @@ SIGNATURES = {
                                                I, I, I, I, I, I, I, P, P, P, P, I, P]),
     "sakv_conv_step": ("recurrent_scan", [P, L, P, P, I, P, P, P, I, I, I, I, I, P]),
     "sakv_decay_attention": ("recurrent_scan", [P, L, I, I, I, P, P, P, P, P, I, I, I, I, I, I,
-                                                I, I, P, I, I, P, P, P, F, P]),
+                                                I, I, P, P, P, F, P]),
     "sakv_dual_scan": ("recurrent_scan", [P, I, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, I,
-                                          I, I, I, I, P, P, P]),
+                                          I, I, P]),
+    "sakv_chunk_fade": ("chunk_scan", [P, L, I, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P,
+                                       I, I, P, P, P, F, P]),
+    "sakv_chunk_dual": ("chunk_scan", [P, I, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I,
+                                       I, I, I, P, P, P]),
     "sakv_norm_gate": ("recurrent_scan", [P, P, I, P, L, P, I, I, I, I, I, I, F, F, P]),
     "sakv_layer_norm": ("layer_norm", [P, P, P, P, P, I, P, I, I, I, F, P]),
     "sakv_latent_prepare": ("latent", [P, L, I, I, I, P, P, I, F, P, P, P, I, P, P, P, P, I, I, I,

@@ -1,12 +1,17 @@
 """The recurrences without feedback from the state into its own update, over a step's tokens
 (`csrc/recurrent_scan.cu`): the selective scan with its convolution and step sizes, attention
-without softmax over a fading state with its norm and gate, and the state-space dual form."""
+without softmax over a fading state with its norm and gate, and the state-space dual form; the
+last two over a long prompt as matrix products a run (`csrc/chunk_scan.cu`)."""
 
 from __future__ import annotations
 
 import torch
 
 from ._lib import KernelError, call, dtype_code, ptr, require_cuda
+
+
+#: most tokens of a run that csrc/chunk_scan.cu takes
+CHUNK = 64
 
 
 def _check(cond: bool, message: str) -> None:
@@ -143,7 +148,8 @@ def decay_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, head
     token's position (pairs (i, i + rot / 2)); `key_scale` multiplies k after that.
     `decay_less_one`: fp32 [heads] holding `decay - 1` (the kernel adds `(decay - 1) S + k
     v^T` to S). `state`: fp32 [slots, heads, vdim, dim] (the state's transpose), read and (with
-    `keep_state`) left. `run`: as in `selective_scan`. Returns fp32 [T, heads * vdim]."""
+    `keep_state`) left. `run`: as in `selective_scan`, a run of up to `CHUNK` tokens as matrix
+    products. Returns fp32 [T, heads * vdim]."""
     require_cuda(proj, decay_less_one, state, cos, sin)
     rot = 0
     if cos is not None:
@@ -161,12 +167,17 @@ def decay_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, head
     _check(state.dtype == torch.float32 and state.is_contiguous()
            and tuple(state.shape[1:]) == (heads, vdim, dim), "state: fp32 [slots, heads, vdim, dim]")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=proj.device)
-    runs, scratch, _ = _runs(run, step, heads * vdim * dim, 0, proj.device)
-    call("sakv_decay_attention", ptr(proj), proj.stride(0), int(q_off), int(k_off), int(v_off),
-         ptr(decay_less_one), ptr(state), ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens,
-         step.sequences, heads, dim, vdim, int(keep_state), int(run) if runs else 0, runs,
-         ptr(scratch), int(bool(activation)), rot, ptr(step.positions) if rot else None, ptr(cos),
-         ptr(sin), float(key_scale))
+    run = min(int(run), CHUNK)
+    runs, scratch, logs = _runs(run, step, heads * vdim * dim, heads, proj.device)
+    args = (ptr(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), ptr(decay_less_one),
+            ptr(state), ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens, step.sequences,
+            heads, dim, vdim, int(keep_state))
+    shape = (int(bool(activation)), rot, ptr(step.positions) if rot else None, ptr(cos), ptr(sin),
+             float(key_scale))
+    if runs:
+        call("sakv_chunk_fade", *args, run, runs, ptr(scratch), ptr(logs), *shape)
+    else:
+        call("sakv_decay_attention", *args, *shape)
     return out
 
 
@@ -179,7 +190,7 @@ def dual_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dt: torch.T
     type with x (heads * vdim columns from `x_off`), B and C (groups * n_state each from `b_off`,
     `c_off`; head h reads group floor(h / (heads / groups))); `dt`: fp32 [T, heads] (any row
     stride); `dt_bias`, `a` (negative), `d_skip`: fp32 [heads]. `state`: fp32 [slots, heads, vdim,
-    n_state], read and (with `keep_state`) left. `run`: as in `selective_scan`. Returns fp32 [T,
+    n_state], read and (with `keep_state`) left. `run`: as in `decay_attention`. Returns fp32 [T,
     heads * vdim]."""
     require_cuda(xbc, dt, dt_bias, a, d_skip, state)
     tokens = xbc.shape[0]
@@ -196,11 +207,16 @@ def dual_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dt: torch.T
            and tuple(state.shape[1:]) == (heads, vdim, n_state),
            "state: fp32 [slots, heads, vdim, n_state]")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=xbc.device)
-    runs, scratch, sums = _runs(run, step, heads * vdim * n_state, heads, xbc.device)
-    call("sakv_dual_scan", ptr(xbc), dtype_code(xbc.dtype), xbc.stride(0), int(x_off), int(b_off),
-         int(c_off), ptr(dt), dt.stride(0), ptr(dt_bias), ptr(a), ptr(d_skip), ptr(state),
-         ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens, step.sequences, heads, groups,
-         n_state, vdim, int(keep_state), int(run) if runs else 0, runs, ptr(scratch), ptr(sums))
+    run = min(int(run), CHUNK)
+    runs, scratch, logs = _runs(run, step, heads * vdim * n_state, heads, xbc.device)
+    args = (ptr(xbc), dtype_code(xbc.dtype), xbc.stride(0), int(x_off), int(b_off), int(c_off),
+            ptr(dt), dt.stride(0), ptr(dt_bias), ptr(a), ptr(d_skip), ptr(state),
+            ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens, step.sequences, heads, groups,
+            n_state, vdim, int(keep_state))
+    if runs:
+        call("sakv_chunk_dual", *args, run, runs, ptr(scratch), ptr(logs))
+    else:
+        call("sakv_dual_scan", *args)
     return out
 
 
