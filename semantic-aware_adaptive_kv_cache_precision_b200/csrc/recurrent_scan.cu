@@ -41,6 +41,32 @@ __device__ __forceinline__ float exp_less_one(float x) {
   return x > -0.125f ? series : __expf(x) - 1.f;
 }
 
+// Eight neighbouring elements as fp32, in 16-byte accesses (p at a multiple of 16 bytes).
+__device__ __forceinline__ void read8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void read8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 raw = *reinterpret_cast<const uint4*>(p);
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __bfloat1622float2(h[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+__device__ __forceinline__ void write8(float* p, const float (&v)[8]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void write8(__nv_bfloat16* p, const float (&v)[8]) {
+  __nv_bfloat162 h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+}
+
 // Between the two passes over a prompt's runs: one number of the state is carried from run to run.
 // What run j left at p[j * step] is replaced by what came before it, which fades by fade(j) + 1
 // over the run. Bound by memory (every run's state is read and written once): the runs' numbers are
@@ -319,22 +345,39 @@ __global__ void selective_scan_kernel(const C* __restrict__ x, const float* __re
   }
   const float skip = widen(d_skip[c]);
   float dt_sum = 0.f;
+  // (16-bit mode: the channel's lanes share out a step size's products, eight neighbouring ones at a
+  // time; one lane's walk over 128 of them took 11 of the kernel's 14 us)
+  const bool share = sizeof(C) == 2 && sizeof(W) == 2 && rank % 8 == 0 && low_stride % 4 == 0 &&
+                     (((uintptr_t)low | (uintptr_t)w_dt) & 15) == 0;
   for (int t = first; t < last; ++t) {
-    float step;
-    if (PHASE == 0 && dt == nullptr) {
-      // the step size made here (a step of few tokens): the same products in the same order
-      // as the tiled kernel adds them
-      const float* lt = low + (long long)t * low_stride;
-      const W* wr = w_dt + (long long)c * rank;
-      float acc = 0.f;
-      for (int r = 0; r < rank; ++r) acc = fmaf(lt[r], widen(wr[r]), acc);
-      step = softplus(acc + (b_dt ? widen(b_dt[c]) : 0.f));
-    } else {
-      step = dt[(long long)t * channels + c];
-    }
     const float xv = widen(x[(long long)t * channels + c]);
     const float* bt = low + (long long)t * low_stride + b_off + n0;
     const float* ct = low + (long long)t * low_stride + c_off + n0;
+    const float zv = PHASE != 1 ? z[(long long)t * z_stride + c] : 0.f;
+    float step;
+    if (PHASE == 0 && dt == nullptr) {
+      const float* lt = low + (long long)t * low_stride;
+      const W* wr = w_dt + (long long)c * rank;
+      const float bias = b_dt ? widen(b_dt[c]) : 0.f;
+      float acc = 0.f;
+      if (share) {
+#pragma unroll 4
+        for (int r = g * 8; r < rank; r += lanes * 8) {
+          float w8[8], l8[8];
+          read8(reinterpret_cast<const __nv_bfloat16*>(wr) + r, w8);
+          read8(lt + r, l8);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc = fmaf(l8[i], w8[i], acc);
+        }
+        for (int o = lanes >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      } else {
+        // the same products in the same order as the tiled kernel adds them
+        for (int r = 0; r < rank; ++r) acc = fmaf(lt[r], widen(wr[r]), acc);
+      }
+      step = softplus(acc + bias);
+    } else {
+      step = dt[(long long)t * channels + c];
+    }
     const float dx = step * xv;
     dt_sum += step;
     float y = 0.f;
@@ -350,7 +393,7 @@ __global__ void selective_scan_kernel(const C* __restrict__ x, const float* __re
       for (int o = lanes >> 1; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
       if (g == 0 && live) {
         y = fmaf(skip, xv, y);
-        out[(long long)t * channels + c] = narrow<C>(y * silu(z[(long long)t * z_stride + c]));
+        out[(long long)t * channels + c] = narrow<C>(y * silu(zv));
       }
     }
   }
@@ -361,6 +404,136 @@ __global__ void selective_scan_kernel(const C* __restrict__ x, const float* __re
   }
   if (PHASE == 1 && live && g == 0)
     dt_sums[((long long)b * max_chunks + run) * channels + c] = dt_sum;
+}
+
+// e^x - 1 of two numbers, as `exp_less_one<false>`.
+__device__ __forceinline__ scan::Two exp_less_one2(scan::Two x) {
+  using scan::two;
+  scan::Two p = scan::fma2(x, two(1.f / 720.f, 1.f / 720.f), two(1.f / 120.f, 1.f / 120.f));
+  p = scan::fma2(x, p, two(1.f / 24.f, 1.f / 24.f));
+  p = scan::fma2(x, p, two(1.f / 6.f, 1.f / 6.f));
+  p = scan::fma2(x, p, two(0.5f, 0.5f));
+  p = scan::fma2(x, p, two(1.f, 1.f));
+  const float2 series = scan::apart(scan::mul2(x, p)), v = scan::apart(x);
+  return two(v.x > -0.125f ? series.x : __expf(v.x) - 1.f, v.y > -0.125f ? series.y : __expf(v.y) - 1.f);
+}
+
+// The two passes over a prompt's runs for up to 16 states a channel in the 16-bit mode: a thread has a
+// channel's states, in pairs for the two-wide arithmetic, and so makes a token's output alone; B and C
+// come through shared memory sixteen tokens at a time, a channel's own numbers eight tokens ahead into
+// registers. Bound by instruction issue (about ten a state and token, one of them an exponential).
+// Four lanes a channel with every number read where it is used took 230 and 430 us over 3,400 tokens of
+// 4,096 channels.
+template <int PHASE, typename W>
+__global__ void __launch_bounds__(128)
+scan_run_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dt,
+                const float* __restrict__ low, long long low_stride, int b_off, int c_off,
+                const float* __restrict__ z, long long z_stride, const W* __restrict__ a_log,
+                const W* __restrict__ d_skip, const int32_t* __restrict__ cu_seqlens,
+                __nv_bfloat16* __restrict__ out, int channels, int n_state, int chunk_len,
+                int max_chunks, float* __restrict__ scratch, float* __restrict__ dt_sums) {
+  constexpr int N = 16, kTile = 16, kAhead = 8;
+  __shared__ __align__(16) float bs[kTile][N], cs[kTile][N];
+  const int b = blockIdx.y / max_chunks, run = blockIdx.y % max_chunks;
+  const int first = cu_seqlens[b] + run * chunk_len;
+  const int last = min(cu_seqlens[b + 1], first + chunk_len);
+  if (first >= last) return;                          // (the whole block)
+  const int c_raw = blockIdx.x * 128 + threadIdx.x;
+  const bool live = c_raw < channels;
+  const int c = live ? c_raw : channels - 1;
+  float* mine = scratch + (((long long)b * max_chunks + run) * channels + c) * n_state;
+  scan::Two a[N / 2], s[N / 2];
+  {
+    float av[N], sv[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      av[k] = k < n_state ? -expf(widen(a_log[(long long)c * n_state + k])) : 0.f;
+      sv[k] = PHASE == 2 && k < n_state ? mine[k] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < N; k += 2) {
+      a[k / 2] = scan::two(av[k], av[k + 1]);
+      s[k / 2] = scan::two(sv[k], sv[k + 1]);
+    }
+  }
+  const float skip = widen(d_skip[c]);
+  float dt_sum = 0.f;
+  float step[kAhead], xv[kAhead], zv[kAhead];
+  auto ask = [&](int t0) {
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      const long long t = min(t0 + q, last - 1);
+      step[q] = dt[t * channels + c];
+      xv[q] = widen(x[t * channels + c]);
+      if (PHASE == 2) zv[q] = z[t * z_stride + c];
+    }
+  };
+  ask(first);
+  for (int t0 = first; t0 < last; t0 += kTile) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < kTile * N; e += 128) {
+      const int t = t0 + e / N, k = e % N;
+      const bool has = t < last && k < n_state;
+      bs[e / N][k] = has ? low[(long long)t * low_stride + b_off + k] : 0.f;
+      if (PHASE == 2) cs[e / N][k] = has ? low[(long long)t * low_stride + c_off + k] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < kTile; h += kAhead) {
+      float st[kAhead], xs[kAhead], zs[kAhead];
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        st[q] = step[q];
+        xs[q] = xv[q];
+        zs[q] = zv[q];
+      }
+      if (t0 + h + kAhead < last) ask(t0 + h + kAhead);
+#pragma unroll
+      for (int q = 0; q < kAhead; ++q) {
+        const int t = t0 + h + q;
+        if (t >= last) break;
+        const float d = st[q], dx = d * xs[q];
+        const scan::Two d2 = scan::two(d, d), dx2 = scan::two(dx, dx);
+        dt_sum += d;
+        scan::Two y2[2] = {0ull, 0ull};
+        const ulonglong2* b4 = reinterpret_cast<const ulonglong2*>(bs[h + q]);
+        const ulonglong2* c4 = reinterpret_cast<const ulonglong2*>(cs[h + q]);
+#pragma unroll
+        for (int k = 0; k < N / 4; ++k) {
+          const ulonglong2 bv = b4[k];
+          const scan::Two bb[2] = {bv.x, bv.y};
+          scan::Two cc[2] = {0ull, 0ull};
+          if (PHASE == 2) {
+            const ulonglong2 cv = c4[k];
+            cc[0] = cv.x;
+            cc[1] = cv.y;
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            // S + (e^(dt A) - 1) S + dt x B: a decay close to 1 keeps its distance from 1 exactly
+            scan::Two& sk = s[2 * k + i];
+            const scan::Two e = exp_less_one2(scan::mul2(d2, a[2 * k + i]));
+            sk = scan::add2(sk, scan::fma2(e, sk, scan::mul2(dx2, bb[i])));
+            if (PHASE == 2) y2[i] = scan::fma2(sk, cc[i], y2[i]);
+          }
+        }
+        if (PHASE == 2 && live) {
+          const float2 y = scan::apart(scan::add2(y2[0], y2[1]));
+          out[(long long)t * channels + c] =
+              narrow<__nv_bfloat16>(fmaf(skip, xs[q], y.x + y.y) * silu(zs[q]));
+        }
+      }
+    }
+  }
+  if (PHASE == 1 && live) {
+#pragma unroll
+    for (int k = 0; k < N; k += 2) {
+      const float2 v = scan::apart(s[k / 2]);
+      if (k < n_state) mine[k] = v.x;
+      if (k + 1 < n_state) mine[k + 1] = v.y;
+    }
+    dt_sums[((long long)b * max_chunks + run) * channels + c] = dt_sum;
+  }
 }
 
 // Between the two passes over a prompt's runs: one thread a (sequence, channel, state) walks
@@ -667,32 +840,6 @@ __global__ void __launch_bounds__(256) dual_scan_kernel(const DualScan<C> p) {
   }
 }
 
-// Eight neighbouring elements as fp32, in 16-byte accesses (p at a multiple of 16 bytes).
-__device__ __forceinline__ void read8(const float* p, float (&v)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void read8(const __nv_bfloat16* p, float (&v)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __bfloat1622float2(h[i]);
-    v[2 * i] = f.x;
-    v[2 * i + 1] = f.y;
-  }
-}
-__device__ __forceinline__ void write8(float* p, const float (&v)[8]) {
-  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-  *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-}
-__device__ __forceinline__ void write8(__nv_bfloat16* p, const float (&v)[8]) {
-  __nv_bfloat162 h[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
-}
-
 // `norm_gate_kernel` below for rows of up to 4,096 numbers, multiples of 8 everywhere: a row's numbers
 // stay in registers, eight or sixteen a thread, read and written 16 bytes at a time, gate and values
 // asked for together. `lanes`: how many neighbouring threads share a part (more than 32: the
@@ -958,10 +1105,18 @@ SAKV_EXPORT int sakv_selective_scan(const void* x, int c_dtype, const float* dt,
                  (const W*)d_skip, state, cu_seqlens, slots, (C*)out, channels, n_state, lanes,  \
                  keep_state, chunk_len, max_chunks, scratch, dt_sums, (const W*)w_dt,            \
                  (const W*)b_dt, rank)
+  // (a prompt's runs, up to 16 states: a thread a channel)
+  const bool whole = c_dtype == SAKV_BF16 && n_state <= 16;
+  const dim3 across((unsigned)((channels + 127) / 128), (unsigned)walks);
+#define SAKV_SCAN_RUN(PHASE, W)                                                                  \
+  launch_ordered(scan_run_kernel<PHASE, W>, across, dim3(128), 0, stream, (const __nv_bfloat16*)x, \
+                 dt, low, low_stride, b_off, c_off, z, z_stride, (const W*)a_log,                \
+                 (const W*)d_skip, cu_seqlens, (__nv_bfloat16*)out, channels, n_state, chunk_len, \
+                 max_chunks, scratch, dt_sums)
 #define SAKV_SCAN_ALL(NPT, W, C)                                                                 \
   do {                                                                                           \
     if (!runs) return SAKV_SCAN(NPT, 0, W, C);                                                   \
-    int code = SAKV_SCAN(NPT, 1, W, C);                                                          \
+    int code = whole ? SAKV_SCAN_RUN(1, W) : SAKV_SCAN(NPT, 1, W, C);                            \
     if (code) return code;                                                                       \
     const long long count = (long long)sequences * channels * n_state;                           \
     code = launch_ordered(scan_carry_kernel<W>, dim3((unsigned)((count + 127) / 128)),           \
@@ -969,7 +1124,7 @@ SAKV_EXPORT int sakv_selective_scan(const void* x, int c_dtype, const float* dt,
                           cu_seqlens, slots, sequences, channels, n_state, chunk_len,            \
                           max_chunks, keep_state);                                               \
     if (code) return code;                                                                       \
-    return SAKV_SCAN(NPT, 2, W, C);                                                              \
+    return whole ? SAKV_SCAN_RUN(2, W) : SAKV_SCAN(NPT, 2, W, C);                                \
   } while (0)
 #define SAKV_SCAN_T(NPT)                                                                         \
   do {                                                                                           \
@@ -983,6 +1138,7 @@ SAKV_EXPORT int sakv_selective_scan(const void* x, int c_dtype, const float* dt,
   else SAKV_SCAN_T(16);
 #undef SAKV_SCAN_T
 #undef SAKV_SCAN_ALL
+#undef SAKV_SCAN_RUN
 #undef SAKV_SCAN
   return cudaErrorInvalidValue;
 }

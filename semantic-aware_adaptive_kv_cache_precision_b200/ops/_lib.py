@@ -64,6 +64,7 @@ SIGNATURES = {
                                           I, I, P]),
     "sakv_chunk_fade": ("chunk_scan", [P, L, I, I, I, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P,
                                        I, I, P, P, P, F, P]),
+    "sakv_chunk_step_size": ("chunk_scan", [P, L, I, P, P, P, I, I, P]),
     "sakv_chunk_dual": ("chunk_scan", [P, I, L, I, I, I, P, L, P, P, P, P, P, P, P, I, I, I, I, I, I,
                                        I, I, I, P, P, P]),
     "sakv_norm_gate": ("recurrent_scan", [P, P, I, P, L, P, I, I, I, I, I, I, F, F, P]),

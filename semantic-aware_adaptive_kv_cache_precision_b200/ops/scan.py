@@ -63,6 +63,10 @@ def step_size(low: torch.Tensor, rank: int, weight: torch.Tensor,
     _check(bias is None or (bias.shape == (channels,) and bias.is_contiguous()
                             and bias.dtype == weight.dtype), "bias: [channels] of the weight's type")
     dt = torch.empty((low.shape[0], channels), dtype=torch.float32, device=low.device)
+    if weight.dtype == torch.bfloat16 and rank <= 256:       # on the tensor cores
+        call("sakv_chunk_step_size", ptr(low), low.stride(0), int(rank), ptr(weight), ptr(bias),
+             ptr(dt), low.shape[0], channels)
+        return dt
     call("sakv_step_size", ptr(low), low.stride(0), int(rank), ptr(weight), ptr(bias),
          dtype_code(weight.dtype), ptr(dt), low.shape[0], channels)
     return dt

@@ -31,7 +31,7 @@ RUN = 64
 
 
 class SelectiveScanMixer(Part):
-    kernel_libraries = ("recurrent_scan", "gemm_f32", "gemm_tc", "gemm_few")
+    kernel_libraries = ("recurrent_scan", "chunk_scan", "gemm_f32", "gemm_tc", "gemm_few")
 
     def __init__(self, spec, prefix, mode):
         super().__init__(spec, prefix, mode)
