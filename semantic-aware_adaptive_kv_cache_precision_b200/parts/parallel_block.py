@@ -10,6 +10,7 @@ leaves the block as `pending`, and the next layer's norm adds it on its way.
 
 from __future__ import annotations
 
+from .. import ops
 from .base import Part, build_part, register_part
 from .block import _normed
 
@@ -48,6 +49,11 @@ class ParallelBlock(Part):
         defer = leave_pending and getattr(last, "can_defer", False)
         if self.ffn is None:
             return self.mixer.forward(h, step, view, x, write_cache, **({"defer": True} if defer else {}))
+        if defer and hasattr(self.ffn, "produce") and ops.goes_aside(step, h.shape[0]):
+            # (the feed-forward reads h alone, and what it gives waits for the next norm)
+            beside = ops.aside(lambda: self.ffn.produce(h, step), step, h.shape[0])
+            self.mixer.forward(h, step, view, x, write_cache)
+            return beside.join()
         self.mixer.forward(h, step, view, x, write_cache)
         return self.ffn.forward(h, step, x, **({"defer": True} if defer else {}))
 

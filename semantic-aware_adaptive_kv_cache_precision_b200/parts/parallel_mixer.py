@@ -81,9 +81,15 @@ class ParallelMixer(Part):
     def produce_branches(self, h, step, view, write_cache=True):
         """The two branches' outputs before their norms and the sum, each fp32 [T, hidden]."""
         proj = ops.linear(h, self.w_in, self.b_in, out_dtype=torch.float32)
-        return tuple(ops.linear(b.mix(proj, offset, h, step, part, write_cache), b.w_o,
-                                out_dtype=torch.float32)
-                     for b, offset, part in zip(self.branches, self.offsets, view.parts))
+
+        def branch(i):
+            b = self.branches[i]
+            return ops.linear(b.mix(proj, self.offsets[i], h, step, view.parts[i], write_cache), b.w_o,
+                              out_dtype=torch.float32)
+
+        second = ops.aside(lambda: branch(1), step, h.shape[0])
+        first = branch(0)
+        return first, second.join()
 
     def produce(self, h, step, view, write_cache=True):
         """The mixer's output, fp32 [T, hidden]."""
@@ -93,13 +99,13 @@ class ParallelMixer(Part):
                 norm.complete(out, y)
             return out if self.spec.scale == 1.0 else ops.scale_cap_(out, self.spec.scale)
         proj = ops.linear(h, self.w_in, self.b_in, out_dtype=torch.float32)
-        out = None
-        for b, offset, part in zip(self.branches, self.offsets, view.parts):
-            mixed = b.mix(proj, offset, h, step, part, write_cache)
-            if out is None:
-                out = ops.linear(mixed, b.w_o, out_dtype=torch.float32)
-            else:
-                ops.linear(mixed, b.w_o, accumulate_into=out)
+
+        def mixed(i):
+            return self.branches[i].mix(proj, self.offsets[i], h, step, view.parts[i], write_cache)
+
+        second = ops.aside(lambda: mixed(1), step, h.shape[0])
+        out = ops.linear(mixed(0), self.branches[0].w_o, out_dtype=torch.float32)
+        ops.linear(second.join(), self.branches[1].w_o, accumulate_into=out)
         return out if self.spec.scale == 1.0 else ops.scale_cap_(out, self.spec.scale)
 
     def forward(self, h, step, view, residual, write_cache=True):

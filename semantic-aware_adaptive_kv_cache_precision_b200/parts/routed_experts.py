@@ -102,6 +102,13 @@ class RoutedExperts(Part):
         """The feed-forward's output, fp32 [T, hidden]; with `into` (the fp32 stream) it is
         added there by the kernel that sums a token's rows."""
         s = self.spec
+        beside = None
+        if s.shared is not None:       # (needs nothing of the routing: a branch of a captured step)
+            def shared_expert():
+                act = ops.gated_up(h, self.w_shared_in,
+                                   (s.shared.limit, s.shared.alpha, s.shared.plus))
+                return ops.linear(act, self.w_shared_down, out_dtype=torch.float32)
+            beside = ops.aside(shared_expert, step, h.shape[0])
         logits = mixture.router_logits(h, self.w_route)
         routing = mixture.route(logits, s.experts, s.top, s.identity, s.score == "softmax",
                                 self.correction, s.groups, s.keep_groups, s.renormalize,
@@ -114,9 +121,7 @@ class RoutedExperts(Part):
         products = mixture.grouped_product(act, routing, self.w_down, None)
         shared = gate = None
         if s.shared is not None:
-            act = ops.gated_up(h, self.w_shared_in,
-                               (s.shared.limit, s.shared.alpha, s.shared.plus))
-            shared = ops.linear(act, self.w_shared_down, out_dtype=torch.float32)
+            shared = beside.join()
             gate = logits[:, self.outputs] if self.has_gate else None
         return mixture.combine(products, routing, not s.weight_input, shared, gate, h, into)
 
