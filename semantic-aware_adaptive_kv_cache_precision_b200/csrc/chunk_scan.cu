@@ -24,12 +24,19 @@
 // All products of a step of 16 are added to a sum of their own, the smallest first, and that sum to the
 // total: the tensor cores cut where they add, and a chain of them loses an ulp of the total a step.
 //
+// Measured (us; walked in runs -> as products): fading state, 3,001 tokens of 16 heads of 128 x 128: 593 +
+// 292 + 26 -> 171 + 89 + 14; dual form, 16 prompts of 500 tokens, 32 heads of 128 x 64: 288 + 165 + 120 ->
+// 135 + 54 + 33; 2,048 tokens of 64 heads: 275 + 157 + 64 -> 117 + 50 + 21. Error against 64 bits 1.6e-7
+// and 1.1e-7 (2.9e-7 and 1.7e-7 walked). What bounds them now is the splitting of fp32 into pieces and the
+// products of those, not memory.
+//
 // A run with an output that is not finite goes through its tokens one by one, in order, so that a value
 // that is not finite (or beyond 3.3e38, whose first piece would not be) is not felt before its token.
 #include "mma.cuh"
 #include "scan.cuh"
 
 #include <initializer_list>
+#include <type_traits>
 
 namespace {
 
@@ -43,15 +50,17 @@ constexpr int kThreads = 128;
 constexpr int kPitchV = kCols + 8;     // (rows 16 bytes apart modulo 128: ldmatrix without conflicts)
 
 // One step's inputs of the fading state: columns of an fp32 projection, shaped on their way in.
+// QUADS: everything in whole pieces of four numbers, so that a thread's loads are straight code.
+template <bool QUADS>
 struct FadeSource {
   static constexpr int kPieces = 3;
+  static constexpr bool kQuads = QUADS;
   const float* proj;
   long long stride;
   int q_off, k_off, v_off;
   const float* less_one;          // [heads]: the decay less one
   int dim, vdim;
   FadeInput in;
-  bool quads;                     // everything in whole 16-byte pieces
 
   __device__ float turned(const float* head, int t, int i) const {
     const float x = fade_act(head[i], in.act);
@@ -65,15 +74,17 @@ struct FadeSource {
   __device__ float4 acted(float4 v) const {
     return in.act ? make_float4(scan::silu(v.x), scan::silu(v.y), scan::silu(v.z), scan::silu(v.w)) : v;
   }
+  // TURN: whether numbers i to i + 3 are turned (any value where they do not come as one quad)
+  template <bool TURN>
   __device__ float4 turned4(const float* head, int t, int i) const {
-    if (!quads) {
+    if constexpr (!QUADS) {
       float v[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) v[k] = i + k < dim ? turned(head, t, i + k) : 0.f;
       return make_float4(v[0], v[1], v[2], v[3]);
     }
     const float4 x = acted(*reinterpret_cast<const float4*>(head + i));
-    if (i >= in.rot) return x;
+    if constexpr (!TURN) return x;
     const int half = in.rot >> 1, pair = i < half ? i : i - half;
     const float4 y = acted(*reinterpret_cast<const float4*>(head + (i < half ? i + half : pair)));
     const long long at = (long long)in.positions[t] * half + pair;
@@ -94,13 +105,18 @@ struct FadeSource {
     return fade_act(proj[(long long)t * stride + v_off + (long long)h * vdim + c], in.act);
   }
   // four neighbouring numbers, 0 beyond the head's
-  __device__ float4 query4(int t, int h, int i) const { return turned4(head_of(t, h, q_off), t, i); }
+  __device__ bool turns(int i) const { return i < in.rot; }
+  template <bool TURN>
+  __device__ float4 query4(int t, int h, int i) const {
+    return turned4<TURN>(head_of(t, h, q_off), t, i);
+  }
+  template <bool TURN>
   __device__ float4 key4(int t, int h, int i) const {
-    const float4 v = turned4(head_of(t, h, k_off), t, i);
+    const float4 v = turned4<TURN>(head_of(t, h, k_off), t, i);
     return make_float4(v.x * in.k_scale, v.y * in.k_scale, v.z * in.k_scale, v.w * in.k_scale);
   }
   __device__ float4 value4(int t, int h, int c) const {
-    if (quads)
+    if constexpr (QUADS)
       return acted(*reinterpret_cast<const float4*>(proj + (long long)t * stride + v_off +
                                                     (long long)h * vdim + c));
     float v[4];
@@ -114,9 +130,10 @@ struct FadeSource {
 };
 
 // One step's inputs of the dual form: x, B and C after the convolution, a step size a (token, head).
-template <typename C>
+template <typename C, bool QUADS>
 struct DualSource {
   static constexpr int kPieces = sizeof(C) == 2 ? 1 : 3;
+  static constexpr bool kQuads = QUADS;
   const C* xbc;
   long long stride;
   int x_off, b_off, c_off;
@@ -126,10 +143,9 @@ struct DualSource {
   const float* a;
   const float* d_skip;
   int dim, vdim, heads_a_group;
-  bool quads;                     // everything in whole pieces of four numbers
 
   __device__ float4 four(const C* row, int i, int size) const {
-    if (quads) {
+    if constexpr (QUADS) {
       if constexpr (sizeof(C) == 4) return *reinterpret_cast<const float4*>(row + i);
       const uint2 raw = *reinterpret_cast<const uint2*>(row + i);
       return make_float4(__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u),
@@ -140,9 +156,12 @@ struct DualSource {
     for (int k = 0; k < 4; ++k) v[k] = i + k < size ? widen(row[i + k]) : 0.f;
     return make_float4(v[0], v[1], v[2], v[3]);
   }
+  __device__ bool turns(int) const { return false; }
+  template <bool TURN>
   __device__ float4 query4(int t, int h, int i) const {
     return four(xbc + (long long)t * stride + c_off + h / heads_a_group * dim, i, dim);
   }
+  template <bool TURN>
   __device__ float4 key4(int t, int h, int i) const {
     return four(xbc + (long long)t * stride + b_off + h / heads_a_group * dim, i, dim);
   }
@@ -212,6 +231,31 @@ __device__ __forceinline__ Deal deal(int wide) {
   d.row = threadIdx.x >> shift;
   d.rows = kThreads >> shift;
   return d;
+}
+
+// Rows `row`, `row` + `step`, ... below `whole` of a tile, four numbers of each a thread (from `to` on, rows
+// `pitch` elements apart), from load(j), j below `n`, and zeros from there on. N rows are asked for before
+// the first is split, whatever j: a load that waited for a branch would be a trip to memory a row, and
+// sixteen of them were most of the kernels' time.
+template <int PIECES, int N, class Load>
+__device__ __forceinline__ void stage(__nv_bfloat16* to, int pitch, int apart, int row, int step, int whole,
+                                      int n, Load load) {
+  for (int j0 = row; j0 < whole; j0 += N * step) {
+    float4 v[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = load(min(j0 + q * step, n - 1));
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const int j = j0 + q * step;
+      if (j < whole) put4<PIECES>(to + j * pitch, apart, j < n ? v[q] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+  }
+}
+// The same of rows that are zeros.
+template <int PIECES>
+__device__ __forceinline__ void stage_zeros(__nv_bfloat16* to, int pitch, int apart, int row, int step,
+                                            int whole) {
+  for (int j = row; j < whole; j += step) put4<PIECES>(to + j * pitch, apart, make_float4(0.f, 0.f, 0.f, 0.f));
 }
 
 // d (two n-tiles) += the products of A's pieces and B's whose orders add up to no more than two.
@@ -332,24 +376,29 @@ __global__ void __launch_bounds__(kThreads) run_states(const Source src, const R
     if (blockIdx.x == 0 && lane == 0)
       r.logs[((long long)s.b * r.max_runs + s.run) * r.heads + h] = hi;
   }
-  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
   const int whole = (s.n + 15) & ~15;            // rows of the products
   const Deal d = deal(wide);
-  if (d.at < wide) {
-#pragma unroll 4
-    for (int j = d.row; j < whole; j += d.rows)
-      put4<NP>(ks + j * pitch + d.at, kTokens * pitch,
-               j < s.n && d.at < r.dim ? src.key4(s.first + j, h, d.at) : none);
+  if (d.at < r.dim) {
+    if (src.turns(d.at))
+      stage<NP, 8>(ks + d.at, pitch, kTokens * pitch, d.row, d.rows, whole, s.n,
+                   [&](int j) { return src.template key4<true>(s.first + j, h, d.at); });
+    else
+      stage<NP, 8>(ks + d.at, pitch, kTokens * pitch, d.row, d.rows, whole, s.n,
+                   [&](int j) { return src.template key4<false>(s.first + j, h, d.at); });
+  } else if (d.at < wide) {
+    stage_zeros<NP>(ks + d.at, pitch, kTokens * pitch, d.row, d.rows, whole);
   }
   __syncthreads();                               // (the weights)
   {
     const int c = (tid & 15) * 4;
-#pragma unroll 4
-    for (int j = tid >> 4; j < whole; j += kThreads / 16) {
-      const float4 v = j < s.n && col0 + c < r.vdim ? src.value4(s.first + j, h, col0 + c) : none;
-      const float w = weight[j];
-      put4<3>(vs + j * kPitchV + c, kTokens * kPitchV, make_float4(w * v.x, w * v.y, w * v.z, w * v.w));
-    }
+    if (col0 + c < r.vdim)
+      stage<3, 8>(vs + c, kPitchV, kTokens * kPitchV, tid >> 4, kThreads / 16, whole, s.n, [&](int j) {
+        const float4 v = src.value4(s.first + j, h, col0 + c);
+        const float w = weight[j];
+        return make_float4(w * v.x, w * v.y, w * v.z, w * v.w);
+      });
+    else
+      stage_zeros<3>(vs + c, kPitchV, kTokens * kPitchV, tid >> 4, kThreads / 16, whole);
   }
   float* state = r.scratch + (((long long)s.b * r.max_runs + s.run) * r.heads + h) *
                                  ((long long)r.vdim * r.dim);
@@ -483,16 +532,21 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
     double total;
     sums_of(src, s, h, steps, g_hi, g_lo, &total);
   }
-  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
   const int whole = (s.n + 15) & ~15;                    // rows of the products
   const Deal d = deal(wide);
-  if (d.at < wide) {
-#pragma unroll 4
-    for (int j = d.row; j < whole; j += d.rows) {
-      const bool in = j < s.n && d.at < r.dim;
-      put4<NP>(qs + j * pitch + d.at, kTokens * pitch, in ? src.query4(s.first + j, h, d.at) : none);
-      put4<NP>(turn + j * pitch + d.at, kTokens * pitch, in ? src.key4(s.first + j, h, d.at) : none);
-    }
+  if (d.at < r.dim) {
+    auto both = [&](auto turned) {
+      constexpr bool T = decltype(turned)::value;
+      stage<NP, 8>(qs + d.at, pitch, kTokens * pitch, d.row, d.rows, whole, s.n,
+                   [&](int j) { return src.template query4<T>(s.first + j, h, d.at); });
+      stage<NP, 8>(turn + d.at, pitch, kTokens * pitch, d.row, d.rows, whole, s.n,
+                   [&](int j) { return src.template key4<T>(s.first + j, h, d.at); });
+    };
+    if (src.turns(d.at)) both(std::true_type());
+    else both(std::false_type());
+  } else if (d.at < wide) {
+    stage_zeros<NP>(qs + d.at, pitch, kTokens * pitch, d.row, d.rows, whole);
+    stage_zeros<NP>(turn + d.at, pitch, kTokens * pitch, d.row, d.rows, whole);
   }
   __syncthreads();
   const uint32_t qs_at = static_cast<uint32_t>(__cvta_generic_to_shared(qs));
@@ -536,24 +590,21 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
 
   // what the state brings
   __syncthreads();
-  if (d.at < wide) {
+  {
     const int columns = min(kCols, (r.vdim - col0 + 15) & ~15);
-#pragma unroll 8
-    for (int c = d.row; c < columns; c += d.rows) {
-      const float* at = state + (long long)(col0 + c) * r.dim + d.at;
-      float4 v = none;
-      if (col0 + c < r.vdim && d.at < r.dim) {
-        if (r.dim % 4 == 0) {
-          v = *reinterpret_cast<const float4*>(at);
-        } else {
-          v.x = at[0];
-          if (d.at + 1 < r.dim) v.y = at[1];
-          if (d.at + 2 < r.dim) v.z = at[2];
-          if (d.at + 3 < r.dim) v.w = at[3];
-        }
-      }
-      put4<3>(turn + c * pitch + d.at, kTokens * pitch, v);
-    }
+    if (d.at < r.dim)
+      stage<3, 8>(turn + d.at, pitch, kTokens * pitch, d.row, d.rows, columns, min(kCols, r.vdim - col0),
+                  [&](int c) {
+                    const float* at = state + (long long)(col0 + c) * r.dim + d.at;
+                    if constexpr (Source::kQuads) return *reinterpret_cast<const float4*>(at);
+                    float4 v = make_float4(at[0], 0.f, 0.f, 0.f);
+                    if (d.at + 1 < r.dim) v.y = at[1];
+                    if (d.at + 2 < r.dim) v.z = at[2];
+                    if (d.at + 3 < r.dim) v.w = at[3];
+                    return v;
+                  });
+    else if (d.at < wide)
+      stage_zeros<3>(turn + d.at, pitch, kTokens * pitch, d.row, d.rows, columns);
   }
   __syncthreads();
   float acc[8][4];
@@ -593,10 +644,11 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
   __syncthreads();
   {
     const int c = (tid & 15) * 4;
-#pragma unroll 8
-    for (int j = tid >> 4; j < whole; j += kThreads / 16)
-      put4<NP>(turn + j * kPitchV + c, kTokens * kPitchV,
-               j < s.n && col0 + c < r.vdim ? src.value4(s.first + j, h, col0 + c) : none);
+    if (col0 + c < r.vdim)
+      stage<NP, 8>(turn + c, kPitchV, kTokens * kPitchV, tid >> 4, kThreads / 16, whole, s.n,
+                   [&](int j) { return src.value4(s.first + j, h, col0 + c); });
+    else
+      stage_zeros<NP>(turn + c, kPitchV, kTokens * kPitchV, tid >> 4, kThreads / 16, whole);
   }
   __syncthreads();
   bool odd = false;
@@ -661,11 +713,12 @@ bool multiples_of_4(std::initializer_list<long long> values) {
 // Step sizes of the selective scan: dt[t, c] = softplus(sum_r low[t, r] W[c, r] + b[c]), low fp32 in three
 // pieces, W bfloat16 as it is. A block has 64 tokens' rows of `low` and goes over `tiles` groups of 64
 // channels; warp w makes 16 tokens.
-// 3,400 tokens of 4,096 channels, rank 128: 185 us on the CUDA cores.
+// 3,400 tokens of 4,096 channels, rank 128: 85 us (on the CUDA cores 185), bound by the pieces and the softplus.
+template <bool QUADS>
 __global__ void __launch_bounds__(kThreads)
 step_sizes(const float* __restrict__ low, long long stride, int rank,
            const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ bias,
-           float* __restrict__ dt, int tokens, int channels, int tiles, bool quads) {
+           float* __restrict__ dt, int tokens, int channels, int tiles) {
   extern __shared__ __align__(16) uint32_t pool[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wide = (rank + 15) / 16 * 16, pitch = wide + 8;
@@ -673,23 +726,19 @@ step_sizes(const float* __restrict__ low, long long stride, int rank,
   __nv_bfloat16* ws = rows + 3 * kTokens * pitch;                        // [64][pitch]
   const int m0 = blockIdx.y * kTokens;
   const Deal d = deal(wide);
-  if (d.at < wide) {
-#pragma unroll 4
-    for (int j = d.row; j < kTokens; j += d.rows) {
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (m0 + j < tokens && d.at < rank) {
-        const float* at = low + (long long)(m0 + j) * stride + d.at;
-        if (quads) {
-          read4(at, v);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (d.at + k < rank) v[k] = at[k];
-        }
-      }
-      put4<3>(rows + j * pitch + d.at, kTokens * pitch, make_float4(v[0], v[1], v[2], v[3]));
-    }
-  }
+  if (d.at < rank)
+    stage<3, 8>(rows + d.at, pitch, kTokens * pitch, d.row, d.rows, kTokens, min(kTokens, tokens - m0),
+                [&](int j) {
+                  const float* at = low + (long long)(m0 + j) * stride + d.at;
+                  if constexpr (QUADS) return *reinterpret_cast<const float4*>(at);
+                  float4 v = make_float4(at[0], 0.f, 0.f, 0.f);
+                  if (d.at + 1 < rank) v.y = at[1];
+                  if (d.at + 2 < rank) v.z = at[2];
+                  if (d.at + 3 < rank) v.w = at[3];
+                  return v;
+                });
+  else if (d.at < wide)
+    stage_zeros<3>(rows + d.at, pitch, kTokens * pitch, d.row, d.rows, kTokens);
   const uint32_t rows_at = static_cast<uint32_t>(__cvta_generic_to_shared(rows));
   const uint32_t ws_at = static_cast<uint32_t>(__cvta_generic_to_shared(ws));
   const uint32_t from = rows_at + ((warp * 16 + a_row(lane)) * pitch + a_col(lane)) * 2;
@@ -698,24 +747,21 @@ step_sizes(const float* __restrict__ low, long long stride, int rank,
     const int n0 = (blockIdx.x * tiles + i) * 64;
     if (n0 >= channels) break;
     if (i) __syncthreads();
-    if (d.at < wide) {
-#pragma unroll 8
-      for (int j = d.row; j < 64; j += d.rows) {
-        uint2 v = make_uint2(0u, 0u);
-        if (n0 + j < channels && d.at < rank) {
-          const __nv_bfloat16* at = w + (long long)(n0 + j) * rank + d.at;
-          if (quads) {
-            v = *reinterpret_cast<const uint2*>(at);
-          } else {
-            float f[4];
+    if (d.at < rank)
+      stage<1, 8>(ws + d.at, pitch, 0, d.row, d.rows, 64, min(64, channels - n0), [&](int j) {
+        const __nv_bfloat16* at = w + (long long)(n0 + j) * rank + d.at;
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (QUADS) {
+          read4(at, f);
+        } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) f[k] = d.at + k < rank ? widen(at[k]) : 0.f;
-            v = make_uint2(mma::pack_bf16(f[0], f[1]), mma::pack_bf16(f[2], f[3]));
-          }
+          for (int k = 0; k < 4; ++k)
+            if (d.at + k < rank) f[k] = widen(at[k]);
         }
-        *reinterpret_cast<uint2*>(ws + j * pitch + d.at) = v;
-      }
-    }
+        return make_float4(f[0], f[1], f[2], f[3]);
+      });
+    else if (d.at < wide)
+      stage_zeros<1>(ws + d.at, pitch, 0, d.row, d.rows, 64);
     __syncthreads();
     float acc[8][4];
 #pragma unroll
@@ -805,9 +851,11 @@ SAKV_EXPORT int sakv_chunk_step_size(const float* low, long long stride, int ran
   if (tokens == 0) return 0;
   static PerDeviceOnce once;
   if (once.needs()) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(step_sizes, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    if (e != cudaSuccess) return static_cast<int>(e);
+    for (const void* kernel : {(const void*)step_sizes<true>, (const void*)step_sizes<false>}) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+      if (e != cudaSuccess) return static_cast<int>(e);
+    }
     once.done();
   }
   const size_t pitch = (rank + 15) / 16 * 16 + 8;
@@ -816,10 +864,10 @@ SAKV_EXPORT int sakv_chunk_step_size(const float* low, long long stride, int ran
   int tiles = 4;                             // (fewer while the blocks do not fill the GPU twice)
   while (tiles > 1 && (long long)((groups + tiles - 1) / tiles) * down < 4LL * sm_count()) tiles /= 2;
   const bool quads = multiples_of_4({stride, rank}) && !((uintptr_t)low & 15) && !((uintptr_t)w & 7);
-  return launch_ordered(step_sizes, dim3((unsigned)((groups + tiles - 1) / tiles), (unsigned)down),
-                        dim3(kThreads), kTokens * pitch * 4 * 2, stream, low, stride, rank,
-                        (const __nv_bfloat16*)w, (const __nv_bfloat16*)bias, dt, tokens, channels,
-                        tiles, quads);
+  return launch_ordered(quads ? step_sizes<true> : step_sizes<false>,
+                        dim3((unsigned)((groups + tiles - 1) / tiles), (unsigned)down), dim3(kThreads),
+                        kTokens * pitch * 4 * 2, stream, low, stride, rank, (const __nv_bfloat16*)w,
+                        (const __nv_bfloat16*)bias, dt, tokens, channels, tiles);
 }
 
 // As `sakv_decay_attention` (csrc/recurrent_scan.cu), a sequence's tokens in runs of run_len (up to 64):
@@ -837,10 +885,13 @@ SAKV_EXPORT int sakv_chunk_fade(const float* proj, long long stride, int q_off, 
   if (tokens == 0 || sequences == 0) return 0;
   const bool quads = multiples_of_4({stride, q_off, k_off, v_off, dim, vdim, rot / 2}) &&
                      !(((uintptr_t)proj | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15);
-  const FadeSource src = {proj, stride, q_off, k_off, v_off, decay, dim, vdim,
-                          FadeInput{act, rot, positions, cos_t, sin_t, k_scale}, quads};
+  const FadeInput in = {act, rot, positions, cos_t, sin_t, k_scale};
   const Runs r = {scratch, logs, cu_seqlens, heads, dim, vdim, run_len, max_runs};
-  return launch_runs(src, r, state, slots, out, sequences, keep_state, stream);
+  if (quads)
+    return launch_runs(FadeSource<true>{proj, stride, q_off, k_off, v_off, decay, dim, vdim, in}, r, state,
+                       slots, out, sequences, keep_state, stream);
+  return launch_runs(FadeSource<false>{proj, stride, q_off, k_off, v_off, decay, dim, vdim, in}, r, state,
+                     slots, out, sequences, keep_state, stream);
 }
 
 // As `sakv_dual_scan`, likewise.
@@ -858,12 +909,19 @@ SAKV_EXPORT int sakv_chunk_dual(const void* xbc, int c_dtype, long long stride, 
   const Runs r = {scratch, logs, cu_seqlens, heads, dim, vdim, run_len, max_runs};
   const bool quads = multiples_of_4({stride, x_off, b_off, c_off, dim, vdim}) &&
                      !((uintptr_t)xbc & (c_dtype == SAKV_F32 ? 15 : 7));
-#define SAKV_DUAL(C)                                                                             \
-  return launch_runs(DualSource<C>{(const C*)xbc, stride, x_off, b_off, c_off, dt, dt_stride,    \
-                                   dt_bias, a, d_skip, dim, vdim, heads / groups, quads},        \
+#define SAKV_DUAL(C, QUADS)                                                                      \
+  return launch_runs(DualSource<C, QUADS>{(const C*)xbc, stride, x_off, b_off, c_off, dt,        \
+                                          dt_stride, dt_bias, a, d_skip, dim, vdim,              \
+                                          heads / groups},                                       \
                      r, state, slots, out, sequences, keep_state, stream)
-  if (c_dtype == SAKV_F32) SAKV_DUAL(float);
-  if (c_dtype == SAKV_BF16) SAKV_DUAL(__nv_bfloat16);
+  if (c_dtype == SAKV_F32) {
+    if (quads) SAKV_DUAL(float, true);
+    SAKV_DUAL(float, false);
+  }
+  if (c_dtype == SAKV_BF16) {
+    if (quads) SAKV_DUAL(__nv_bfloat16, true);
+    SAKV_DUAL(__nv_bfloat16, false);
+  }
 #undef SAKV_DUAL
   return cudaErrorInvalidValue;
 }
