@@ -17,7 +17,7 @@ from . import attention_mma, gemm_tc
 from .branch import aside, goes_aside
 from .streams import streams_spread, streams_step, token_shift
 from .recurrent import delta_rule, gated_delta
-from .scan import causal_conv, decay_attention, dual_scan, norm_gate, selective_scan, step_size
+from .scan import causal_conv, decay_attention, dual_scan, norm_gate, run_length, selective_scan, step_size
 from . import mixture
 from .mixture import latent_prepare, rotate_heads
 from .attention import (attention_decode, attention_prefill, attention_prefill_tc, decode_splits,
@@ -32,7 +32,7 @@ __all__ = ["CACHE_BLOCK", "KernelError", "embed", "rms_norm", "rope_store", "att
            "kernel_errors", "gated_silu", "gelu_tanh", "relu_squared", "dense_up", "embed_pairs", "gated_delta", "streams_step", "streams_spread", "token_shift",
            "delta_rule", "kv_store", "layer_norm", "cached_attention", "mixture", "latent_prepare",
            "rotate_heads", "distance_attention", "rms_update", "rms_join", "qk_prepare", "causal_conv",
-           "decay_attention", "dual_scan", "norm_gate", "selective_scan", "step_size", "gated_up", "gemm_tc", "add_into", "scale_cap_", "linear", "per_head", "choose", "Deferred", "aside", "goes_aside"]
+           "decay_attention", "dual_scan", "norm_gate", "run_length", "selective_scan", "step_size", "gated_up", "gemm_tc", "add_into", "scale_cap_", "linear", "per_head", "choose", "Deferred", "aside", "goes_aside"]
 
 
 def _check(cond: bool, message: str) -> None:

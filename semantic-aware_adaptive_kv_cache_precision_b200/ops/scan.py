@@ -14,6 +14,16 @@ from ._lib import KernelError, call, dtype_code, ptr, require_cuda
 CHUNK = 64
 
 
+def run_length(max_new: int) -> int:
+    """Tokens a run for the fading state and the dual form, by the longest part of the step: runs as matrix
+    products are the faster form from 64 tokens on, in shorter runs up to 128, so that some go side by side
+    (us, one walk / runs; fading state, 16 heads of 128 x 128: 64 tokens 86 / 35, 128 tokens 169 / 43; dual
+    form, four prompts, 32 heads of 128 x 64: 59 / 31, 114 / 37; prompt steps of three designs of width
+    1,024, one prompt of 250: 2.08 / 1.03, 2.07 / 1.04 and 1.91 / 1.21 ms, 16 prompts of up to 100 tokens 2.28 /
+    2.28, 1.71 / 1.55 and 1.62 / 1.61; 8 of up to 40, in runs of 16: 0.98 / 1.05 and 0.77 / 0.85). 0: one walk."""
+    return 0 if max_new < 64 else 32 if max_new < 128 else CHUNK
+
+
 def _check(cond: bool, message: str) -> None:
     if not cond:
         raise KernelError(message)

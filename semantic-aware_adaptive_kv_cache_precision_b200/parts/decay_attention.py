@@ -9,7 +9,7 @@ The fused projection leaves fp32 (its accumulator, unrounded); the silus, the re
 norm and the gate are fp32 in both modes (`csrc/recurrent_scan.cu`). The state lives in the
 cache as fixed-size per-sequence state, stored as its transpose [heads, value_dim, dim]. The
 state moves by its change, `S += (decay - 1) S + k v^T`, with `decay - 1` rounded once from the
-exact number; in bfloat16 a long part of a prompt is walked in runs of `RUN` tokens side by side.
+exact number; in bfloat16 a long part of a prompt is walked in runs (`ops.run_length`) side by side.
 
 The spec's fields turn this into its relatives: no activation on q, k, v; the first numbers of
 every head of q and k turned by the token's position (the tables of a `RotaryHalf`, rotation in
@@ -30,10 +30,6 @@ from .. import ops
 from ..cache.needs import StateNeed
 from ..weights.decl import TensorDecl
 from .base import Part, build_part, register_part
-
-
-#: tokens a run when a long prompt is walked in runs side by side
-RUN = 64
 
 
 class DecayAttention(Part):
@@ -129,9 +125,7 @@ class DecayAttention(Part):
         """Tokens a run of a long prompt: in bfloat16 a sequence's part of the step is walked
         in runs side by side (the states carried between them in fp32). In the 32-bit mode,
         and for short parts, one walk, whose sums do not depend on how the sequence was cut."""
-        if self.act_dtype == torch.float32 or getattr(step, "max_new", 0) < 4 * RUN:
-            return 0
-        return RUN
+        return 0 if self.act_dtype == torch.float32 else ops.run_length(getattr(step, "max_new", 0))
 
     def prepare(self, device, max_positions):
         if self.position is not None:

@@ -12,7 +12,7 @@ exponentials, the state, the sums over it, the gate and the norm are fp32 in bot
 stored as its transpose [heads, vdim, state]) lives in the cache as two fixed-size states. The
 state moves by its change, `S += (e^(dt A) - 1) S + dt B x^T`.
 
-In bfloat16 a long part of a prompt is walked in runs of `RUN` tokens side by side. The part is a
+In bfloat16 a long part of a prompt is walked in runs (`ops.run_length`) side by side. The part is a
 mixer of its own (`produce`) and a branch of a `ParallelMixer`.
 """
 
@@ -24,9 +24,6 @@ from .. import ops
 from ..cache.needs import MultiNeed, StateNeed
 from ..weights.decl import TensorDecl
 from .base import Part, register_part
-
-#: tokens a run when a long prompt is walked in runs side by side
-RUN = 64
 
 
 class DualScanMixer(Part):
@@ -95,9 +92,7 @@ class DualScanMixer(Part):
         """Tokens a run of a long prompt: in bfloat16 a sequence's part of the step is walked
         in runs side by side (the states carried between them in fp32). In the 32-bit mode,
         and for short parts, one walk, whose sums do not depend on how the sequence was cut."""
-        if self.act_dtype == torch.float32 or getattr(step, "max_new", 0) < 4 * RUN:
-            return 0
-        return RUN
+        return 0 if self.act_dtype == torch.float32 else ops.run_length(getattr(step, "max_new", 0))
 
     # -- the part alone ---------------------------------------------------------------------
 
