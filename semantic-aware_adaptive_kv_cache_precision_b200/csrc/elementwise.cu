@@ -197,6 +197,50 @@ __global__ void relu_squared_bf16x8_kernel(const uint4* __restrict__ in, uint4* 
   }
 }
 
+// A bias on the rows of an fp32 product: a thread four neighbouring columns (QUADS, else one) of every
+// gridDim.y-th row, four rows asked for at a time. Columns whose biases are zero are left alone (the vector
+// of a product of several projections has them for those without one, most of it). Bound by memory: 3,400
+// rows of a prompt of two mixers side by side, width 2,048: 14 us, 104 as a broadcast addition of every column.
+template <bool QUADS, typename B>
+__global__ void __launch_bounds__(128)
+add_bias_kernel(float* __restrict__ y, long long ld, const B* __restrict__ bias, int tokens, int n) {
+  constexpr int kWide = QUADS ? 4 : 1;
+  const int c = (blockIdx.x * 128 + threadIdx.x) * kWide;
+  if (c >= n) return;
+  float b[kWide];
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < kWide; ++k) {
+    b[k] = widen(bias[c + k]);
+    any |= b[k] != 0.f;
+  }
+  if (!any) return;
+  const int step = gridDim.y;
+  for (int t0 = blockIdx.y; t0 < tokens; t0 += 4 * step) {
+    float v[4][kWide];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float* at = y + (long long)min(t0 + r * step, tokens - 1) * ld + c;
+      if constexpr (QUADS) {
+        const float4 f = *reinterpret_cast<const float4*>(at);
+        v[r][0] = f.x; v[r][1] = f.y; v[r][2] = f.z; v[r][3] = f.w;
+      } else {
+        v[r][0] = at[0];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (t0 + r * step >= tokens) break;
+      float* at = y + (long long)(t0 + r * step) * ld + c;
+      if constexpr (QUADS)
+        *reinterpret_cast<float4*>(at) =
+            make_float4(v[r][0] + b[0], v[r][1] + b[1], v[r][2] + b[2], v[r][3] + b[3]);
+      else
+        at[0] = v[r][0] + b[0];
+    }
+  }
+}
+
 }  // namespace
 
 // out = relu(in)^2 (in place is fine).
@@ -320,4 +364,26 @@ SAKV_EXPORT int sakv_add_into(float* acc, const void* y, int dtype, long long co
   else
     return cudaErrorInvalidValue;
   return launch_status();
+}
+
+// y[t, :] += bias: y fp32 rows `ld` apart, bias [n] of `bias_dtype`.
+SAKV_EXPORT int sakv_add_bias(float* y, long long ld, const void* bias, int bias_dtype, int tokens, int n,
+                              cudaStream_t stream) {
+  if (tokens < 0 || n < 0 || ld < n) return cudaErrorInvalidValue;
+  if (tokens == 0 || n == 0) return 0;
+  const bool quads = n % 4 == 0 && ld % 4 == 0 && !((uintptr_t)y & 15);
+  const int across = ((quads ? n / 4 : n) + 127) / 128;
+  int down = (tokens + 3) / 4;
+  if (down > 65535) down = 65535;
+  const dim3 grid(across, down);
+#define SAKV_BIAS(B)                                                                             \
+  do {                                                                                           \
+    if (quads) add_bias_kernel<true, B><<<grid, 128, 0, stream>>>(y, ld, (const B*)bias, tokens, n); \
+    else add_bias_kernel<false, B><<<grid, 128, 0, stream>>>(y, ld, (const B*)bias, tokens, n);  \
+    return launch_status();                                                                      \
+  } while (0)
+  if (bias_dtype == SAKV_F32) SAKV_BIAS(float);
+  if (bias_dtype == SAKV_BF16) SAKV_BIAS(__nv_bfloat16);
+#undef SAKV_BIAS
+  return cudaErrorInvalidValue;
 }

@@ -24,6 +24,7 @@ SIGNATURES = {
     "sakv_embed": ("elementwise", [P, P, I, P, I, I, I, F, P, P, I, P]),
     "sakv_gated_silu": ("elementwise", [P, P, I, I, I, P]),
     "sakv_add_into": ("elementwise", [P, P, I, L, P]),
+    "sakv_add_bias": ("elementwise", [P, L, P, I, I, I, P]),
     "sakv_scale_cap": ("elementwise", [P, L, F, F, P]),
     "sakv_gelu_tanh": ("elementwise", [P, P, I, L, P]),
     "sakv_relu_squared": ("elementwise", [P, P, I, L, P]),

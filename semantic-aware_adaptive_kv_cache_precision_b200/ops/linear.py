@@ -16,7 +16,7 @@ from __future__ import annotations
 import torch
 
 from . import gemm_few, gemm_tc, gemm_wide
-from ._lib import KernelError, call, ptr, require_cuda
+from ._lib import KernelError, call, dtype_code, ptr, require_cuda
 
 #: up to this many tokens the library's own tcgen05 kernel runs (weights on the MMA's rows:
 #: made for decode); above it cuBLAS, whose 2-CTA kernels win once the tensor cores matter
@@ -134,6 +134,15 @@ def per_head(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> torch.
     return out
 
 
+def _add_bias(y: torch.Tensor, bias: torch.Tensor) -> None:
+    """`y += bias` for an fp32 product [T, N]."""
+    if bias.dtype not in (torch.float32, torch.bfloat16) or not bias.is_contiguous() \
+            or bias.shape != y.shape[1:]:
+        y += bias.float()
+        return
+    call("sakv_add_bias", ptr(y), y.stride(0), ptr(bias), dtype_code(bias.dtype), y.shape[0], y.shape[1])
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, *,
            out_dtype: torch.dtype | None = None,
            accumulate_into: torch.Tensor | None = None, may_defer: bool = False):
@@ -214,7 +223,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         from . import add_into
         y = torch.mm(xb, weight.t(), out_dtype=torch.float32)
         if bias is not None:
-            y += bias.float()
+            _add_bias(y, bias)
         if may_defer and acc.is_contiguous():
             return Deferred(y)
         add_into(acc, y)
@@ -222,7 +231,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     if out_dtype == torch.float32:
         y = torch.mm(xb, weight.t(), out_dtype=torch.float32)
         if bias is not None:
-            y += bias.float()
+            _add_bias(y, bias)
         return y
     if bias is not None:
         return torch.addmm(bias.to(torch.bfloat16), xb, weight.t())
