@@ -17,14 +17,15 @@ LARGE = 20_000_000     # bytes of a weight, from which on more than 8 tokens go 
 def takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether this kernel is the one for the product.
 
-    Its gain is at the ends of a kernel, and it reads x once for every 16 rows of the weight, so it is
-    for short rows and for products that one wave of blocks makes. Decode steps, us (this kernel for
-    every product / `csrc/gemm_tc.cu` for every product): width 1,536, one user 955 / 1,101 and 8 users
-    1,095 / 1,254; width 1,024 and 4 users 425 / 481; width 3,584 and 8 users, whose products have rows of
-    3,584 in more than a wave, 6,831 / 3,401 (between other kernels of a step they fall to a third of the
-    memory's rate, alone they are as fast as there: 44 / 43; with only one of a layer taken
-    no better). With more than 8 tokens x is as much to read as the weights, and a large product takes longer
-    (46 MB, 16 tokens: 14.9 / 11.3; 4 MB: 3.1 / 3.4; a step of 16 users 692 / 680, with the limit 688)."""
+    Its gain is at the ends of a kernel, and it reads x once for every 16 rows of the weight with more
+    instructions a byte than `csrc/gemm_tc.cu`, so it is for short rows and for products that one wave of
+    blocks makes. Decode steps, us (this kernel for every product / that one): width 1,536, one user 955 /
+    1,101 and 8 users 1,095 / 1,254; width 1,024 and 4 users 425 / 481. Width 3,584 and 8 users, rows of 3,584 in
+    more than a wave: alone the products are as fast (44 / 43), but in the steps after a prompt of 9,216
+    tokens, whose power holds the clocks down (every kernel of a step takes 1.7 times what it does after
+    2,560), instructions are what bounds this one and a step takes 6,831 / 3,401. With more than 8 tokens x
+    is as much to read as the weights, and a large product takes longer (46 MB, 16 tokens: 14.9 / 11.3; 4
+    MB: 3.1 / 3.4; a step of 16 users 692 / 680, with the limit 688)."""
     tokens = x.shape[0]
     if tokens > MAX_TOKENS or not gemm_tc.takes(x, weight):
         return False
