@@ -156,6 +156,7 @@ struct RouteForm {
   float scale;
 };
 
+constexpr int kKeys = 4;             // ranks a lane holds
 __device__ __forceinline__ void route_token(const float* __restrict__ z, int experts, int top,
                                             int32_t* __restrict__ chosen,
                                             float* __restrict__ weights,
@@ -218,25 +219,58 @@ __device__ __forceinline__ void route_token(const float* __restrict__ z, int exp
   }
   float sum_chosen = 0.f;
   uint32_t taken = 0;                              // bit i: this lane's i-th expert is chosen
-  for (int k = 0; k < top; ++k) {
-    float best = -INFINITY;
-    int at = 0x7fffffff;
-    for (int i = 0, e = lane; e < experts; ++i, e += 32) {
-      if (taken >> i & 1) continue;
-      if (form.groups > 1 && !(open >> (e / per_group) & 1)) continue;
-      const float v = rank_of(e);
-      if (v > best || (at == 0x7fffffff && !(v != v))) {
-        best = v;
-        at = e;
+  // Up to 128 outputs: the ranks once, as whole numbers in the floats' order (0: not a number, closed or
+  // taken), so that a choice is two reductions of the warp in hardware, not ten shuffles in a chain.
+  // (Decode steps, us a launch: one token 9.7 -> 7.5, 16 tokens 8.0 -> 7.2; alone, 64 tokens of 16 outputs 7.7 -> 7.0.)
+  uint32_t key[kKeys];
+  const bool by_key = experts <= 32 * kKeys;
+  if (by_key) {
+#pragma unroll
+    for (int i = 0; i < kKeys; ++i) {
+      const int e = lane + 32 * i;
+      key[i] = 0;
+      if (e < experts && (form.groups <= 1 || (open >> (e / per_group) & 1))) {
+        const float v = rank_of(e) + 0.f;          // (one zero)
+        const uint32_t bits = __float_as_uint(v);
+        if (v == v) key[i] = bits ^ (bits >> 31 ? 0xffffffffu : 0x80000000u);
       }
     }
+  }
+  for (int k = 0; k < top; ++k) {
+    int at = 0x7fffffff;
+    if (by_key) {
+      uint32_t mine = key[0];
+      int index = lane;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oa = __shfl_xor_sync(0xffffffffu, at, o);
-      if (ob > best || (ob == best && oa < at)) {
-        best = ob;
-        at = oa;
+      for (int i = 1; i < kKeys; ++i)
+        if (key[i] > mine) {
+          mine = key[i];
+          index = lane + 32 * i;
+        }
+      const uint32_t best = __reduce_max_sync(0xffffffffu, mine);
+      at = (int)__reduce_min_sync(0xffffffffu, best != 0 && mine == best ? (uint32_t)index : 0x7fffffffu);
+#pragma unroll
+      for (int i = 0; i < kKeys; ++i)
+        if (at == lane + 32 * i) key[i] = 0;
+    } else {
+      float best = -INFINITY;
+      for (int i = 0, e = lane; e < experts; ++i, e += 32) {
+        if (taken >> i & 1) continue;
+        if (form.groups > 1 && !(open >> (e / per_group) & 1)) continue;
+        const float v = rank_of(e);
+        if (v > best || (at == 0x7fffffff && !(v != v))) {
+          best = v;
+          at = e;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+        if (ob > best || (ob == best && oa < at)) {
+          best = ob;
+          at = oa;
+        }
       }
     }
     if (at == 0x7fffffff) at = k;                  // (a row without a finite logit)
