@@ -29,12 +29,16 @@ constexpr int kRows = 16;
 enum : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_ACCUM = 2, EPI_GATED = 3, EPI_CLAMPED = 4, EPI_RELU2 = 5 };
 constexpr bool gated_epi(int epi) { return epi == EPI_GATED || epi == EPI_CLAMPED; }
 
+// groups of columns a warp asks for at a time, at most
+constexpr int ahead(int epi) { return gated_epi(epi) ? 3 : 6; }
+
 struct Few {
   const __nv_bfloat16* x;
   long long ldx;
   const __nv_bfloat16* w;            // [rows, K]
   int M, N, K;
   int groups;                        // groups of 32 columns of one part
+  int each;                          // groups a warp takes at a time
   int dual_offset;
   float limit, alpha, plus;
   const void* bias;
@@ -57,11 +61,15 @@ __device__ __forceinline__ float bias_of(const Few& p, int n) {
                                   : widen(static_cast<const __nv_bfloat16*>(p.bias)[n]);
 }
 
-// NT: groups of eight tokens.
-template <int NT, int kEpi>
+// NT: groups of eight tokens. FULL: a warp takes as many groups of columns at a time as it has room for, known
+// when compiled (with the number an argument, steps of width 1,536 took 1,004 us for 959); else `each` of
+// them, so that all warps have the same (K 1,024: four, not six for five warps and two for the sixth; steps of
+// width 1,024 466 us for 503 and 550 for 571, and at K 512 the error against 64 bits is 7.4e-8, not 9.9e-8).
+template <int NT, int kEpi, bool FULL>
 __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
   constexpr int kSets = gated_epi(kEpi) ? 2 : 1;       // gate and up rows
-  constexpr int kAhead = kSets == 2 ? 3 : 6;           // groups of columns asked for at a time
+  constexpr int kAhead = ahead(kEpi);
+  const int each = FULL ? kAhead : p.each;
   __shared__ float sums[kSets][kWarps][NT * 8][kRows + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * kRows, part = blockIdx.y;
@@ -77,14 +85,14 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
   uint4 w[kAhead][kSets][2], x[kAhead][NT];
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
   auto ask = [&](int i, int g) {
-    const bool in = g < last && g * 32 + col < p.K;
+    const bool in = (FULL || i < each) && g < last && g * 32 + col < p.K;
 #pragma unroll
     for (int s = 0; s < kSets; ++s)
 #pragma unroll
       for (int h = 0; h < 2; ++h) w[i][s][h] = in ? stream16(from[s][h] + g * 32) : none;
   };
   auto ask_x = [&](int i, int g) {
-    const bool in = g < last && g * 32 + col < p.K;
+    const bool in = (FULL || i < each) && g < last && g * 32 + col < p.K;
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
       const int m = t * 8 + row;
@@ -104,17 +112,18 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
       for (int k = 0; k < 4; ++k) acc[s][t][0][k] = acc[s][t][1][k] = 0.f;
 
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) ask(i, first + warp * kAhead + i);
+  for (int i = 0; i < kAhead; ++i) ask(i, first + warp * each + i);
   float bias = 0.f;
   if (threadIdx.x < NT * 8 * kRows && n0 + (int)(threadIdx.x & 15) < p.N && part == 0)
     bias = bias_of(p, n0 + (threadIdx.x & 15));
   wait_for_previous_kernel();
   let_next_kernel_start();
 #pragma unroll
-  for (int i = 0; i < kAhead; ++i) ask_x(i, first + warp * kAhead + i);
-  for (int g0 = first + warp * kAhead; g0 < last; g0 += kAhead * kWarps) {
+  for (int i = 0; i < kAhead; ++i) ask_x(i, first + warp * each + i);
+  for (int g0 = first + warp * each; g0 < last; g0 += each * kWarps) {
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
+      if (!FULL && i >= each) break;
 #pragma unroll
       for (int s = 0; s < kSets; ++s) {
         const uint32_t a0[4] = {w[i][s][0].x, w[i][s][1].x, w[i][s][0].y, w[i][s][1].y};
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_few_kernel(const Few p) {
           mma::bf16_16816(acc[s][t][1], a1, x[i][t].z, x[i][t].w);
         }
       }
-      const int next = g0 + kAhead * kWarps + i;
+      const int next = g0 + each * kWarps + i;
       if (next < last) {
         ask(i, next);
         ask_x(i, next);
@@ -189,13 +198,18 @@ SAKV_EXPORT int sakv_gemm_few(const void* x, long long ldx, const void* w, int M
       (((uintptr_t)x | (uintptr_t)w) & 15))
     return cudaErrorInvalidValue;
   const int groups = (K + 31) / 32;
-  Few p = {(const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, (groups + parts - 1) / parts,
+  Few p = {(const __nv_bfloat16*)x, ldx, (const __nv_bfloat16*)w, M, N, K, (groups + parts - 1) / parts, 1,
            dual_offset, limit, alpha, plus, bias, bias_dtype, out, ldo, part_stride};
+  const int most = kWarps * ahead(epi), rounds = (p.groups + most - 1) / most;
+  p.each = (p.groups + kWarps * rounds - 1) / (kWarps * rounds);     // (the same for all warps, nearly)
   const dim3 grid((unsigned)((N + kRows - 1) / kRows), (unsigned)parts);
+  const bool full = p.each == ahead(epi);
+#define SAKV_FEW_AS(NT, EPI, FULL)                                                               \
+  launch_overlapped(gemm_few_kernel<NT, EPI, FULL>, grid, dim3(kThreads), 0, stream, 1, p)
 #define SAKV_FEW(EPI)                                                                            \
   if (epi == EPI)                                                                                \
-    return M <= 8 ? launch_overlapped(gemm_few_kernel<1, EPI>, grid, dim3(kThreads), 0, stream, 1, p) \
-                  : launch_overlapped(gemm_few_kernel<2, EPI>, grid, dim3(kThreads), 0, stream, 1, p)
+    return M <= 8 ? full ? SAKV_FEW_AS(1, EPI, true) : SAKV_FEW_AS(1, EPI, false)                \
+                  : full ? SAKV_FEW_AS(2, EPI, true) : SAKV_FEW_AS(2, EPI, false)
   SAKV_FEW(EPI_BF16);
   SAKV_FEW(EPI_F32);
   SAKV_FEW(EPI_ACCUM);
@@ -203,5 +217,6 @@ SAKV_EXPORT int sakv_gemm_few(const void* x, long long ldx, const void* w, int M
   SAKV_FEW(EPI_CLAMPED);
   SAKV_FEW(EPI_RELU2);
 #undef SAKV_FEW
+#undef SAKV_FEW_AS
   return cudaErrorInvalidValue;
 }
