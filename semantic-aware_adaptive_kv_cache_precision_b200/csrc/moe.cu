@@ -66,9 +66,9 @@ __global__ void logits_kernel(const T* __restrict__ h, const float* __restrict__
 }
 
 // Whether rows go by in groups of four neighbouring numbers (both kernels alike: a sum's order depends
-// on the width alone).
+// on the width alone; in the 32-bit mode it stays what one by one makes it).
 bool logits_by_fours(const void* h, int dtype, const float* w, int width) {
-  return width % 4 == 0 && (uintptr_t)h % (dtype == SAKV_F32 ? 16 : 8) == 0 && (uintptr_t)w % 16 == 0;
+  return dtype == SAKV_BF16 && width % 4 == 0 && (uintptr_t)h % 8 == 0 && (uintptr_t)w % 16 == 0;
 }
 
 // Whether sixteen sums a warp are the faster split: with 80 sums an SM there are warps enough, and a

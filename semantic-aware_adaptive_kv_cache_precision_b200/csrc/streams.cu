@@ -254,7 +254,8 @@ int launch_step(float* xs, long long stride, int streams, int tokens, int width,
                            (out_dtype == SAKV_F32 ? (uintptr_t)out : 0) |
                            (sizeof(W) == 4 ? (uintptr_t)norm_w | (uintptr_t)shift_w : 0);
     const uintptr_t narrow = (uintptr_t)out | (uintptr_t)norm_w | (uintptr_t)shift_w;
-    if (streams == S && width % 4 == 0 && width <= 4096 && stride % 4 == 0 && !(wide & 15) &&
+    // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
+    if (sizeof(W) == 2 && streams == S && width % 4 == 0 && width <= 4096 && stride % 4 == 0 && !(wide & 15) &&
         !(narrow & 7)) {
       auto go = [&](auto kernel, auto* o) {
         return launch_overlapped(kernel, dim3(tokens), dim3(kThreads), 0, stream, 1, xs, stride, width,
