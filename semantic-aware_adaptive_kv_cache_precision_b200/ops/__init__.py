@@ -14,7 +14,7 @@ from ._lib import (BF16, CACHE_BLOCK, F32, KernelError, call, dtype_code, plain_
                    require_cuda, sm_count)
 from .linear import Deferred, dense_up, gated_up, linear, per_head
 from . import attention_mma, gemm_tc
-from .branch import aside, goes_aside
+from .branch import apart, aside, goes_aside
 from .streams import streams_spread, streams_step, token_shift
 from .recurrent import delta_rule, gated_delta
 from .scan import causal_conv, decay_attention, dual_scan, norm_gate, run_length, selective_scan, step_size
@@ -536,10 +536,13 @@ def cached_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tens
         groups = tokens * kv_heads * (heads * maps // kv_heads + 3)
         floats = groups * key_splits * (max(dim, vdim + 2) + 4)
         scratch = torch.empty(floats, dtype=torch.float32, device=q.device)
-        tickets = _attention_tickets.get(q.device)
-        if tickets is None or tickets.numel() < groups:    # zero between calls: the last
-            tickets = _attention_tickets[q.device] = torch.zeros(        # block clears its own
-                max(groups, 4096), dtype=torch.int32, device=q.device)
+        if apart():                # (the blocks of another call may be counting at the same time)
+            tickets = torch.zeros(groups, dtype=torch.int32, device=q.device)
+        else:
+            tickets = _attention_tickets.get(q.device)
+            if tickets is None or tickets.numel() < groups:    # zero between calls: the last
+                tickets = _attention_tickets[q.device] = torch.zeros(        # block clears its own
+                    max(groups, 4096), dtype=torch.int32, device=q.device)
     else:
         key_splits = 1
     call("sakv_cached_attention", ptr(q), dtype_code(q.dtype), q.stride(0), q.stride(1), ptr(q2),

@@ -11,9 +11,7 @@ import threading
 
 import torch
 
-from .linear import TC_MAX_TOKENS
-
-_local = threading.local()      # the streams are a thread's own: captures of two threads never meet
+_local = threading.local()      # `streams`: a thread's own, by device; `open`: its branches not yet joined
 
 
 def _other_stream(main: torch.cuda.Stream) -> torch.cuda.Stream:
@@ -29,6 +27,13 @@ def _other_stream(main: torch.cuda.Stream) -> torch.cuda.Stream:
     return streams[at]
 
 
+def apart() -> bool:
+    """Whether what this thread launches now may run at the same time as another piece of its step (a
+    branch that is not joined yet). Scratch memory that calls share, one after another in stream order,
+    is not to be used then."""
+    return getattr(_local, "open", 0) > 0
+
+
 class Aside:
     """What `aside` started; `join()` lets the stream it started from wait for it and gives its result."""
 
@@ -39,14 +44,16 @@ class Aside:
 
     def join(self):
         if self.stream is not None:
-            self.main.wait_stream(self.stream)
-            self.stream = None
+            _local.open -= 1
+            stream, self.stream = self.stream, None
+            self.main.wait_stream(stream)
         return self.result
 
 
 def goes_aside(step, tokens: int) -> bool:
     """Whether `aside` gives work of this step a branch of its own: a decode step of few tokens that is
-    being captured (its products are this library's own, which share no scratch memory)."""
+    being captured."""
+    from .linear import TC_MAX_TOKENS
     return bool(getattr(step, "is_decode", False)) and tokens <= TC_MAX_TOKENS \
         and torch.cuda.is_current_stream_capturing()
 
@@ -58,12 +65,17 @@ def aside(work, step, tokens: int) -> Aside:
     Memory: the caller keeps whatever `work` reads until it has joined. `work`'s launches come before the
     main path's, so what the main path gives back meanwhile can only be given to a later branch, which
     begins after it; what the branch itself made is given to later branches only, which begin after
-    whoever read it."""
+    whoever read it. Neither side uses memory that calls share (`apart`)."""
     if not goes_aside(step, tokens):
         return Aside(work())
     main = torch.cuda.current_stream()
     stream = _other_stream(main)
     stream.wait_stream(main)
-    with torch.cuda.stream(stream):
-        result = work()
+    _local.open = getattr(_local, "open", 0) + 1
+    try:
+        with torch.cuda.stream(stream):
+            result = work()
+    except BaseException:
+        _local.open -= 1
+        raise
     return Aside(result, main, stream)

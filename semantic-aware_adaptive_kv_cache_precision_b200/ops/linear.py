@@ -17,6 +17,7 @@ import torch
 
 from . import gemm_few, gemm_tc, gemm_wide
 from ._lib import KernelError, call, dtype_code, ptr, require_cuda
+from .branch import apart
 
 #: up to this many tokens the library's own tcgen05 kernel runs (weights on the MMA's rows:
 #: made for decode); above it cuBLAS, whose 2-CTA kernels win once the tensor cores matter
@@ -53,6 +54,8 @@ def _library_adds(device) -> bool:
 
 
 def _library_workspace(device) -> torch.Tensor:
+    if apart():                # (another branch's product may be using the one that calls share)
+        return torch.empty(_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
     space = _workspaces.get(device)
     if space is None:
         space = _workspaces[device] = torch.empty(_WORKSPACE_BYTES, dtype=torch.uint8, device=device)
@@ -216,8 +219,9 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     if accumulate_into is not None and bias is None and LIBRARY_ADDS_IN_PLACE \
             and xb.stride(1) == 1 and acc.stride(1) == 1 and _library_adds(x.device):
         # the library adds into the stream itself (beta = 1), as the reference's products do
+        space = _library_workspace(x.device)
         call("sakv_lib_accumulate", ptr(xb), xb.stride(0), ptr(weight), ptr(acc), acc.stride(0),
-             tokens, n, k, ptr(_library_workspace(x.device)), _WORKSPACE_BYTES)
+             tokens, n, k, ptr(space), _WORKSPACE_BYTES)
         return acc
     if accumulate_into is not None:
         from . import add_into

@@ -1,0 +1,91 @@
+"""Branches of a captured step (`ops/branch.py`): they share no scratch memory with what runs beside them."""
+
+from __future__ import annotations
+
+import sys
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from semantic_aware_adaptive_kv_cache_precision_b200 import ops
+from semantic_aware_adaptive_kv_cache_precision_b200.ops import _lib
+
+DEV = "cuda"
+STEP = SimpleNamespace(is_decode=True)
+
+
+def captured(run):
+    """`run()` in a graph, after one run outside; (graph, the captured run's result)."""
+    run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = run()
+    return graph, out
+
+
+def attention_case(dim, seed, keys=700, tokens=2, heads=2):
+    """A decoded token of each of two sequences over caches in blocks, its keys shared out over four blocks."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    blocks = -(-keys // ops.CACHE_BLOCK)
+    cache = [torch.randn((tokens * blocks, heads, ops.CACHE_BLOCK, dim), generator=g, device=DEV).bfloat16()
+             for _ in range(2)]
+    q = torch.randn((tokens, heads, dim), generator=g, device=DEV).bfloat16()
+    table = torch.arange(tokens * blocks, dtype=torch.int32, device=DEV).view(tokens, blocks)
+    at = torch.full((tokens,), keys - 1, dtype=torch.int32, device=DEV)
+    seq = torch.arange(tokens, dtype=torch.int32, device=DEV)
+    return lambda: ops.cached_attention(q, *cache, at, seq, table, heads, dim, dim, dim ** -0.5,
+                                        heads_first=True, key_splits=4)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [80, 96, 256])
+def test_two_attentions_side_by_side(dim):
+    """Two calls whose blocks count how many of them are done, one in a branch: the same bits as one after
+    the other, whatever the count that calls in plain order share holds meanwhile."""
+    left, right = attention_case(dim, 1), attention_case(dim, 2)
+    want = [left().clone(), right().clone()]
+
+    def both():
+        beside = ops.aside(right, STEP, 2)
+        first = left()
+        return first, beside.join()
+
+    graph, out = captured(both)
+    shared = ops._attention_tickets[out[0].device]
+    shared.fill_(12345)          # (blocks that counted here would never be the last ones)
+    try:
+        for _ in range(20):
+            graph.replay()
+            assert torch.equal(out[0], want[0]) and torch.equal(out[1], want[1])
+            out[0].zero_(), out[1].zero_()
+    finally:
+        shared.zero_()
+    assert torch.equal(left(), want[0])
+
+
+@pytest.mark.gpu
+def test_the_library_s_workspace_is_not_shared_by_branches(monkeypatch):
+    """Products that only the library takes (rows of no whole 16 bytes), added into a stream."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x, w = (torch.randn(s, 12, generator=g, device=DEV).bfloat16() for s in (4, 20))
+    spaces = []
+    monkeypatch.setattr(sys.modules[ops.linear.__module__], "call", lambda name, *args: (
+        spaces.append(args[8]) if name == "sakv_lib_accumulate" else None, _lib.call(name, *args)))
+
+    def product():
+        return ops.linear(x, w, accumulate_into=torch.ones((4, 20), device=DEV))
+
+    def both():
+        spaces.clear()
+        beside = ops.aside(product, STEP, 4)
+        first = product()
+        return first, beside.join(), product()
+
+    graph, out = captured(both)
+    assert len(set(spaces)) == len(spaces) == 3
+    graph.replay()
+    want = 1 + x.double() @ w.double().T
+    for y in out:                                            # (12 products, fp32)
+        assert ((y.double() - want).abs() <= 16 * 2.0 ** -23 * (1 + want.abs())).all()
