@@ -35,19 +35,28 @@ def apart() -> bool:
 
 
 class Aside:
-    """What `aside` started; `join()` lets the stream it started from wait for it and gives its result."""
+    """What `aside` started. As a context: the stream it started from waits for it at the end (also when
+    something fails in between: what is captured then can still be ended, and the failure is what the
+    caller sees); from there on `result` may be read."""
 
     __slots__ = ("result", "main", "stream")
 
-    def __init__(self, result, main=None, stream=None):
-        self.result, self.main, self.stream = result, main, stream
+    def __init__(self, main=None, stream=None):
+        self.result, self.main, self.stream = None, main, stream
 
-    def join(self):
+    def __enter__(self):
+        return self
+
+    def __exit__(self, kind, value, trace):
         if self.stream is not None:
             _local.open -= 1
             stream, self.stream = self.stream, None
-            self.main.wait_stream(stream)
-        return self.result
+            try:
+                self.main.wait_stream(stream)
+            except Exception:
+                if kind is None:           # (else the capture itself has failed, and `value` says why)
+                    raise
+        return False
 
 
 def goes_aside(step, tokens: int) -> bool:
@@ -59,23 +68,26 @@ def goes_aside(step, tokens: int) -> bool:
 
 
 def aside(work, step, tokens: int) -> Aside:
-    """Start `work()` beside what the caller launches from here to `join()`; where it has no branch of its
-    own (`goes_aside`), run it here and now.
+    """`with aside(work, step, tokens) as beside: ...`: start `work()` beside what is launched in the
+    context; where it has no branch of its own (`goes_aside`), run it here and now. `work` None: nothing.
 
-    Memory: the caller keeps whatever `work` reads until it has joined. `work`'s launches come before the
+    Memory: the caller keeps whatever `work` reads until the context ends. `work`'s launches come before the
     main path's, so what the main path gives back meanwhile can only be given to a later branch, which
     begins after it; what the branch itself made is given to later branches only, which begin after
     whoever read it. Neither side uses memory that calls share (`apart`)."""
-    if not goes_aside(step, tokens):
-        return Aside(work())
+    if work is None or not goes_aside(step, tokens):
+        beside = Aside()
+        beside.result = work() if work is not None else None
+        return beside
     main = torch.cuda.current_stream()
     stream = _other_stream(main)
     stream.wait_stream(main)
     _local.open = getattr(_local, "open", 0) + 1
+    beside = Aside(main, stream)
     try:
         with torch.cuda.stream(stream):
-            result = work()
-    except BaseException:
-        _local.open -= 1
+            beside.result = work()
+    except BaseException as failure:
+        beside.__exit__(type(failure), failure, None)
         raise
-    return Aside(result, main, stream)
+    return beside

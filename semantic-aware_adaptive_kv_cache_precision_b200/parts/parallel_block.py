@@ -51,9 +51,9 @@ class ParallelBlock(Part):
             return self.mixer.forward(h, step, view, x, write_cache, **({"defer": True} if defer else {}))
         if defer and hasattr(self.ffn, "produce") and ops.goes_aside(step, h.shape[0]):
             # (the feed-forward reads h alone, and what it gives waits for the next norm)
-            beside = ops.aside(lambda: self.ffn.produce(h, step), step, h.shape[0])
-            self.mixer.forward(h, step, view, x, write_cache)
-            return beside.join()
+            with ops.aside(lambda: self.ffn.produce(h, step), step, h.shape[0]) as beside:
+                self.mixer.forward(h, step, view, x, write_cache)
+            return beside.result
         self.mixer.forward(h, step, view, x, write_cache)
         return self.ffn.forward(h, step, x, **({"defer": True} if defer else {}))
 

@@ -87,9 +87,9 @@ class ParallelMixer(Part):
             return ops.linear(b.mix(proj, self.offsets[i], h, step, view.parts[i], write_cache), b.w_o,
                               out_dtype=torch.float32)
 
-        second = ops.aside(lambda: branch(1), step, h.shape[0])
-        first = branch(0)
-        return first, second.join()
+        with ops.aside(lambda: branch(1), step, h.shape[0]) as second:
+            first = branch(0)
+        return first, second.result
 
     def produce(self, h, step, view, write_cache=True):
         """The mixer's output, fp32 [T, hidden]."""
@@ -103,9 +103,9 @@ class ParallelMixer(Part):
         def mixed(i):
             return self.branches[i].mix(proj, self.offsets[i], h, step, view.parts[i], write_cache)
 
-        second = ops.aside(lambda: mixed(1), step, h.shape[0])
-        out = ops.linear(mixed(0), self.branches[0].w_o, out_dtype=torch.float32)
-        ops.linear(second.join(), self.branches[1].w_o, accumulate_into=out)
+        with ops.aside(lambda: mixed(1), step, h.shape[0]) as second:
+            out = ops.linear(mixed(0), self.branches[0].w_o, out_dtype=torch.float32)
+        ops.linear(second.result, self.branches[1].w_o, accumulate_into=out)
         return out if self.spec.scale == 1.0 else ops.scale_cap_(out, self.spec.scale)
 
     def forward(self, h, step, view, residual, write_cache=True):

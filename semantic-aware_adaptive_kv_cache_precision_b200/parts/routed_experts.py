@@ -102,27 +102,24 @@ class RoutedExperts(Part):
         """The feed-forward's output, fp32 [T, hidden]; with `into` (the fp32 stream) it is
         added there by the kernel that sums a token's rows."""
         s = self.spec
-        beside = None
-        if s.shared is not None:       # (needs nothing of the routing: a branch of a captured step)
-            def shared_expert():
-                act = ops.gated_up(h, self.w_shared_in,
-                                   (s.shared.limit, s.shared.alpha, s.shared.plus))
-                return ops.linear(act, self.w_shared_down, out_dtype=torch.float32)
-            beside = ops.aside(shared_expert, step, h.shape[0])
-        logits = mixture.router_logits(h, self.w_route)
-        routing = mixture.route(logits, s.experts, s.top, s.identity, s.score == "softmax",
-                                self.correction, s.groups, s.keep_groups, s.renormalize,
-                                s.group_top, s.scale)
-        # (a checkpoint stored in 32 bits keeps its matrices so: the experts then run in 32 bits)
-        rows = mixture.gather_rows(h if h.dtype == self.w_gate.dtype else h.to(self.w_gate.dtype),
-                                   routing, s.weight_input)
-        act = mixture.grouped_product(rows, routing, self.w_gate, self.w_up, s.expert.limit,
-                                      s.expert.alpha, s.expert.plus)
-        products = mixture.grouped_product(act, routing, self.w_down, None)
-        shared = gate = None
-        if s.shared is not None:
-            shared = beside.join()
-            gate = logits[:, self.outputs] if self.has_gate else None
+        def shared_expert():
+            act = ops.gated_up(h, self.w_shared_in, (s.shared.limit, s.shared.alpha, s.shared.plus))
+            return ops.linear(act, self.w_shared_down, out_dtype=torch.float32)
+
+        # (the shared expert needs nothing of the routing: a branch of a captured step)
+        with ops.aside(shared_expert if s.shared is not None else None, step, h.shape[0]) as beside:
+            logits = mixture.router_logits(h, self.w_route)
+            routing = mixture.route(logits, s.experts, s.top, s.identity, s.score == "softmax",
+                                    self.correction, s.groups, s.keep_groups, s.renormalize,
+                                    s.group_top, s.scale)
+            # (a checkpoint stored in 32 bits keeps its matrices so: the experts then run in 32 bits)
+            rows = mixture.gather_rows(h if h.dtype == self.w_gate.dtype else h.to(self.w_gate.dtype),
+                                       routing, s.weight_input)
+            act = mixture.grouped_product(rows, routing, self.w_gate, self.w_up, s.expert.limit,
+                                          s.expert.alpha, s.expert.plus)
+            products = mixture.grouped_product(act, routing, self.w_down, None)
+        shared = beside.result
+        gate = logits[:, self.outputs] if s.shared is not None and self.has_gate else None
         return mixture.combine(products, routing, not s.weight_input, shared, gate, h, into)
 
     def forward(self, h, step, residual):

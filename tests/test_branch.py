@@ -10,6 +10,7 @@ import torch
 
 from semantic_aware_adaptive_kv_cache_precision_b200 import ops
 from semantic_aware_adaptive_kv_cache_precision_b200.ops import _lib
+from semantic_aware_adaptive_kv_cache_precision_b200.ops.branch import apart
 
 DEV = "cuda"
 STEP = SimpleNamespace(is_decode=True)
@@ -48,9 +49,9 @@ def test_two_attentions_side_by_side(dim):
     want = [left().clone(), right().clone()]
 
     def both():
-        beside = ops.aside(right, STEP, 2)
-        first = left()
-        return first, beside.join()
+        with ops.aside(right, STEP, 2) as beside:
+            first = left()
+        return first, beside.result
 
     graph, out = captured(both)
     shared = ops._attention_tickets[out[0].device]
@@ -79,9 +80,9 @@ def test_the_library_s_workspace_is_not_shared_by_branches(monkeypatch):
 
     def both():
         spaces.clear()
-        beside = ops.aside(product, STEP, 4)
-        first = product()
-        return first, beside.join(), product()
+        with ops.aside(product, STEP, 4) as beside:
+            first = product()
+        return first, beside.result, product()
 
     graph, out = captured(both)
     assert len(set(spaces)) == len(spaces) == 3
@@ -89,3 +90,76 @@ def test_the_library_s_workspace_is_not_shared_by_branches(monkeypatch):
     want = 1 + x.double() @ w.double().T
     for y in out:                                            # (12 products, fp32)
         assert ((y.double() - want).abs() <= 16 * 2.0 ** -23 * (1 + want.abs())).all()
+
+
+def small(x):
+    """Some of this library's kernels with temporaries that come and go."""
+    y = ops.linear(x, x, out_dtype=torch.float32)
+    ops.add_into(y, ops.linear(x, x, out_dtype=torch.float32))
+    return ops.linear(y.bfloat16(), x.T.contiguous(), out_dtype=torch.float32)
+
+
+@pytest.mark.gpu
+def test_a_branch_inside_a_branch():
+    """An outer and an inner branch in turn, twice, what they made given back in between: the bits of the
+    same calls one after the other."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    xs = [torch.randn(64, 64, generator=g, device=DEV).bfloat16() for _ in range(6)]
+
+    def outer(a, b):
+        with ops.aside(lambda: small(a), STEP, 64) as inner:
+            own = small(b)
+        return own + inner.result
+
+    def step():
+        outs = []
+        for a, b, c in (xs[:3], xs[3:]):
+            with ops.aside(lambda: outer(a, b), STEP, 64) as beside:
+                own = small(c)
+            outs.append(own - beside.result)
+            del own, beside
+        return outs
+
+    want = [y.clone() for y in step()]
+    graph, out = captured(step)
+    for _ in range(10):
+        graph.replay()
+        for y, w in zip(out, want):
+            assert torch.equal(y, w)
+            y.zero_()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["in the branch", "beside it", "in an inner branch"])
+def test_a_failure_ends_the_branch(where):
+    """What fails inside a capture is what the caller sees; afterwards everything works as before."""
+    x = torch.ones(64, 64, device=DEV).bfloat16()
+
+    def failing():
+        ops.linear(x, x)
+        raise ops.KernelError("a part says no")
+
+    def inner():
+        with ops.aside(failing, STEP, 64):
+            return small(x)
+
+    def step():
+        first = {"in the branch": failing, "beside it": lambda: small(x), "in an inner branch": inner}[where]
+        with ops.aside(first, STEP, 64):
+            return failing() if where == "beside it" else small(x)
+
+    small(x)
+    torch.cuda.synchronize()
+    with pytest.raises(ops.KernelError, match="a part says no"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            step()
+    assert not apart()
+
+    def fine():
+        with ops.aside(lambda: small(x), STEP, 64) as beside:
+            own = small(x)
+        return own, beside.result
+
+    graph, out = captured(fine)
+    graph.replay()
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], small(x))
