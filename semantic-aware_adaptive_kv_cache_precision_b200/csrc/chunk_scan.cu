@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kThreads) run_states(const Source src, const R
 }
 
 // From run to run: what run j left is replaced by what came before it, which fades by exp(log_j) over
-// the run. VEC neighbouring numbers of a (sequence, head) a thread, eight runs asked for before the
+// the run (`scan::Fade`). VEC neighbouring numbers of a (sequence, head) a thread, eight runs asked for before the
 // first is used, since a store keeps the compiler from asking for what follows it.
 template <int VEC>
 __global__ void __launch_bounds__(256)
@@ -491,20 +491,20 @@ carry(const Runs r, float* __restrict__ states, const int32_t* __restrict__ slot
   };
   read(home, s);
   for (int j0 = 0; j0 < runs; j0 += kAhead) {
-    float left[kAhead][VEC], fade[kAhead];
+    float left[kAhead][VEC], log[kAhead];
 #pragma unroll
     for (int k = 0; k < kAhead; ++k)
       if (j0 + k < runs) {
         read(p + (j0 + k) * apart, left[k]);
-        fade[k] = logs[(long long)(j0 + k) * r.heads];
+        log[k] = logs[(long long)(j0 + k) * r.heads];
       }
 #pragma unroll
     for (int k = 0; k < kAhead; ++k)
       if (j0 + k < runs) {
-        fade[k] = expm1f(fade[k]);
+        const scan::Fade fade(log[k]);
         write(p + (j0 + k) * apart, s);
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) s[i] += fmaf(fade[k], s[i], left[k][i]);
+        for (int i = 0; i < VEC; ++i) s[i] = fade.carried(s[i], left[k][i]);
       }
   }
   if (keep_state) write(home, s);

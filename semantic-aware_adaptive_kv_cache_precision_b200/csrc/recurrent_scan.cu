@@ -68,14 +68,14 @@ __device__ __forceinline__ void write8(__nv_bfloat16* p, const float (&v)[8]) {
 }
 
 // Between the two passes over a prompt's runs: one number of the state is carried from run to run.
-// What run j left at p[j * step] is replaced by what came before it, which fades by fade(j) + 1
-// over the run. Bound by memory (every run's state is read and written once): the runs' numbers are
+// What run j left at p[j * step] is replaced by what came before it, which fades by exp(log(j))
+// over the run (`scan::Fade`). Bound by memory (every run's state is read and written once): the runs' numbers are
 // asked for eight at a time before the first is used, since the store of one keeps the compiler
 // from asking for the next (the dual form, 16 sequences of up to 8 runs of 1 MB of state: 350 us
 // one by one, 120 now; one sequence of 47 runs of the fading state: 162 and 25).
-template <typename Fade>
+template <typename Log>
 __device__ __forceinline__ float carry_runs(float* __restrict__ p, long long step, int runs, float s,
-                                            Fade fade) {
+                                            Log log) {
   constexpr int kAhead = 8;
   for (int j0 = 0; j0 < runs; j0 += kAhead) {
     float left[kAhead], f[kAhead];
@@ -84,12 +84,12 @@ __device__ __forceinline__ float carry_runs(float* __restrict__ p, long long ste
       if (j0 + k < runs) left[k] = p[(j0 + k) * step];
 #pragma unroll
     for (int k = 0; k < kAhead; ++k)
-      if (j0 + k < runs) f[k] = fade(j0 + k);
+      if (j0 + k < runs) f[k] = log(j0 + k);
 #pragma unroll
     for (int k = 0; k < kAhead; ++k)
       if (j0 + k < runs) {
         p[(j0 + k) * step] = s;
-        s += fmaf(f[k], s, left[k]);
+        s = scan::Fade(f[k]).carried(s, left[k]);
       }
   }
   return s;
@@ -556,7 +556,7 @@ __global__ void scan_carry_kernel(const W* __restrict__ a_log, float* __restrict
   float* home = state + (long long)slots[b] * per + cn;
   const float* sums = dt_sums + (long long)b * max_chunks * channels + c;
   const float s = carry_runs(scratch + (long long)b * max_chunks * per + cn, per, runs, *home,
-                             [&](int j) { return expm1f(a * sums[(long long)j * channels]); });
+                             [&](int j) { return a * sums[(long long)j * channels]; });
   if (keep_state) *home = s;
 }
 

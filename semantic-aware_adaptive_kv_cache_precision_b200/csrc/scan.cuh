@@ -23,6 +23,21 @@ struct FadeInput {
 
 __device__ __forceinline__ float fade_act(float x, int act) { return act ? silu(x) : x; }
 
+// What is left over a run whose decays' logarithms add up to `log`: a state s becomes exp(log) s + left.
+// Near 1 by its change, so that a decay keeps its distance from 1; where the run forgets, by the product: the
+// change would take the state off itself, and half a unit of the last place of the OLD state stayed in the
+// new one (s = 1e4, log = -18.4, left = 1e-2: 3 % of the new one).
+struct Fade {
+  bool change;
+  float factor;
+  __device__ __forceinline__ explicit Fade(float log)
+      : change(log > -0.5f), factor(change ? expm1f(log) : expf(log)) {}
+  __device__ __forceinline__ float carried(float s, float left) const {
+    const float moved = fmaf(factor, s, left);
+    return change ? s + moved : moved;
+  }
+};
+
 // Two fp32 numbers in one register pair, for the two-wide arithmetic of sm_100.
 using Two = unsigned long long;
 __device__ __forceinline__ Two two(float x, float y) {

@@ -112,3 +112,66 @@ def test_selective_scan_in_runs(lengths, run, channels, n_state, rank):
     want, last = torch.stack(outs), torch.stack(states)
     assert (state.double() - last).abs().max() <= TOL * last.abs().max()
     assert (got.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()     # (rounded once to 16 bits)
+
+
+@pytest.mark.parametrize("lengths,run", [((300, 90), 64), ((100,), 32)])
+def test_what_a_run_forgets_leaves_no_rest(lengths, run):
+    """One very large token early in a sequence, strong decays and small tokens after it: every number's
+    error is bounded by the sum of what it is made of (the same recurrence over absolute values), not by
+    the largest number of the step. (Such a bound is what fp32 sums in any order keep; a state taken off
+    itself keeps an ulp of what it was.)"""
+    heads, dim, vdim, T = 2, 32, 40, sum(lengths)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    proj = 0.1 * torch.randn(T, heads * (2 * dim + vdim), generator=g, device=DEV)
+    at = 0
+    for n in lengths:
+        proj[at + 3] *= 1e4
+        at += n
+    less_one = torch.tensor([-0.25, -0.375], device=DEV)
+    got, state = fading(proj, heads, dim, vdim, less_one, lengths, run)
+    p = proj.double()
+    q, k = (p[:, i * heads * dim:(i + 1) * heads * dim].view(T, heads, dim) for i in (0, 1))
+    v = p[:, 2 * heads * dim:].view(T, heads, vdim)
+    decay = (1 + less_one.double()).expand(T, heads)
+    one = torch.ones_like(decay)
+    want, last = walked(decay, one, k, v, q, lengths)
+    bound, last_bound = walked(decay, one, k.abs(), v.abs(), q.abs(), lengths)
+    assert ((got.double() - want).abs() <= TOL * bound).all()
+    assert ((state.double() - last).abs() <= TOL * last_bound).all()
+
+    # the dual form and the selective scan, whose tokens choose how much is forgotten
+    dt = torch.full((T, heads), 0.5, device=DEV)
+    a, zero = torch.tensor([-0.6, -1.3], device=DEV), torch.zeros(heads, device=DEV)
+    xbc = torch.cat([v[:, :].reshape(T, -1).float(), k[:, 0].float(), q[:, 0].float()], 1).contiguous()
+    state = torch.zeros(len(lengths), heads, vdim, dim, device=DEV)
+    got = ops.dual_scan(xbc, 0, heads * vdim, heads * vdim + dim, dt, zero, a, zero, heads, 1, dim, vdim,
+                        state, step_of(lengths), run=run).view(T, heads, vdim)
+    d = torch.nn.functional.softplus(dt.double())
+    decay = torch.exp(d * a.double())
+    k1, q1 = (z[:, :1].expand(T, heads, dim) for z in (k, q))
+    want, last = walked(decay, d, k1, v, q1, lengths)
+    bound, last_bound = walked(decay, d, k1.abs(), v.abs(), q1.abs(), lengths)
+    assert ((got.double() - want).abs() <= TOL * bound).all()
+    assert ((state.double() - last).abs() <= TOL * last_bound).all()
+
+    channels, n_state = 64, 16
+    x = torch.ones(T, channels, device=DEV)
+    at = 0
+    for n in lengths:
+        x[at + 3] = 1e4
+        at += n
+    x = x.bfloat16()
+    low = 0.1 * torch.rand(T, 2 * n_state, generator=g, device=DEV)
+    dt = torch.full((T, channels), 0.75, device=DEV)
+    a_log = torch.zeros(channels, n_state, device=DEV)
+    state = torch.zeros(len(lengths), channels, n_state, device=DEV)
+    ops.selective_scan(x, dt, low, 0, n_state, n_state, torch.ones(T, channels, device=DEV), a_log,
+                       torch.zeros(channels, device=DEV), state, step_of(lengths), run=run)
+    fade = torch.exp(-dt[0, 0].double())                     # (all terms are positive)
+    at = 0
+    for b, n in enumerate(lengths):
+        S = torch.zeros(channels, n_state, dtype=torch.float64, device=DEV)
+        for t in range(at, at + n):
+            S = fade * S + dt[t].double()[:, None] * x[t].double()[:, None] * low[t, :n_state].double()
+        at += n
+        assert ((state[b].double() - S).abs() <= TOL * S).all()
