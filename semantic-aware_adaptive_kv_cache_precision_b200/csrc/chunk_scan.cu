@@ -125,7 +125,12 @@ struct FadeSource {
     return make_float4(v[0], v[1], v[2], v[3]);
   }
   __device__ float step(int, int) const { return 1.f; }
-  __device__ double rate(float, int h) const { return log1p((double)less_one[h]); }
+  // (of the decay's size; a decay below zero also changes the state's sign, every token)
+  __device__ double rate(float, int h) const {
+    return flips(h) ? log(-1.0 - (double)less_one[h]) : log1p((double)less_one[h]);
+  }
+  __device__ bool flips(int h) const { return less_one[h] < -1.f; }
+  __device__ float change(float, int h) const { return less_one[h]; }      // the decay less one
   __device__ float skip(int) const { return 0.f; }
 };
 
@@ -181,12 +186,15 @@ struct DualSource {
     return softplus(dt[(long long)t * dt_stride + h] + dt_bias[h]);
   }
   __device__ double rate(float step, int h) const { return (double)step * a[h]; }
+  __device__ bool flips(int) const { return false; }
+  __device__ float change(float step, int h) const { return (float)expm1(rate(step, h)); }
   __device__ float skip(int h) const { return d_skip[h]; }
 };
 
 struct Runs {
   float* scratch;                  // [sequences, max_runs, heads, vdim, dim]
   float* logs;                     // [sequences, max_runs, heads]: the sum of a run's g
+  const float* less_one;           // [heads]: the decay less one, where decays may be below zero (else null)
   const int32_t* cu_seqlens;
   int heads, dim, vdim, run_len, max_runs;
 };
@@ -333,7 +341,7 @@ __device__ __noinline__ void walk(const Source& src, const Runs& r, const Span& 
     float* mine = state + (long long)c * r.dim;
     for (int t = s.first; t < s.first + s.n; ++t) {
       const float d = src.step(t, h), x = src.value(t, h, c), v = d * x;
-      const float fade = (float)expm1(src.rate(d, h));
+      const float fade = src.change(d, h);
       float o = 0.f;
       for (int i = 0; i < r.dim; ++i) {
         const float m = fmaf(src.key(t, h, i), v, fmaf(fade, mine[i], mine[i]));
@@ -371,8 +379,10 @@ __global__ void __launch_bounds__(kThreads) run_states(const Source src, const R
     sums_of(src, s, h, steps, g_hi, g_lo, &total);
     __syncwarp();
     const float hi = (float)total, lo = (float)(total - (double)hi);
-    for (int i = lane; i < kTokens; i += 32)
-      weight[i] = i < s.n ? steps[i] * expf((hi - g_hi[i]) + (lo - g_lo[i])) : 0.f;
+    for (int i = lane; i < kTokens; i += 32) {
+      const float w = i < s.n ? steps[i] * expf((hi - g_hi[i]) + (lo - g_lo[i])) : 0.f;
+      weight[i] = src.flips(h) && ((s.n - 1 - i) & 1) ? -w : w;
+    }
     if (blockIdx.x == 0 && lane == 0)
       r.logs[((long long)s.b * r.max_runs + s.run) * r.heads + h] = hi;
   }
@@ -471,7 +481,9 @@ carry(const Runs r, float* __restrict__ states, const int32_t* __restrict__ slot
   const int e = (blockIdx.x * 256 + threadIdx.x) * VEC;
   if (e >= per_head) return;
   const int h = blockIdx.y, b = blockIdx.z;
-  const int runs = (r.cu_seqlens[b + 1] - r.cu_seqlens[b] + r.run_len - 1) / r.run_len;
+  const int tokens = r.cu_seqlens[b + 1] - r.cu_seqlens[b];
+  const int runs = (tokens + r.run_len - 1) / r.run_len;
+  const bool flips = r.less_one && r.less_one[h] < -1.f;
   const long long apart = (long long)r.heads * per_head;
   float* p = r.scratch + ((long long)b * r.max_runs * r.heads + h) * per_head + e;
   const float* logs = r.logs + (long long)b * r.max_runs * r.heads + h;
@@ -503,6 +515,12 @@ carry(const Runs r, float* __restrict__ states, const int32_t* __restrict__ slot
       if (j0 + k < runs) {
         const scan::Fade fade(log[k]);
         write(p + (j0 + k) * apart, s);
+        if (flips && (min(tokens - (j0 + k) * r.run_len, r.run_len) & 1)) {    // (an odd number of tokens)
+          const float factor = -expf(log[k]);
+#pragma unroll
+          for (int i = 0; i < VEC; ++i) s[i] = fmaf(factor, s[i], left[k][i]);
+          continue;
+        }
 #pragma unroll
         for (int i = 0; i < VEC; ++i) s[i] = fade.carried(s[i], left[k][i]);
       }
@@ -552,6 +570,7 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
   const uint32_t qs_at = static_cast<uint32_t>(__cvta_generic_to_shared(qs));
   const uint32_t turn_at = static_cast<uint32_t>(__cvta_generic_to_shared(turn));
   const bool rows = warp * 16 < s.n;                     // (a warp without rows still fills buffers)
+  const bool flips = src.flips(h);
   const uint32_t q_from = qs_at + ((warp * 16 + a_row(lane)) * pitch + a_col(lane)) * 2;
   const int piece = kTokens * pitch * 2;                 // bytes
 
@@ -583,7 +602,8 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int i = warp * 16 + (lane >> 2) + (k >> 1) * 8, j = n * 8 + (lane & 3) * 2 + (k & 1);
-        sc[n][k] = j <= i ? sc[n][k] * steps[j] * expf((g_hi[i] - g_hi[j]) + (g_lo[i] - g_lo[j])) : 0.f;
+        const float w = sc[n][k] * steps[j] * expf((g_hi[i] - g_hi[j]) + (g_lo[i] - g_lo[j]));
+        sc[n][k] = j > i ? 0.f : flips && ((i - j) & 1) ? -w : w;
       }
     }
   }
@@ -632,7 +652,7 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int i = warp * 16 + (lane >> 2) + half * 8;
-      f[half] = expf(g_hi[i] + g_lo[i]);
+      f[half] = flips && !(i & 1) ? -expf(g_hi[i] + g_lo[i]) : expf(g_hi[i] + g_lo[i]);
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n)
@@ -886,7 +906,7 @@ SAKV_EXPORT int sakv_chunk_fade(const float* proj, long long stride, int q_off, 
   const bool quads = multiples_of_4({stride, q_off, k_off, v_off, dim, vdim, rot / 2}) &&
                      !(((uintptr_t)proj | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15);
   const FadeInput in = {act, rot, positions, cos_t, sin_t, k_scale};
-  const Runs r = {scratch, logs, cu_seqlens, heads, dim, vdim, run_len, max_runs};
+  const Runs r = {scratch, logs, decay, cu_seqlens, heads, dim, vdim, run_len, max_runs};
   if (quads)
     return launch_runs(FadeSource<true>{proj, stride, q_off, k_off, v_off, decay, dim, vdim, in}, r, state,
                        slots, out, sequences, keep_state, stream);
@@ -906,7 +926,7 @@ SAKV_EXPORT int sakv_chunk_dual(const void* xbc, int c_dtype, long long stride, 
       heads % groups)
     return cudaErrorInvalidValue;
   if (tokens == 0 || sequences == 0) return 0;
-  const Runs r = {scratch, logs, cu_seqlens, heads, dim, vdim, run_len, max_runs};
+  const Runs r = {scratch, logs, nullptr, cu_seqlens, heads, dim, vdim, run_len, max_runs};
   const bool quads = multiples_of_4({stride, x_off, b_off, c_off, dim, vdim}) &&
                      !((uintptr_t)xbc & (c_dtype == SAKV_F32 ? 15 : 7));
 #define SAKV_DUAL(C, QUADS)                                                                      \

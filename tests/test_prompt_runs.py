@@ -65,6 +65,25 @@ def test_a_run_s_edges(lengths, run, dim, vdim):
         assert (a.double() - b).abs().max() <= TOL * b.abs().max()
 
 
+@pytest.mark.parametrize("lengths,run", [((64, 131, 1), 64), ((100, 33), 32)])
+def test_decays_of_any_sign_and_size(lengths, run):
+    """Decays below zero change the state's sign with every token; a decay of zero forgets it at once."""
+    heads, dim, vdim, T = 6, 24, 20, sum(lengths)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    proj = torch.randn(T, heads * (2 * dim + vdim), generator=g, device=DEV)
+    less_one = torch.tensor([-1.5, -1.96875, -1.0, -2.0, 0.0, 0.015625], device=DEV)     # -0.5, -0.97, 0, -1, 1 ...
+    got, state = fading(proj, heads, dim, vdim, less_one, lengths, run)
+    p = proj.double()
+    q, k = (p[:, i * heads * dim:(i + 1) * heads * dim].view(T, heads, dim) for i in (0, 1))
+    v = p[:, 2 * heads * dim:].view(T, heads, vdim)
+    decay = (1 + less_one.double()).expand(T, heads)
+    one = torch.ones_like(decay)
+    want, last = walked(decay, one, k, v, q, lengths)
+    bound, last_bound = walked(decay.abs(), one, k.abs(), v.abs(), q.abs(), lengths)
+    assert ((got.double() - want).abs() <= TOL * bound).all()
+    assert ((state.double() - last).abs() <= TOL * last_bound).all()
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan"), 3.4e38])
 @pytest.mark.parametrize("where", ["key", "value", "query"])
 def test_a_value_that_is_not_finite_is_not_felt_before(value, where):
