@@ -194,3 +194,26 @@ def test_what_a_run_forgets_leaves_no_rest(lengths, run):
             S = fade * S + dt[t].double()[:, None] * x[t].double()[:, None] * low[t, :n_state].double()
         at += n
         assert ((state[b].double() - S).abs() <= TOL * S).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38])
+@pytest.mark.parametrize("where", ["low", "weight"])
+def test_step_sizes_of_values_that_are_not_finite(value, where):
+    """On the tensor cores as number by number (the kernel for fp32 weights): the same numbers are not
+    finite, and in the same way."""
+    T, channels, rank = 70, 66, 40
+    g = torch.Generator(device=DEV).manual_seed(11)
+    low = torch.randn(T, rank + 4, generator=g, device=DEV)
+    w = (0.3 * torch.randn(channels, rank, generator=g, device=DEV)).bfloat16()
+    b = torch.randn(channels, generator=g, device=DEV).bfloat16()
+    w[5, 3] = 0.0
+    if where == "low":
+        low[17, 3], low[69, 39] = value, value
+    else:
+        w[9, 3], w[65, 39] = value, value             # (3.4e38 is infinite in 16 bits)
+    got = ops.step_size(low, rank, w, b)
+    want = ops.step_size(low, rank, w.float(), b.float())
+    odd = ~torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), ~odd)
+    assert torch.equal(got[odd].nan_to_num(nan=-1.0), want[odd].nan_to_num(nan=-1.0))
+    assert ((got[~odd] - want[~odd]).abs() <= TOL * (8 + want[~odd].abs())).all()      # (sums of some units)
