@@ -206,8 +206,9 @@ int launch(const float* proj, long long stride, int q_off, int k_off, int v_off,
   const int most = q_count > v_count ? q_count : v_count;
   const bool whole = norm_kind == 1 && most <= 4096;
   const bool pieces = norm_kind == 0 || (norm_kind == 2 && dim <= 128 && (dim & (dim - 1)) == 0);
-  // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
-  if (sizeof(W) == 2 && fours && (whole || pieces) && most <= 16 * 1024 * 1024) {
+  // (16-bit mode, which the queries and the cache tell: weights may be absent. In the 32-bit mode a row's
+  // sums keep the order they have in the kernel below)
+  if constexpr (sizeof(C) == 2) if (fours && (whole || pieces) && most <= 16 * 1024 * 1024) {
     const int n = !whole || most <= 1024 ? 1 : most <= 2048 ? 2 : 4, size = n * kThreads * 4;
     const int qb = (q_count + size - 1) / size, kb = (k_count + size - 1) / size;
     const int vb = (v_count + size - 1) / size;
