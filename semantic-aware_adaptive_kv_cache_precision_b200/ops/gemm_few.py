@@ -1,5 +1,5 @@
-"""Host side of the product of a step of few tokens (`csrc/gemm_few.cu`): weights from memory straight
-into registers, nothing to set up."""
+"""Host side of the product of a step of few tokens (`csrc/gemm_few.cu`): every thread its own numbers from
+memory to the tensor cores, nothing to set up."""
 
 from __future__ import annotations
 
@@ -10,7 +10,8 @@ from ._lib import BF16, call, dtype_code, ptr, sm_count
 
 MAX_TOKENS = 16        # what the kernel takes
 ROWS = 16              # weight rows a block
-SHORT_ROW = 2048       # up to this K any number of rows; beyond, what one wave of blocks makes
+LONGEST_ROW = 3072     # up to this K any number of rows; beyond, what one wave of blocks makes
+SHORT_ROW = 2048       # the same for more than 8 tokens
 LARGE = 20_000_000     # bytes of a weight, from which on more than 8 tokens go elsewhere
 
 
@@ -19,20 +20,19 @@ def takes(x: torch.Tensor, weight: torch.Tensor) -> bool:
 
     Its gain is at the ends of a kernel, and it reads x once for every 16 rows of the weight with more
     instructions a byte than `csrc/gemm_tc.cu`, so it is for short rows and for products that one wave of
-    blocks makes. Decode steps, us (this kernel for every product / that one): width 1,536, one user 955 /
-    1,101 and 8 users 1,095 / 1,254; width 1,024 and 4 users 425 / 481. Width 3,584 and 8 users, rows of 3,584 in
-    more than a wave: alone the products are as fast (44 / 43), but in the steps after a prompt of 9,216
-    tokens, whose power holds the clocks down (every kernel of a step takes 1.7 times what it does after
-    2,560), instructions are what bounds this one and a step takes 6,831 / 3,401. With more than 8 tokens x
-    is as much to read as the weights, and a large product takes longer (46 MB, 16 tokens: 14.9 / 11.3; 4
-    MB: 3.1 / 3.4; a step of 16 users 692 / 680, with the limit 688)."""
+    blocks makes (by the rows of the weight: a gated product has half as many blocks). Decoded steps after
+    1,024 tokens of models of the Qwen2 layout, us, every product by this kernel / by that one, for 1, 8 and
+    16 tokens: width 1,024 481 / 737, 587 / 772, 731 / 856; 1,536 924 / 1,083, 1,057 / 1,185, 1,249 / 1,292; 2,048 879 /
+    1,080, 1,003 / 1,132, 1,109 / 1,212; 2,560 963 / 1,094, 1,093 / 1,148, 1,284 / 1,241; 3,072 792 / 875, 899 / 931, 1,011
+    / 1,005; 3,584 1,289 / 1,261, 1,444 / 1,361, 1,570 / 1,407. With more than 8 tokens x is as much to read as the
+    weights (46 MB, 16 tokens, alone: 14.9 / 11.3; 4 MB: 3.1 / 3.4)."""
     tokens = x.shape[0]
     if tokens > MAX_TOKENS or not gemm_tc.takes(x, weight):
         return False
     n, k = weight.shape
     if tokens > 8 and n * k * weight.element_size() > LARGE:
         return False
-    return k <= SHORT_ROW or n <= ROWS * sm_count()
+    return k <= (LONGEST_ROW if tokens <= 8 else SHORT_ROW) or n <= ROWS * sm_count()
 
 
 def choose_parts(n: int, k: int) -> int:
