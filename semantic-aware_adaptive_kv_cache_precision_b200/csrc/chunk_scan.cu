@@ -192,12 +192,18 @@ struct DualSource {
 };
 
 struct Runs {
-  float* scratch;                  // [sequences, max_runs, heads, vdim, dim]
-  float* logs;                     // [sequences, max_runs, heads]: the sum of a run's g
+  float* scratch;                  // [rows, heads, vdim, dim], a row a run (`row_of`)
+  float* logs;                     // [rows, heads]: the sum of a run's g
   const float* less_one;           // [heads]: the decay less one, where decays may be below zero (else null)
   const int32_t* cu_seqlens;
   int heads, dim, vdim, run_len, max_runs;
 };
+
+// The scratch row of a sequence's first run; its further runs follow. (Runs of the sequences before it: no
+// more than their tokens / run_len, and one each that is not full.)
+__device__ __forceinline__ long long row_of(const Runs& r, int b) {
+  return r.cu_seqlens[b] / r.run_len + b;
+}
 
 __device__ __forceinline__ bool odd_value(float x) { return !(fabsf(x) < INFINITY); }
 
@@ -384,7 +390,7 @@ __global__ void __launch_bounds__(kThreads) run_states(const Source src, const R
       weight[i] = src.flips(h) && ((s.n - 1 - i) & 1) ? -w : w;
     }
     if (blockIdx.x == 0 && lane == 0)
-      r.logs[((long long)s.b * r.max_runs + s.run) * r.heads + h] = hi;
+      r.logs[(row_of(r, s.b) + s.run) * r.heads + h] = hi;
   }
   const int whole = (s.n + 15) & ~15;            // rows of the products
   const Deal d = deal(wide);
@@ -410,7 +416,7 @@ __global__ void __launch_bounds__(kThreads) run_states(const Source src, const R
     else
       stage_zeros<3>(vs + c, kPitchV, kTokens * kPitchV, tid >> 4, kThreads / 16, whole);
   }
-  float* state = r.scratch + (((long long)s.b * r.max_runs + s.run) * r.heads + h) *
+  float* state = r.scratch + ((row_of(r, s.b) + s.run) * r.heads + h) *
                                  ((long long)r.vdim * r.dim);
   __syncthreads();
   bool odd = false;
@@ -485,8 +491,8 @@ carry(const Runs r, float* __restrict__ states, const int32_t* __restrict__ slot
   const int runs = (tokens + r.run_len - 1) / r.run_len;
   const bool flips = r.less_one && r.less_one[h] < -1.f;
   const long long apart = (long long)r.heads * per_head;
-  float* p = r.scratch + ((long long)b * r.max_runs * r.heads + h) * per_head + e;
-  const float* logs = r.logs + (long long)b * r.max_runs * r.heads + h;
+  float* p = r.scratch + (row_of(r, b) * r.heads + h) * per_head + e;
+  const float* logs = r.logs + row_of(r, b) * r.heads + h;
   float* home = states + ((long long)slots[b] * r.heads + h) * per_head + e;
   float s[VEC];
   auto read = [](const float* at, float (&v)[VEC]) {
@@ -544,7 +550,7 @@ run_outputs(const Source src, const Runs r, float* __restrict__ out) {
   const int wide = (r.dim + 15) / 16 * 16, pitch = wide + 8;
   __nv_bfloat16* qs = reinterpret_cast<__nv_bfloat16*>(pool);             // [NP][64][pitch]
   __nv_bfloat16* turn = qs + NP * kTokens * pitch;       // k [NP][64][pitch], S0 [3][64][pitch], v
-  float* state = r.scratch + (((long long)s.b * r.max_runs + s.run) * r.heads + h) *
+  float* state = r.scratch + ((row_of(r, s.b) + s.run) * r.heads + h) *
                                  ((long long)r.vdim * r.dim);
   if (warp == 0) {
     double total;
@@ -904,7 +910,8 @@ SAKV_EXPORT int sakv_chunk_step_size(const float* low, long long stride, int ran
 }
 
 // As `sakv_decay_attention` (csrc/recurrent_scan.cu), a sequence's tokens in runs of run_len (up to 64):
-// scratch: fp32 [sequences, max_runs, heads, vdim, dim]; logs: fp32 [sequences, max_runs, heads].
+// max_runs the most a sequence has. scratch: fp32 [tokens / run_len + sequences, heads, vdim, dim]; logs: fp32
+// [tokens / run_len + sequences, heads].
 SAKV_EXPORT int sakv_chunk_fade(const float* proj, long long stride, int q_off, int k_off, int v_off,
                                 const float* decay, float* state, const int32_t* cu_seqlens,
                                 const int32_t* slots, float* out, int tokens, int sequences, int heads,

@@ -14,14 +14,23 @@ from ._lib import KernelError, call, dtype_code, ptr, require_cuda
 CHUNK = 64
 
 
-def run_length(max_new: int) -> int:
+def run_length(max_new: int, tokens: int | None = None, sequences: int = 1) -> int:
     """Tokens a run for the fading state and the dual form, by the longest part of the step: runs as matrix
     products are the faster form from 64 tokens on, in shorter runs up to 128, so that some go side by side
     (us, one walk / runs; fading state, 16 heads of 128 x 128: 64 tokens 86 / 35, 128 tokens 169 / 43; dual
     form, four prompts, 32 heads of 128 x 64: 59 / 31, 114 / 37; prompt steps of three designs of width
     1,024, one prompt of 250: 2.08 / 1.03, 2.07 / 1.04 and 1.91 / 1.21 ms, 16 prompts of up to 100 tokens 2.28 /
-    2.28, 1.71 / 1.55 and 1.62 / 1.61; 8 of up to 40, in runs of 16: 0.98 / 1.05 and 0.77 / 0.85). 0: one walk."""
-    return 0 if max_new < 64 else 32 if max_new < 128 else CHUNK
+    2.28, 1.71 / 1.55 and 1.62 / 1.61; 8 of up to 40, in runs of 16: 0.98 / 1.05 and 0.77 / 0.85). 0: one walk.
+
+    A sequence of few tokens has its state through memory three times more in runs, so where the step's
+    `tokens` are fewer than eight for each of its `sequences` (a prompt beside many decoded tokens) it is one
+    walk (fading state, one prompt of 64 tokens beside 8 / 16 / 32 decoded ones 78 / 96, 86 / 105, 105 / 177; of 200
+    beside 16 / 32 / 64 182 / 130, 204 / 198, 259 / 340; of 500 beside 64 / 128 451 / 394, 586 / 692; dual form, 200
+    beside 32 / 64 172 / 131, 184 / 232). That bounds the runs' memory too: a state for every `run` tokens and
+    one a sequence."""
+    if max_new < 64 or (tokens is not None and tokens < 8 * sequences):
+        return 0
+    return 32 if max_new < 128 else CHUNK
 
 
 def _check(cond: bool, message: str) -> None:
@@ -136,17 +145,18 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor | None, low: torch.Tensor, 
     return out
 
 
-def _runs(run: int, step, state_size: int, sum_size: int, device):
+def _runs(run: int, step, state_size: int, sum_size: int, device, tokens: int | None = None):
     """(runs a sequence at most, scratch for every run's state, scratch for its sums) of a
-    step walked in runs of `run` tokens; (0, None, None) where one walk does."""
+    step walked in runs of `run` tokens; (0, None, None) where one walk does. Scratch rows: for every
+    sequence as many as the longest has, or with `tokens`, the step's, one for every run there can be."""
     if not run:
         return 0, None, None
     runs = -(-int(step.max_new) // int(run))
     if runs <= 1 or step.sequences * runs > 65535:
         return 0, None, None
-    scratch = torch.empty((step.sequences * runs, state_size), dtype=torch.float32, device=device)
-    sums = torch.empty((step.sequences * runs, sum_size), dtype=torch.float32,
-                       device=device) if sum_size else None
+    rows = step.sequences * runs if tokens is None else tokens // int(run) + step.sequences
+    scratch = torch.empty((rows, state_size), dtype=torch.float32, device=device)
+    sums = torch.empty((rows, sum_size), dtype=torch.float32, device=device) if sum_size else None
     return runs, scratch, sums
 
 
@@ -182,7 +192,7 @@ def decay_attention(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, head
            and tuple(state.shape[1:]) == (heads, vdim, dim), "state: fp32 [slots, heads, vdim, dim]")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=proj.device)
     run = min(int(run), CHUNK)
-    runs, scratch, logs = _runs(run, step, heads * vdim * dim, heads, proj.device)
+    runs, scratch, logs = _runs(run, step, heads * vdim * dim, heads, proj.device, tokens)
     args = (ptr(proj), proj.stride(0), int(q_off), int(k_off), int(v_off), ptr(decay_less_one),
             ptr(state), ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens, step.sequences,
             heads, dim, vdim, int(keep_state))
@@ -222,7 +232,7 @@ def dual_scan(xbc: torch.Tensor, x_off: int, b_off: int, c_off: int, dt: torch.T
            "state: fp32 [slots, heads, vdim, n_state]")
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=xbc.device)
     run = min(int(run), CHUNK)
-    runs, scratch, logs = _runs(run, step, heads * vdim * n_state, heads, xbc.device)
+    runs, scratch, logs = _runs(run, step, heads * vdim * n_state, heads, xbc.device, tokens)
     args = (ptr(xbc), dtype_code(xbc.dtype), xbc.stride(0), int(x_off), int(b_off), int(c_off),
             ptr(dt), dt.stride(0), ptr(dt_bias), ptr(a), ptr(d_skip), ptr(state),
             ptr(step.cu_seqlens), ptr(step.slots), ptr(out), tokens, step.sequences, heads, groups,

@@ -91,8 +91,11 @@ class DualScanMixer(Part):
     def _run(self, step) -> int:
         """Tokens a run of a long prompt: in bfloat16 a sequence's part of the step is walked
         in runs side by side (the states carried between them in fp32). In the 32-bit mode,
-        and for short parts, one walk, whose sums do not depend on how the sequence was cut."""
-        return 0 if self.act_dtype == torch.float32 else ops.run_length(getattr(step, "max_new", 0))
+        for short parts and beside many of few tokens, one walk, whose sums do not depend on how the
+        sequence was cut."""
+        if self.act_dtype == torch.float32:
+            return 0
+        return ops.run_length(getattr(step, "max_new", 0), getattr(step, "tokens", None), step.sequences)
 
     # -- the part alone ---------------------------------------------------------------------
 
