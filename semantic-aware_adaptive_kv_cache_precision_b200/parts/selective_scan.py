@@ -28,7 +28,7 @@ from .base import Part, register_part
 
 #: tokens a run when a long prompt is walked in runs side by side
 RUN = 64
-FEW_WALKS = 16384     # channels, all sequences together
+WALKS_AN_SM = 64      # channels, all sequences together, up to which shorter runs are side by side
 
 
 class SelectiveScanMixer(Part):
@@ -67,10 +67,12 @@ class SelectiveScanMixer(Part):
             return 0
         if most >= 4 * RUN:
             return RUN
-        # (from 128 tokens on shorter runs are faster while the step's walks do not fill the GPU: prompt
-        # steps of width 1,024, 2,048 channels, one walk / runs of 32: one prompt of 130 tokens 0.93 / 0.85
-        # ms, of 250 1.23 / 0.91, 4 of up to 200 1.31 / 1.15, 16 of up to 250 3.00 / 3.16)
-        return RUN // 2 if self.spec.state <= 16 and step.sequences * self.spec.inner <= FEW_WALKS else 0
+        # (from 128 tokens on shorter runs are faster while the step's walks do not fill the GPU; us, one walk /
+        # runs of 32, prompts of 250 tokens, at 8,192 and 12,288 channels together: 1,024 channels a sequence
+        # 124 / 110 and 134 / 140, 2,048 125 / 112 and 133 / 136, 4,096 125 / 110 and 211 / 235 at 24,576; one prompt
+        # 121 / 74, 117 / 68, 117 / 72; of 128 tokens 72 / 72 up to 8,192)
+        few = step.sequences * self.spec.inner <= WALKS_AN_SM * ops.sm_count()
+        return RUN // 2 if self.spec.state <= 16 and few else 0
 
     def cache_need(self):
         s = self.spec
