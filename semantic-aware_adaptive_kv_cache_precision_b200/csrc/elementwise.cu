@@ -387,3 +387,16 @@ SAKV_EXPORT int sakv_add_bias(float* y, long long ld, const void* bias, int bias
 #undef SAKV_BIAS
   return cudaErrorInvalidValue;
 }
+
+// A stream of its own on the current device, also while this thread captures (a stream is made at once, and
+// nothing that is captured depends on it).
+SAKV_EXPORT int sakv_stream_create(void** out) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) return static_cast<int>(e);
+  cudaStream_t stream = nullptr;
+  e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+  const cudaError_t back = cudaThreadExchangeStreamCaptureMode(&mode);
+  *out = stream;
+  return static_cast<int>(e != cudaSuccess ? e : back);
+}

@@ -104,6 +104,7 @@ SIGNATURES = {
 #: functions without a stream argument: (library, argument types)
 PLAIN_SIGNATURES = {
     "sakv_choose_chunks": ("sampling", [I]),
+    "sakv_stream_create": ("elementwise", [P]),
     "sakv_moe_tile_rows": ("moe", []),
     "sakv_delta_coefficients": ("gated_delta", []),
     "sakv_decode_attention_map": ("attention_decode", [P, P, L, I, I]),

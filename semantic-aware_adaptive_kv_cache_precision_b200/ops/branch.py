@@ -7,24 +7,58 @@ result is read."""
 
 from __future__ import annotations
 
+import ctypes
 import threading
 
 import torch
 
-_local = threading.local()      # `streams`: a thread's own, by device; `open`: its branches not yet joined
+from ._lib import KernelError, plain_function
+
+_local = threading.local()      # `streams`: a thread's own; `open`: its branches not yet joined
+_idle: dict = {}                # streams of threads that have ended, by device
+_idle_lock = threading.Lock()
+
+
+class _Streams:
+    """One thread's streams for branches, by device, outermost first. They are not from PyTorch's pool, which
+    deals its streams out again: what another thread launched on such a stream while this one captures on
+    it would be captured with it. A thread that ends leaves them to the next."""
+
+    def __init__(self):
+        self.of: dict = {}
+
+    def beside(self, main: torch.cuda.Stream) -> torch.cuda.Stream:
+        """The first of `main`'s device, or if `main` is one of them (a branch inside a branch) the one
+        after it."""
+        streams = self.of.setdefault(main.device, [])
+        at = next((i + 1 for i, s in enumerate(streams) if s.cuda_stream == main.cuda_stream), 0)
+        if at == len(streams):
+            with _idle_lock:
+                idle = _idle.setdefault(main.device, [])
+                stream = idle.pop() if idle else None
+            streams.append(stream if stream is not None else self._make(main.device))
+        return streams[at]
+
+    @staticmethod
+    def _make(device) -> torch.cuda.Stream:
+        handle = ctypes.c_void_p()
+        with torch.cuda.device(device):
+            code = plain_function("sakv_stream_create")(ctypes.addressof(handle))
+        if code != 0:
+            raise KernelError(f"could not make a stream (CUDA error {code})")
+        return torch.cuda.ExternalStream(handle.value, device)
+
+    def __del__(self):
+        with _idle_lock:
+            for device, streams in self.of.items():
+                _idle.setdefault(device, []).extend(streams)
 
 
 def _other_stream(main: torch.cuda.Stream) -> torch.cuda.Stream:
-    """A stream for work beside `main`'s: the first of this thread's and device's, or if `main` is one of
-    them (a branch inside a branch) the one after it."""
     kept = getattr(_local, "streams", None)
     if kept is None:
-        kept = _local.streams = {}
-    streams = kept.setdefault(main.device, [])
-    at = next((i + 1 for i, s in enumerate(streams) if s == main), 0)
-    if at == len(streams):
-        streams.append(torch.cuda.Stream(main.device))
-    return streams[at]
+        kept = _local.streams = _Streams()
+    return kept.beside(main)
 
 
 def apart() -> bool:

@@ -2,14 +2,16 @@
 
 from __future__ import annotations
 
+import gc
 import sys
+import threading
 from types import SimpleNamespace
 
 import pytest
 import torch
 
 from semantic_aware_adaptive_kv_cache_precision_b200 import ops
-from semantic_aware_adaptive_kv_cache_precision_b200.ops import _lib
+from semantic_aware_adaptive_kv_cache_precision_b200.ops import _lib, branch
 from semantic_aware_adaptive_kv_cache_precision_b200.ops.branch import apart
 
 DEV = "cuda"
@@ -163,3 +165,31 @@ def test_a_failure_ends_the_branch(where):
     graph, out = captured(fine)
     graph.replay()
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], small(x))
+
+
+@pytest.mark.gpu
+def test_a_branch_s_stream_is_its_thread_s_own():
+    """No two threads', and none that PyTorch deals out; a thread that has ended leaves its streams to the next."""
+    from concurrent.futures import ThreadPoolExecutor
+    main = torch.cuda.current_stream()
+
+    def mine():
+        first = branch._other_stream(main)
+        return first.cuda_stream, branch._other_stream(first).cuda_stream
+
+    dealt = {torch.cuda.Stream().cuda_stream for _ in range(80)}
+    meet = threading.Barrier(3, timeout=60)
+
+    def held():
+        both = mine()
+        meet.wait()
+        assert mine() == both
+        return both
+
+    with ThreadPoolExecutor(3) as pool:
+        taken = [s for f in [pool.submit(held) for _ in range(3)] for s in f.result()]
+    assert len(set(taken)) == 6 and not dealt & set(taken)
+    gc.collect()
+    with ThreadPoolExecutor(1) as pool:
+        again = pool.submit(mine).result()
+    assert set(again) <= set(taken)
