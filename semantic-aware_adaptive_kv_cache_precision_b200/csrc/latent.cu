@@ -156,10 +156,10 @@ int prepare(const float* down, long long stride, int q_rank, int rank, int rot,
             const float* cos_t, const float* sin_t, void* q_latent, void* cache, int write_cache,
             int interleaved, int tokens, cudaStream_t stream) {
   // (by the sizes alone: how a row is summed must not depend on the step)
-  auto aligned = [](const void* p, size_t bytes) { return (uintptr_t)p % bytes == 0; };
-  const int most = q_rank > rank ? q_rank : rank;
+  [[maybe_unused]] auto aligned = [](const void* p, size_t bytes) { return (uintptr_t)p % bytes == 0; };
+  [[maybe_unused]] const int most = q_rank > rank ? q_rank : rank;
   // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
-  if (sizeof(W) == 2 && stride % 4 == 0 && q_rank % 4 == 0 && rank % 4 == 0 && rot % 4 == 0 && rot <= 2 * kThreads &&
+  if constexpr (sizeof(W) == 2) if (stride % 4 == 0 && q_rank % 4 == 0 && rank % 4 == 0 && rot % 4 == 0 && rot <= 2 * kThreads &&
       most <= 4096 && aligned(down, 16) && aligned(q_weight, 4 * sizeof(W)) &&
       aligned(kv_weight, 4 * sizeof(W)) && aligned(q_latent, 4 * sizeof(T)) &&
       aligned(cache, 4 * sizeof(T))) {

@@ -132,7 +132,7 @@ int launch(float* x, const float* y, const void* w_after, const int32_t* rows,
            const void* w_before, void* out, int n, int hidden, float eps, cudaStream_t stream) {
   const uintptr_t weights = (uintptr_t)w_after | (uintptr_t)w_before;
   // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
-  if (sizeof(W) == 2 && hidden % 4 == 0 && hidden <= 4096 && !(((uintptr_t)x | (uintptr_t)y) & 15) &&
+  if constexpr (sizeof(W) == 2) if (hidden % 4 == 0 && hidden <= 4096 && !(((uintptr_t)x | (uintptr_t)y) & 15) &&
       !(weights & (4 * sizeof(W) - 1)) && !((uintptr_t)out & (4 * sizeof(Out) - 1))) {
     auto go = [&](auto kernel) {
       return launch_ordered(kernel, dim3(n), dim3(kThreads), 0, stream, x, y, (const W*)w_after, rows,

@@ -65,10 +65,10 @@ __global__ void logits_kernel(const T* __restrict__ h, const float* __restrict__
   if (lane == 0) out[item] = sum;
 }
 
-// Whether rows go by in groups of four neighbouring numbers (both kernels alike: a sum's order depends
-// on the width alone; in the 32-bit mode it stays what one by one makes it).
-bool logits_by_fours(const void* h, int dtype, const float* w, int width) {
-  return dtype == SAKV_BF16 && width % 4 == 0 && (uintptr_t)h % 8 == 0 && (uintptr_t)w % 16 == 0;
+// Whether rows in 16 bits go by in groups of four neighbouring numbers (both kernels alike: a sum's order
+// depends on the width alone; in the 32-bit mode it stays what one by one makes it).
+bool logits_by_fours(const void* h, const float* w, int width) {
+  return width % 4 == 0 && (uintptr_t)h % 8 == 0 && (uintptr_t)w % 16 == 0;
 }
 
 // Whether sixteen sums a warp are the faster split: with 80 sums an SM there are warps enough, and a
@@ -748,7 +748,6 @@ SAKV_EXPORT int sakv_moe_logits(const void* h, int dtype, const float* w, float*
   const bool in_tiles = logits_in_tiles(tokens, outputs);
   const long long tiles = (tokens + 3LL) / 4 * ((outputs + 3) / 4);
   const dim3 grid4((unsigned)((tiles * 32 + 255) / 256));
-  const bool fours = logits_by_fours(h, dtype, w, width);
 #define SAKV_LOGITS(FOURS, T)                                                                    \
   do {                                                                                           \
     if (in_tiles)                                                                                \
@@ -757,12 +756,9 @@ SAKV_EXPORT int sakv_moe_logits(const void* h, int dtype, const float* w, float*
     return launch_ordered(logits_kernel<FOURS, T>, grid, block, 0, stream, (const T*)h, w, out,  \
                           outputs, width, count);                                                \
   } while (0)
-  if (dtype == SAKV_F32) {
-    if (fours) SAKV_LOGITS(true, float);
-    SAKV_LOGITS(false, float);
-  }
+  if (dtype == SAKV_F32) SAKV_LOGITS(false, float);
   if (dtype == SAKV_BF16) {
-    if (fours) SAKV_LOGITS(true, __nv_bfloat16);
+    if (logits_by_fours(h, w, width)) SAKV_LOGITS(true, __nv_bfloat16);
     SAKV_LOGITS(false, __nv_bfloat16);
   }
 #undef SAKV_LOGITS

@@ -248,14 +248,13 @@ int launch_step(float* xs, long long stride, int streams, int tokens, int width,
                 const void* norm_w, float eps, void* out, int out_dtype, float* shift_state,
                 const void* shift_w, const int32_t* token_seq, const int32_t* slots,
                 int keep_state, cudaStream_t stream) {
-  if constexpr (S <= 4) {
+  // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
+  if constexpr (S <= 4 && sizeof(W) == 2) {
     // whole groups of four, aligned everywhere (bf16 constants and outputs: to 8 bytes)
     const uintptr_t wide = (uintptr_t)xs | (uintptr_t)y | (uintptr_t)shift_state |
-                           (out_dtype == SAKV_F32 ? (uintptr_t)out : 0) |
-                           (sizeof(W) == 4 ? (uintptr_t)norm_w | (uintptr_t)shift_w : 0);
+                           (out_dtype == SAKV_F32 ? (uintptr_t)out : 0);
     const uintptr_t narrow = (uintptr_t)out | (uintptr_t)norm_w | (uintptr_t)shift_w;
-    // (16-bit mode: in the 32-bit mode a row's sums keep the order they have in the kernel below)
-    if (sizeof(W) == 2 && streams == S && width % 4 == 0 && width <= 4096 && stride % 4 == 0 && !(wide & 15) &&
+    if (streams == S && width % 4 == 0 && width <= 4096 && stride % 4 == 0 && !(wide & 15) &&
         !(narrow & 7)) {
       auto go = [&](auto kernel, auto* o) {
         return launch_overlapped(kernel, dim3(tokens), dim3(kThreads), 0, stream, 1, xs, stride, width,
