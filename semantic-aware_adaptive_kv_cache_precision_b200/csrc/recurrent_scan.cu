@@ -16,9 +16,10 @@
 //
 // Everything that enters a recurrence is fp32: decays, exponentials, softplus, step sizes, the
 // states and the sums over them. The projections' outputs come as fp32 (their accumulators,
-// unrounded). A sequence's tokens are taken in order by the threads that own a piece of its
-// state, so the result of a token does not depend on how its sequence was cut into steps or
-// on what else is in the step.
+// unrounded). In one walk a sequence's tokens are taken in order by the threads that own a piece of its
+// state, so in the 32-bit mode the result of a token does not depend on how its sequence was cut into
+// steps or on what else is in the step. (In the 16-bit mode long parts go in runs, and a step size's
+// products are added in another order in a decoded step than in a prompt.)
 #include "scan.cuh"
 
 namespace {
@@ -71,8 +72,8 @@ __device__ __forceinline__ void write8(__nv_bfloat16* p, const float (&v)[8]) {
 // What run j left at p[j * step] is replaced by what came before it, which fades by exp(log(j))
 // over the run (`scan::Fade`). Bound by memory (every run's state is read and written once): the runs' numbers are
 // asked for eight at a time before the first is used, since the store of one keeps the compiler
-// from asking for the next (the dual form, 16 sequences of up to 8 runs of 1 MB of state: 350 us
-// one by one, 120 now; one sequence of 47 runs of the fading state: 162 and 25).
+// from asking for the next (16 sequences of up to 8 runs of 1 MB of state: 350 us one by one, 120 so;
+// one sequence of 47 runs: 162 and 25).
 template <typename Log>
 __device__ __forceinline__ float carry_runs(float* __restrict__ p, long long step, int runs, float s,
                                             Log log) {
@@ -371,7 +372,7 @@ __global__ void selective_scan_kernel(const C* __restrict__ x, const float* __re
         }
         for (int o = lanes >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       } else {
-        // the same products in the same order as the tiled kernel adds them
+        // one after another, as the tiled kernel adds them
         for (int r = 0; r < rank; ++r) acc = fmaf(lt[r], widen(wr[r]), acc);
       }
       step = softplus(acc + bias);

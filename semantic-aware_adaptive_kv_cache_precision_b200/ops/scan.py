@@ -109,7 +109,10 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor | None, low: torch.Tensor, 
 
     `dt` None (a step of few tokens, one walk): the kernel makes the step sizes itself,
     `softplus(low[:, :rank] dt_weight^T + dt_bias)` with `dt_weight` [channels, rank] of
-    a_log's type, adding the products in the order `step_size` adds them."""
+    a_log's type. In the 32-bit mode it adds the products in the order `step_size` adds them, so a
+    token's result does not depend on the step it came with; with 16-bit weights each form adds the
+    same fp32 products in an order of its own (a channel's lanes share them out; the tensor cores),
+    and the two differ by the rounding of those sums."""
     require_cuda(x, dt, low, z, a_log, d_skip, state, dt_weight, dt_bias)
     tokens, channels = x.shape
     rank = 0

@@ -1,4 +1,5 @@
-"""The bias of a prompt's fp32 product (`csrc/elementwise.cu`): one addition an element, the same bits."""
+"""The bias of a prompt's fp32 product (`csrc/elementwise.cu`): one addition an element, the same bits (but for a
+-0 that a bias of zero is not added to)."""
 
 import pytest
 import torch
