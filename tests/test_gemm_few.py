@@ -92,3 +92,16 @@ def test_the_rule_and_the_ops_that_follow_it():
     assert isinstance(left, ops.Deferred) and left.delta.shape == (2, 4, 64)
     close(left.delta.sum(0), x.double() @ w.double().T, 32, 8192)
     assert (stream == 1).all()
+
+
+@pytest.mark.parametrize("m,k,taken", [(1, 3072, True), (8, 3072, True), (8, 3080, False), (9, 2048, True),
+                                       (9, 2056, False), (16, 2048, True), (17, 1024, False)])
+def test_the_rule_s_lines(m, k, taken):
+    """By tokens and columns where the rows are more than a wave of blocks makes; any columns up to there."""
+    wave = gemm_few.ROWS * ops.sm_count()
+    x = torch.zeros((m, k), dtype=torch.bfloat16, device=DEV)
+    w = torch.zeros((wave + 16, k), dtype=torch.bfloat16, device=DEV)
+    assert gemm_few.takes(x, w) == taken
+    assert gemm_few.takes(x, w[:wave]) == (m <= gemm_few.MAX_TOKENS)
+    large = torch.zeros((gemm_few.LARGE // (2 * k) + 1, k), dtype=torch.bfloat16, device=DEV)
+    assert gemm_few.takes(x, large) == (taken and m <= 8)
