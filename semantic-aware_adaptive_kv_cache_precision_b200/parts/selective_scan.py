@@ -61,7 +61,8 @@ class SelectiveScanMixer(Part):
     def _run(self, step) -> int:
         """Tokens a run of a long prompt: in bfloat16 a sequence's part of the step is walked
         in runs side by side (the states carried between them in fp32). In the 32-bit mode,
-        and for short parts, one walk, whose sums do not depend on how the sequence was cut."""
+        and for short parts, one walk, whose sums do not depend on how the sequence was cut (in
+        bfloat16 the step sizes' do: `ops.selective_scan`)."""
         most = getattr(step, "max_new", 0)
         if self.act_dtype == torch.float32 or most < 2 * RUN:
             return 0

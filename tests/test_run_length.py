@@ -36,3 +36,21 @@ def test_the_runs_of_a_step_and_their_memory():
             row = first + -(-n // 32) - 1
             at += n
         assert row < scratch.shape[0]
+
+
+@pytest.mark.parametrize("longest,sequences,inner,state,run", [
+    (127, 1, 64, 16, 0), (128, 1, 64, 16, 32), (255, 4, 2048, 16, 32), (255, 4, 2369, 16, 0), (128, 37, 256, 16, 32),
+    (128, 38, 256, 16, 0), (255, 1, 64, 17, 0), (256, 64, 4096, 16, 64), (256, 1, 64, 128, 64)])
+def test_the_selective_scan_s_runs(monkeypatch, longest, sequences, inner, state, run):
+    """Shorter runs up to 64 channels an SM, all sequences together; one walk in the 32-bit mode."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from semantic_aware_adaptive_kv_cache_precision_b200.parts.selective_scan import SelectiveScanMixer
+    monkeypatch.setattr(ops, "sm_count", lambda: 148)
+    step = SimpleNamespace(max_new=longest, sequences=sequences)
+    part = SimpleNamespace(act_dtype=torch.bfloat16, spec=SimpleNamespace(inner=inner, state=state))
+    assert SelectiveScanMixer._run(part, step) == run
+    part.act_dtype = torch.float32
+    assert SelectiveScanMixer._run(part, step) == 0
